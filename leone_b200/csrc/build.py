@@ -28,7 +28,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 
 MODULES: Dict[str, List[str]] = {
     # every run needs these: both dtypes, every size
-    "core": ["elementwise.cu", "gemm_simt.cu", "attention_generic.cu", "sampling_pipeline.cu", "random_weights.cu"],
+    "core": ["elementwise.cu", "gemm_simt.cu", "attention_generic.cu", "attention_f32.cu", "sampling_pipeline.cu", "random_weights.cu"],
     # the bfloat16 serving path: tensor-core products and tiled attention
     "bf16": ["gemm_tc.cu", "gemm_pair.cu", "attention_tiled.cu", "attention_prefill_pingpong.cu"],
     # mixers and feed-forwards beyond softmax attention over K/V pages and the dense gated layer:

@@ -67,6 +67,28 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// Sums of V values (V a power of two) over a warp by halving exchanges: at each step a lane gives away half of the
+// values it still has, so V values cost about V exchanges instead of 5 V.  Afterwards v[0] of lane l is the whole
+// sum of value l / (32 / V) for V <= 32; for more, v[i] is that of value l * (V / 32) + i.  Called with O = 16.
+template <int V, int O>
+__device__ __forceinline__ void warp_sum_scatter(float* v, int lane) {
+  if constexpr (O >= 1) {
+    if constexpr (V > 1) {
+      const bool upper = lane & O;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) {
+        const float give = upper ? v[i] : v[i + V / 2];
+        const float keep = upper ? v[i + V / 2] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+      }
+      warp_sum_scatter<V / 2, O / 2>(v, lane);
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+      warp_sum_scatter<1, O / 2>(v, lane);
+    }
+  }
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.
 // `scratch` is 33 floats of shared memory.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

@@ -424,12 +424,40 @@ class CudaOps:
             self.launches += 1
             return
         _need(fuse is None, "the any-size attention kernel needs q/k norm and cache write done before")
+        if self._attention_f32(ctx, qkv, out, n_q, n_kv, d, scale, window, cache):
+            return
         self.launches += 1
         _check(self.core.leone_attention_generic(
             _dt(qkv.dtype), _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp),
             _ptr(bt), bt.shape[1], _ptr(ctx.seq_of_token), _ptr(ctx.positions), n, n_q, n_kv, d,
             c_float(scale), int(window or 0), cache.page_tokens, kp.shape[0], bt.shape[0],
             _ptr(ctx.status), self._stream()), "attention_generic")
+
+    def _attention_f32(self, ctx, qkv, out, n_q, n_kv, d, scale, window, cache) -> bool:
+        """The 32-bit kernels for head sizes 64 and 128.  False: the any-size kernel's case.  In a mixed step the leading
+        rows of one token each (the scheduler puts decode rows first) run in the decode form, which streams a sequence's
+        keys, and the rest in the prompt form, which would spend a tile of 64 rows on each of them."""
+        if (qkv.dtype != torch.float32 or d not in (64, 128) or qkv.stride(0) % 4 or qkv.data_ptr() % 16
+                or out.data_ptr() % 16 or n_kv * -(-(n_q // n_kv) // 8) > 65535
+                or getattr(ctx, "q_start", None) is None or ctx.n_seqs > 65535):
+            return False                    # (the any-size kernel needs no sequence starts)
+        kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
+        parts = [(0, ctx.n_seqs, ctx.max_q_len, ctx.max_ctx_len)]
+        q_lens = getattr(ctx, "q_lens", None)
+        if not ctx.decode_only and not getattr(ctx, "fixed_shapes", False) and q_lens is not None:
+            n = 0
+            while n < len(q_lens) and q_lens[n] == 1:
+                n += 1
+            if 0 < n < len(q_lens):
+                parts = [(0, n, 1, int(ctx.ctx_lens[:n].max())),
+                         (n, ctx.n_seqs - n, int(q_lens[n:].max()), int(ctx.ctx_lens[n:].max()))]
+        for first, count, q_len, ctx_len in parts:
+            self.launches += 1
+            _check(self.core.leone_attention_f32(
+                _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt[first:]), bt.stride(0),
+                _ptr(ctx.q_start[first:]), _ptr(ctx.ctx_len[first:]), count, q_len, ctx_len, n_q, n_kv, d, c_float(scale),
+                int(window or 0), cache.page_tokens, kp.shape[0], _ptr(ctx.status), self._stream()), "attention_f32")
+        return True
 
     _MASKS = {"causal": 0, "window": 1, "chunk": 2}
     _WEIGHTS = {"softmax": 0, "softmax_plus_one": 1, "sigmoid": 2}

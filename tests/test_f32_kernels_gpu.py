@@ -1,0 +1,102 @@
+"""The 32-bit path's matrix product and attention at the sizes where their forms change, against float64."""
+import math
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from tests.test_kernels_gpu import DEV, _paged_setup, _randn, _ref_attention, ops32  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# m: the last and first size of every form (1, 2, 4, 8 | 16 | 32 | 64 | 128 tokens a tile) and ragged ones; n: fewer than a
+# block's four rows, a tile's edge, ragged; k: one piece, a ragged stage, several rounds of 256 threads, enough for eight splits
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 33, 64, 65, 130, 257])
+@pytest.mark.parametrize("n,k", [(3, 4), (129, 100), (256, 2052), (1030, 4096)])
+def test_product_in_32_bits(ops32, m, n, k):  # noqa: F811
+    x, w = _randn((m, k + 4), 1)[:, :k], _randn((n, k), 2)
+    bias, res = _randn((n,), 3), _randn((m, n + 5), 4)[:, :n]
+    want = x.double() @ w.double().t()
+    # a sum of k products in any order is within k 2^-24 of the sum of their magnitudes, to first order
+    bound = (k + 4) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t() + bias.double().abs() + res.double().abs())
+    out = torch.full((m, n), 9.0, device=DEV)
+    ops32._gemm_simt(x, w, out, 0, None)
+    assert ((out.double() - want).abs() <= bound).all()
+    ops32._gemm_simt(x, w, out, 1, None, bias)
+    assert ((out.double() - want - bias.double()).abs() <= bound).all()
+    got = _randn((m, n + 5), 4)[:, :n]
+    ops32._gemm_simt(x, w, got, 2, got, bias)
+    assert ((got.double() - want - bias.double() - res.double()).abs() <= bound).all()
+
+
+def test_a_row_of_the_product_with_an_infinity_stays_its_own(ops32):  # noqa: F811
+    for m in (4, 40):
+        x, w = _randn((m, 64), 5), _randn((130, 64), 6)
+        x[1, 3] = float("inf")
+        out = torch.empty((m, 130), device=DEV)
+        ops32._gemm_simt(x, w, out, 0, None)
+        keep = [i for i in range(m) if i != 1]
+        assert torch.isfinite(out[keep]).all() and torch.equal(out[1], torch.copysign(torch.tensor(float("inf"), device=DEV), w[:, 3]))
+
+
+# groups of 1, 2, 3 (padded to 4) and 9 (two runs of 8) heads; pages that no tile of 64 divides; windows inside and across tiles
+@pytest.mark.parametrize("n_q,n_kv,d,pt,window", [(4, 4, 64, 16, None), (16, 8, 128, 16, None), (6, 2, 128, 5, 70),
+                                                  (9, 1, 64, 3, 1), (32, 4, 128, 16, 300)])
+@pytest.mark.parametrize("seq_lens,starts", [([1, 65, 700, 33], [0, 64, 699, 32]),          # one token each: the decode form
+                                             ([150, 3, 131, 64], [0, 0, 100, 0]),           # prompts
+                                             ([640, 9, 200], [639, 8, 71])])                # decode rows, then a portion
+def test_attention_in_32_bits(ops32, n_q, n_kv, d, pt, window, seq_lens, starts):  # noqa: F811
+    table, k_pool, v_pool = _paged_setup(seq_lens, pt, n_kv, d, torch.float32, 9)
+    k_pool.fill_(float("inf"))                          # rows that no sequence holds must not be read into a sum
+    v_pool.fill_(float("inf"))
+    keys = [_randn((l, n_kv, d), 30 + s) for s, l in enumerate(seq_lens)]
+    vals = [_randn((l, n_kv, d), 40 + s) for s, l in enumerate(seq_lens)]
+    positions, q_start = [], [0]
+    for s, (l, st) in enumerate(zip(seq_lens, starts)):
+        pos = torch.arange(l)
+        pages = table[s, (pos // pt).to(DEV)].long()
+        k_pool[pages, :, (pos % pt).to(DEV)] = keys[s]
+        v_pool[pages, :, (pos % pt).to(DEV)] = vals[s]
+        if window:
+            table[s, :max(0, st - window + 1) // pt] = -1          # pages the window has passed are gone
+        positions += [(s, p) for p in range(st, l)]
+        q_start.append(len(positions))
+    n = len(positions)
+    qkv = _randn((n, (n_q + 2 * n_kv) * d), 50)
+    for s in range(len(seq_lens)):                      # a far key that dominates: a wrong page would show
+        qkv.view(n, -1, d)[q_start[s], 0] = keys[s][min(3, starts[s]), 0] * 3
+    out = torch.full((n, n_q * d), 7.0, device=DEV)
+    q_lens = np.diff(q_start)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(q_start=torch.tensor(q_start, **i32), ctx_len=torch.tensor(seq_lens, **i32), n_seqs=len(seq_lens),
+                                max_q_len=int(q_lens.max()), max_ctx_len=max(seq_lens), decode_only=int(q_lens.max()) == 1,
+                                fixed_shapes=False, q_lens=q_lens, ctx_lens=np.array(seq_lens), status=torch.zeros(4, **i32))
+    cache = types.SimpleNamespace(k_pool=k_pool, v_pool=v_pool, block_table=table, page_tokens=pt)
+    scale = 1 / math.sqrt(d)
+    assert ops32._attention_f32(ctx, qkv, out, n_q, n_kv, d, scale, window, cache)
+    assert ctx.status.tolist() == [0, 0, 0, 0]
+    for i, (s, p) in enumerate(positions):
+        q = qkv[i].double().view(-1, d)[:n_q]
+        want = _ref_attention(q, keys[s][:p + 1].double(), vals[s][:p + 1].double(), n_q, n_kv, scale,
+                              max(0, p - window + 1) if window else 0)
+        # a score is a sum of d products (|s| <= |q| |k| scale, error d 2^-24 of it), a weight moves by as much relatively;
+        # the weighted mean of values moves by twice that of the largest value, plus its own sum's rounding
+        s_err = d * 2.0 ** -24 * scale * q.norm(dim=1).max() * keys[s][:p + 1].double().norm(dim=2).max()
+        bound = (2 * s_err + (p + 8) * 2.0 ** -23) * vals[s][:p + 1].abs().max().double()
+        assert ((out[i].view(n_q, d).double() - want).abs() <= bound).all(), (s, p)
+
+
+def test_attention_in_32_bits_reports_a_missing_page(ops32):  # noqa: F811
+    i32 = dict(dtype=torch.int32, device=DEV)
+    for q_len in (1, 2):
+        table, k_pool, v_pool = _paged_setup([20], 16, 1, 64, torch.float32, 1)
+        table[0, 1] = -1
+        ctx = types.SimpleNamespace(q_start=torch.tensor([0, q_len], **i32), ctx_len=torch.tensor([20], **i32), n_seqs=1,
+                                    max_q_len=q_len, max_ctx_len=20, decode_only=q_len == 1, fixed_shapes=True,
+                                    status=torch.zeros(4, **i32))
+        cache = types.SimpleNamespace(k_pool=k_pool, v_pool=v_pool, block_table=table, page_tokens=16)
+        out = torch.empty((q_len, 64), device=DEV)
+        assert ops32._attention_f32(ctx, _randn((q_len, 192), 1), out, 1, 1, 64, 0.1, None, cache)
+        assert ctx.status[0].item() == 2
