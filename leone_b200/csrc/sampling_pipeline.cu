@@ -8,7 +8,8 @@
 // row in id order with u = uniform(seed, position, Select) (:803-857).  The same here:
 //
 //   sort      one row = P (a power of two >= vocab) pairs (fp64 key, id), bitonic network:
-//             tiles of 2,048 pairs in shared memory, larger strides in global memory
+//             tiles of 2,048 pairs in shared memory, larger strides in global memory; a list that
+//             starts with a top-k of up to 1,024 finds and sorts those k alone
 //   stages    one block per row walks the stage list over the sorted row with block-wide
 //             fp64 sums and scans; "typical" needs a second sort (by |surprise - entropy|),
 //             so the stage list is cut there and the host entry launches the pieces in order
@@ -156,49 +157,16 @@ __global__ void bitonic_global_kernel(int which, int vocab, int P, int n_sort, u
 }
 
 // Sorts the first n_sort (a power of two) pairs of every row's first or second pair of arrays.
-// tiles_only: stop when every tile of 2,048 is sorted in itself.
-static int sort_rows(int which, int vocab, int P, int n_sort, int rows, uint8_t* scratch, cudaStream_t stream,
-                     bool tiles_only = false) {
+static int sort_rows(int which, int vocab, int P, int n_sort, int rows, uint8_t* scratch, cudaStream_t stream) {
   const int tile = n_sort < kTile ? n_sort : kTile;
   bitonic_tile_kernel<<<dim3(n_sort / tile, rows), kThreads, 0, stream>>>(which, vocab, P, n_sort, scratch, 2, tile);
-  for (int k = 2 * tile; k <= n_sort && !tiles_only; k <<= 1) {
+  for (int k = 2 * tile; k <= n_sort; k <<= 1) {
     for (int j = k >> 1; j >= tile; j >>= 1)
       bitonic_global_kernel<<<dim3((n_sort / 2 + 255) / 256, rows), 256, 0, stream>>>(which, vocab, P, n_sort,
                                                                                        scratch, k, j);
     bitonic_tile_kernel<<<dim3(n_sort / tile, rows), kThreads, 0, stream>>>(which, vocab, P, n_sort, scratch, k, k);
   }
   return (int)cudaGetLastError();
-}
-
-// After the tiles are sorted in themselves, every tile alternately descending and ascending
-// (the network's direction at level kTile): the `take` best pairs of every tile, which hold the
-// row's `take` best, go to the front of the second pair of arrays (padded to n_out with pairs
-// that sort last).
-__global__ void gather_tile_heads_kernel(int vocab, int P, uint8_t* scratch, int take, int n_out) {
-  const Row r = row_of(scratch, blockIdx.y, P, vocab);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_out) return;
-  const int tiles = P / kTile;
-  const int t = i / take, e = i - t * take;
-  if (t < tiles) {
-    // tile t is sorted descending ("up") if bit kTile of its base is clear, else ascending
-    const int base = t * kTile;
-    const int at = (base & kTile) == 0 ? base + e : base + kTile - 1 - e;
-    r.skeys[i] = r.keys[at];
-    r.sidx[i] = r.order[at];
-  } else {
-    r.skeys[i] = -INFINITY;
-    r.sidx[i] = vocab + P + i;
-  }
-}
-
-__global__ void take_heads_kernel(int vocab, int P, uint8_t* scratch, int count) {
-  const Row r = row_of(scratch, blockIdx.y, P, vocab);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P) return;
-  // the sorted heads become the row; what follows them is marked as excluded
-  r.keys[i] = i < count ? r.skeys[i] : -INFINITY;
-  r.order[i] = i < count ? r.sidx[i] : vocab + i;
 }
 
 // ---- block-wide fp64 helpers (one block of kThreads per row) ----------------------------------
@@ -322,6 +290,117 @@ __device__ void renormalize(double* kept, int n, Shared& sh) {
   const double total = sum_of(kept, n, sh);
   for (int i = threadIdx.x; i < n; i += kThreads) kept[i] /= total;
   __syncthreads();
+}
+
+// ---- the k best of a row ------------------------------------------------------------------------
+// A block per row, in place of ordering the whole row.  Bound by two readings of the row through one SM (about 5 us each at
+// 151,936 logits); a full sort moves the row 36 times.  Every thread keeps the largest of its share of the row; the k-th
+// largest of the 1,024 such maxima is a lower bound of the row's k-th largest value, so few values reach it; those
+// are collected and sorted as 64-bit words (value as an ordered integer, then the smaller id first).  Where more
+// reach it than fit (a few threads hold most of the best values, or thousands of ties), the k-th value and the
+// last id among its ties are found bit by bit with counts over the row.
+// Measured with all that follows (64 rows of 151,936 logits, top-k 40 and top-p): 2.29 ms with tiles of 2,048 sorted and their
+// heads gathered, now 0.24 ms of which the host's share is most.
+constexpr int kMaxTopK = 1024, kCandidates = 4096;
+
+// Finite values in order; 0 for the others.  (-0 and 0 are equal keys.)
+__device__ __forceinline__ unsigned ordered(float v) {
+  if (!isfinite(v)) return 0u;
+  const unsigned u = __float_as_uint(v + 0.f);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(unsigned o) {
+  return __uint_as_float(o & 0x80000000u ? o & 0x7fffffffu : ~o);
+}
+
+__global__ void __launch_bounds__(kThreads)
+top_k_kernel(const float* __restrict__ logits, const int* __restrict__ row_map, int vocab, int P, uint8_t* scratch, int k) {
+  __shared__ unsigned long long cand[kCandidates];
+  __shared__ Shared sh;
+  __shared__ int count_s;
+  const int row = blockIdx.x, tid = threadIdx.x;
+  const Row r = row_of(scratch, row, P, vocab);
+  const float* l = logits + (size_t)(row_map != nullptr ? row_map[row] : row) * vocab;
+  unsigned top = 0;
+  int finite = 0;
+#pragma unroll 8
+  for (int i = tid; i < vocab; i += kThreads) {
+    const unsigned o = ordered(l[i]);
+    finite += o != 0;
+    top = max(top, o);
+  }
+  finite = block_sum_int(finite, sh);
+  const int want = min(k, finite);
+  if (tid == 0) {
+    *r.n = want;
+    count_s = 0;
+  }
+  if (want == 0) return;
+  // the largest bound that at least `want` threads reach (1, the least finite value's lower neighbour, if too few do)
+  unsigned bound = 0;
+  for (int b = 31; b >= 0; --b) {
+    const unsigned t = bound | 1u << b;
+    if (__syncthreads_count(top >= t) >= want) bound = t;
+  }
+  bound = max(bound, 1u);
+#pragma unroll 8
+  for (int i = tid; i < vocab; i += kThreads) {
+    const unsigned o = ordered(l[i]);
+    if (o >= bound) {
+      const int at = atomicAdd(&count_s, 1);
+      if (at < kCandidates) cand[at] = (unsigned long long)o << 32 | (0xffffffffu - (unsigned)i);
+    }
+  }
+  __syncthreads();
+  int count = count_s;
+  if (count > kCandidates) {
+    auto reach = [&](unsigned t) {
+      int c = 0;
+      for (int i = tid; i < vocab; i += kThreads) c += ordered(l[i]) >= t;
+      return block_sum_int(c, sh);
+    };
+    unsigned kth = 0;
+    for (int b = 31; b >= 0; --b)
+      if (reach(kth | 1u << b) >= want) kth |= 1u << b;
+    const int ties = want - (kth == 0xffffffffu ? 0 : reach(kth + 1));       // at least one
+    // the id of the last tie that belongs: the largest t with fewer than `ties` ties below it
+    unsigned last = 0;
+    for (int b = 30; b >= 0; --b) {
+      const unsigned t = last | 1u << b;
+      int c = 0;
+      for (int i = tid; i < vocab; i += kThreads) c += ordered(l[i]) == kth && (unsigned)i < t;
+      if (block_sum_int(c, sh) < ties) last = t;
+    }
+    if (tid == 0) count_s = 0;
+    __syncthreads();
+    for (int i = tid; i < vocab; i += kThreads) {
+      const unsigned o = ordered(l[i]);
+      if (o > kth || (o == kth && (unsigned)i <= last))
+        cand[atomicAdd(&count_s, 1)] = (unsigned long long)o << 32 | (0xffffffffu - (unsigned)i);
+    }
+    __syncthreads();
+    count = count_s;                       // = want
+  }
+  int n_sort = 2;
+  while (n_sort < count) n_sort <<= 1;
+  for (int i = count + tid; i < n_sort; i += kThreads) cand[i] = 0;
+  __syncthreads();
+  for (int size = 2; size <= n_sort; size <<= 1)
+    for (int j = size >> 1; j >= 1; j >>= 1) {
+      for (int t = tid; t < (n_sort >> 1); t += kThreads) {
+        const int i = 2 * j * (t / j) + (t % j);
+        const unsigned long long a = cand[i], b = cand[i + j];
+        if ((i & size) == 0 ? a < b : a > b) {
+          cand[i] = b;
+          cand[i + j] = a;
+        }
+      }
+      __syncthreads();
+    }
+  for (int i = tid; i < want; i += kThreads) {
+    r.keys[i] = (double)from_ordered((unsigned)(cand[i] >> 32));
+    r.order[i] = (int)(0xffffffffu - (unsigned)cand[i]);
+  }
 }
 
 // ---- the stages -------------------------------------------------------------------------------
@@ -510,6 +589,8 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long v) {
   return z ^ (z >> 31);
 }
 
+constexpr int kFewSurvivors = 1024;
+
 // Probabilities back in id order, and the draw: the first id whose running sum exceeds u, else
 // the last id with any probability.
 __global__ void __launch_bounds__(kThreads)
@@ -521,27 +602,85 @@ select_kernel(int vocab, int P, uint8_t* scratch, const long long* __restrict__ 
   const int dst = row_map != nullptr ? row_map[row] : row;      // where the row's id goes
   const Row r = row_of(scratch, row, P, vocab);
   const int n = *r.n;
-  for (int i = threadIdx.x; i < vocab; i += kThreads) r.dense[i] = 0.0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += kThreads) r.dense[r.order[i]] = r.kept[i];
-  __syncthreads();
-  if (probs != nullptr)
-    for (int i = threadIdx.x; i < vocab; i += kThreads) probs[(size_t)row * vocab + i] = r.dense[i];
-  if (n <= 0) {
-    if (threadIdx.x == 0) out[dst] = -1;
-    return;
-  }
   const unsigned long long purpose = 0xbf58476d1ce4e5b9ull;
   const unsigned long long mixed =
       splitmix64((unsigned long long)seeds[row] ^ splitmix64((unsigned long long)positions[row] ^ purpose));
   const double u = (double)(mixed >> 11) * (1.0 / 9007199254740992.0);
-  const double* dense = r.dense;
-  const int at = first_where(vocab, [&](int i) { return dense[i]; }, [&](double c) { return u < c; }, sh);
-  int last = -1;
-  for (int i = threadIdx.x; i < vocab; i += kThreads)
-    if (dense[i] > 0.0) last = i;
-  last = -block_min(-last, sh);
-  const int token = at == INT_MAX ? last : at;     // a zero entry cannot make the sum pass u
+  int token;
+  if (n > 0 && n <= kFewSurvivors && probs == nullptr) {
+    // few survivors: sorted by id here instead of scattered over the vocabulary.  The sums are the other branch's,
+    // whose zeros change none of them: a thread's share of the ids in order, from the prefix of the shares before it.
+    __shared__ int ids[kFewSurvivors];
+    __shared__ double p[kFewSurvivors];
+    int n_sort = 2;
+    while (n_sort < n) n_sort <<= 1;
+    for (int i = threadIdx.x; i < n_sort; i += kThreads) {
+      ids[i] = i < n ? r.order[i] : INT_MAX;
+      p[i] = i < n ? r.kept[i] : 0.0;
+    }
+    __syncthreads();
+    for (int size = 2; size <= n_sort; size <<= 1)
+      for (int j = size >> 1; j >= 1; j >>= 1) {
+        for (int t = threadIdx.x; t < (n_sort >> 1); t += kThreads) {
+          const int i = 2 * j * (t / j) + (t % j);
+          const int a = ids[i], b = ids[i + j];
+          if ((i & size) == 0 ? a > b : a < b) {
+            ids[i] = b;
+            ids[i + j] = a;
+            const double pa = p[i];
+            p[i] = p[i + j];
+            p[i + j] = pa;
+          }
+        }
+        __syncthreads();
+      }
+    auto first_at_least = [&](int id) {
+      int lo = 0, hi = n;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ids[mid] < id) lo = mid + 1;
+        else hi = mid;
+      }
+      return lo;
+    };
+    int lo, hi;
+    chunk_of(vocab, &lo, &hi);
+    const int from = first_at_least(lo), to = first_at_least(hi);
+    double local = 0.0, total;
+    int last = -1;
+    for (int i = from; i < to; ++i) {
+      local += p[i];
+      if (p[i] > 0.0) last = ids[i];
+    }
+    double run = block_scan(local, sh, &total);
+    int found = INT_MAX;
+    if (lo < hi && (from == to || ids[from] != lo) && u < run) found = lo;
+    for (int i = from; i < to && found == INT_MAX; ++i) {
+      run += p[i];
+      if (u < run) found = ids[i];
+    }
+    const int at = block_min(found, sh);
+    last = -block_min(-last, sh);
+    token = at == INT_MAX ? last : at;
+  } else {
+    for (int i = threadIdx.x; i < vocab; i += kThreads) r.dense[i] = 0.0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kThreads) r.dense[r.order[i]] = r.kept[i];
+    __syncthreads();
+    if (probs != nullptr)
+      for (int i = threadIdx.x; i < vocab; i += kThreads) probs[(size_t)row * vocab + i] = r.dense[i];
+    if (n <= 0) {
+      if (threadIdx.x == 0) out[dst] = -1;
+      return;
+    }
+    const double* dense = r.dense;
+    const int at = first_where(vocab, [&](int i) { return dense[i]; }, [&](double c) { return u < c; }, sh);
+    int last = -1;
+    for (int i = threadIdx.x; i < vocab; i += kThreads)
+      if (dense[i] > 0.0) last = i;
+    last = -block_min(-last, sh);
+    token = at == INT_MAX ? last : at;             // a zero entry cannot make the sum pass u
+  }
   if (threadIdx.x == 0) out[dst] = token;
   if (chosen_prob != nullptr)                      // the token's probability before the surprise filter
     for (int i = threadIdx.x; i < n; i += kThreads)
@@ -617,28 +756,19 @@ extern "C" int leone_sample_truncated(const float* logits, int rows, int vocab, 
   }
   const int P = pow2_at_least(vocab);
   uint8_t* sc = static_cast<uint8_t*>(scratch);
-  sort_init_logits_kernel<<<dim3((P + 255) / 256, rows), 256, 0, stream>>>(logits, row_map, vocab, P, sc);
-  // A pipeline that starts with a small top-k and has no raw-logit stage needs only the row's k
-  // best pairs, which are among the k best of every tile: the tiles are sorted in themselves,
-  // their heads gathered and sorted, and the rest of the row is never ordered.
+  // A list that starts with a top-k and has no raw-logit stage needs only the row's k best pairs.  (A larger k than a block
+  // collects orders the whole row.)
   bool raw = false;
   for (int s = 0; s < n_stages; ++s) raw = raw || st.type[s] == kMinK || st.type[s] == kTopNSigma;
-  const int tiles = P / kTile;
   int e;
-  if (!raw && n_stages > 0 && st.type[0] == kTopK && P > kTile && st.value[0] * tiles <= 4 * kTile) {
-    const int take = (int)st.value[0];
-    const int n_out = pow2_at_least(take * tiles);
-    e = sort_rows(0, vocab, P, P, rows, sc, stream, true);
-    if (e != 0) return e;
-    gather_tile_heads_kernel<<<dim3((n_out + 255) / 256, rows), 256, 0, stream>>>(vocab, P, sc, take, n_out);
-    e = sort_rows(1, vocab, P, n_out, rows, sc, stream);
-    if (e != 0) return e;
-    take_heads_kernel<<<dim3((P + 255) / 256, rows), 256, 0, stream>>>(vocab, P, sc, take);
+  if (!raw && n_stages > 0 && st.type[0] == kTopK && st.value[0] <= kMaxTopK) {
+    top_k_kernel<<<rows, kThreads, 0, stream>>>(logits, row_map, vocab, P, sc, (int)st.value[0]);
   } else {
+    sort_init_logits_kernel<<<dim3((P + 255) / 256, rows), 256, 0, stream>>>(logits, row_map, vocab, P, sc);
     e = sort_rows(0, vocab, P, P, rows, sc, stream);
     if (e != 0) return e;
+    count_finite_kernel<<<dim3((P + 255) / 256, rows), 256, 0, stream>>>(vocab, P, sc);
   }
-  count_finite_kernel<<<dim3((P + 255) / 256, rows), 256, 0, stream>>>(vocab, P, sc);
   int done = 0;
   bool begun = false;
   while (true) {

@@ -243,12 +243,14 @@ class Sampler:
         host[self._cap:self._cap + rows] = np.array([p.seed & 0xFFFF_FFFF_FFFF_FFFF for p in params],
                                                     dtype=np.uint64).view(np.int64)
         host[2 * self._cap:2 * self._cap + rows] = np.asarray(positions, dtype=np.int64)
-        self._dev.copy_(self._host, non_blocking=True)
-        t = self._dev[:self._cap].view(torch.float32)[:rows]
-        seeds = self._dev[self._cap:self._cap + rows]
-        pos = self._dev[2 * self._cap:2 * self._cap + rows]
         out = self._out[:rows]
-        self.ops.sample(logits, t, seeds, pos, out)
+        # rows without stages and without Mirostat; where there are none the plain kernel has nothing to draw
+        if not all(p.temperature > 0 and (p.truncations or p.mirostat) for p in params):
+            self._dev.copy_(self._host, non_blocking=True)
+            t = self._dev[:self._cap].view(torch.float32)[:rows]
+            seeds = self._dev[self._cap:self._cap + rows]
+            pos = self._dev[2 * self._cap:2 * self._cap + rows]
+            self.ops.sample(logits, t, seeds, pos, out)
         # rows with truncation stages: grouped by their stage list, through the fp64 pipeline
         if any(p.mirostat for p in params) and (states is None or len(states) != rows or any(
                 p.mirostat and states[i] is None for i, p in enumerate(params))):
