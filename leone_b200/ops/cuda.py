@@ -607,6 +607,28 @@ class CudaOps:
         _need(state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, dim, vdim)
               and decay.dtype == torch.float32 and decay.numel() == heads, "linear_attention state/decay")
         n_chunks, chunk_state = 0, None
+        if (self.fast is not None and proj.dtype == torch.bfloat16 and not ctx.decode_only and ctx.max_q_len >= 16
+                and self.mixers.leone_linear_attention_mma_supported(dim, vdim) and proj.data_ptr() % 16 == 0
+                and not any(o % 8 for o in (proj.stride(0), q_off, k_off, v_off))):
+            # Prompt portions in bfloat16: 64 tokens at a time on tensor cores.  Chunks as short as still leave about
+            # two rounds of blocks (two a SM): a chunk's state costs as much traffic as 64 tokens' outputs.
+            chunk_decay = None
+            chunk = 64
+            q_lens = [int(q) for q in ctx.q_lens]
+            while sum(-(-q // chunk) for q in q_lens) * heads * -(-vdim // 64) > 4 * self.fast.sm_count:
+                chunk *= 2
+            if max(q_lens) <= chunk:
+                chunk = 0
+            else:
+                n_chunks = sum(-(-q // chunk) for q in q_lens)
+                chunk_state = self._scratch("linattn_chunks", n_chunks, heads * dim * vdim, torch.float32)
+                chunk_decay = self._scratch("linattn_chunk_decay", n_chunks, heads * dim, torch.float32)
+            self.launches += 1 if chunk == 0 else 3
+            _check(self.mixers.leone_linear_attention_mma(
+                _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state), _ptr(ctx.q_start),
+                _ptr(ctx.slot_ids), _ptr(decay), ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk, n_chunks,
+                _ptr(chunk_state), _ptr(chunk_decay), _ptr(ctx.status), self._stream()), "linear_attention_mma")
+            return
         if chunk > 0:
             n_chunks = int(sum(-(-int(q) // chunk) for q in ctx.q_lens))
             chunk_state = self._scratch("linattn_chunks", n_chunks, heads * dim * vdim, torch.float32)

@@ -1,0 +1,51 @@
+"""Linear attention with a decaying state on tensor cores, against the recurrence in float64."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from tests.test_kernels_gpu import DEV, _randn, ops16  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _walk(q, k, v, decay, state):
+    out = torch.empty((q.shape[0], q.shape[1], v.shape[2]), dtype=torch.float64, device=q.device)
+    for t in range(q.shape[0]):
+        state = decay[:, None, None] * state + k[t][:, :, None] * v[t][:, None, :]
+        out[t] = torch.einsum("hdv,hd->hv", state, q[t])
+    return out, state
+
+
+# dim: below, at and above the widths of the kernel's forms; vdim: a part of a block's 64 columns, one block, a block and a part.
+# Lengths: one token, around a tile of 64, several tiles in one chunk and in several; decays of 0, weak, 1 and above 1.
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 8), (3, 40, 72), (2, 64, 64), (4, 128, 128), (1, 88, 24)])
+@pytest.mark.parametrize("q_lens", [[16], [63, 1, 65], [200, 64, 130], [700]])
+def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens):  # noqa: F811
+    n, slots = sum(q_lens), [4, 1, 3][:len(q_lens)]
+    cols = 2 * heads * dim + heads * vdim
+    proj = _randn((n, cols + 8), 3, torch.bfloat16, 1.5)[:, :cols]
+    state = _randn((6, heads, dim, vdim), 4)
+    decay = torch.tensor([0.97, 0.0, 1.0, 1.01][:heads], device=DEV)
+    before = state.clone()
+    starts = np.concatenate([[0], np.cumsum(q_lens)])
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(q_start=torch.tensor(starts, **i32), slot_ids=torch.tensor(slots, **i32), n_seqs=len(q_lens),
+                                q_lens=np.array(q_lens), max_q_len=max(q_lens), decode_only=False, status=torch.zeros(4, **i32))
+    out = torch.full((n, heads * vdim), 9.0, device=DEV)
+    ops16.linear_attention(ctx, proj, out, state, decay, heads, dim, vdim, 0, heads * dim, 2 * heads * dim, chunk=64)
+    assert ctx.status.tolist() == [0, 0, 0, 0]
+    act = torch.nn.functional.silu(proj.double())
+    q, k = (act[:, i * heads * dim:(i + 1) * heads * dim].view(n, heads, dim) for i in (0, 1))
+    v = act[:, 2 * heads * dim:].view(n, heads, vdim)
+    for s, (a, b, slot) in enumerate(zip(starts[:-1], starts[1:], slots)):
+        want, end = _walk(q[a:b], k[a:b], v[a:b], decay.double(), before[slot].double())
+        size, end_size = _walk(q[a:b].abs(), k[a:b].abs(), v[a:b].abs(), decay.double(), before[slot].double().abs())
+        # two terms hold an operand to 2^-17 of it; an output has up to four such operands (q, k or the state, the weighted
+        # score, v), and the dropped products of two lo terms are 2^-18; sums of n terms in fp32 add n 2^-24
+        rel = 5 * 2.0 ** -17 + (b - a + dim) * 2.0 ** -24
+        got = out[a:b].view(b - a, heads, vdim).double()
+        assert ((got - want).abs() <= rel * size + 1e-30).all(), s
+        assert ((state[slot].double() - end).abs() <= rel * end_size + 1e-30).all(), s
+    assert torch.equal(state[[0, 2, 5]], before[[0, 2, 5]])
