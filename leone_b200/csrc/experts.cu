@@ -15,6 +15,7 @@
 // to be empty return at once).  A row of the grouped products is computed from its own token only,
 // with k ascending, so a token's result does not depend on what else is in the step.
 #include "common.cuh"
+#include "experts_tc.h"
 #include "mma_tile.cuh"
 
 namespace leone {
@@ -338,7 +339,43 @@ __global__ void experts_combine_kernel(float* __restrict__ hidden, const float* 
     hidden[i] = top < 0 ? sum : hidden[i] + sum;
   }
 }
-
+// The same four columns a thread (width a multiple of 4, 16-byte aligned rows): a pass over the pairs' rows at the memory's rate.
+template <typename T>
+__global__ void __launch_bounds__(256)
+experts_combine_vec_kernel(float* hidden, const float* pair_out, long long total4, int width4, int top, const T* x, int ldx,
+                           const int* chosen, const float* weight, int experts) {
+  pdl_trigger();
+  pdl_wait();
+  const float4* src = reinterpret_cast<const float4*>(pair_out);
+  float4* dst = reinterpret_cast<float4*>(hidden);
+  const int n = top < 0 ? -top : top;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
+    const long long t = i / width4;
+    const int c = (int)(i - t * width4);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const size_t p = (size_t)t * n + j;
+      float4 v;
+      if (x != nullptr && chosen[p] >= experts) {
+        const float w = weight[p];
+        const T* row = x + (size_t)t * ldx + 4 * c;
+        v = make_float4(w * to_float<T>(row[0]), w * to_float<T>(row[1]), w * to_float<T>(row[2]), w * to_float<T>(row[3]));
+      } else {
+        v = src[p * width4 + c];
+      }
+      sum.x += v.x;
+      sum.y += v.y;
+      sum.z += v.z;
+      sum.w += v.w;
+    }
+    if (top >= 0) {
+      const float4 h = dst[i];
+      sum = make_float4(h.x + sum.x, h.y + sum.y, h.z + sum.z, h.w + sum.w);
+    }
+    dst[i] = sum;
+  }
+}
 
 // ---- the grouped products on tensor cores (bfloat16) ----------------------------------------------
 // A row tile of 64 sorted pairs of one expert times 64 output columns; four warps of 16 rows each;
@@ -545,12 +582,13 @@ extern "C" int leone_experts_select(const float* logits, int ldl, const float* b
 // are experts without tensors whose output is their input (weighted at the output).  fresh: hidden is
 // written, not added to.
 // x: [n_tokens, ldx]; chosen, weight: [n_tokens * top]; scratch: offsets int [experts + 1], order int
-// [pairs], act [pairs, ff] in the run dtype, pair_out fp32 [pairs, width]; hidden fp32 [n_tokens, width].
+// [pairs], act [pairs, ff] in the run dtype, pair_out fp32 [pairs, width]; hidden fp32 [n_tokens, width].  tensor_cores: 0 none,
+// 1 chosen by size, 2 the mma.sync form only.
 extern "C" int leone_experts_forward(int dtype, const void* x, int ldx, const void* w_gate, const void* w_up,
                                      const void* w_down, const int* chosen, const float* weight, int n_tokens,
                                      int width, int ff, int experts, int top, int scale_input, int* offsets,
                                      int* order, void* act, float* pair_out, float* hidden, int tensor_cores,
-                                     int identity, int fresh, cudaStream_t stream) {
+                                     int identity, int fresh, int* status, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (identity < 0 || (identity > 0 && scale_input)) return kRefusedSize;
   if (width <= 0 || ff <= 0 || experts <= 0 || top <= 0 || experts > 8192) return kRefusedSize;
@@ -560,6 +598,35 @@ extern "C" int leone_experts_forward(int dtype, const void* x, int ldx, const vo
   launch_kernel(group_pairs_kernel, dim3(1), dim3(1024), sizeof(int) * (size_t)experts, stream, chosen, (int)pairs, experts, offsets, order);
   const int combine_top = fresh ? -top : top;
   if (tensor_cores && dtype == 1 && width % 8 == 0 && ff % 8 == 0 && ldx % 8 == 0) {
+    const long long total = (long long)n_tokens * width;
+    const long long blocks = (total + 255) / 256;
+    const dim3 combine_grid((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8));
+    auto combine = [&] {
+      if (width % 4 == 0 && ((uintptr_t)hidden | (uintptr_t)pair_out) % 16 == 0) {
+        const long long blocks4 = (total / 4 + 255) / 256;
+        launch_kernel(experts_combine_vec_kernel<__nv_bfloat16>, dim3((unsigned)(blocks4 < 148 * 8 ? blocks4 : 148 * 8)), dim3(256), 0,
+                      stream, hidden, pair_out, total / 4, width / 4, combine_top, identity > 0 ? (const __nv_bfloat16*)x : nullptr,
+                      ldx, chosen, weight, experts);
+        return launch_result();
+      }
+      launch_kernel(experts_combine_kernel<__nv_bfloat16>, combine_grid, dim3(256), 0, stream, hidden, pair_out, total, width,
+                    combine_top, identity > 0 ? (const __nv_bfloat16*)x : nullptr, ldx, chosen, weight, experts);
+      return launch_result();
+    };
+    // From a pair an expert on, tcgen05 is the faster form (32 experts of 512, 8 tokens with 4 pairs each: 50 us against 62; 64 of
+    // 1,024, 32 tokens: 276 against 346); with fewer pairs its 128 x 256 tiles are too few blocks to stream the weights.
+    const uintptr_t starts = (uintptr_t)x | (uintptr_t)w_gate | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)pair_out;
+    if (tensor_cores != 2 && experts <= kExpertsTcMost && pairs >= experts && starts % 16 == 0) {
+      int e = w_gate == nullptr
+                  ? experts_tc_product(1, x, ldx, w_up, nullptr, offsets, order, weight, n_tokens, experts, top, ff, width,
+                                       scale_input, act, pair_out, status, stream)
+                  : experts_tc_product(0, x, ldx, w_gate, w_up, offsets, order, weight, n_tokens, experts, top, ff, width,
+                                       scale_input, act, pair_out, status, stream);
+      if (e == 0)
+        e = experts_tc_product(2, act, ff, w_down, nullptr, offsets, order, weight, n_tokens, experts, top, width, ff, scale_input,
+                               pair_out, nullptr, status, stream);
+      return e != 0 ? e : combine();
+    }
     const long long tiles = (pairs + TM - 1) / TM + (experts < pairs ? experts : pairs);
     if (tiles > 65535) return kRefusedSize;
     const size_t smem_up = (size_t)TSTAGES * (TM + 2 * TN) * TPITCH, smem_down = (size_t)TSTAGES * (TM + TN) * TPITCH;
@@ -581,12 +648,7 @@ extern "C" int leone_experts_forward(int dtype, const void* x, int ldx, const vo
     launch_kernel(experts_down_mma_kernel, dim3((width + TN - 1) / TN, (unsigned)tiles), dim3(128), smem_down, stream, 
         (const __nv_bfloat16*)act, (const __nv_bfloat16*)w_down, pair_out, offsets, order, weight, experts, width, ff,
         scale_input);
-    const long long total = (long long)n_tokens * width;
-    const long long blocks = (total + 255) / 256;
-    launch_kernel(experts_combine_kernel<__nv_bfloat16>, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream,
-                  hidden, pair_out, total, width, combine_top, identity > 0 ? (const __nv_bfloat16*)x : nullptr, ldx, chosen,
-                  weight, experts);
-    return launch_result();
+    return combine();
   }
   // every expert may end with a partly filled tile
   const long long max_tiles = (pairs + GM - 1) / GM + (experts < pairs ? experts : pairs);

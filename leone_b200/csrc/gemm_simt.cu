@@ -98,7 +98,7 @@ __device__ __forceinline__ float4 ld_stream(const float* p) {
 
 template <int MT, int R>
 __global__ void __launch_bounds__(256, MT == 8 ? 3 : 4)
-gemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C, const float* residual,
+gemm_rows_kernel(const float* A, const float* __restrict__ W, float* C, const float* residual,
                  const float* __restrict__ bias, int M, int N, int K, int lda, int ldw, int ldc) {
   constexpr int V = R * MT;
   static_assert((V & (V - 1)) == 0 && V <= 64, "the exchanges halve the values");

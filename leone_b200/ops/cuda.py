@@ -1245,7 +1245,7 @@ class CudaOps:
             _dt(x.dtype), _ptr(x), x.stride(0), _ptr(w_gate), _ptr(w_up), _ptr(w_down), _ptr(chosen), _ptr(weight), n,
             width, ff, experts, top, 1 if scale_input else 0, _ptr(offsets), _ptr(order), _ptr(act), _ptr(pair_out),
             _ptr(hidden), 0 if os.environ.get("LEONE_NO_EXPERT_MMA", "0") == "1" else 1, int(identity),
-            1 if fresh else 0, self._stream()), "experts_forward")
+            1 if fresh else 0, _ptr(self.status), self._stream()), "experts_forward")
 
     def sample(self, logits, temperature, seeds, positions, out):
         rows, vocab = logits.shape
