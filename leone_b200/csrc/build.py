@@ -28,7 +28,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 
 MODULES: Dict[str, List[str]] = {
     # every run needs these: both dtypes, every size
-    "core": ["elementwise.cu", "gemm_simt.cu", "attention_generic.cu", "attention_f32.cu", "sampling_pipeline.cu", "random_weights.cu"],
+    "core": ["elementwise.cu", "gemm_simt.cu", "gemm_f32_tc.cu", "attention_generic.cu", "attention_f32.cu", "sampling_pipeline.cu", "random_weights.cu"],
     # the bfloat16 serving path: tensor-core products and tiled attention
     "bf16": ["gemm_tc.cu", "gemm_pair.cu", "attention_tiled.cu", "attention_prefill_pingpong.cu"],
     # mixers and feed-forwards beyond softmax attention over K/V pages and the dense gated layer:
@@ -48,7 +48,7 @@ MODULES: Dict[str, List[str]] = {
 }
 HOST_ONLY = {"host"}
 HEADERS = ["common.cuh", "mma_tile.cuh", "tc_common.cuh", "gemm_parts.cuh", "leone_static.h", "attention_tiled.cu", "random_draw.h",
-           "gla_parts.cuh", "ssd_parts.cuh", "experts_tc.h"]
+           "gla_parts.cuh", "ssd_parts.cuh", "experts_tc.h", "gemm_f32.h"]
 
 # -fno-gnu-unique: statics inside inline functions and templates (the once-per-kernel set-up
 # flags, the launch mode switch) must belong to one library image each; with GNU unique

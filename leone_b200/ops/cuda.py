@@ -241,7 +241,7 @@ class CudaOps:
         self.launches += 1
         _check(self.core.leone_gemm_simt(_dt(x.dtype), epilogue, _ptr(x), _ptr(w), _ptr(out),
                                          _ptr(residual), _ptr(bias), m, n, k, x.stride(0), w.stride(0),
-                                         out.stride(0), self._stream()), "gemm_simt")
+                                         out.stride(0), _ptr(self.status), self._stream()), "gemm_simt")
 
     def linear_fuses_norm(self, n_tokens: int, w: PreparedMatrix) -> bool:
         """True if a product of ``n_tokens`` tokens with ``w`` can take part in a fused RMSNorm:

@@ -11,9 +11,9 @@ from tests.test_kernels_gpu import DEV, _paged_setup, _randn, _ref_attention, op
 pytestmark = pytest.mark.gpu
 
 
-# m: the last and first size of every form (1, 2, 4, 8 | 16 | 32 | 64 | 128 tokens a tile) and ragged ones; n: fewer than a
+# m: the last and first size of every form (1, 2, 4, 8 tokens a block | 128 a tile) and ragged ones; n: fewer than a
 # block's four rows, a tile's edge, ragged; k: one piece, a ragged stage, several rounds of 256 threads, enough for eight splits
-@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 33, 64, 65, 130, 257])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 24, 25, 64, 128, 129, 257])
 @pytest.mark.parametrize("n,k", [(3, 4), (129, 100), (256, 2052), (1030, 4096)])
 def test_product_in_32_bits(ops32, m, n, k):  # noqa: F811
     x, w = _randn((m, k + 4), 1)[:, :k], _randn((n, k), 2)
