@@ -47,3 +47,28 @@ def test_top_k_keeps_the_best_ids_and_draws_among_them(ops32, vocab, k):  # noqa
         few = min(np.count_nonzero(got), len(keep))
         assert (got[best[:few]] > 0).all() and abs(got.sum() - 1.0) < 1e-12
         assert out[i].item() == select(got, uniform(seeds[i], positions[i]))
+
+
+@pytest.mark.parametrize("vocab", [2049, 4096, 4097, 9001, 151936])      # the first radix-sorted size, a tile of 4,096, remainders
+def test_rows_sorted_whole_keep_equal_logits_in_id_order(ops32, vocab):  # noqa: F811
+    from leone_b200.sampling.sampler import TRUNCATION_STAGES
+    logits = _rows(vocab)
+    logits[3] = torch.round(logits[3])                                   # many ties
+    logits[1, ::7] = -3e38
+    n, t = logits.shape[0], 1.3
+    # an epsilon of nearly nothing keeps every finite logit: the distribution is the whole row's
+    out, probs = ops32.sample_truncated(logits, [t] * n, list(range(n)), [5] * n, [(TRUNCATION_STAGES["epsilon"], 1e-300)],
+                                        want_probs=True)
+    # a top-k longer than a block collects is cut from the sorted row: ties at the cut keep the lower ids
+    k = min(1500, vocab)
+    _, cut = ops32.sample_truncated(logits, [t] * n, list(range(n)), [5] * n, [(TRUNCATION_STAGES["top_k"], float(k))], want_probs=True)
+    for i, row in enumerate(logits.cpu().numpy().astype(np.float64)):
+        ids = np.flatnonzero(np.isfinite(row))
+        if not len(ids):
+            assert out[i].item() == -1
+            continue
+        p = np.zeros(vocab)
+        p[ids] = np.exp((row[ids] - row[ids].max()) / t)
+        assert np.abs(probs[i].cpu().numpy() - p / p.sum()).max() < 1e-13
+        best = ids[np.lexsort((ids, -row[ids]))][:k]
+        assert set(np.flatnonzero(cut[i].cpu().numpy())) == set(best[p[best] > 0])
