@@ -56,6 +56,12 @@ class DecodeGraph:
         self._filled_rids = None           # what fill() last wrote into the host copy
         self._filled_pages = [[0] * batch for _ in engine.cache.groups]
         self._tables_at = min((o for o, _ in self.bt_offsets), default=None)   # where the block tables start
+        # A row as wide as a design without a position limit needs (65,536 entries and more) costs more to clear and to
+        # copy whole than a copy call of its own for the entries in use: 2 to 4 MB a refill, 44 us on the GPU and more on the
+        # host.  Nothing reads a table past its sequence's length.
+        self._wide = self._tables_at is not None and max(self.widths) > 16384
+        if self._wide:
+            self.meta[self._tables_at:].fill_(-1)
         self._events = [torch.cuda.Event(), torch.cuda.Event()]
         self._advance_host = [torch.zeros((2, batch), dtype=torch.int32, pin_memory=True) for _ in range(2)]
         self.launches_per_step = 0
@@ -141,15 +147,13 @@ class DecodeGraph:
         appended = []                       # [lo, hi) ranges of the host copy that gained entries
         for gi, (g, w, (o, shape)) in enumerate(zip(e.cache.groups, self.widths, self.bt_offsets)):
             view = host[o:o + shape[0] * shape[1]].reshape(shape)
-            windowed = g.spec.kind == "window"
-            if windowed:
-                same = False                # a window's table also loses entries at its front: rewrite
             for i, r in enumerate(rids):
                 n = int(table_lens[gi][i]) if table_lens is not None else g.tables.length(r)
                 if n > w:
                     raise ValueError(f"block table needs {n} columns, only {w} given")
-                done = 0 if (not same or windowed) else self._filled_pages[gi][i]
-                if done == 0:
+                # (a window's table that lost entries at its front has a new version, so it is not the same)
+                done = self._filled_pages[gi][i] if same else 0
+                if done == 0 and not self._wide:
                     view[i, :] = -1
                 if n > done:
                     view[i, done:n] = g.tables.tail(r, done)
@@ -164,9 +168,9 @@ class DecodeGraph:
             records.set_sampling(int(slot), p.seed, p.temperature)
             records.set_progress(int(slot), int(length), int(length), int(tok))
         records.sync()
-        if same and self._tables_at is not None:
-            # same requests in the same rows: the per-token and per-sequence vectors, and the
-            # block-table entries that were appended
+        if (same or self._wide) and self._tables_at is not None:
+            # the per-token and per-sequence vectors, and the block-table entries that are new: those appended since the last
+            # call for the same requests in the same rows, or all that are in use
             self.meta[:self._tables_at].copy_(self.meta_host[:self._tables_at], non_blocking=True)
             for lo, hi in appended:
                 self.meta[lo:hi].copy_(self.meta_host[lo:hi], non_blocking=True)
