@@ -278,6 +278,52 @@ gate_norm_kernel(const float* __restrict__ o, int width, const TW* __restrict__ 
   }
 }
 
+// The same with four neighbouring columns a load (rows of up to 4,096 columns in registers, 16-byte aligned), one reading of the
+// row: bound by the bytes, 2,048 rows of 2,048 in 9.1 us (33 MB, 5 us at the copy rate); element by
+// element 18.7.
+template <typename TW>
+__global__ void __launch_bounds__(256)
+gate_norm_vec_kernel(const float* o, int width, const TW* __restrict__ w, const __nv_bfloat16* gate, int ldg, __nv_bfloat16* out,
+                     float eps) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float scratch[33];
+  constexpr int kMost = 4;
+  const int t = blockIdx.x, pieces = width >> 2;
+  const float4* row = reinterpret_cast<const float4*>(o + (size_t)t * width);
+  float4 v[kMost];
+  uint2 g[kMost];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c < pieces) {
+      v[i] = row[c];
+      g[i] = *reinterpret_cast<const uint2*>(gate + (size_t)t * ldg + 4 * c);
+      ss = fmaf(v[i].x, v[i].x, ss);
+      ss = fmaf(v[i].y, v[i].y, ss);
+      ss = fmaf(v[i].z, v[i].z, ss);
+      ss = fmaf(v[i].w, v[i].w, ss);
+    }
+  }
+  ss = block_sum(ss, scratch);
+  const float r = 1.f / sqrtf(ss / (float)width + eps);
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const int c = threadIdx.x + i * 256;
+    if (c < pieces) {
+      const float g0 = sigmoid_f(__uint_as_float(g[i].x << 16)), g1 = sigmoid_f(__uint_as_float(g[i].x & 0xffff0000u)),
+                  g2 = sigmoid_f(__uint_as_float(g[i].y << 16)), g3 = sigmoid_f(__uint_as_float(g[i].y & 0xffff0000u));
+      const __nv_bfloat162 a = __floats2bfloat162_rn(v[i].x * r * to_float<TW>(w[4 * c]) * g0, v[i].y * r * to_float<TW>(w[4 * c + 1]) * g1);
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[i].z * r * to_float<TW>(w[4 * c + 2]) * g2, v[i].w * r * to_float<TW>(w[4 * c + 3]) * g3);
+      uint2 packed;
+      packed.x = *reinterpret_cast<const uint32_t*>(&a);
+      packed.y = *reinterpret_cast<const uint32_t*>(&b);
+      *reinterpret_cast<uint2*>(out + (size_t)t * width + 4 * c) = packed;
+    }
+  }
+}
+
 }  // namespace leone
 
 using namespace leone;
@@ -367,6 +413,14 @@ extern "C" int leone_gate_norm(int dtype, const float* o, int n_tokens, int widt
   if (width <= 0) return kRefusedSize;
 #define GN(T, TW) \
   launch_kernel(gate_norm_kernel<T, TW>, dim3(n_tokens), dim3(256), 0, stream, o, width, (const TW*)w, (const T*)gate, ldg, (T*)out, eps)
+  if (dtype == 1 && width % 4 == 0 && width <= 4096 && ldg % 4 == 0 && (uintptr_t)o % 16 == 0 && (uintptr_t)gate % 8 == 0 &&
+      (uintptr_t)out % 8 == 0 && (w_dtype == 0 || w_dtype == 1)) {
+    if (w_dtype == 0)
+      return launch_kernel(gate_norm_vec_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, o, width, (const float*)w,
+                           (const __nv_bfloat16*)gate, ldg, (__nv_bfloat16*)out, eps);
+    return launch_kernel(gate_norm_vec_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, o, width,
+                         (const __nv_bfloat16*)w, (const __nv_bfloat16*)gate, ldg, (__nv_bfloat16*)out, eps);
+  }
   if (dtype == 0 && w_dtype == 0) GN(float, float);
   else if (dtype == 1 && w_dtype == 0) GN(__nv_bfloat16, float);
   else if (dtype == 1 && w_dtype == 1) GN(__nv_bfloat16, __nv_bfloat16);

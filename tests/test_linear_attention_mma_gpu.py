@@ -49,3 +49,18 @@ def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens)
         assert ((got - want).abs() <= rel * size + 1e-30).all(), s
         assert ((state[slot].double() - end).abs() <= rel * end_size + 1e-30).all(), s
     assert torch.equal(state[[0, 2, 5]], before[[0, 2, 5]])
+
+
+# the smallest vector row, one that fills no round of 256 threads, the widest in registers, and the first that is not
+@pytest.mark.parametrize("width", [4, 1028, 4096, 4100])
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+def test_gate_norm(ops16, width, wdtype):  # noqa: F811
+    n, eps = 5, 1e-6
+    o, w = _randn((n, width), 1, scale=3.0), _randn((width,), 2).to(wdtype)
+    gate = _randn((n, width + 12), 3, torch.bfloat16)[:, 8:8 + width]
+    out = torch.empty((n, width), device=DEV, dtype=torch.bfloat16)
+    ops16.gate_norm(o, w, gate, out, eps)
+    x = o.double()
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps) * w.double() * torch.sigmoid(gate.double())
+    # the result's own rounding, and a few units of fp32 before it
+    assert ((out.double() - want).abs() <= (2.0 ** -8 + 1e-5) * want.abs() + 1e-30).all()
