@@ -12,12 +12,14 @@
 // An operand that is not finite (or rounds to infinity) has no such terms; a block that meets one forms its tile from
 // the operands in global memory instead, with fp32 FMA in the order of k.
 //
-// A block owns 128 tokens x 128 weight rows.  Warp 0 brings 32 k of both operands at a time by TMA (128-byte swizzle, three stages),
-// warps 2..9 replace a stage's words by their hi terms and leave the lo terms beside them (the same place in a second
-// tile, so nothing depends on the swizzle), warp 1 issues the MMAs, warps 10..17 add up.  Bound by shared memory: 32 KB
-// in, 32 KB read and 64 KB written by the split, 96 KB read by the MMAs, 224 KB of 128 bytes a cycle for 768 cycles of MMAs.
+// A block owns 128 tokens x 128 weight rows.  Warp 0 brings 32 k of both operands at a time by TMA (128-byte swizzle, four stages).
+// Warps 2..5 split the tokens' words and leave both terms in tensor memory, from where the MMAs read their A operand; warps
+// 6..9 replace the weights' words by their hi terms and leave the lo terms beside them (the same place in a second tile, so
+// nothing depends on the swizzle); warp 1 issues the MMAs, warps 10..17 add up.  Bound by shared memory: 32 KB in, 32 KB read and
+// 32 KB written by the split, 48 KB read by the MMAs, 144 KB at 128 bytes a cycle for 768 cycles of MMAs.  (With the tokens' terms
+// in shared memory too it was 224 KB, and 70 us where this takes 57.)
 // Where tiles are fewer than SMs a cluster of `splits` blocks shares a tile's K, as in gemm_simt.cu.  Every wait is bounded.
-// Measured (509 tokens): 12,288 x 2,048 202 us (126 TFLOP/s), 4,096 x 2,048 70 us, 2,048 x 6,144 109 us (two splits); tiles of packed
+// Measured (509 tokens): 12,288 x 2,048 169 us (151 TFLOP/s), 4,096 x 2,048 57 us, 2,048 x 6,144 89 us (two splits); tiles of packed
 // FMA (fma.rn.f32x2, 8 x 8 sums a thread) 617, 206 and 320 us.
 #include "gemm_f32.h"
 #include "tc_common.cuh"
@@ -25,25 +27,41 @@
 namespace leone {
 namespace tc {
 
-constexpr int kFtM = 128, kFtN = 128, kFtK = 32, kFtStages = 3;
+constexpr int kFtM = 128, kFtN = 128, kFtK = 32, kFtStages = 4;
 constexpr int kFtSplitWarps = 8, kFtSumWarps = 8, kFtThreads = 32 * (2 + kFtSplitWarps + kFtSumWarps);
-constexpr int kFtTile = kFtM * kFtK * 4;                  // one operand of a stage; hi and lo of both: 4 of them
-constexpr int kFtStage = 4 * kFtTile;
+constexpr int kFtTile = kFtM * kFtK * 4;                  // the tokens' words, the weights' hi terms, their lo terms
+constexpr int kFtStage = 3 * kFtTile;
+// tensor memory: two sums of hi hi, the sum of the small products, two sets of the tokens' hi and lo terms
+constexpr int kFtSmall = 2 * kFtN, kFtTerms = 3 * kFtN, kFtTermCols = 2 * kFtK;
 constexpr int kFtPitch = kFtN + 4;                        // floats of a row of the tile's sums
 constexpr int kFtSmem = kFtStages * kFtStage + 1024 + 256;
 static_assert(kFtM * kFtPitch * 4 <= kFtStages * kFtStage, "the sums fit where the stages were");
 
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
+// The nearest number of 11 significant bits (of two as near the larger), in integer steps: the conversion instruction runs at a
+// fraction of their rate.  For finite words; the caller looks for the others in the words' magnitudes.
+__device__ __forceinline__ uint32_t to_tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
+constexpr uint32_t kFtStrange = 0x7f7ff000u;              // from this magnitude on a word rounds to infinity, or is not finite
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo, uint32_t& most) {
+  hi = to_tf32(x);
+  lo = to_tf32(x - __uint_as_float(hi));
+  most = max(most, __float_as_uint(x) & 0x7fffffffu);
 }
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem]^T: row m of A in lane m, an element a column.
+__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 16 consecutive 32-bit columns of this thread's lane.
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 // tf32 x tf32 -> fp32, both operands K-major.
@@ -61,7 +79,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   uint8_t* tiles = smem_raw + (tiles_base - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + kFtStages * kFtStage);
   const uint32_t raw_full0 = smem_u32(bars), split_full0 = raw_full0 + 8 * kFtStages, empty0 = split_full0 + 8 * kFtStages;
-  const uint32_t sum_full0 = empty0 + 8 * kFtStages, sum_empty0 = sum_full0 + 16;
+  const uint32_t sum_full0 = empty0 + 8 * kFtStages, sum_empty0 = sum_full0 + 16, terms_empty0 = sum_empty0 + 16;
   __shared__ uint32_t tmem_holder;
   __shared__ int gave_up, odd;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,6 +98,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     for (int b = 0; b < 2; ++b) {
       mbar_init(sum_full0 + 8 * b, 1);
       mbar_init(sum_empty0 + 8 * b, kFtSumWarps);
+      mbar_init(terms_empty0 + 8 * b, 1);
     }
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
@@ -120,7 +139,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // ---------------- MMAs ----------------
     if (lane == 0) {
       const uint32_t idesc = instr_desc_tf32(kFtM, kFtN);
-      const uint32_t small = tmem_base + 2 * kFtN;
+      const uint32_t small = tmem_base + kFtSmall;
       int stage = 0;
       uint32_t phase = 0;
       for (int step = first; step < last; ++step) {
@@ -129,44 +148,81 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (!mbar_wait(split_full0 + 8 * stage, phase, giveup)) break;
         tc_fence_after();
         const uint32_t at = tiles_base + stage * kFtStage, big = tmem_base + buf * kFtN;
-        const uint64_t a_hi = smem_desc_sw128(at), w_hi = smem_desc_sw128(at + kFtTile);
-        const uint64_t a_lo = smem_desc_sw128(at + 2 * kFtTile), w_lo = smem_desc_sw128(at + 3 * kFtTile);
+        const uint32_t a_hi = tmem_base + kFtTerms + (i & 1) * kFtTermCols, a_lo = a_hi + kFtK;
+        const uint64_t w_hi = smem_desc_sw128(at + kFtTile), w_lo = smem_desc_sw128(at + 2 * kFtTile);
 #pragma unroll
         for (int k = 0; k < kFtK / 8; ++k) {
-          umma_tf32(big, a_hi + 2 * k, w_hi + 2 * k, idesc, (i & 1) || k > 0 ? 1u : 0u);
-          umma_tf32(small, a_hi + 2 * k, w_lo + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
-          umma_tf32(small, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
+          umma_tf32(big, a_hi + 8 * k, w_hi + 2 * k, idesc, (i & 1) || k > 0 ? 1u : 0u);
+          umma_tf32(small, a_hi + 8 * k, w_lo + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+          umma_tf32(small, a_lo + 8 * k, w_hi + 2 * k, idesc, 1u);
         }
+        umma_commit(terms_empty0 + 8 * (i & 1));
         umma_commit(empty0 + 8 * stage);
         if ((i & 1) || step + 1 == last) umma_commit(sum_full0 + 8 * buf);
         if (++stage == kFtStages) { stage = 0; phase ^= 1; }
       }
     }
+  } else if (warp < 6) {
+    // ---------------- split of the tokens: a thread's row of 32 words, both terms to its lane of tensor memory ----------------
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int step = first; step < last; ++step) {
+      const int i = step - first;
+      bool ok = mbar_wait(terms_empty0 + 8 * (i & 1), ((i >> 1) & 1) ^ 1, giveup) && mbar_wait(raw_full0 + 8 * stage, phase, giveup);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const float4* words = reinterpret_cast<const float4*>(tiles + stage * kFtStage + row * 128);
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kFtTerms + (i & 1) * kFtTermCols;
+      uint32_t most = 0;
+#pragma unroll
+      for (int c0 = 0; c0 < 8; c0 += 4) {
+        uint32_t h[16], l[16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 x = words[(c0 + c) ^ (row & 7)];            // the 128-byte swizzle: 16-byte pieces by row
+          split_tf32(x.x, h[4 * c], l[4 * c], most);
+          split_tf32(x.y, h[4 * c + 1], l[4 * c + 1], most);
+          split_tf32(x.z, h[4 * c + 2], l[4 * c + 2], most);
+          split_tf32(x.w, h[4 * c + 3], l[4 * c + 3], most);
+        }
+        tmem_store16(taddr + 4 * c0, h);
+        tmem_store16(taddr + kFtK + 4 * c0, l);
+      }
+      if (most >= kFtStrange) odd = 1;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(split_full0 + 8 * stage);
+      if (++stage == kFtStages) { stage = 0; phase ^= 1; }
+    }
   } else if (warp < 2 + kFtSplitWarps) {
-    // ---------------- split: words to hi terms in place, lo terms two tiles further on ----------------
-    const int at = (warp - 2) * 32 + lane;
+    // ---------------- split of the weights: words to hi terms in place, lo terms in the next tile ----------------
+    const int at = (warp - 6) * 32 + lane;
     int stage = 0;
     uint32_t phase = 0;
     for (int step = first; step < last; ++step) {
       bool ok = mbar_wait(raw_full0 + 8 * stage, phase, giveup);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      float4* words = reinterpret_cast<float4*>(tiles + stage * kFtStage);
+      float4* words = reinterpret_cast<float4*>(tiles + stage * kFtStage + kFtTile);
       uint4* hi = reinterpret_cast<uint4*>(words);
-      uint4* lo = hi + 2 * kFtTile / 16;
-      bool strange = false;
+      uint4* lo = hi + kFtTile / 16;
+      uint32_t most = 0;
 #pragma unroll
-      for (int j = 0; j < 2 * kFtTile / 16 / (32 * kFtSplitWarps); ++j) {
-        const int i = at + j * 32 * kFtSplitWarps;
+      for (int j = 0; j < kFtTile / 16 / 128; ++j) {
+        const int i = at + j * 128;
         const float4 x = words[i];
-        const uint4 h = make_uint4(to_tf32(x.x), to_tf32(x.y), to_tf32(x.z), to_tf32(x.w));
+        uint4 h, l;
+        split_tf32(x.x, h.x, l.x, most);
+        split_tf32(x.y, h.y, l.y, most);
+        split_tf32(x.z, h.z, l.z, most);
+        split_tf32(x.w, h.w, l.w, most);
         hi[i] = h;
-        lo[i] = make_uint4(to_tf32(x.x - __uint_as_float(h.x)), to_tf32(x.y - __uint_as_float(h.y)),
-                           to_tf32(x.z - __uint_as_float(h.z)), to_tf32(x.w - __uint_as_float(h.w)));
-        strange |= (h.x & 0x7f800000u) == 0x7f800000u || (h.y & 0x7f800000u) == 0x7f800000u ||
-                   (h.z & 0x7f800000u) == 0x7f800000u || (h.w & 0x7f800000u) == 0x7f800000u;
+        lo[i] = l;
       }
-      if (strange) odd = 1;
+      if (most >= kFtStrange) odd = 1;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(split_full0 + 8 * stage);
@@ -197,7 +253,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       if (!ok) break;
       tc_fence_after();
       add(taddr + buf * kFtN);
-      if (pair + 1 == pairs) add(taddr + 2 * kFtN);      // the last commit covers the small products too
+      if (pair + 1 == pairs) add(taddr + kFtSmall);      // the last commit covers the small products too
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(sum_empty0 + 8 * buf);

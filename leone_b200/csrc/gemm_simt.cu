@@ -6,7 +6,7 @@
 //
 // Three forms, chosen by leone_gemm_simt from dtype, sizes and alignment:
 //  * gemm_rows: 32 bits, up to 24 tokens.  A stream over the weights;
-//  * gemm_f32_tc.cu: 32 bits, more tokens.  Tiles on tensor cores, operands split into exact terms;
+//  * gemm_f32_tc.cu: 32 bits, more tokens, K of 256 and more.  Tiles on tensor cores, operands split into exact terms;
 //  * gemm_simt_kernel: bfloat16, and any size or alignment (4-byte loads).
 // In every form a row of C is computed from its own row of A only.  How its sum over k is grouped depends on the
 // form and the split, so a token's result in another batch differs by fp32 rounding at most.
@@ -163,9 +163,13 @@ gemm_rows_kernel(const float* A, const float* __restrict__ W, float* C, const fl
 }
 
 // The 32-bit product with 16-byte loads of up to 24 tokens: the stream is read again for every 8 tokens (its blocks share the
-// weights through the L2).  Beyond, tensor cores are faster: at 24 tokens 27 / 15 / 73 / 37 us here against 31 / 29 / 68 / 61 there
-// for 4,096, 2,048 and 12,288 rows of 2,048 and 2,048 of 6,144; they take the same at 64 tokens, where the stream is read 8 times.
+// weights through the L2).  Beyond, tensor cores are faster: at 24 tokens 27 / 15 / 73 / 37 us here against 29 / 26 / 58 / 51 there
+// (at 25) for 4,096, 2,048 and 12,288 rows of 2,048 and 2,048 of 6,144; they take the same at 64 tokens, where the stream is
+// read 8 times.
 constexpr int kStreamTokens = 24;
+// From here on the tensor cores' sums are nearer to 64 bits than a chain of FMA is (2.1e-7 at any K against 2.8e-7 at 256, growing
+// with its root; below, a chain is as near, and the product is small).
+constexpr int kTensorCoresFrom = 256;
 
 inline int launch_rows(const float* a, const float* w, float* c, const float* residual, const float* bias, int m, int n,
                        int k, int lda, int ldw, int ldc, cudaStream_t stream) {
@@ -195,8 +199,10 @@ extern "C" int leone_gemm_simt(int dtype, int epilogue, const void* a, const voi
     const float *x = (const float*)a, *y = (const float*)w, *r = epilogue == 2 ? residual : nullptr;
     if (m <= kStreamTokens && n <= 65535 * 4)
       return launch_rows(x, y, (float*)c, r, bias, m, n, k, lda, ldw, ldc, stream);
-    const int code = gemm_f32_tc(x, y, (float*)c, r, bias, m, n, k, lda, ldw, ldc, status, stream);
-    if (code >= 0) return code;            // (refused: nothing was launched)
+    if (k >= kTensorCoresFrom) {
+      const int code = gemm_f32_tc(x, y, (float*)c, r, bias, m, n, k, lda, ldw, ldc, status, stream);
+      if (code >= 0) return code;          // (refused: nothing was launched)
+    }
   }
   dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
   if (grid.y > 65535) return kRefusedSize;

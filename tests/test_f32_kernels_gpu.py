@@ -12,9 +12,10 @@ pytestmark = pytest.mark.gpu
 
 
 # m: the last and first size of every form (1, 2, 4, 8 tokens a block | 128 a tile) and ragged ones; n: fewer than a
-# block's four rows, a tile's edge, ragged; k: one piece, a ragged stage, several rounds of 256 threads, enough for eight splits
+# block's four rows, a tile's edge, ragged; k: one piece, the
+# last of the any-size kernel and the first of the tensor cores', a ragged stage, several rounds of 256 threads, enough for eight splits
 @pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 24, 25, 64, 128, 129, 257])
-@pytest.mark.parametrize("n,k", [(3, 4), (129, 100), (256, 2052), (1030, 4096)])
+@pytest.mark.parametrize("n,k", [(3, 4), (129, 252), (129, 256), (256, 2052), (1030, 4096)])
 def test_product_in_32_bits(ops32, m, n, k):  # noqa: F811
     x, w = _randn((m, k + 4), 1)[:, :k], _randn((n, k), 2)
     bias, res = _randn((n,), 3), _randn((m, n + 5), 4)[:, :n]
@@ -31,9 +32,25 @@ def test_product_in_32_bits(ops32, m, n, k):  # noqa: F811
     assert ((got.double() - want - bias.double() - res.double()).abs() <= bound).all()
 
 
+def test_values_at_the_edge_of_the_range_pass_through_the_product(ops32):  # noqa: F811
+    """The largest number, one that rounds past it at 11 bits, and NaNs of any payload, alone in their row and column."""
+    m, n, k = 40, 300, 256
+    for word in (0x7f7fffff, 0x7f7ff000, 0x7f7fefff, 0xff7fffff, 0x7fffffff, 0x7f800001, 0x7fc00000):
+        x, w = torch.zeros((m, k), device=DEV), torch.eye(n, k, device=DEV)
+        x.view(torch.int32)[7, 3] = word - (1 << 32) if word >> 31 else word
+        x[8, 5] = 1.5
+        out = torch.empty((m, n), device=DEV)
+        ops32._gemm_simt(x, w, out, 0, None)
+        if word & 0x7fffffff > 0x7f800000:
+            assert torch.isnan(out[7]).any()
+        else:                                          # two terms of 11 bits hold a word to 2^-23 of it
+            assert ((out[7, :k].double() - x[7].double()).abs() <= 2.0 ** -23 * x[7].double().abs()).all()
+        assert torch.equal(out[8, :k], x[8]) and torch.isfinite(out[:7]).all() and torch.isfinite(out[9:]).all()
+
+
 def test_a_row_of_the_product_with_an_infinity_stays_its_own(ops32):  # noqa: F811
     for m in (4, 40):
-        x, w = _randn((m, 64), 5), _randn((130, 64), 6)
+        x, w = _randn((m, 260), 5), _randn((130, 260), 6)
         x[1, 3] = float("inf")
         out = torch.empty((m, 130), device=DEV)
         ops32._gemm_simt(x, w, out, 0, None)
