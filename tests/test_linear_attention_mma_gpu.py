@@ -64,3 +64,15 @@ def test_gate_norm(ops16, width, wdtype):  # noqa: F811
     want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps) * w.double() * torch.sigmoid(gate.double())
     # the result's own rounding, and a few units of fp32 before it
     assert ((out.double() - want).abs() <= (2.0 ** -8 + 1e-5) * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("width", [4, 1028, 4096, 4100])
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+def test_two_norms_of_the_same_rows(ops16, width, wdtype):  # noqa: F811
+    n, eps = 5, 1e-6
+    x, a, b = _randn((n, width), 1, scale=3.0), _randn((width,), 2).to(wdtype), _randn((width,), 3).to(wdtype)
+    out = [torch.empty((n, width), device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    ops16.rms_norm_pair(x, a, b, *out, eps)
+    y = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + eps)
+    for got, w in zip(out, (a, b)):
+        assert ((got.double() - y * w.double()).abs() <= (2.0 ** -8 + 1e-5) * (y * w.double()).abs() + 1e-30).all()
