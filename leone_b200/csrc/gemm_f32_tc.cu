@@ -18,7 +18,8 @@
 // nothing depends on the swizzle); warp 1 issues the MMAs, warps 10..17 add up.  Bound by shared memory: 32 KB in, 32 KB read and
 // 32 KB written by the split, 48 KB read by the MMAs, 144 KB at 128 bytes a cycle for 768 cycles of MMAs.  (With the tokens' terms
 // in shared memory too it was 224 KB, and 70 us where this takes 57.)
-// Where tiles are fewer than SMs a cluster of `splits` blocks shares a tile's K, as in gemm_simt.cu.  Every wait is bounded.
+// Where tiles are fewer than SMs a cluster of `splits` blocks shares a tile's K: every block leaves its sums in its own shared
+// memory, and each adds a share of the rows over the ranks, in rank order.  Every wait is bounded.
 // Measured (509 tokens): 12,288 x 2,048 169 us (151 TFLOP/s), 4,096 x 2,048 57 us, 2,048 x 6,144 89 us (two splits); tiles of packed
 // FMA (fma.rn.f32x2, 8 x 8 sums a thread) 617, 206 and 320 us.
 #include "gemm_f32.h"
