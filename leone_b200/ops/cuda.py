@@ -611,11 +611,12 @@ class CudaOps:
                 and self.mixers.leone_linear_attention_mma_supported(dim, vdim) and proj.data_ptr() % 16 == 0
                 and not any(o % 8 for o in (proj.stride(0), q_off, k_off, v_off))):
             # Prompt portions in bfloat16: 64 tokens at a time on tensor cores.  Chunks as short as still leave about
-            # two rounds of blocks (two a SM): a chunk's state costs as much traffic as 64 tokens' outputs.
+            # two rounds of blocks (two a SM): a chunk's state costs as much traffic as 64 tokens' outputs.  Once no
+            # sequence is cut any more, longer chunks make no fewer blocks.
             chunk_decay = None
             chunk = 64
             q_lens = [int(q) for q in ctx.q_lens]
-            while sum(-(-q // chunk) for q in q_lens) * heads * -(-vdim // 64) > 4 * self.fast.sm_count:
+            while chunk < max(q_lens) and sum(-(-q // chunk) for q in q_lens) * heads * -(-vdim // 64) > 4 * self.fast.sm_count:
                 chunk *= 2
             if max(q_lens) <= chunk:
                 chunk = 0
