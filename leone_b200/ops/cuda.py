@@ -433,6 +433,18 @@ class CudaOps:
             c_float(scale), int(window or 0), cache.page_tokens, kp.shape[0], bt.shape[0],
             _ptr(ctx.status), self._stream()), "attention_generic")
 
+    @staticmethod
+    def _leading_single_rows(ctx) -> int:
+        """How many sequences of one token stand in front of a mixed step's portions (the scheduler puts decode rows first);
+        0 for a step of one kind or of fixed shapes."""
+        q_lens = getattr(ctx, "q_lens", None)
+        if ctx.decode_only or getattr(ctx, "fixed_shapes", False) or q_lens is None:
+            return 0
+        n = 0
+        while n < len(q_lens) and q_lens[n] == 1:
+            n += 1
+        return n if n < len(q_lens) else 0
+
     def _attention_f32(self, ctx, qkv, out, n_q, n_kv, d, scale, window, cache) -> bool:
         """The 32-bit kernels for head sizes 64 and 128.  False: the any-size kernel's case.  In a mixed step the leading
         rows of one token each (the scheduler puts decode rows first) run in the decode form, which streams a sequence's
@@ -443,14 +455,10 @@ class CudaOps:
             return False                    # (the any-size kernel needs no sequence starts)
         kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
         parts = [(0, ctx.n_seqs, ctx.max_q_len, ctx.max_ctx_len)]
-        q_lens = getattr(ctx, "q_lens", None)
-        if not ctx.decode_only and not getattr(ctx, "fixed_shapes", False) and q_lens is not None:
-            n = 0
-            while n < len(q_lens) and q_lens[n] == 1:
-                n += 1
-            if 0 < n < len(q_lens):
-                parts = [(0, n, 1, int(ctx.ctx_lens[:n].max())),
-                         (n, ctx.n_seqs - n, int(q_lens[n:].max()), int(ctx.ctx_lens[n:].max()))]
+        n = self._leading_single_rows(ctx)
+        if n:
+            parts = [(0, n, 1, int(ctx.ctx_lens[:n].max())),
+                     (n, ctx.n_seqs - n, int(ctx.q_lens[n:].max()), int(ctx.ctx_lens[n:].max()))]
         for first, count, q_len, ctx_len in parts:
             self.launches += 1
             _check(self.core.leone_attention_f32(
@@ -612,10 +620,18 @@ class CudaOps:
                 and not any(o % 8 for o in (proj.stride(0), q_off, k_off, v_off))):
             # Prompt portions in bfloat16: 64 tokens at a time on tensor cores.  Chunks as short as still leave about
             # two rounds of blocks (two a SM): a chunk's state costs as much traffic as 64 tokens' outputs.  Once no
-            # sequence is cut any more, longer chunks make no fewer blocks.
+            # sequence is cut any more, longer chunks make no fewer blocks.  A decode row in front of the portions would
+            # be a tile of 64 tokens here: those rows are walked.
+            lead = self._leading_single_rows(ctx)
+            if lead:
+                self.launches += 1
+                _check(self.mixers.leone_linear_attention(
+                    _dt(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
+                    _ptr(ctx.q_start), _ptr(ctx.slot_ids), _ptr(decay), lead, heads, dim, vdim, state.shape[0], 0, 0,
+                    c_void_p(0), _ptr(ctx.status), self._stream()), "linear_attention")
             chunk_decay = None
             chunk = 64
-            q_lens = [int(q) for q in ctx.q_lens]
+            q_lens = [int(q) for q in ctx.q_lens[lead:]]
             while chunk < max(q_lens) and sum(-(-q // chunk) for q in q_lens) * heads * -(-vdim // 64) > 4 * self.fast.sm_count:
                 chunk *= 2
             if max(q_lens) <= chunk:
@@ -626,9 +642,10 @@ class CudaOps:
                 chunk_decay = self._scratch("linattn_chunk_decay", n_chunks, heads * dim, torch.float32)
             self.launches += 1 if chunk == 0 else 3
             _check(self.mixers.leone_linear_attention_mma(
-                _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state), _ptr(ctx.q_start),
-                _ptr(ctx.slot_ids), _ptr(decay), ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk, n_chunks,
-                _ptr(chunk_state), _ptr(chunk_decay), _ptr(ctx.status), self._stream()), "linear_attention_mma")
+                _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
+                _ptr(ctx.q_start[lead:]), _ptr(ctx.slot_ids[lead:]), _ptr(decay), len(q_lens), heads, dim, vdim, state.shape[0],
+                chunk, n_chunks, _ptr(chunk_state), _ptr(chunk_decay), _ptr(ctx.status), self._stream()),
+                "linear_attention_mma")
             return
         if chunk > 0:
             n_chunks = int(sum(-(-int(q) // chunk) for q in ctx.q_lens))

@@ -19,14 +19,16 @@ def _walk(q, k, v, decay, state):
 
 
 # dim: below, at and above the widths of the kernel's forms; vdim: a part of a block's 64 columns, one block, a block and a part.
-# Lengths: one token, around a tile of 64, several tiles in one chunk and in several; decays of 0, weak, 1 and above 1.
+# Lengths: one token, around a tile of 64, several tiles in one chunk and in several; decode rows in front
+# of a portion and more sequences than two rounds of blocks hold; decays of 0, weak, 1 and above 1.
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 8), (3, 40, 72), (2, 64, 64), (4, 128, 128), (1, 88, 24)])
-@pytest.mark.parametrize("q_lens", [[16], [63, 1, 65], [200, 64, 130], [700]])
+@pytest.mark.parametrize("q_lens", [[16], [63, 1, 65], [200, 64, 130], [700],
+                                    [1] * 24 + [100], [17, 1] * 160])
 def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens):  # noqa: F811
-    n, slots = sum(q_lens), [4, 1, 3][:len(q_lens)]
+    n, slots = sum(q_lens), [4, 1, 3][:len(q_lens)] if len(q_lens) <= 3 else [6 + i for i in range(len(q_lens))]
     cols = 2 * heads * dim + heads * vdim
     proj = _randn((n, cols + 8), 3, torch.bfloat16, 1.5)[:, :cols]
-    state = _randn((6, heads, dim, vdim), 4)
+    state = _randn((6 + len(q_lens), heads, dim, vdim), 4)
     decay = torch.tensor([0.97, 0.0, 1.0, 1.01][:heads], device=DEV)
     before = state.clone()
     starts = np.concatenate([[0], np.cumsum(q_lens)])
@@ -48,7 +50,8 @@ def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens)
         got = out[a:b].view(b - a, heads, vdim).double()
         assert ((got - want).abs() <= rel * size + 1e-30).all(), s
         assert ((state[slot].double() - end).abs() <= rel * end_size + 1e-30).all(), s
-    assert torch.equal(state[[0, 2, 5]], before[[0, 2, 5]])
+    others = [i for i in range(6 + len(q_lens)) if i not in slots]
+    assert torch.equal(state[others], before[others])
 
 
 # the smallest vector row, one that fills no round of 256 threads, the widest in registers, and the first that is not

@@ -61,4 +61,20 @@ def test_the_choice_of_a_chunk_ends(q_lens, heads, vdim):
     assert calls
     # every sequence has at least one chunk, and a chunk holds at least 64 tokens of one
     if "linattn_chunks" in scratch:
-        assert len(q_lens) <= scratch["linattn_chunks"][0] <= sum(-(-q // 64) for q in q_lens)
+        assert scratch["linattn_chunks"][0] <= sum(-(-q // 64) for q in q_lens)
+
+
+# decode rows lead a mixed step: they are walked, and only what follows goes through tiles of 64 tokens; a row of one token
+# between portions stays with them
+@pytest.mark.parametrize("q_lens,walked", [([1] * 24 + [100], 24), ([1, 16], 1), ([100], 0), ([100, 1, 1], 0), ([1, 1, 70, 1, 16], 2)])
+def test_decode_rows_of_a_mixed_step_are_walked(q_lens, walked):
+    _, calls = _plan(q_lens, 4, 64, 64)
+    walks = [args for name, args in calls if name == "leone_linear_attention"]
+    assert [args[12] for args in walks] == ([walked] if walked else [])        # (its sequences)
+    assert len(calls) == len(walks) + 1
+
+
+def test_steps_of_one_kind_are_one_launch():
+    for q_lens, dtype in (([1] * 8, torch.bfloat16), ([15, 1, 2], torch.bfloat16), ([1, 100], torch.float32)):
+        _, calls = _plan(q_lens, 4, 64, 64, dtype)
+        assert [(name, args[12]) for name, args in calls] == [("leone_linear_attention", len(q_lens))]
