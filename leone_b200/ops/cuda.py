@@ -616,12 +616,12 @@ class CudaOps:
               and decay.dtype == torch.float32 and decay.numel() == heads, "linear_attention state/decay")
         n_chunks, chunk_state = 0, None
         if (self.fast is not None and proj.dtype == torch.bfloat16 and not ctx.decode_only and ctx.max_q_len >= 16
-                and self.mixers.leone_linear_attention_mma_supported(dim, vdim) and proj.data_ptr() % 16 == 0
+                and self.mixers.leone_linear_attention_tiles_supported(dim, vdim)
+                and not any(t.data_ptr() % 16 for t in (proj, out, state))
                 and not any(o % 8 for o in (proj.stride(0), q_off, k_off, v_off))):
-            # Prompt portions in bfloat16: 64 tokens at a time on tensor cores.  Chunks as short as still leave about
-            # two rounds of blocks (two a SM): a chunk's state costs as much traffic as 64 tokens' outputs.  Once no
-            # sequence is cut any more, longer chunks make no fewer blocks.  A decode row in front of the portions would
-            # be a tile of 64 tokens here: those rows are walked.
+            # Prompt portions in bfloat16: 64 tokens at a time.  A decode row in front of the portions would be a tile of
+            # 64 tokens here: those rows are walked.  A chunk's start state stands in scratch, but for a sequence's first
+            # chunk, which starts from the slot.
             lead = self._leading_single_rows(ctx)
             if lead:
                 self.launches += 1
@@ -629,23 +629,15 @@ class CudaOps:
                     _dt(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
                     _ptr(ctx.q_start), _ptr(ctx.slot_ids), _ptr(decay), lead, heads, dim, vdim, state.shape[0], 0, 0,
                     c_void_p(0), _ptr(ctx.status), self._stream()), "linear_attention")
-            chunk_decay = None
-            chunk = 64
-            q_lens = [int(q) for q in ctx.q_lens[lead:]]
-            while chunk < max(q_lens) and sum(-(-q // chunk) for q in q_lens) * heads * -(-vdim // 64) > 4 * self.fast.sm_count:
-                chunk *= 2
-            if max(q_lens) <= chunk:
-                chunk = 0
-            else:
-                n_chunks = sum(-(-q // chunk) for q in q_lens)
-                chunk_state = self._scratch("linattn_chunks", n_chunks, heads * dim * vdim, torch.float32)
-                chunk_decay = self._scratch("linattn_chunk_decay", n_chunks, heads * dim, torch.float32)
-            self.launches += 1 if chunk == 0 else 3
-            _check(self.mixers.leone_linear_attention_mma(
+            chunks = [-(-int(q) // 64) for q in ctx.q_lens[lead:]]
+            entries = sum(c - 1 for c in chunks if c > 1)
+            if entries:
+                chunk_state = self._scratch("linattn_chunks", entries, heads * dim * vdim, torch.float32)
+            self.launches += 4 if entries else 2
+            _check(self.mixers.leone_linear_attention_tiles(
                 _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
-                _ptr(ctx.q_start[lead:]), _ptr(ctx.slot_ids[lead:]), _ptr(decay), len(q_lens), heads, dim, vdim, state.shape[0],
-                chunk, n_chunks, _ptr(chunk_state), _ptr(chunk_decay), _ptr(ctx.status), self._stream()),
-                "linear_attention_mma")
+                _ptr(ctx.q_start[lead:]), _ptr(ctx.slot_ids[lead:]), _ptr(decay), len(chunks), heads, dim, vdim, state.shape[0],
+                sum(chunks), entries, _ptr(chunk_state), _ptr(ctx.status), self._stream()), "linear_attention_tiles")
             return
         if chunk > 0:
             n_chunks = int(sum(-(-int(q) // chunk) for q in ctx.q_lens))

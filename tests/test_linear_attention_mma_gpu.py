@@ -1,4 +1,4 @@
-"""Linear attention with a decaying state on tensor cores, against the recurrence in float64."""
+"""Linear attention with a decaying state in prompt portions, and the row kernels beside it, against float64."""
 import types
 
 import numpy as np
@@ -18,23 +18,28 @@ def _walk(q, k, v, decay, state):
     return out, state
 
 
-# dim: below, at and above the widths of the kernel's forms; vdim: a part of a block's 64 columns, one block, a block and a part.
-# Lengths: one token, around a tile of 64, several tiles in one chunk and in several; decode rows in front
-# of a portion and more sequences than two rounds of blocks hold; decays of 0, weak, 1 and above 1.
-@pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 8), (3, 40, 72), (2, 64, 64), (4, 128, 128), (1, 88, 24)])
-@pytest.mark.parametrize("q_lens", [[16], [63, 1, 65], [200, 64, 130], [700],
-                                    [1] * 24 + [100], [17, 1] * 160])
-def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens):  # noqa: F811
+def _step(heads, dim, vdim, q_lens):
     n, slots = sum(q_lens), [4, 1, 3][:len(q_lens)] if len(q_lens) <= 3 else [6 + i for i in range(len(q_lens))]
     cols = 2 * heads * dim + heads * vdim
     proj = _randn((n, cols + 8), 3, torch.bfloat16, 1.5)[:, :cols]
     state = _randn((6 + len(q_lens), heads, dim, vdim), 4)
     decay = torch.tensor([0.97, 0.0, 1.0, 1.01][:heads], device=DEV)
-    before = state.clone()
-    starts = np.concatenate([[0], np.cumsum(q_lens)])
     i32 = dict(dtype=torch.int32, device=DEV)
-    ctx = types.SimpleNamespace(q_start=torch.tensor(starts, **i32), slot_ids=torch.tensor(slots, **i32), n_seqs=len(q_lens),
-                                q_lens=np.array(q_lens), max_q_len=max(q_lens), decode_only=False, status=torch.zeros(4, **i32))
+    ctx = types.SimpleNamespace(q_start=torch.tensor(np.concatenate([[0], np.cumsum(q_lens)]), **i32),
+                                slot_ids=torch.tensor(slots, **i32), n_seqs=len(q_lens), q_lens=np.array(q_lens),
+                                max_q_len=max(q_lens), decode_only=False, status=torch.zeros(4, **i32))
+    return proj, state, decay, ctx, slots
+
+
+# dim: below, at and above the widths of the kernels' forms; vdim: a part of a block's 64 or 128 columns, one block, a block and a part.
+# Lengths: one token, around a tile of 64, several tiles; decode rows in front
+# of a portion and more sequences than two rounds of blocks hold; decays of 0, weak, 1 and above 1.
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 8), (3, 40, 72), (2, 64, 64), (4, 128, 128), (1, 88, 24), (2, 72, 136)])
+@pytest.mark.parametrize("q_lens", [[16], [63, 1, 65], [200, 64, 130], [700],
+                                    [1] * 24 + [100], [17, 1] * 160])
+def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens):  # noqa: F811
+    proj, state, decay, ctx, slots = _step(heads, dim, vdim, q_lens)
+    n, before, starts = sum(q_lens), state.clone(), ctx.q_start.tolist()
     out = torch.full((n, heads * vdim), 9.0, device=DEV)
     ops16.linear_attention(ctx, proj, out, state, decay, heads, dim, vdim, 0, heads * dim, 2 * heads * dim, chunk=64)
     assert ctx.status.tolist() == [0, 0, 0, 0]
@@ -44,14 +49,46 @@ def test_prompt_portions_against_the_recurrence(ops16, heads, dim, vdim, q_lens)
     for s, (a, b, slot) in enumerate(zip(starts[:-1], starts[1:], slots)):
         want, end = _walk(q[a:b], k[a:b], v[a:b], decay.double(), before[slot].double())
         size, end_size = _walk(q[a:b].abs(), k[a:b].abs(), v[a:b].abs(), decay.double(), before[slot].double().abs())
-        # two terms hold an operand to 2^-17 of it; an output has up to four such operands (q, k or the state, the weighted
-        # score, v), and the dropped products of two lo terms are 2^-18; sums of n terms in fp32 add n 2^-24
-        rel = 5 * 2.0 ** -17 + (b - a + dim) * 2.0 ** -24
+        # a silu is within 2^-21 (an exponential of two units of the last place, a sum, a division), an output has three; sums
+        # of n terms in fp32 add n 2^-24, the weights a rounding each
+        rel = 3 * 2.0 ** -21 + (b - a + dim + 8) * 2.0 ** -24
         got = out[a:b].view(b - a, heads, vdim).double()
         assert ((got - want).abs() <= rel * size + 1e-30).all(), s
         assert ((state[slot].double() - end).abs() <= rel * end_size + 1e-30).all(), s
+        # roundings of either sign grow with the root of their number; operands short of 32 bits show (two bfloat16 terms: 1.5e-6 to 5e-6)
+        assert (got - want).norm() <= 8e-7 * want.norm() and (state[slot].double() - end).norm() <= 8e-7 * end.norm()
     others = [i for i in range(6 + len(q_lens)) if i not in slots]
     assert torch.equal(state[others], before[others])
+
+
+# in the first tile, at its end, and in the last of several; an infinity or a NaN in a key, a query or a value
+@pytest.mark.parametrize("at", [5, 63, 130])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_a_token_that_is_not_finite_reaches_no_earlier_one(ops16, at, bad):  # noqa: F811
+    heads, dim, vdim = 2, 64, 72
+    hd, c = heads * dim, 9                             # channel or column 9 of head 0
+    runs = []
+    for column in (None, c, hd + c, 2 * hd + c):
+        proj, state, decay, ctx, slots = _step(heads, dim, vdim, [150])
+        decay.fill_(0.9)
+        proj = proj.clone()
+        if column is not None:
+            proj[at, column] = bad
+        out = torch.full((150, heads * vdim), 9.0, device=DEV)
+        ops16.linear_attention(ctx, proj, out, state, decay, heads, dim, vdim, 0, hd, 2 * hd, chunk=64)
+        assert ctx.status.tolist() == [0, 0, 0, 0]
+        runs.append((out.view(150, heads, vdim), state[slots[0]]))
+    (clean, end), (q, q_end), (k, k_end), (v, v_end) = runs
+    for out, state in runs[1:]:
+        assert torch.equal(out[:at], clean[:at]) and torch.equal(out[:, 1], clean[:, 1]) and torch.equal(state[1], end[1])
+    # a query is its own token's; a key's channel is a row of the state and reaches every later output; a value's column stays one
+    others = [i for i in range(vdim) if i != c]
+    assert torch.equal(q[at + 1:], clean[at + 1:]) and not torch.isfinite(q[at, 0]).any() and torch.equal(q_end, end)
+    rows = [i for i in range(dim) if i != c]
+    assert torch.equal(k_end[0, rows], end[0, rows]) and not torch.isfinite(k_end[0, c]).any()
+    assert not torch.isfinite(k[at:, 0]).any()
+    assert torch.equal(v[:, 0, others], clean[:, 0, others]) and torch.equal(v_end[0][:, others], end[0][:, others])
+    assert not torch.isfinite(v[at:, 0, c]).any() and not torch.isfinite(v_end[0, :, c]).any()
 
 
 # the smallest vector row, one that fills no round of 256 threads, the widest in registers, and the first that is not
