@@ -61,6 +61,7 @@ __device__ __forceinline__ long long key_row(const Params& p, int s, int kvh, in
 // itself) 1,155 us.
 constexpr int kRowsQ = 64, kKeys = 64;
 
+template <bool B> struct Masked { static constexpr bool value = B; };
 template <int D>
 struct PromptShape {
   static constexpr int kPitch = D + 4, kPitchP = kKeys + 4;
@@ -199,27 +200,35 @@ attention_f32_prompt_kernel(const Params p) {
     __syncthreads();                       // values have landed, weights are written, the keys' readers are done
     if (t + 1 < tiles) load(p.k_pool, k_at, S::kPitch, buf ^ 1);
     cp_commit();
+    // Of a tile on the diagonal or at the window's edge a row takes its own keys only: a masked key's weight is 0, but its value
+    // may be infinite.  (A missing page's values are zeros.)
+    auto add = [&](auto some_masked) {
 #pragma unroll 2
-    for (int j = 0; j < kKeys; j += 4) {
-      float w[4][4];
+      for (int j = 0; j < kKeys; j += 4) {
+        float w[4][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *(float4*)w[i] = *(const float4*)(p_s + (ty + 16 * i) * S::kPitchP + j);
+        for (int i = 0; i < 4; ++i) *(float4*)w[i] = *(const float4*)(p_s + (ty + 16 * i) * S::kPitchP + j);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        float4 v[kCols / 4];
+        for (int jj = 0; jj < 4; ++jj) {
+          float4 v[kCols / 4];
 #pragma unroll
-        for (int c = 0; c < kCols / 4; ++c) v[c] = *(const float4*)(v_s + (j + jj) * D + 64 * c + 4 * tx);
+          for (int c = 0; c < kCols / 4; ++c) v[c] = *(const float4*)(v_s + (j + jj) * D + 64 * c + 4 * tx);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 ww = make_float2(w[i][jj], w[i][jj]);
+          for (int i = 0; i < 4; ++i) {
+            const float2 ww = make_float2(w[i][jj], w[i][jj]);
+            const int key = j0 + j + jj;
+            if (decltype(some_masked)::value && (key > pos[i] || (p.window > 0 && key <= pos[i] - p.window))) continue;
 #pragma unroll
-          for (int c = 0; c < kCols / 4; ++c) {
-            fma2(acc[i][2 * c], ww, make_float2(v[c].x, v[c].y));
-            fma2(acc[i][2 * c + 1], ww, make_float2(v[c].z, v[c].w));
+            for (int c = 0; c < kCols / 4; ++c) {
+              fma2(acc[i][2 * c], ww, make_float2(v[c].x, v[c].y));
+              fma2(acc[i][2 * c + 1], ww, make_float2(v[c].z, v[c].w));
+            }
           }
         }
       }
-    }
+    };
+    if (j0 + kKeys - 1 > start + row0 / g || (p.window > 0 && j0 <= hi - p.window)) add(Masked<true>());
+    else add(Masked<false>());
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

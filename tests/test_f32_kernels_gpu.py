@@ -105,6 +105,39 @@ def test_attention_in_32_bits(ops32, n_q, n_kv, d, pt, window, seq_lens, starts)
         assert ((out[i].view(n_q, d).double() - want).abs() <= bound).all(), (s, p)
 
 
+# a position at the start, inside and at the end of a tile of 64 keys; windows that leave it inside the tile and across tiles
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("n_q,n_kv,d", [(4, 2, 128), (3, 1, 64)])
+@pytest.mark.parametrize("at,window", [(40, None), (64, None), (127, None), (40, 9), (64, 70), (127, 33)])
+def test_a_position_that_is_not_finite_reaches_only_the_rows_that_see_it(ops32, n_q, n_kv, d, at, window, bad):  # noqa: F811
+    length, pt = 200, 16
+    i32 = dict(dtype=torch.int32, device=DEV)
+    qkv = _randn((length, (n_q + 2 * n_kv) * d), 3)
+    runs = []
+    for pool in (None, 0, 1):
+        table, *pools = _paged_setup([length], pt, n_kv, d, torch.float32, 9)
+        for i, p in enumerate(pools):
+            p.copy_(_randn(p.shape, 10 + i))
+        if pool is not None:
+            pools[pool][table[0, at // pt], :, at % pt, d // 2] = bad
+        ctx = types.SimpleNamespace(q_start=torch.tensor([0, length], **i32), ctx_len=torch.tensor([length], **i32), n_seqs=1,
+                                    max_q_len=length, max_ctx_len=length, decode_only=False, fixed_shapes=False,
+                                    q_lens=np.array([length]), ctx_lens=np.array([length]), status=torch.zeros(4, **i32))
+        cache = types.SimpleNamespace(k_pool=pools[0], v_pool=pools[1], block_table=table, page_tokens=pt)
+        out = torch.full((length, n_q * d), 7.0, device=DEV)
+        assert ops32._attention_f32(ctx, qkv, out, n_q, n_kv, d, 0.1, window, cache)
+        runs.append(out)
+    sees = [p for p in range(length) if at <= p and (window is None or at > p - window)]
+    others = [p for p in range(length) if p not in sees]
+    clean, key, value = runs
+    assert torch.isfinite(clean).all()
+    assert torch.equal(key[others], clean[others]) and torch.equal(value[others], clean[others])
+    column = [h * d + d // 2 for h in range(n_q)]
+    assert not torch.isfinite(value[sees][:, column]).any()
+    value[:, column] = clean[:, column]
+    assert torch.equal(value, clean)
+
+
 def test_attention_in_32_bits_reports_a_missing_page(ops32):  # noqa: F811
     i32 = dict(dtype=torch.int32, device=DEV)
     for q_len in (1, 2):
