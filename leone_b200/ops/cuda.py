@@ -449,11 +449,11 @@ class CudaOps:
         """The 32-bit kernels for head sizes 64 and 128.  False: the any-size kernel's case.  In a mixed step the leading
         rows of one token each (the scheduler puts decode rows first) run in the decode form, which streams a sequence's
         keys, and the rest in the prompt form, which would spend a tile of 64 rows on each of them."""
-        if (qkv.dtype != torch.float32 or d not in (64, 128) or qkv.stride(0) % 4 or qkv.data_ptr() % 16
-                or out.data_ptr() % 16 or n_kv * -(-(n_q // n_kv) // 8) > 65535
-                or getattr(ctx, "q_start", None) is None or ctx.n_seqs > 65535):
-            return False                    # (the any-size kernel needs no sequence starts)
         kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
+        if (qkv.dtype != torch.float32 or d not in (64, 128) or qkv.stride(0) % 4 or out.stride(0) % 4
+                or any(t.data_ptr() % 16 for t in (qkv, out, kp, vp)) or n_kv * -(-(n_q // n_kv) // 8) > 65535
+                or getattr(ctx, "q_start", None) is None or ctx.n_seqs > 65535):
+            return False                    # (the any-size kernel needs no alignment and no sequence starts)
         parts = [(0, ctx.n_seqs, ctx.max_q_len, ctx.max_ctx_len)]
         n = self._leading_single_rows(ctx)
         if n:

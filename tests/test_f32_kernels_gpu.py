@@ -138,6 +138,27 @@ def test_a_position_that_is_not_finite_reaches_only_the_rows_that_see_it(ops32, 
     assert torch.equal(value, clean)
 
 
+def test_attention_on_pools_of_any_alignment(ops32):  # noqa: F811
+    """Pools that do not start on 16 bytes are the any-size kernel's."""
+    length, n_q, n_kv, d, pt = 21, 2, 1, 64, 4
+    table, k_pool, v_pool = _paged_setup([length], pt, n_kv, d, torch.float32, 9)
+    k_pool.copy_(_randn(k_pool.shape, 1))
+    v_pool.copy_(_randn(v_pool.shape, 2))
+    shifted = [torch.empty(p.numel() + 1, device=DEV)[1:].view(p.shape).copy_(p) for p in (k_pool, v_pool)]
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(q_start=torch.tensor([0, length], **i32), ctx_len=torch.tensor([length], **i32), n_seqs=1,
+                                max_q_len=length, max_ctx_len=length, decode_only=False, fixed_shapes=False,
+                                q_lens=np.array([length]), ctx_lens=np.array([length]), status=torch.zeros(4, **i32),
+                                positions=torch.arange(length, **i32), seq_of_token=torch.zeros(length, **i32))
+    qkv, outs = _randn((length, (n_q + 2 * n_kv) * d), 3), []
+    for k, v in ((k_pool, v_pool), shifted):
+        cache = types.SimpleNamespace(k_pool=k, v_pool=v, block_table=table, page_tokens=pt)
+        outs.append(torch.empty((length, n_q * d), device=DEV))
+        ops32.attention(ctx, qkv, outs[-1], n_q, n_kv, d, 0.125, None, cache)
+    # both within (2 d 2^-24 |q| |k| scale + length 2^-23) of the largest value; |q| |k| scale is below 20 for these
+    assert (outs[0] - outs[1]).abs().max() <= 2 * (2 * d * 2.0 ** -24 * 20 + length * 2.0 ** -23) * v_pool.abs().max()
+
+
 def test_attention_in_32_bits_reports_a_missing_page(ops32):  # noqa: F811
     i32 = dict(dtype=torch.int32, device=DEV)
     for q_len in (1, 2):
