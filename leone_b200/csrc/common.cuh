@@ -89,6 +89,16 @@ __device__ __forceinline__ void warp_sum_scatter(float* v, int lane) {
   }
 }
 
+// z / (1 + exp(-z)) without the branches of a division, which keep neighbouring values from overlapping: of exp(-|z|) the divisor
+// is between 1 and 2, and a Newton step on the approximate reciprocal's quotient (Markstein) leaves its rounding.
+__device__ __forceinline__ float silu_branchless(float z) {
+  const float e = expf(-fabsf(z)), n = z < 0.f ? z * e : z, d = 1.f + e;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r;
+  return z > 3.0e38f ? z : fmaf(fmaf(-q, d, n), r, q);     // (an infinite quotient has no remainder)
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.
 // `scratch` is 33 floats of shared memory.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

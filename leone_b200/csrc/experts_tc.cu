@@ -38,10 +38,6 @@ struct ExpertParams {
   int* status;
 };
 
-// (The exact division and exponential branch on every value, which kept 16 values a thread from overlapping: 25 us a tile.
-// These are within a few units of the last place, ahead of a rounding to bfloat16.)
-__device__ __forceinline__ float silu_exp(float z) { return __fdividef(z, 1.f + __expf(-z)); }
-
 // sorted[row] = x[token of the row's pair].  (What the kernels before this one write is not declared read-only: such a load
 // may be moved ahead of the wait for them.  The count of rows is the first thing read, so it would be.)
 __global__ void __launch_bounds__(256)
@@ -213,7 +209,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             const float s = __uint_as_float(a[j]);
             float f;
             if (p.mode == 0) {
-              f = silu_exp(round_to<__nv_bfloat16>(s * w)) * round_to<__nv_bfloat16>(__uint_as_float(b[j]) * w);
+              f = silu_branchless(round_to<__nv_bfloat16>(s * w)) * round_to<__nv_bfloat16>(__uint_as_float(b[j]) * w);
             } else if (p.mode == 1) {
               const float u = fmaxf(round_to<__nv_bfloat16>(s), 0.f);
               f = u * u;

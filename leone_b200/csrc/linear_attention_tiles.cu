@@ -86,15 +86,6 @@ __device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {
       : "+l"(reinterpret_cast<unsigned long long&>(acc))
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
 }
-// z / (1 + exp(-z)) without the branches of a division, which keep neighbouring values from overlapping: of exp(-|z|) the divisor
-// is between 1 and 2, and a Newton step on the approximate reciprocal's quotient (Markstein) leaves its rounding.
-__device__ __forceinline__ float silu_of(float z) {
-  const float e = expf(-fabsf(z)), n = z < 0.f ? z * e : z, d = 1.f + e;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = n * r;
-  return z > 3.0e38f ? z : fmaf(fmaf(-q, d, n), r, q);     // (an infinite quotient has no remainder)
-}
 // d^n, rounded once; a decay above one may overflow: 0 times it must stay 0.
 __device__ __forceinline__ float power(float d, int n) {
   double f = 1.0, b = (double)d;
@@ -108,8 +99,8 @@ __device__ __forceinline__ void silu8(uint4 raw, float* dst, float w = 1.f) {
   float v[8];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    v[2 * e] = silu_of(__uint_as_float(in[e] << 16)) * w;
-    v[2 * e + 1] = silu_of(__uint_as_float(in[e] & 0xffff0000u)) * w;
+    v[2 * e] = silu_branchless(__uint_as_float(in[e] << 16)) * w;
+    v[2 * e + 1] = silu_branchless(__uint_as_float(in[e] & 0xffff0000u)) * w;
   }
   *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
   *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);

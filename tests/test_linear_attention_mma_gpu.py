@@ -91,6 +91,26 @@ def test_a_token_that_is_not_finite_reaches_no_earlier_one(ops16, at, bad):  # n
     assert not torch.isfinite(v[at:, 0, c]).any() and not torch.isfinite(v_end[0, :, c]).any()
 
 
+def test_silu_of_every_bfloat16(ops16):  # noqa: F811
+    """A state that is forgotten at once (decay 0), keys and values of 128, whose silu is 128: outputs are 2^14 silu(q)."""
+    words = torch.arange(1 << 16, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    z = words[(words.float().abs() < 2.0 ** 80)]
+    n = z.numel()
+    proj = torch.zeros((n, 24), device=DEV, dtype=torch.bfloat16)
+    proj[:, 0], proj[:, 8], proj[:, 16:] = z, 128.0, 128.0
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(q_start=torch.tensor([0, n], **i32), slot_ids=torch.zeros(1, **i32), n_seqs=1, q_lens=np.array([n]),
+                                max_q_len=n, decode_only=False, status=torch.zeros(4, **i32))
+    out = torch.empty((n, 8), device=DEV)
+    ops16.linear_attention(ctx, proj, out, torch.zeros((1, 1, 8, 8), device=DEV), torch.zeros(1, device=DEV), 1, 8, 8, 0, 8, 16)
+    want = torch.nn.functional.silu(z.double())[:, None]
+    # the exponential's two units of the last place, its product, the divisor's sum and the quotient: four; an exponential below
+    # 2^-126 is held to 2^-149, and |z| times it
+    bound = 2.0 ** -21 * want.abs() + (z.double().abs()[:, None] + 2) * 2.0 ** -149
+    wrong = ((out.double() * 2.0 ** -14 - want).abs() > bound).any(1)
+    assert not wrong.any(), (z[wrong][:8], out[wrong][:8, 0] * 2.0 ** -14, want[wrong][:8])
+
+
 # the smallest vector row, one that fills no round of 256 threads, the widest in registers, and the first that is not
 @pytest.mark.parametrize("width", [4, 1028, 4096, 4100])
 @pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
