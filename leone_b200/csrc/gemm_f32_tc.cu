@@ -1,7 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T in 32 bits on tensor cores: the 32-bit product of prompt steps (gemm_simt.cu has the others).
 //
-// Every operand is the sum of two numbers of 11 significant bits, x = hi + lo + r with |r| <= 2^-23 |x| (both rounded to nearest),
-// and a product of two is hi hi + hi lo + lo hi; the dropped lo lo is at most 2^-24 of it, of either sign.  The three run as
+// Every operand is the sum of two numbers of 11 significant bits, x = hi + lo + r with |lo| <= 2^-11 |x| and |r| <= 2^-23 |x| (both
+// rounded to nearest), and a product of two is hi hi + hi lo + lo hi; the dropped lo lo is at most 2^-22 of it, of either
+// sign, so that a product is within about 2^-21 (of sums of normal inputs the drops are 8e-8 in the 2-norm).  The three run as
 // tcgen05.mma kind::tf32, whose operands these numbers are exactly.  What tensor cores lose is in their sums, not in
 // the products, so sums stay short there: hi hi of 64 k is summed in tensor memory (8 additions) and then added to fp32
 // registers, which hold the running sum over K; the small products (2^-12 of the result) are summed in tensor memory to the
@@ -9,8 +10,9 @@
 // of which 1.5e-7 is a bias towards zero (the sums in tensor memory are cut off, not rounded); a chain of fp32 FMA over 32-k tiles
 // with two sums an output 5.7e-7 to 9.9e-7.
 //
-// An operand that is not finite (or rounds to infinity) has no such terms; a block that meets one forms its tile from
-// the operands in global memory instead, with fp32 FMA in the order of k.
+// A word that is not finite has no such terms, a word near the least normal number loses its second one, and products beyond
+// the range of fp32 cancel as inf - inf; outputs whose rows hold such words (terms_suffice) are formed from the operands in
+// global memory instead, with fp32 FMA in the order of k.
 //
 // A block owns 128 tokens x 128 weight rows.  Warp 0 brings 32 k of both operands at a time by TMA (128-byte swizzle, four stages).
 // Warps 2..5 split the tokens' words and leave both terms in tensor memory, from where the MMAs read their A operand; warps
@@ -20,7 +22,7 @@
 // in shared memory too it was 224 KB, and 70 us where this takes 57.)
 // Where tiles are fewer than SMs a cluster of `splits` blocks shares a tile's K: every block leaves its sums in its own shared
 // memory, and each adds a share of the rows over the ranks, in rank order.  Every wait is bounded.
-// Measured (509 tokens): 12,288 x 2,048 169 us (151 TFLOP/s), 4,096 x 2,048 57 us, 2,048 x 6,144 89 us (two splits); tiles of packed
+// Measured (509 tokens): 12,288 x 2,048 170 us (150 TFLOP/s), 4,096 x 2,048 56 us, 2,048 x 6,144 88 us (two splits); tiles of packed
 // FMA (fma.rn.f32x2, 8 x 8 sums a thread) 617, 206 and 320 us.
 #include "gemm_f32.h"
 #include "tc_common.cuh"
@@ -41,12 +43,30 @@ static_assert(kFtM * kFtPitch * 4 <= kFtStages * kFtStage, "the sums fit where t
 // The nearest number of 11 significant bits (of two as near the larger), in integer steps: the conversion instruction runs at a
 // fraction of their rate.  For finite words; the caller looks for the others in the words' magnitudes.
 __device__ __forceinline__ uint32_t to_tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
-constexpr uint32_t kFtStrange = 0x7f7ff000u;              // from this magnitude on a word rounds to infinity, or is not finite
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo, uint32_t& most) {
+
+// The two terms hold a word to 2^-23 of it while the second stays above the least normal number, and products and sums must stay
+// below the largest: what an output can meet is told by the largest magnitudes of its token's and its weight row's words
+// (over the block's K).  lo, hi: the least but zero, and the largest, of several weight rows.  False too for an infinity or a NaN.
+constexpr float kFtLeast = 0x1p-100f, kFtMostProduct = 0x1p110f, kFtMostWord = 0x1p126f;
+__device__ __forceinline__ bool terms_suffice(float x, float lo, float hi) {
+  if (x == 0.f || hi == 0.f) return x < kFtMostWord && hi < kFtMostWord;
+  return x >= kFtLeast && x < kFtMostWord && lo >= kFtLeast && hi < kFtMostWord && x * hi < kFtMostProduct && x * lo >= kFtLeast;
+}
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
   hi = to_tf32(x);
   lo = to_tf32(x - __uint_as_float(hi));
-  most = max(most, __float_as_uint(x) & 0x7fffffffu);
 }
+// The largest magnitude of words in two running maxima of three operands an instruction: as signed integers the largest
+// positive word wins, as unsigned ones the largest negative, if there is one.
+struct Largest {
+  int s = 0;
+  uint32_t u = 0;
+  __device__ __forceinline__ void add(const float4& x) {
+    s = __vimax3_s32(__vimax3_s32(s, __float_as_int(x.x), __float_as_int(x.y)), __float_as_int(x.z), __float_as_int(x.w));
+    u = __vimax3_u32(__vimax3_u32(u, __float_as_uint(x.x), __float_as_uint(x.y)), __float_as_uint(x.z), __float_as_uint(x.w));
+  }
+  __device__ __forceinline__ uint32_t magnitude() const { return max((uint32_t)s, u & 0x7fffffffu); }
+};
 // D[tmem] (+)= A[tmem] * B[smem]^T: row m of A in lane m, an element a column.
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -82,7 +102,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t raw_full0 = smem_u32(bars), split_full0 = raw_full0 + 8 * kFtStages, empty0 = split_full0 + 8 * kFtStages;
   const uint32_t sum_full0 = empty0 + 8 * kFtStages, sum_empty0 = sum_full0 + 16, terms_empty0 = sum_empty0 + 16;
   __shared__ uint32_t tmem_holder;
-  __shared__ int gave_up, odd;
+  __shared__ int gave_up;
+  __shared__ uint32_t x_most[kFtM], w_most[kFtN], w_low, w_high;      // magnitudes: of every row, and over the weight rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = splits > 1 ? (int)cluster_ctarank() : 0;
   const int m0 = blockIdx.y * kFtM, n0 = (blockIdx.x / splits) * kFtN;
@@ -90,7 +111,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int first = (int)((long long)steps * rank / splits), last = (int)((long long)steps * (rank + 1) / splits);
   if (threadIdx.x == 0) {
     gave_up = 0;
-    odd = 0;
+    w_low = 0x7f7fffffu;
+    w_high = 0;
     for (int s = 0; s < kFtStages; ++s) {
       mbar_init(raw_full0 + 8 * s, 1);
       mbar_init(split_full0 + 8 * s, kFtSplitWarps);
@@ -168,6 +190,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int quarter = warp & 3, row = quarter * 32 + lane;
     int stage = 0;
     uint32_t phase = 0;
+    Largest most;
     for (int step = first; step < last; ++step) {
       const int i = step - first;
       bool ok = mbar_wait(terms_empty0 + 8 * (i & 1), ((i >> 1) & 1) ^ 1, giveup) && mbar_wait(raw_full0 + 8 * stage, phase, giveup);
@@ -176,22 +199,22 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       tc_fence_after();
       const float4* words = reinterpret_cast<const float4*>(tiles + stage * kFtStage + row * 128);
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kFtTerms + (i & 1) * kFtTermCols;
-      uint32_t most = 0;
 #pragma unroll
       for (int c0 = 0; c0 < 8; c0 += 4) {
         uint32_t h[16], l[16];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const float4 x = words[(c0 + c) ^ (row & 7)];            // the 128-byte swizzle: 16-byte pieces by row
-          split_tf32(x.x, h[4 * c], l[4 * c], most);
-          split_tf32(x.y, h[4 * c + 1], l[4 * c + 1], most);
-          split_tf32(x.z, h[4 * c + 2], l[4 * c + 2], most);
-          split_tf32(x.w, h[4 * c + 3], l[4 * c + 3], most);
+          most.add(x);
+          split_tf32(x.x, h[4 * c], l[4 * c]);
+          split_tf32(x.y, h[4 * c + 1], l[4 * c + 1]);
+          split_tf32(x.z, h[4 * c + 2], l[4 * c + 2]);
+          split_tf32(x.w, h[4 * c + 3], l[4 * c + 3]);
         }
         tmem_store16(taddr + 4 * c0, h);
         tmem_store16(taddr + kFtK + 4 * c0, l);
       }
-      if (most >= kFtStrange) odd = 1;
+      if (step + 1 == last) x_most[row] = most.magnitude();
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
@@ -201,8 +224,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   } else if (warp < 2 + kFtSplitWarps) {
     // ---------------- split of the weights: words to hi terms in place, lo terms in the next tile ----------------
     const int at = (warp - 6) * 32 + lane;
+    constexpr int kPieces = kFtTile / 16 / 128;            // a thread's, each of another row
     int stage = 0;
     uint32_t phase = 0;
+    Largest most[kPieces];
     for (int step = first; step < last; ++step) {
       bool ok = mbar_wait(raw_full0 + 8 * stage, phase, giveup);
       ok = __all_sync(0xffffffffu, ok);
@@ -210,20 +235,32 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       float4* words = reinterpret_cast<float4*>(tiles + stage * kFtStage + kFtTile);
       uint4* hi = reinterpret_cast<uint4*>(words);
       uint4* lo = hi + kFtTile / 16;
-      uint32_t most = 0;
 #pragma unroll
-      for (int j = 0; j < kFtTile / 16 / 128; ++j) {
+      for (int j = 0; j < kPieces; ++j) {
         const int i = at + j * 128;
         const float4 x = words[i];
         uint4 h, l;
-        split_tf32(x.x, h.x, l.x, most);
-        split_tf32(x.y, h.y, l.y, most);
-        split_tf32(x.z, h.z, l.z, most);
-        split_tf32(x.w, h.w, l.w, most);
+        most[j].add(x);
+        split_tf32(x.x, h.x, l.x);
+        split_tf32(x.y, h.y, l.y);
+        split_tf32(x.z, h.z, l.z);
+        split_tf32(x.w, h.w, l.w);
         hi[i] = h;
         lo[i] = l;
       }
-      if (most >= kFtStrange) odd = 1;
+      if (step + 1 == last) {
+#pragma unroll
+    for (int j = 0; j < kPieces; ++j) {                    // a row's eight pieces are neighbouring lanes'
+      uint32_t m = most[j].magnitude();
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if ((lane & 7) == 0) {
+        w_most[(at + j * 128) / 8] = m;
+        atomicMax(&w_high, m);
+        if (m != 0) atomicMin(&w_low, m);
+      }
+    }
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(split_full0 + 8 * stage);
@@ -263,17 +300,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // (every MMA is done, so the stages are free)
     const int row = quarter * 32 + lane;
     float* dst = reinterpret_cast<float*>(tiles) + row * kFtPitch + half * (kFtN / 2);
-    if (*(volatile int*)&odd) {
+#pragma unroll
+    for (int c = 0; c < kFtN / 2; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+    const float x = __uint_as_float(x_most[row]);
+    if (!terms_suffice(x, __uint_as_float(w_low), __uint_as_float(w_high))) {
       const float* a = A + (size_t)min(m0 + row, M - 1) * lda;
       for (int c = 0; c < kFtN / 2; ++c) {
+        const float most = __uint_as_float(w_most[half * (kFtN / 2) + c]);
+        if (terms_suffice(x, most, most)) continue;
         const float* w = W + (size_t)min(n0 + half * (kFtN / 2) + c, N - 1) * ldw;
         float sum = 0.f;
         for (int k = first * kFtK; k < min(last * kFtK, K); ++k) sum = fmaf(a[k], w[k], sum);
         dst[c] = sum;
       }
-    } else {
-#pragma unroll
-      for (int c = 0; c < kFtN / 2; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
     }
   }
   __syncwarp();

@@ -32,6 +32,49 @@ def test_product_in_32_bits(ops32, m, n, k):  # noqa: F811
     assert ((got.double() - want - bias.double() - res.double()).abs() <= bound).all()
 
 
+# 1, 2, 4 and 8 blocks over K, the last three with an odd number of steps of 32; a whole stage ring and a ragged last step
+@pytest.mark.parametrize("k", [256, 544, 1056, 2080, 2052, 6116])
+def test_product_on_tensor_cores_keeps_the_small_terms(ops32, k):  # noqa: F811
+    x, w = _randn((40, k), 11), _randn((256, k), 12)
+    out = torch.empty((40, 256), device=DEV)
+    ops32._gemm_simt(x, w, out, 0, None)
+    want = x.double() @ w.double().t()
+    # 2.0e-7 to 2.7e-7 measured at any K; one term of 11 bits alone, or a lost product of the small terms in one of the
+    # blocks, is 1e-4 and more
+    assert (out.double() - want).norm() <= 5e-7 * want.norm()
+    half = out[:, ::2].double() - want[:, ::2]
+    assert half.norm() <= 5e-7 * want[:, ::2].norm() and (out.double() - want).abs().max() <= 3e-6 * want.norm() / want.numel() ** 0.5
+
+
+def test_rows_of_any_magnitude_keep_their_bits(ops32):  # noqa: F811
+    """Token rows and weight rows of every magnitude in one tile: where the second terms would be lost or products leave the range
+    the result is a chain of FMA's."""
+    k = 288
+    ex = torch.tensor([0, -60, -99, -101, -110, -120, -126, 60, 100, 125, 0, 0], device=DEV)
+    ew = torch.tensor([0, -60, -99, -101, -115, -126, 50, 90, 124], device=DEV)
+    x = (_randn((48, k), 13).clamp(-2, 2).double() * 2.0 ** ex.repeat(4).double()[:, None]).float()
+    w = (_randn((180, k), 14).clamp(-2, 2).double() * 2.0 ** ew.repeat(20).double()[:, None]).float()
+    x[10::12] = 0
+    w[5] = 0
+    out = torch.empty((48, 180), device=DEV)
+    ops32._gemm_simt(x, w, out, 0, None)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    inside = size < 2.0 ** 126
+    assert inside.sum() > 4000 and (~inside).sum() > 500
+    # a sum of k products within k 2^-24 of their magnitudes; what falls below the least number is lost, 2^-149 a product
+    bound = (k + 4) * 2.0 ** -24 * size + 2 * k * 2.0 ** -149
+    assert ((out.double() - want).abs() <= bound)[inside].all()
+    small = inside & (size < 2.0 ** -90) & (size > 2.0 ** -110)
+    assert small.sum() > 100 and (out.double() - want)[small].norm() <= 1e-6 * want[small].norm()
+    x, w = torch.full((40, k), 1e30, device=DEV), torch.full((130, k), 1e30, device=DEV)
+    x[3], w[7] = 1.0 + 2.0 ** -11, -1e30
+    out = torch.empty((40, 130), device=DEV)
+    ops32._gemm_simt(x, w, out, 0, None)
+    inf = float("inf")
+    assert (out[:3, :7] == inf).all() and (out[:3, 7] == -inf).all()
+    assert ((out[3].double() - x[3].double() @ w.double().t()).abs() <= (k + 4) * 2.0 ** -24 * k * 1.001e30).all()
+
+
 def test_values_at_the_edge_of_the_range_pass_through_the_product(ops32):  # noqa: F811
     """The largest number, one that rounds past it at 11 bits, and NaNs of any payload, alone in their row and column."""
     m, n, k = 40, 300, 256
