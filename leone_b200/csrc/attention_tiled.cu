@@ -694,14 +694,12 @@ __device__ __forceinline__ void norm_rope_row(const __nv_bfloat16* src, __nv_bfl
 // block's range rounded up to a multiple of 4.
 template <int D, int NT> struct DecodeInbox { static constexpr int kFloats = 8 * NT * D + 4 * 8; };
 
-constexpr int kLongestFirstMost = 1024;      // sequences that are put in order
-
 template <int D, int NT, bool kFuse>
 __global__ void __launch_bounds__(kThreads)
 attention_decode_cluster_kernel(const __nv_bfloat16* __restrict__ qkv, int row_stride,
                                 __nv_bfloat16* __restrict__ out, int out_stride, PagedArgs pa,
                                 const int* __restrict__ q_start, const int* __restrict__ ctx_len,
-                                int n_q, float scale, int window, int splits, int longest_first,
+                                int n_q, float scale, int window, int splits, const int* __restrict__ order,
                                 DecodeFuse fz, int* status) {
   constexpr int kRow = D + 8;
   constexpr int kChunks = D / 8;
@@ -727,26 +725,11 @@ attention_decode_cluster_kernel(const __nv_bfloat16* __restrict__ qkv, int row_s
   const int head0 = kvh * g + hg * 16, heads = min(16, g - hg * 16);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int seq = blockIdx.z;
-  if (longest_first) {
-    // Blocks of several rounds start in order, so the z-th of them takes the z-th longest sequence: contexts of 64 to 2,048
-    // tokens in the order of the batch left the last round's SMs to a few long ones (64 such sequences, 8 kv heads of 128: a
-    // step of the 1.7B shape 4.17 ms, now 3.68).
-    __shared__ int seq_s;
-    int* lens = reinterpret_cast<int*>(smem_raw);
-    const int n = gridDim.z;
-    for (int i = tid; i < n; i += kThreads) lens[i] = ctx_len[i];
-    __syncthreads();
-    for (int i = tid; i < n; i += kThreads) {
-      const int mine = lens[i];
-      int before = 0;
-#pragma unroll 8
-      for (int j = 0; j < n; ++j) before += (lens[j] > mine || (lens[j] == mine && j < i)) ? 1 : 0;
-      if (before == seq) seq_s = i;
-    }
-    __syncthreads();
-    seq = seq_s;
-  }
+  // Blocks of several rounds start in order, so the z-th of them takes the z-th longest sequence: contexts of 64 to 2,048
+  // tokens in the order of the batch leave the last round's SMs to a few long ones (64 / 128 / 1,024 such sequences, 8 kv heads
+  // of 128: 54, 64 and 404 us, now 44, 49 and 395; equal lengths within 2 %).  The host ranks them once a step: ranked by every
+  // block, n^2 comparisons each, 256 took 146 and 1,024 2,400 us.
+  const int seq = order != nullptr ? order[blockIdx.z] : blockIdx.z;
   const int row_token = q_start[seq];
   const int ctx = ctx_len[seq];
   const int pos = ctx - 1;                              // the query's (and the new key's) position
@@ -987,8 +970,8 @@ template <int D, int NT> constexpr int decode_cluster_smem() {
 template <int D, int NT, bool kFuse>
 int launch_decode_cluster_nt(const __nv_bfloat16* qkv, int row_stride, __nv_bfloat16* out, int out_stride,
                           const PagedArgs& pa, const int* q_start, const int* ctx_len, int n_seqs, int n_q,
-                          float scale, int window, int splits, const DecodeFuse& fz, int* status,
-                          cudaStream_t stream) {
+                          float scale, int window, int splits, const int* order, const DecodeFuse& fz,
+                          int* status, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attention_decode_cluster_kernel<D, NT, kFuse>,
@@ -998,28 +981,28 @@ int launch_decode_cluster_nt(const __nv_bfloat16* qkv, int row_stride, __nv_bflo
   }
   const int g = n_q / pa.n_kv;
   dim3 grid(pa.n_kv * ((g + 15) / 16), splits, n_seqs);
-  // more blocks than the two places an SM has: the order in which sequences start matters
-  const int longest_first = splits == 1 && (long long)grid.x * n_seqs > 2 * 148 && n_seqs <= kLongestFirstMost;
+  // with no more blocks than the two places an SM has, all start at once and the order is one more load
+  if (splits > 1 || (long long)grid.x * n_seqs <= 2 * 148) order = nullptr;
   if (splits == 1)
     return launch_kernel(attention_decode_cluster_kernel<D, NT, kFuse>, grid, dim3(kThreads), decode_cluster_smem<D, NT>(),
                          stream, qkv, row_stride, out, out_stride, pa, q_start, ctx_len, n_q, scale, window,
-                         splits, longest_first, fz, status);
+                         splits, order, fz, status);
   return launch_kernel_cluster(attention_decode_cluster_kernel<D, NT, kFuse>, grid, dim3(kThreads),
                                decode_cluster_smem<D, NT>(), stream, dim3(1, splits, 1), qkv, row_stride, out,
-                               out_stride, pa, q_start, ctx_len, n_q, scale, window, splits, 0, fz, status);
+                               out_stride, pa, q_start, ctx_len, n_q, scale, window, splits, order, fz, status);
 }
 
 // Up to 8 query heads per block take one tile of 8 heads (NT = 1), up to 16 take two.
 template <int D, bool kFuse>
 int launch_decode_cluster(const __nv_bfloat16* qkv, int row_stride, __nv_bfloat16* out, int out_stride,
                           const PagedArgs& pa, const int* q_start, const int* ctx_len, int n_seqs, int n_q,
-                          float scale, int window, int splits, const DecodeFuse& fz, int* status,
-                          cudaStream_t stream) {
+                          float scale, int window, int splits, const int* order, const DecodeFuse& fz,
+                          int* status, cudaStream_t stream) {
   if (n_q / pa.n_kv <= 8)
     return launch_decode_cluster_nt<D, 1, kFuse>(qkv, row_stride, out, out_stride, pa, q_start, ctx_len, n_seqs,
-                                                 n_q, scale, window, splits, fz, status, stream);
+                                                 n_q, scale, window, splits, order, fz, status, stream);
   return launch_decode_cluster_nt<D, 2, kFuse>(qkv, row_stride, out, out_stride, pa, q_start, ctx_len, n_seqs,
-                                               n_q, scale, window, splits, fz, status, stream);
+                                               n_q, scale, window, splits, order, fz, status, stream);
 }
 
 template <int D, int NT>
@@ -1141,14 +1124,17 @@ extern "C" int leone_attention_decode(const void* qkv, int row_stride, void* out
 // `adjacent`) to the queries and to the new key at position
 // ctx_len-1, uses the new key and value in place of what the cache holds there and, if
 // `write_cache`, stores them into the pools.  fuse needs d of 64 or 128.
-extern "C" int leone_attention_decode_cluster(const void* qkv, int row_stride, void* out, int out_stride,
-                                              void* k_pool, void* v_pool, const int* block_table,
-                                              int table_width, const int* q_start, const int* ctx_len,
-                                              int n_seqs, int n_q, int n_kv, int d, float scale, int window,
-                                              int page_tokens, int num_pages, int splits, int fuse,
-                                              const float* q_norm_w, const float* k_norm_w, float eps,
-                                              const float* rope, int max_positions, int write_cache,
-                                              int adjacent, int* status, cudaStream_t stream) {
+// order: a permutation of the sequences, the longest first (int32 [n_seqs], as old as the lengths), or null: the order in
+// which their blocks start.
+extern "C" int leone_attention_decode_cluster_ordered(const void* qkv, int row_stride, void* out, int out_stride,
+                                                      void* k_pool, void* v_pool, const int* block_table,
+                                                      int table_width, const int* q_start, const int* ctx_len,
+                                                      int n_seqs, int n_q, int n_kv, int d, float scale, int window,
+                                                      int page_tokens, int num_pages, int splits, int fuse,
+                                                      const float* q_norm_w, const float* k_norm_w, float eps,
+                                                      const float* rope, int max_positions, int write_cache,
+                                                      int adjacent, const int* order, int* status,
+                                                      cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   int r = check_common(d, n_q, n_kv, row_stride, out_stride, qkv, k_pool, v_pool, page_tokens, table_width);
   if (r != 0) return r;
@@ -1162,13 +1148,27 @@ extern "C" int leone_attention_decode_cluster(const void* qkv, int row_stride, v
     if (d == 64)
       return launch_decode_cluster<64, true>((const __nv_bfloat16*)qkv, row_stride, (__nv_bfloat16*)out,
                                              out_stride, pa, q_start, ctx_len, n_seqs, n_q, scale, window,
-                                             splits, fz, status, stream);
+                                             splits, order, fz, status, stream);
     return launch_decode_cluster<128, true>((const __nv_bfloat16*)qkv, row_stride, (__nv_bfloat16*)out,
                                             out_stride, pa, q_start, ctx_len, n_seqs, n_q, scale, window,
-                                            splits, fz, status, stream);
+                                            splits, order, fz, status, stream);
   }
   LEONE_DISPATCH_D(d, return (launch_decode_cluster<DD, false>((const __nv_bfloat16*)qkv, row_stride,
                                                                (__nv_bfloat16*)out, out_stride, pa, q_start,
                                                                ctx_len, n_seqs, n_q, scale, window, splits,
-                                                               fz, status, stream)));
+                                                               order, fz, status, stream)));
+}
+
+extern "C" int leone_attention_decode_cluster(const void* qkv, int row_stride, void* out, int out_stride,
+                                              void* k_pool, void* v_pool, const int* block_table,
+                                              int table_width, const int* q_start, const int* ctx_len,
+                                              int n_seqs, int n_q, int n_kv, int d, float scale, int window,
+                                              int page_tokens, int num_pages, int splits, int fuse,
+                                              const float* q_norm_w, const float* k_norm_w, float eps,
+                                              const float* rope, int max_positions, int write_cache,
+                                              int adjacent, int* status, cudaStream_t stream) {
+  return leone_attention_decode_cluster_ordered(qkv, row_stride, out, out_stride, k_pool, v_pool, block_table, table_width,
+                                                q_start, ctx_len, n_seqs, n_q, n_kv, d, scale, window, page_tokens,
+                                                num_pages, splits, fuse, q_norm_w, k_norm_w, eps, rope, max_positions,
+                                                write_cache, adjacent, nullptr, status, stream);
 }

@@ -41,6 +41,7 @@ class StepContext:
         self.token_ids = self.positions = self.seq_of_token = None
         self.q_start = self.ctx_len = self.slot_ids = self.logit_rows = None
         self.block_tables: List[torch.Tensor] = []
+        self.seq_order = None          # the leading sequences of one token each, the longest first (see longest_first)
         self.q_lens: np.ndarray = None
         self.starts: np.ndarray = None
         self.ctx_lens: np.ndarray = None
@@ -58,6 +59,15 @@ class StepContext:
     def cache_view(self, run_position: int):
         """The cache of the layer at this position of the run order (None if it has none)."""
         return self.layer_caches.get(run_position)
+
+
+def longest_first(ctx_lens: np.ndarray) -> np.ndarray:
+    """The order in which the blocks of a decode attention start: the longest sequence first, equal ones as they stand."""
+    return np.argsort(-ctx_lens, kind="stable").astype(np.int32)
+
+
+# fewer sequences' blocks all start at once (two an SM, up to 37 heads of keys and values): the order does not matter
+ORDER_FROM = 9
 
 
 def pack_metadata(token_lists: Sequence[Sequence[int]], starts: Sequence[int], slots: Sequence[int],

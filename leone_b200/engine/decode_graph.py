@@ -27,7 +27,7 @@ from typing import Hashable, List, Sequence
 import numpy as np
 import torch
 
-from .batch import StepContext, pack_metadata
+from .batch import ORDER_FROM, StepContext, longest_first, pack_metadata
 
 
 class DecodeGraph:
@@ -38,9 +38,13 @@ class DecodeGraph:
         dev = engine.device
         self.widths = [-(-engine.spec.max_positions // engine.page_tokens) for _ in engine.cache.groups]
         tables = [np.full((batch, w), -1, dtype=np.int32) for w in self.widths]
-        packed, self.offsets, self.bt_offsets, _ = pack_metadata(
+        packed, offsets, bt_offsets, _ = pack_metadata(
             [[0]] * batch, [0] * batch, [0] * batch, [[0]] * batch, tables)
-        self.size = packed.size
+        # in front of them, the order in which the sequences' attention starts.  Every sequence grows by a token a step, so an
+        # order holds until the next fill
+        self.offsets = {"seq_order": (0, batch), **{name: (batch + o, s) for name, (o, s) in offsets.items()}}
+        self.bt_offsets = [(batch + o, shape) for o, shape in bt_offsets]
+        self.size = batch + packed.size
         self.meta = torch.zeros(self.size, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(self.size, dtype=torch.int32, pin_memory=True)
         self.sampled = torch.zeros(batch, dtype=torch.int32, device=dev)
@@ -139,11 +143,14 @@ class DecodeGraph:
         key = (tuple(rids), tuple(int(v) for v in versions))
         same = key == self._filled_rids
         if not same:
+            put("seq_order", np.arange(b, dtype=np.int32))
             put("seq_of_token", np.arange(b, dtype=np.int32))
             put("q_start", np.arange(b + 1, dtype=np.int32))
             put("slot_ids", np.asarray(slots if slots is not None else [e.cache.slot(r) for r in rids],
                                        dtype=np.int32))
             put("logit_rows", np.arange(b, dtype=np.int32))
+        if b >= ORDER_FROM:
+            put("seq_order", longest_first(lengths))
         appended = []                       # [lo, hi) ranges of the host copy that gained entries
         for gi, (g, w, (o, shape)) in enumerate(zip(e.cache.groups, self.widths, self.bt_offsets)):
             view = host[o:o + shape[0] * shape[1]].reshape(shape)

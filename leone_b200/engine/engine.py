@@ -27,7 +27,7 @@ from ..parts.spec import ModelSpec
 from ..registry import config_from_folder, spec_from_config
 from ..weights.loader import check_names_and_shapes, load_checkpoint, target_dtype
 from .budget import check_memory_budget, plan_memory
-from .batch import StepContext, StepEntry, pack_metadata
+from .batch import ORDER_FROM, StepContext, StepEntry, longest_first, pack_metadata
 from .model import Model
 
 _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16,
@@ -259,6 +259,12 @@ class Engine:
         tables = [self.cache.block_table(g.gid, rids) for g in self.cache.groups]
         packed, offsets, bt_offsets, stats = pack_metadata(
             [e.tokens for e in entries], starts, slots, [e.want for e in entries], tables)
+        # decode rows stand in front of a mixed step's portions
+        longer = np.flatnonzero(stats["q_lens"] != 1)
+        single = int(longer[0]) if longer.size else stats["b"]
+        if single >= ORDER_FROM:
+            offsets["seq_order"] = (packed.size, single)
+            packed = np.concatenate([packed, longest_first(stats["ctx_lens"][:single])])
         dev = self._stage(packed)
         ctx = StepContext()
         for name, (o, s) in offsets.items():

@@ -500,22 +500,25 @@ class FastKernels:
         bt = cache.block_table
         args = (qkv, out, n_q, n_kv, d, scale, window, cache)
         if ctx.decode_only:
-            self._attention_decode(*args, ctx.q_start, ctx.ctx_len, bt, ctx.n_seqs, ctx.max_ctx_len, ctx.status, fuse)
+            self._attention_decode(*args, ctx.q_start, ctx.ctx_len, bt, ctx.n_seqs, ctx.max_ctx_len, ctx.status, fuse,
+                                   getattr(ctx, "seq_order", None))
             return True
         if fuse is not None:
             raise RuntimeError("fused q/k preparation is a decode-step feature")
         n_dec = self.leading_decode_rows(ctx)
         if n_dec:
             self._attention_decode(*args, ctx.q_start[:n_dec + 1], ctx.ctx_len[:n_dec], bt[:n_dec], n_dec,
-                                   int(ctx.ctx_lens[:n_dec].max()), ctx.status, None)
+                                   int(ctx.ctx_lens[:n_dec].max()), ctx.status, None, getattr(ctx, "seq_order", None))
         self._attention_prompt(*args, ctx.q_start[n_dec:], ctx.ctx_len[n_dec:], bt[n_dec:], ctx.n_seqs - n_dec,
                                int(ctx.q_lens[n_dec:].max()) if n_dec else ctx.max_q_len, ctx.status)
         return True
 
     def _attention_decode(self, qkv, out, n_q, n_kv, d, scale, window, cache, q_start, ctx_len, bt, n_seqs,
-                          max_ctx, status, fuse) -> None:
-        """Sequences with one query token each (row ``q_start[s]``)."""
+                          max_ctx, status, fuse, order=None) -> None:
+        """Sequences with one query token each (row ``q_start[s]``); ``order``: these sequences, the longest first."""
         from ctypes import c_float
+        if order is not None and order.numel() != n_seqs:
+            raise ValueError(f"an order of {order.numel()} sequences for {n_seqs}")
         g = n_q // n_kv
         kp, vp = cache.k_pool, cache.v_pool
         common = (_ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt),
@@ -530,9 +533,9 @@ class FastKernels:
                 fz = (1, _ptr(fuse["q_w"]), _ptr(fuse["k_w"]), c_float(fuse["eps"]), _ptr(rope),
                       rope.shape[0] if rope is not None else 0, 1 if fuse["write_cache"] else 0,
                       1 if fuse.get("pairing", "half_split") == "adjacent" else 0)
-            code = self.lib.leone_attention_decode_cluster(
+            code = self.lib.leone_attention_decode_cluster_ordered(
                 *common, n_q, n_kv, d, c_float(scale), int(window or 0), cache.page_tokens,
-                kp.shape[0], splits, *fz, _ptr(status), self._stream())
+                kp.shape[0], splits, *fz, _ptr(order), _ptr(status), self._stream())
         else:
             if fuse is not None:
                 raise RuntimeError("fused decode attention asked for where decode_fusable() is false")
