@@ -62,7 +62,7 @@ class DecodeGraph:
         self._tables_at = min((o for o, _ in self.bt_offsets), default=None)   # where the block tables start
         # A row as wide as a design without a position limit needs (65,536 entries and more) costs more to clear and to
         # copy whole than a copy call of its own for the entries in use: 2 to 4 MB a refill, 44 us on the GPU and more on the
-        # host.  Nothing reads a table past its sequence's length.
+        # host.  What a row no longer uses is set to -1 with it, so a read past a sequence's length is reported as in other rows.
         self._wide = self._tables_at is not None and max(self.widths) > 16384
         if self._wide:
             self.meta[self._tables_at:].fill_(-1)
@@ -159,12 +159,18 @@ class DecodeGraph:
                 if n > w:
                     raise ValueError(f"block table needs {n} columns, only {w} given")
                 # (a window's table that lost entries at its front has a new version, so it is not the same)
-                done = self._filled_pages[gi][i] if same else 0
+                before = self._filled_pages[gi][i]
+                done = before if same else 0
+                end = n                     # a wide row is cleared as far as it was in use
                 if done == 0 and not self._wide:
                     view[i, :] = -1
+                elif not same and before > n:
+                    view[i, n:before] = -1
+                    end = before
                 if n > done:
                     view[i, done:n] = g.tables.tail(r, done)
-                    appended.append((o + i * shape[1] + done, o + i * shape[1] + n))
+                if end > done:
+                    appended.append((o + i * shape[1] + done, o + i * shape[1] + end))
                 self._filled_pages[gi][i] = n
         self._filled_rids = key
         # the requests' slot records: sampling parameters, and where each stands (the position

@@ -23,6 +23,15 @@ def test_captured_steps_equal_eager_ones_as_the_batch_changes(which):
         got = engines[0].decode_logits(rids, fed) if captured else engines[0].step([(r, [t], [0]) for r, t in zip(rids, fed)])
         for r in rids:
             at[r] += 1
+        if captured:
+            # a row holds its request's pages and -1 behind them, whoever was in it before
+            graph = engines[0]._decode_graphs[len(rids)]
+            for group, (o, shape) in zip(engines[0].cache.groups, graph.bt_offsets):
+                rows = graph.meta[o:o + shape[0] * shape[1]].view(shape)
+                for row, r in zip(rows, rids):
+                    n = group.tables.length(r)
+                    held = [(a, int(b)) for a, b in zip(row[:n].tolist(), group.tables.tail(r, 0)) if b >= 0]   # (a window lets pages go)
+                    assert held and all(a == b for a, b in held) and int(row[n:].max()) == -1
         assert torch.allclose(got, want, rtol=0, atol=2e-5 * float(want.abs().max()))
 
     def begin(rid, n):
