@@ -32,7 +32,7 @@ struct ExpertParams {
   const int* order;            // [pairs]: sorted row -> pair
   const float* weight;         // [pairs]
   void* out;                   // modes 0, 1: bf16 [pairs, cols] by sorted row; mode 2: fp32 [pairs, cols] by pair
-  int experts, top, n_tokens;
+  int experts, top;
   int cols, K;                 // output columns (weight rows of one expert), inner size
   int scale_input, mode;
   int* status;
@@ -280,19 +280,19 @@ int leone::experts_tc_product(int mode, const void* x, int ldx, const void* w, c
   using namespace leone::tc;
   const long long pairs = (long long)n_tokens * top;
   CUtensorMap mx, mw, mw2;
-  if (mode != 2) {
-    launch_kernel(experts_sort_rows_kernel, dim3((unsigned)(pairs < 148 * 8 ? pairs : 148 * 8)), dim3(256), 0, stream,
-                  (const __nv_bfloat16*)x, ldx, K, top, order, offsets + experts, (__nv_bfloat16*)sorted);
-    x = sorted;
-  }
-  int e = make_tensor_map_2d(&mx, x, pairs, K, K, kExRows);
+  int e = make_tensor_map_2d(&mx, mode == 2 ? x : sorted, pairs, K, K, kExRows);
   if (e == 0) e = make_tensor_map_2d(&mw, w, (uint64_t)experts * cols, K, K, mode == 0 ? kExCols / 2 : kExCols);
   if (e == 0 && mode == 0) e = make_tensor_map_2d(&mw2, w2, (uint64_t)experts * cols, K, K, kExCols / 2);
   if (e != 0) return e;
   if (mode != 0) mw2 = mw;
   static const cudaError_t ready = cudaFuncSetAttribute(experts_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExSmem);
   if (ready != cudaSuccess) return (int)ready;
-  const ExpertParams p = {offsets, order, weight, out, experts, top, n_tokens, cols, K, scale_input, mode, status};
+  if (mode != 2) {
+    e = launch_kernel(experts_sort_rows_kernel, dim3((unsigned)(pairs < 148 * 8 ? pairs : 148 * 8)), dim3(256), 0, stream,
+                      (const __nv_bfloat16*)x, ldx, K, top, order, offsets + experts, (__nv_bfloat16*)sorted);
+    if (e != 0) return e;
+  }
+  const ExpertParams p = {offsets, order, weight, out, experts, top, cols, K, scale_input, mode, status};
   const int per = mode == 0 ? kExCols / 2 : kExCols;
   const long long most = (pairs / kExRows + (experts < pairs ? experts : pairs)) * ((cols + per - 1) / per);
   return launch_kernel(experts_tc_kernel, dim3((unsigned)(most < 148 ? most : 148)), dim3(kExThreads), kExSmem, stream, mx, mw, mw2,
