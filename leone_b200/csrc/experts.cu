@@ -578,6 +578,17 @@ extern "C" int leone_experts_select(const float* logits, int ldl, const float* b
   return launch_result();
 }
 
+// 1 if leone_experts_forward takes these arguments on tcgen05 (experts_tc.cu; a launch more, which sorts the rows).  From a pair an
+// expert on that is the faster form (32 experts of 512, 8 tokens with 4 pairs each: 50 us against 62; 64 of
+// 1,024, 32 tokens: 276 against 346); with fewer pairs its 128 x 256 tiles are too few blocks to stream the weights.
+extern "C" int leone_experts_on_tcgen05(int dtype, const void* x, int ldx, const void* w_gate, const void* w_up, const void* w_down,
+                                        int n_tokens, int width, int ff, int experts, int top, const void* act,
+                                        const void* pair_out, int tensor_cores) {
+  const uintptr_t starts = (uintptr_t)x | (uintptr_t)w_gate | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)pair_out;
+  return tensor_cores == 1 && dtype == 1 && width % 8 == 0 && ff % 8 == 0 && ldx % 8 == 0 && experts <= kExpertsTcMost &&
+         (long long)n_tokens * top >= experts && starts % 16 == 0;
+}
+
 // w_gate null: ungated experts (see the top of the file).  identity: choices `experts .. experts + identity - 1`
 // are experts without tensors whose output is their input (weighted at the output).  fresh: hidden is
 // written, not added to.
@@ -613,10 +624,7 @@ extern "C" int leone_experts_forward(int dtype, const void* x, int ldx, const vo
                     combine_top, identity > 0 ? (const __nv_bfloat16*)x : nullptr, ldx, chosen, weight, experts);
       return launch_result();
     };
-    // From a pair an expert on, tcgen05 is the faster form (32 experts of 512, 8 tokens with 4 pairs each: 50 us against 62; 64 of
-    // 1,024, 32 tokens: 276 against 346); with fewer pairs its 128 x 256 tiles are too few blocks to stream the weights.
-    const uintptr_t starts = (uintptr_t)x | (uintptr_t)w_gate | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)pair_out;
-    if (tensor_cores != 2 && experts <= kExpertsTcMost && pairs >= experts && starts % 16 == 0) {
+    if (leone_experts_on_tcgen05(dtype, x, ldx, w_gate, w_up, w_down, n_tokens, width, ff, experts, top, act, pair_out, tensor_cores)) {
       int e = w_gate == nullptr
                   ? experts_tc_product(1, x, ldx, w_up, nullptr, offsets, order, weight, n_tokens, experts, top, ff, width,
                                        scale_input, act, pair_out, status, stream)

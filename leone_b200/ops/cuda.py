@@ -1250,11 +1250,15 @@ class CudaOps:
         order = rt.flat_buffer("experts_order", pairs, torch.int32, reserve=cap)
         act = rt.flat_buffer("experts_act", pairs * ff, x.dtype, reserve=cap * ff)
         pair_out = rt.flat_buffer("experts_pair_out", pairs * width, torch.float32, reserve=cap * width)
-        self.launches += 4
+        tensor_cores = 0 if os.environ.get("LEONE_NO_EXPERT_MMA", "0") == "1" else 1
+        # grouping, two products, the sum over a token's experts; on tcgen05 the rows are sorted first
+        self.launches += 4 + self.mixers.leone_experts_on_tcgen05(
+            _dt(x.dtype), _ptr(x), x.stride(0), _ptr(w_gate), _ptr(w_up), _ptr(w_down), n, width, ff, experts, top, _ptr(act),
+            _ptr(pair_out), tensor_cores)
         _check(self.mixers.leone_experts_forward(
             _dt(x.dtype), _ptr(x), x.stride(0), _ptr(w_gate), _ptr(w_up), _ptr(w_down), _ptr(chosen), _ptr(weight), n,
             width, ff, experts, top, 1 if scale_input else 0, _ptr(offsets), _ptr(order), _ptr(act), _ptr(pair_out),
-            _ptr(hidden), 0 if os.environ.get("LEONE_NO_EXPERT_MMA", "0") == "1" else 1, int(identity),
+            _ptr(hidden), tensor_cores, int(identity),
             1 if fresh else 0, _ptr(self.status), self._stream()), "experts_forward")
 
     def sample(self, logits, temperature, seeds, positions, out):

@@ -36,9 +36,10 @@ def test_grouped_products(ops16, form, scale_input, n, experts, top, width, ff, 
         want = want.index_add(0, row, y)
         size = size.index_add(0, row, (act.abs() @ down[e].double().abs().t()) * (1.0 if scale_input else w))
     rt = Runtime(torch.device(DEV), torch.bfloat16, ops16, n)
-    got = hidden.clone()
+    got, before = hidden.clone(), ops16.launches
     ops16.experts_forward(x, gate if form == "gated" else None, up, down, chosen.int().flatten(), weight.flatten(), top, scale_input,
                           got, rt)
+    assert ops16.launches - before == 5                 # grouping, the rows in order, two products, the sum over a token's experts
     # a projection near a rounding boundary may fall on its other side: 2^-8 of it, through silu and a product of two, twice;
     # the activation's own rounding likewise
     assert ((got.double() - want).abs() <= 3 * 2.0 ** -8 * size + 1e-6).all()
