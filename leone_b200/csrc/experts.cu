@@ -13,7 +13,9 @@
 // Nothing is read back by the host: the pairs are counted and placed per expert on the device, and
 // the grouped products take a grid that is large enough for any assignment (row tiles that turn out
 // to be empty return at once).  A row of the grouped products is computed from its own token only,
-// with k ascending, so a token's result does not depend on what else is in the step.
+// with k ascending.  How its sum over k is grouped depends on the form, which depends on the step's number of pairs, so with
+// other tokens in the step a token's result differs by fp32 rounding at most (ahead of the roundings to bfloat16); in the
+// same form it has the same bits.
 #include "common.cuh"
 #include "experts_tc.h"
 #include "mma_tile.cuh"

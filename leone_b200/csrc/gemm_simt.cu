@@ -6,7 +6,7 @@
 //
 // Three forms, chosen by leone_gemm_simt from dtype, sizes and alignment:
 //  * gemm_rows: 32 bits, up to 24 tokens.  A stream over the weights;
-//  * gemm_f32_tc.cu: 32 bits, more tokens, K of 256 and more.  Tiles on tensor cores, operands split into exact terms;
+//  * gemm_f32_tc.cu: 32 bits, more tokens, K of 256 and more.  Tiles on tensor cores, operands split into two terms;
 //  * gemm_simt_kernel: bfloat16, and any size or alignment (4-byte loads).
 // In every form a row of C is computed from its own row of A only.  How its sum over k is grouped depends on the
 // form and the split, so a token's result in another batch differs by fp32 rounding at most.
@@ -163,9 +163,9 @@ gemm_rows_kernel(const float* A, const float* __restrict__ W, float* C, const fl
 }
 
 // The 32-bit product with 16-byte loads of up to 24 tokens: the stream is read again for every 8 tokens (its blocks share the
-// weights through the L2).  Beyond, tensor cores are faster: at 24 tokens 27 / 15 / 73 / 37 us here against 29 / 26 / 58 / 51 there
-// (at 25) for 4,096, 2,048 and 12,288 rows of 2,048 and 2,048 of 6,144; they take the same at 64 tokens, where the stream is
-// read 8 times.
+// weights through the L2), tensor cores take the same time for any part of a tile of 128.  One line for all shapes, where a layer's four
+// products break even: at 24 tokens 27 / 15 / 73 / 37 us here (152) and 29 / 26 / 58 / 51 there (164; at 25) for 4,096, 2,048 and
+// 12,288 rows of 2,048 and 2,048 of 6,144; the next 8 tokens cost the stream a third more.
 constexpr int kStreamTokens = 24;
 // From here on the tensor cores' sums are nearer to 64 bits than a chain of FMA is (2.1e-7 at any K against 2.8e-7 at 256, growing
 // with its root; below, a chain is as near, and the product is small).

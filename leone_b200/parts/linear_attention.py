@@ -53,8 +53,9 @@ class DecayLinearAttention(Mixer):
         return (self.cols * self.hidden + self.hidden * self.hv) * self.rt.dtype.itemsize
 
     def scratch_bytes(self, max_tokens):
-        # a state for every chunk but a sequence's first; prompt portions in bfloat16 run in chunks of 64
-        chunks = max_tokens // max(min(self.chunk, 64), 1) + 1
+        # a state for every chunk but a sequence's first; prompt portions in bfloat16 run in chunks of 64.  (The buffer
+        # starts with room for 64.)
+        chunks = max(max_tokens // max(min(self.chunk, 64), 1) + 1, 64)
         return max_tokens * (self.cols * self.rt.dtype.itemsize + self.hv * (4 + self.rt.dtype.itemsize)) \
             + chunks * self.heads * self.dim * self.vdim * 4
 

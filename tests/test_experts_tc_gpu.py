@@ -1,4 +1,4 @@
-"""The routed experts' grouped products on tcgen05, against float64, and the same bits as a token alone would get."""
+"""The routed experts' grouped products on tcgen05, against float64; which other tokens are in the step, and the other form."""
 import pytest
 import torch
 
@@ -44,9 +44,16 @@ def test_grouped_products(ops16, form, scale_input, n, experts, top, width, ff, 
     # the activation's own rounding likewise
     assert ((got.double() - want).abs() <= 3 * 2.0 ** -8 * size + 1e-6).all()
     assert (got.double() - want).norm() <= 1e-3 * (want - hidden.double()).norm()
-    # which other tokens are in the step does not change a token's bits, only the form of the products may
+    # which other tokens are in the step does not change a token's bits while the form is the same
     part = hidden.clone()[: n // 2 + 1]
     m = part.shape[0]
     ops16.experts_forward(x[:m], gate if form == "gated" else None, up, down, chosen[:m].int().flatten().contiguous(),
                           weight[:m].flatten().contiguous(), top, scale_input, part, rt)
-    assert (part - got[:m]).norm() <= 2e-3 * (got[:m] - hidden[:m]).norm()
+    assert m * top >= experts and torch.equal(part, got[:m])
+    # fewer pairs than experts: the mma.sync form, whose sums over k are grouped differently; a projection near a rounding
+    # boundary may fall on its other side
+    if top < experts:
+        alone = hidden[:1].clone()
+        ops16.experts_forward(x[:1], gate if form == "gated" else None, up, down, chosen[:1].int().flatten().contiguous(),
+                              weight[:1].flatten().contiguous(), top, scale_input, alone, rt)
+        assert (alone - got[:1]).norm() <= 2e-3 * (got[:1] - hidden[:1]).norm()
