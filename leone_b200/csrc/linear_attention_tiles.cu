@@ -12,12 +12,12 @@
 // of a later token does not reach an earlier one.  The powers of d are products in fp64, rounded once.
 //
 // Why fp32: tensor cores take q, k, v and the state as sums of short terms.  Two bfloat16 terms (2^-17 of an operand) were further
-// from 64 bits than the walk (outputs 1.5e-6 to 5e-6 in the 2-norm; the walk 0.8e-7 to 4.9e-7, this 1.2e-7 to 2.5e-7), and an
-// infinity has no such terms.
+// from 64 bits than the walk (outputs 1.5e-6 to 5e-6 in the 2-norm; the walk 0.8e-7 at 60 tokens to 4.9e-7 at 2,048, this 0.8e-7
+// to 1.9e-7; states 1.5e-6 to 5e-6, 1.3e-7 to 5.0e-7, 0.8e-7 to 1.6e-7), and an infinity has no such terms.
 // Bound by the FMA pipes and by latency: (3) is 1.6 M multiply-adds a chunk and head of 128 x 128 where the walk takes 2.1 M, one
-// after another; (1) 1.0 M.  A block is 256 threads with 4 x 8 outputs (3) or 8 x 8 (1) each, two blocks an SM; the state
-// comes through shared memory in slabs of 8 channels, two slabs ahead.
-// Measured (16 heads of 128 x 128): 2,048 tokens 131 us ((1) 40, (2) 11, (3) 73, (4) 16; the walk, in chunks of 64, 349), 500 tokens 53
+// after another; (1) 1.0 M.  A block is 256 threads with 8 x 8 outputs each, in (3) of half of the sums, two blocks an SM; the
+// state comes through shared memory in slabs of 8 channels, two slabs ahead.
+// Measured (16 heads of 128 x 128): 2,048 tokens 131 us ((1) 39, (2) 11, (3) 72, (4) 15; the walk, in chunks of 64, 349), 500 tokens 53
 // (140), 77 tokens 47 (89), 16 sequences of 200 tokens 215 (545).
 #include "common.cuh"
 
@@ -232,8 +232,10 @@ linear_attention_states_kernel(const LinTileParams p) {
   }
 }
 
-// (3): a thread owns tokens ty, 16 + ty, 32 + ty, 48 + ty times 4 * VH columns, so every warp has the same share of the
-// tokens' triangle.
+// (3): two groups of 128 threads; a thread owns tokens ty, 8 + ty, .. 56 + ty times 4 * VH columns, of every other four channels and
+// tokens that are summed, so every warp has the same share of the tokens' triangle and no sum is a chain of more than
+// 96 (the walk's are of 16 channels); the groups' halves meet in shared memory.  (Chains of 192 were 1.2e-7 to 2.5e-7 from 64 bits,
+// in the same time.)
 template <int VH> struct LinOutLayout {
   static constexpr int V = 64 * VH;
   static constexpr int kFloats = 2 * kLtTokens * kLtPitch + kLtTokens * V + kLtSlabs * kLtSlab * V + kLtTokens + 4;
@@ -252,7 +254,7 @@ linear_attention_outputs_kernel(const LinTileParams p) {
   float* v_s = k_s + kLtTokens * kLtPitch;         // [kLtTokens][V]
   float* s_s = v_s + kLtTokens * V;                // [kLtSlabs][kLtSlab][V]
   float* pow_s = s_s + kLtSlabs * kLtSlab * V;     // d^0 .. d^64
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid & 15, group = tid >> 7, ty = tid >> 4 & 7;
   const int h = blockIdx.y, v0 = blockIdx.z * V, dim = p.dim, vdim = p.vdim;
   LinChunk c;
   if (!find_chunk(p, blockIdx.x, c)) return;
@@ -299,41 +301,50 @@ linear_attention_outputs_kernel(const LinTileParams p) {
   }
   __syncthreads();
   {
-    // scores of tokens ty + 16 i with tokens tx + 16 j, j <= i
-    float2 sc[4][4];
+    // scores of tokens row + 16 i with tokens tx + 16 j, j <= i, each in eight sums
+    const int row = tid >> 4;
+    float2 sc[4][4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j <= i; ++j) sc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 2
-    for (int d = 0; d < dim; d += 4) {
-      float4 a[4], b[4];
+      for (int j = 0; j <= i; ++j)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        a[i] = *reinterpret_cast<const float4*>(q_s + (ty + 16 * i) * kLtPitch + d);
-        b[i] = *reinterpret_cast<const float4*>(k_s + (tx + 16 * i) * kLtPitch + d);
-      }
+        for (int e = 0; e < 4; ++e) sc[i][j][e] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int d = 0; d < dim; d += 8) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int e = 0; e < 4; e += 2) {
+        float4 a[4], b[4];
 #pragma unroll
-        for (int j = 0; j <= i; ++j) {
-          fma2(sc[i][j], lower(a[i]), lower(b[j]));
-          fma2(sc[i][j], upper(a[i]), upper(b[j]));
+        for (int i = 0; i < 4; ++i) {
+          a[i] = *reinterpret_cast<const float4*>(q_s + (row + 16 * i) * kLtPitch + d + 2 * e);
+          b[i] = *reinterpret_cast<const float4*>(k_s + (tx + 16 * i) * kLtPitch + d + 2 * e);
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j <= i; ++j) {
+            fma2(sc[i][j][e], lower(a[i]), lower(b[j]));
+            fma2(sc[i][j][e + 1], upper(a[i]), upper(b[j]));
+          }
+      }
     }
     __syncthreads();                               // the keys are read
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j <= i; ++j) {
-        const int t = ty + 16 * i, s = tx + 16 * j;
-        k_s[t * kLtPitchA + s] = (sc[i][j].x + sc[i][j].y) * pow_s[max(t - s, 0)];
+        const int t = row + 16 * i, s = tx + 16 * j;
+        float sum[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] = sc[i][j][e].x + sc[i][j][e].y;
+        k_s[t * kLtPitchA + s] = ((sum[0] + sum[1]) + (sum[2] + sum[3])) * pow_s[max(t - s, 0)];
       }
   }
-  // the read-out of the state before these tokens
-  float2 acc[4][2 * VH];
+  // the read-out of the state before these tokens: four channels of a slab a group
+  float2 acc[8][2 * VH];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 2 * VH; ++j) acc[i][j] = make_float2(0.f, 0.f);
   const int slabs = dim / kLtSlab;
@@ -341,73 +352,87 @@ linear_attention_outputs_kernel(const LinTileParams p) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kLtSlabs - 2) : "memory");
     __syncthreads();                               // this slab has landed, the last one's readers are done (and the scores are there)
     request(slab + kLtSlabs - 1);
-    const float* rows = s_s + (slab % kLtSlabs) * kLtSlab * V;
+    const float* rows = s_s + ((slab % kLtSlabs) * kLtSlab + 4 * group) * V;
 #pragma unroll
-    for (int d = 0; d < kLtSlab; d += 4) {
-      float q[4][4];
+    for (int d = 0; d < 4; d += 2) {
+      float2 q[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(q[i]) = *reinterpret_cast<const float4*>(q_s + (ty + 16 * i) * kLtPitch + slab * kLtSlab + d);
+      for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const float2*>(q_s + (ty + 8 * i) * kLtPitch + slab * kLtSlab + 4 * group + d);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         float4 s[VH];
 #pragma unroll
         for (int b = 0; b < VH; ++b) s[b] = *reinterpret_cast<const float4*>(rows + (d + e) * V + 64 * b + 4 * tx);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
           for (int b = 0; b < VH; ++b) {
-            fma2(acc[i][2 * b], twice(q[i][e]), lower(s[b]));
-            fma2(acc[i][2 * b + 1], twice(q[i][e]), upper(s[b]));
+            fma2(acc[i][2 * b], twice(e ? q[i].y : q[i].x), lower(s[b]));
+            fma2(acc[i][2 * b + 1], twice(e ? q[i].y : q[i].x), upper(s[b]));
           }
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float f = pow_s[ty + 16 * i + 1];
+  for (int i = 0; i < 8; ++i) {
+    const float f = pow_s[ty + 8 * i + 1];
 #pragma unroll
     for (int j = 0; j < 2 * VH; ++j) {
       acc[i][j].x *= f;
       acc[i][j].y *= f;
     }
   }
-  // the chunk's own tokens up to each one
+  // the chunk's own tokens up to each one: four of eight a group
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (16 * j >= nt) break;
+  for (int j = 0; j < 8; ++j) {
+    if (8 * j >= nt) break;
 #pragma unroll
-    for (int s0 = 0; s0 < 16; s0 += 4) {
-      float a[4][4];
+    for (int e2 = 0; e2 < 4; e2 += 2) {
+      const int s0 = 4 * group + e2;
+      float2 a[8];
 #pragma unroll
-      for (int i = j; i < 4; ++i) *reinterpret_cast<float4*>(a[i]) = *reinterpret_cast<const float4*>(k_s + (ty + 16 * i) * kLtPitchA + 16 * j + s0);
+      for (int i = j; i < 8; ++i) a[i] = *reinterpret_cast<const float2*>(k_s + (ty + 8 * i) * kLtPitchA + 8 * j + s0);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         float4 v[VH];
 #pragma unroll
-        for (int b = 0; b < VH; ++b) v[b] = *reinterpret_cast<const float4*>(v_s + (16 * j + s0 + e) * V + 64 * b + 4 * tx);
+        for (int b = 0; b < VH; ++b) v[b] = *reinterpret_cast<const float4*>(v_s + (8 * j + s0 + e) * V + 64 * b + 4 * tx);
 #pragma unroll
-        for (int i = j; i < 4; ++i) {
+        for (int i = j; i < 8; ++i) {
           if (i > j || s0 + e <= ty) {
 #pragma unroll
             for (int b = 0; b < VH; ++b) {
-              fma2(acc[i][2 * b], twice(a[i][e]), lower(v[b]));
-              fma2(acc[i][2 * b + 1], twice(a[i][e]), upper(v[b]));
+              fma2(acc[i][2 * b], twice(e ? a[i].y : a[i].x), lower(v[b]));
+              fma2(acc[i][2 * b + 1], twice(e ? a[i].y : a[i].x), upper(v[b]));
             }
           }
         }
       }
     }
   }
+  // each group finishes four of a thread's tokens: the other group's part of them comes through where the queries were
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if ((i < 4) == (group == 1)) {
+#pragma unroll
+      for (int b = 0; b < VH; ++b)
+        *reinterpret_cast<float4*>(q_s + (ty + 8 * i) * kLtPitch + 64 * b + 4 * tx) =
+            make_float4(acc[i][2 * b].x, acc[i][2 * b].y, acc[i][2 * b + 1].x, acc[i][2 * b + 1].y);
+    }
+  __syncthreads();
   float* dst = p.out + (size_t)c.t0 * p.ldo + (size_t)h * vdim + v0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = ty + 16 * i;
-    if (t >= nt) break;
+  for (int i = 0; i < 8; ++i) {
+    const int t = ty + 8 * i;
+    if ((i < 4) != (group == 0) || t >= nt) continue;
 #pragma unroll
     for (int b = 0; b < VH; ++b)
-      if (64 * b + 4 * tx < cols)
+      if (64 * b + 4 * tx < cols) {
+        const float4 o = *reinterpret_cast<const float4*>(q_s + t * kLtPitch + 64 * b + 4 * tx);
         *reinterpret_cast<float4*>(dst + (size_t)t * p.ldo + 64 * b + 4 * tx) =
-            make_float4(acc[i][2 * b].x, acc[i][2 * b].y, acc[i][2 * b + 1].x, acc[i][2 * b + 1].y);
+            make_float4(acc[i][2 * b].x + o.x, acc[i][2 * b].y + o.y, acc[i][2 * b + 1].x + o.z, acc[i][2 * b + 1].y + o.w);
+      }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
