@@ -8,6 +8,9 @@ step lives in one int32 device buffer, filled by a single host→device copy:
     token_ids[N] positions[N] seq_of_token[N] q_start[B+1] ctx_len[B]
     slot_ids[B] logit_rows[M] block_table_g[B, W_g] for every cache group g
 
+An engine's step appends ``seq_order`` where it starts with enough sequences of one token (see :func:`longest_first`); a
+captured step keeps it in front.
+
 ``positions`` are absolute (crates/leone/src/cpu.rs:1759-1765: prefill position
 = start + t); ``ctx_len`` is a sequence's length after this step, so the query
 at position p reads keys ``..p`` (the reference masks by loop bound,

@@ -86,7 +86,7 @@ def test_values_at_the_edge_of_the_range_pass_through_the_product(ops32):  # noq
         ops32._gemm_simt(x, w, out, 0, None)
         if word & 0x7fffffff > 0x7f800000:
             assert torch.isnan(out[7]).any()
-        else:                                          # two terms of 11 bits hold a word to 2^-23 of it
+        else:                                          # (such a row is summed by FMA; two terms would hold a word to 2^-23 of it)
             assert ((out[7, :k].double() - x[7].double()).abs() <= 2.0 ** -23 * x[7].double().abs()).all()
         assert torch.equal(out[8, :k], x[8]) and torch.isfinite(out[:7]).all() and torch.isfinite(out[9:]).all()
 
