@@ -248,12 +248,15 @@ attention_f32_prompt_kernel(const Params p) {
 
 // ---- one token a sequence --------------------------------------------------------------------------------------
 // Bound by the keys' and values' bytes.  A cluster of `splits` blocks owns a (sequence, kv head, up to GT heads of its
-// group); the warps of all its blocks take runs of 32 keys in turn.  A lane holds D / 32 elements of every query, looks up
-// one of the 32 keys' pages, and reads its piece of four keys and four values at a time, each a whole row per warp.
-// Every warp keeps its own running maximum, sum and outputs; they meet in shared memory, then across the cluster, in rank
-// order.  Measured: 4 sequences of 300, 16 heads on 8 of 128: under 10 us in the
-// step; the any-size kernel 74 us.
-constexpr int kWarps = 4;
+// group); the warps of all its blocks take runs of eight keys in turn (four with eight heads).  A lane holds D / 32 elements of every
+// query and reads its piece of a run's keys and values, each a whole row per warp, all at once; the rows of the next run are
+// looked up meanwhile.  With few short sequences the time is a chain of such reads, one after another, so runs are short and
+// many warps are at work: runs of 32 keys in steps of four took a sequence of 300 through eight reads in a row, these
+// through three.  Every warp keeps its own running maximum, sum and outputs; a block's meet in shared memory, then the blocks' across
+// the cluster, in rank order.  Measured in the step of 4
+// sequences of 300, 16 heads on 8 of 128: 17 us before the next kernel can start with runs of 32, 8 with runs of 8 (the
+// any-size kernel 74).
+constexpr int kWarps = 4, kMostSplits = 8;
 
 template <int D, int GT>
 __global__ void __launch_bounds__(kWarps * 32)
@@ -261,6 +264,8 @@ attention_f32_decode_kernel(const Params p, int head_groups, int splits) {
   constexpr int E = D / 32;                     // elements of a row a lane holds
   __shared__ float m_s[kWarps][GT], l_s[kWarps][GT];
   __shared__ __align__(16) float o_s[kWarps][GT][D];
+  __shared__ float m_b[GT], l_b[GT];            // of the whole block
+  constexpr int kRun = GT <= 4 ? 8 : 4;         // keys a warp reads at a time
   pdl_trigger();
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -290,62 +295,63 @@ attention_f32_decode_kernel(const Params p, int head_groups, int splits) {
       dst[0] = v.x; dst[1] = v.y;
     }
   };
-  for (int j0 = lo + (rank * kWarps + warp) * 32; j0 <= pos; j0 += splits * kWarps * 32) {
-    const long long mine = j0 + lane <= pos ? key_row(p, s, kvh, j0 + lane, row) : -1;
-    const int there = min(32, pos - j0 + 1);
-    for (int j = 0; j < there; j += 4) {
-      long long at[4];
-      float k[4][E], v[4][E];
+  const int step = splits * kWarps * kRun;
+  auto lookup = [&](int j0) { return lane < kRun && j0 + lane <= pos ? key_row(p, s, kvh, j0 + lane, row) : -1ll; };
+  int j0 = lo + (rank * kWarps + warp) * kRun;
+  long long mine = lookup(j0);
+  for (; j0 <= pos; j0 += step) {
+    long long at[kRun];
+    float k[kRun][E], v[kRun][E];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        at[i] = __shfl_sync(0xffffffffu, mine, j + i);
-        piece(p.k_pool + (at[i] < 0 ? 0 : at[i]) * D + lane * E, k[i]);
+    for (int i = 0; i < kRun; ++i) {
+      at[i] = __shfl_sync(0xffffffffu, mine, i);
+      piece(p.k_pool + (at[i] < 0 ? 0 : at[i]) * D + lane * E, k[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) piece(p.v_pool + (at[i] < 0 ? 0 : at[i]) * D + lane * E, v[i]);
+    mine = lookup(j0 + step);
+#pragma unroll
+    for (int i = 0; i < kRun; ++i)
+      if (at[i] < 0)
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[i][e] = 0.f;         // another row's value may be infinite
+    float sc[kRun * GT];
+#pragma unroll
+    for (int h = 0; h < GT; ++h)
+#pragma unroll
+      for (int i = 0; i < kRun; ++i) {
+        float a = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) a = fmaf(q[h][e], k[i][e], a);
+        sc[h * kRun + i] = a;
       }
+    warp_sum_scatter<kRun * GT, 16>(sc, lane);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        piece(p.v_pool + (at[i] < 0 ? 0 : at[i]) * D + lane * E, v[i]);
-        if (at[i] < 0)
+    for (int h = 0; h < GT; ++h) {
+      float w[kRun], top = -INFINITY;
 #pragma unroll
-          for (int e = 0; e < E; ++e) v[i][e] = 0.f;     // another row's value may be infinite
+      for (int i = 0; i < kRun; ++i) {
+        w[i] = __shfl_sync(0xffffffffu, sc[0], (h * kRun + i) * (32 / (kRun * GT))) * p.scale;
+        if (at[i] < 0) w[i] = -INFINITY;
+        top = fmaxf(top, w[i]);
       }
-      float sc[4 * GT];
+      const float m_new = fmaxf(m_run[h], top);
+      const float base = m_new == -INFINITY ? 0.f : m_new;
+      const float alpha = expf(m_run[h] - base);
+      m_run[h] = m_new;
+      float sum = 0.f;
 #pragma unroll
-      for (int h = 0; h < GT; ++h)
+      for (int i = 0; i < kRun; ++i) {
+        w[i] = expf(w[i] - base);
+        sum += w[i];
+      }
+      l_run[h] = l_run[h] * alpha + sum;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float a = 0.f;
+      for (int e = 0; e < E; ++e) {
+        float a = acc[h][e] * alpha;
 #pragma unroll
-          for (int e = 0; e < E; ++e) a = fmaf(q[h][e], k[i][e], a);
-          sc[h * 4 + i] = a;
-        }
-      warp_sum_scatter<4 * GT, 16>(sc, lane);
-#pragma unroll
-      for (int h = 0; h < GT; ++h) {
-        float w[4], top = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          w[i] = __shfl_sync(0xffffffffu, sc[0], (h * 4 + i) * (32 / (4 * GT))) * p.scale;
-          if (at[i] < 0) w[i] = -INFINITY;
-          top = fmaxf(top, w[i]);
-        }
-        const float m_new = fmaxf(m_run[h], top);
-        const float base = m_new == -INFINITY ? 0.f : m_new;
-        const float alpha = expf(m_run[h] - base);
-        m_run[h] = m_new;
-        float sum = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          w[i] = expf(w[i] - base);
-          sum += w[i];
-        }
-        l_run[h] = l_run[h] * alpha + sum;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          float a = acc[h][e] * alpha;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) a = fmaf(w[i], v[i][e], a);
-          acc[h][e] = a;
-        }
+        for (int i = 0; i < kRun; ++i) a = fmaf(w[i], v[i][e], a);
+        acc[h][e] = a;
       }
     }
   }
@@ -358,33 +364,58 @@ attention_f32_decode_kernel(const Params p, int head_groups, int splits) {
 #pragma unroll
     for (int e = 0; e < E; ++e) o_s[warp][h][lane * E + e] = acc[h][e];
   }
-  if (splits > 1) cluster_sync_all();
-  else __syncthreads();
-  const uint32_t m_at = (uint32_t)__cvta_generic_to_shared(&m_s[0][0]), l_at = (uint32_t)__cvta_generic_to_shared(&l_s[0][0]),
-                 o_at = (uint32_t)__cvta_generic_to_shared(&o_s[0][0][0]);
-  // the cluster's threads share out the heads' elements
-  for (int i = rank * kWarps * 32 + tid; i < heads * D; i += splits * kWarps * 32) {
+  __syncthreads();
+  // The block's warps become one: thread tid owns elements tid, tid + 128, .. of the heads' outputs and leaves them in warp 0's place
+  // (nobody else reads those elements; the maxima and sums go to a place of their own).
+  for (int i = tid; i < GT * D; i += kWarps * 32) {
     const int h = i / D, c = i % D;
     float top = -INFINITY, l = 0.f, o = 0.f;
-    for (int r = 0; r < splits; ++r)
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const float m = splits > 1 ? cluster_ld_f32(cluster_map(m_at + (w * GT + h) * 4, r)) : m_s[w][h];
-        top = fmaxf(top, m);
-      }
-    if (top > -INFINITY)
-      for (int r = 0; r < splits; ++r)
+    for (int w = 0; w < kWarps; ++w) top = fmaxf(top, m_s[w][h]);
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-          const float m = splits > 1 ? cluster_ld_f32(cluster_map(m_at + (w * GT + h) * 4, r)) : m_s[w][h];
-          if (m == -INFINITY) continue;
-          const float f = expf(m - top);
-          l += f * (splits > 1 ? cluster_ld_f32(cluster_map(l_at + (w * GT + h) * 4, r)) : l_s[w][h]);
-          o += f * (splits > 1 ? cluster_ld_f32(cluster_map(o_at + ((w * GT + h) * D + c) * 4, r)) : o_s[w][h][c]);
-        }
-    p.out[(size_t)row * p.out_stride + (size_t)(kvh * g + h0 + h) * D + c] = l > 0.f ? o / l : 0.f;
+    for (int w = 0; w < kWarps; ++w) {
+      if (m_s[w][h] == -INFINITY) continue;
+      const float f = expf(m_s[w][h] - top);
+      l += f * l_s[w][h];
+      o += f * o_s[w][h][c];
+    }
+    o_s[0][h][c] = o;
+    if (c == 0) {
+      m_b[h] = top;
+      l_b[h] = l;
+    }
+    if (splits == 1 && h < heads)
+      p.out[(size_t)row * p.out_stride + (size_t)(kvh * g + h0 + h) * D + c] = l > 0.f ? o / l : 0.f;
   }
-  if (splits > 1) cluster_sync_all();      // a block's sums stay until everyone has read them
+  if (splits == 1) return;
+  cluster_sync_all();
+  const uint32_t m_at = (uint32_t)__cvta_generic_to_shared(m_b), l_at = (uint32_t)__cvta_generic_to_shared(l_b),
+                 o_at = (uint32_t)__cvta_generic_to_shared(&o_s[0][0][0]);
+  // The cluster's threads share out the heads' elements; a thread's loads from the other blocks are in flight together.
+  for (int i = rank * kWarps * 32 + tid; i < heads * D; i += splits * kWarps * 32) {
+    const int h = i / D, c = i % D;
+    float m[kMostSplits], l[kMostSplits], o[kMostSplits], top = -INFINITY, sum = 0.f, out = 0.f;
+#pragma unroll
+    for (int r = 0; r < kMostSplits; ++r) {
+      if (r < splits) {
+        m[r] = cluster_ld_f32(cluster_map(m_at + h * 4, r));
+        l[r] = cluster_ld_f32(cluster_map(l_at + h * 4, r));
+        o[r] = cluster_ld_f32(cluster_map(o_at + (h * D + c) * 4, r));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kMostSplits; ++r)
+      if (r < splits) top = fmaxf(top, m[r]);
+#pragma unroll
+    for (int r = 0; r < kMostSplits; ++r) {
+      if (r >= splits || m[r] == -INFINITY) continue;
+      const float f = expf(m[r] - top);
+      sum += f * l[r];
+      out += f * o[r];
+    }
+    p.out[(size_t)row * p.out_stride + (size_t)(kvh * g + h0 + h) * D + c] = sum > 0.f ? out / sum : 0.f;
+  }
+  cluster_sync_all();                      // a block's sums stay until everyone has read them
 }
 
 template <int D>
@@ -402,10 +433,10 @@ template <int D, int GT>
 int launch_decode(const Params& p, int n_seqs, int max_ctx, cudaStream_t stream) {
   const int groups = (p.n_q / p.n_kv + GT - 1) / GT;
   if ((long long)p.n_kv * groups > 65535) return kRefusedSize;
-  // Splits until two blocks an SM are there, while every warp of a split has a run of 32 keys of its own.
+  // Splits until two blocks an SM are there, while every warp of a split has two runs of its own.
   int splits = 1;
   const long long blocks = (long long)n_seqs * p.n_kv * groups;
-  while (splits < 8 && blocks * splits < 2 * 148 && max_ctx > splits * kWarps * 32) splits *= 2;
+  while (splits < kMostSplits && blocks * splits < 2 * 148 && max_ctx > splits * kWarps * 16) splits *= 2;
   const dim3 grid(splits, p.n_kv * groups, n_seqs);
   if (splits == 1)
     return launch_kernel(attention_f32_decode_kernel<D, GT>, grid, dim3(kWarps * 32), 0, stream, p, groups, 1);
