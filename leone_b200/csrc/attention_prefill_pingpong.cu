@@ -289,7 +289,7 @@ attention_prefill_pingpong_kernel(const __nv_bfloat16* __restrict__ qkv, int row
 
     if (warp == kMmaWarp) {
       // ---------------- the warp that issues the tensor-core work ----------------
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc_s = instr_desc_bf16(kRows, kKeys);
         constexpr uint32_t idesc_o = instr_desc_bf16_b_mn(kRows, D);
         auto issue_s = [&](int j, int t) {     // S_j = Q_j . K(t)^T

@@ -127,7 +127,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 
   if (warp == 0) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -149,7 +149,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(kExRows, kExCols);
       int stage = 0, it = 0;
       uint32_t phase = 0;
@@ -160,7 +160,6 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         bool ok = true;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
-          tc_fence_after();
           const uint32_t a_addr = tiles_base + stage * kExStage;
           const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(a_addr + kExStageA);
 #pragma unroll

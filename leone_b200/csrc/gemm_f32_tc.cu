@@ -138,7 +138,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == 0) {
     // ---------------- copies: the first stages' weights before the wait for the kernel before this one ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const int early = min(kFtStages, last - first);
       for (int i = 0; i < early; ++i) {
         mbar_expect_tx(raw_full0 + 8 * i, 2 * kFtTile);
@@ -160,7 +160,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else if (warp == 1) {
     // ---------------- MMAs ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_tf32(kFtM, kFtN);
       const uint32_t small = tmem_base + kFtSmall;
       int stage = 0;

@@ -185,7 +185,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // ---------------- producer (both blocks) ----------------
     // As in the single-block kernel the weight halves of the first stages are requested before
     // the wait for the kernel before this one, whose output is the token operand.
-    if (lane == 0) {
+    if (elect_one()) {
       int early = 0;
       for (int pass = 0; pass < 2; ++pass) {
         int stage = 0, filled = 0;
@@ -220,7 +220,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // the second block's warp 1 has nothing to do between allocating and freeing tensor memory
   } else if (warp == 1) {
     // ---------------- MMA issuer (the first block) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(2 * kTileW, BN);
       int stage = 0;
       uint32_t phase = 0;
@@ -233,7 +233,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         bool ok = true;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait_cluster(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
-          tc_fence_after();
           const uint32_t a_addr = tiles_base + stage * cfg.stage_bytes;
           const uint32_t b_addr = a_addr + kTileW * kTileK * 2;
           const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(b_addr);

@@ -108,7 +108,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // first stages are requested at once, and only then does the producer wait for the
     // predecessor (whose output is the token operand).  Pass 0 issues those early weight
     // loads, pass 1 is the steady loop, which for the first stages adds the token half only.
-    if (lane == 0) {
+    if (elect_one()) {
       int early = 0;                       // stages whose weight half was requested in pass 0
       for (int pass = 0; pass < 2; ++pass) {
         int stage = 0, filled = 0;
@@ -151,7 +151,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc_bf16(kTileW, BN);
       int stage = 0;
       uint32_t phase = 0;
@@ -168,7 +168,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         bool ok = true;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
-          tc_fence_after();
           if (it == 0 && kb == kb0) stamp(p, 3);           // first stage complete in shared memory
           const uint32_t a_addr = tiles_base + stage * Cfg::kStageBytes;
           const uint32_t b_addr = a_addr + kTileW * kTileK * 2;

@@ -12,6 +12,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// True in one thread of a warp, always the same; called by the whole warp.  A branch on it is how code that one thread of a warp runs is
+// to be written where it issues tcgen05 and TMA instructions: the compiler knows of elect.sync that a single thread goes on, so their
+// operands stay in uniform registers.  Behind `lane == 0` it cannot know: four MMAs, a commit and a wait took 547 cycles there,
+// 377 here, whatever the width of the MMAs below 256.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 r;\n\telect.sync r|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(yes));
+  return yes != 0;
+}
+
 // ---- mbarrier -------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
