@@ -401,6 +401,16 @@ class CacheManager:
                                                  out.ctypes.data_as(ctypes.POINTER(c_int))))
         return out
 
+    def copy_table_tails(self, gid: int, rids: Sequence[Hashable], done: np.ndarray, end: np.ndarray, rows: np.ndarray) -> None:
+        """Into row ``i`` of ``rows`` (int32, a row per request): the request's entries from ``done[i]`` on and -1 behind them up
+        to ``end[i]`` (``done``, ``end``: int32)."""
+        if rows.shape[0] < len(rids) or rows.dtype != np.int32 or not rows.flags.c_contiguous:
+            raise CacheError("a mirror of the tables is contiguous int32 with a row per request")
+        ci = ctypes.POINTER(c_int)
+        _check(self._lib.leone_cache_table_tails(
+            self._h, gid, len(rids), _ll(self._id(r) for r in rids), done.ctypes.data_as(ci), end.ctypes.data_as(ci),
+            rows.ctypes.data_as(ci), c_longlong(rows.shape[1])))
+
     # -- accounting -------------------------------------------------------------------
     def free_pages(self) -> List[int]:
         return [g.pool.num_free for g in self.groups]

@@ -29,6 +29,7 @@ from __future__ import annotations
 import struct
 from typing import Iterable, Optional
 
+import numpy as np
 import torch
 
 FIELDS = 8
@@ -75,6 +76,17 @@ class SlotRecords:
         if last_token is not None:
             self._rows[slot, LAST_TOKEN] = last_token
         self._dirty.add(slot)
+
+    def set_rows(self, slots, params, lengths, last_tokens) -> None:
+        """:meth:`set_sampling` and :meth:`set_progress` (position = length) of many slots at once."""
+        at = np.asarray(slots, dtype=np.int64)
+        bits = {t: struct.unpack("<I", struct.pack("<f", float(t)))[0] for t in {p.temperature for p in params}}
+        rows = self._rows
+        rows[at, SEED] = [_signed(int(p.seed)) for p in params]
+        rows[at, TEMPERATURE] = [bits[p.temperature] for p in params]
+        rows[at, LENGTH] = rows[at, POSITION] = lengths
+        rows[at, LAST_TOKEN] = last_tokens
+        self._dirty.update(at.tolist())
 
     def set_sampler_state(self, slot: int, value: float) -> None:
         self._rows[slot, SAMPLER] = struct.unpack("<q", struct.pack("<d", float(value)))[0]

@@ -18,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -45,8 +46,11 @@ MODULES: Dict[str, List[str]] = {
     # the host side of the runtime (pages, block tables, step metadata, the scheduler's decisions,
     # seeded random weights for CPU tensors): plain C++, no device code
     "host": ["host_runtime.cpp", "random_weights_host.cpp"],
+    # a CPython extension that calls the entry points of the others (ops/entry_points.py)
+    "call": ["launch_call.cpp"],
 }
-HOST_ONLY = {"host"}
+HOST_ONLY = {"host", "call"}
+OPTIONAL = {"call"}                # what the package does without where it cannot be built
 HEADERS = ["common.cuh", "mma_tile.cuh", "tc_common.cuh", "gemm_parts.cuh", "leone_static.h", "attention_tiled.cu", "random_draw.h",
            "gla_parts.cuh", "ssd_parts.cuh", "experts_tc.h", "gemm_f32.h"]
 
@@ -211,6 +215,8 @@ def _build_host(module, lib, stamp, digest, fresh, out_dir, verbose) -> str:
             flags = ["-O2", "-std=c++17", "-shared", "-Xcompiler", ",".join(HOST_FLAGS)] \
                 if os.path.basename(cxx).startswith("nvcc") \
                 else ["-O2", "-std=c++17", "-shared", "-fno-gnu-unique", *HOST_FLAGS]
+            if module == "call":
+                flags += ["-I", sysconfig.get_paths()["include"]]
             _run_with_heartbeat([cxx, *flags, "-I", HERE, *srcs, "-o", tmp_lib], MODULES[module][0])
             os.replace(tmp_lib, lib)
             with open(stamp, "w") as fh:
@@ -224,5 +230,12 @@ def _build_host(module, lib, stamp, digest, fresh, out_dir, verbose) -> str:
 
 
 def build_all(verbose: bool = True) -> List[str]:
-    return [ensure_built(m, verbose) for m in MODULES
-            if all(os.path.isfile(os.path.join(HERE, s)) for s in MODULES[m])]
+    built = []
+    for m in MODULES:
+        if all(os.path.isfile(os.path.join(HERE, s)) for s in MODULES[m]):
+            try:
+                built.append(ensure_built(m, verbose))
+            except BuildError:
+                if m not in OPTIONAL:
+                    raise
+    return built

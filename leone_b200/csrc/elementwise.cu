@@ -614,11 +614,12 @@ sample_kernel(const float* __restrict__ logits, int vocab,
 // (crates/leone-cuda/cuda/ie_cuda.cu:2940); this is the same idea for a whole batch.
 // ---------------------------------------------------------------------------
 // With slot records (records != null) the request's record is advanced instead of sample_pos:
-// its position and length by one, its last token set.
+// its position and length by one, its last token set.  status_out (or null): the four status words as the step left
+// them, beside the history, so that the host reads both in one copy.
 __global__ void decode_advance_kernel(int* token_ids, int* positions, int* ctx_len,
                                       long long* sample_pos, const int* sampled, int* history,
                                       int* step_counter, int n, int max_steps, const int* slot_ids,
-                                      long long* records) {
+                                      long long* records, const int* status, int* status_out) {
   pdl_trigger();
   pdl_wait();
   const int step = *step_counter;
@@ -639,6 +640,7 @@ __global__ void decode_advance_kernel(int* token_ids, int* positions, int* ctx_l
     if (step < max_steps) history[(size_t)step * n + i] = tok;
   }
   if (threadIdx.x == 0) *step_counter = step + 1;
+  if (status_out != nullptr && threadIdx.x < 4) status_out[threadIdx.x] = status[threadIdx.x];
 }
 
 // out[t] = scale * table[id_t] + pairs[row_t] + places[position_t]: a token's row, a row of a second table chosen by
@@ -713,12 +715,13 @@ using namespace leone;
 extern "C" int leone_decode_advance(int* token_ids, int* positions, int* ctx_len,
                                     long long* sample_pos, const int* sampled, int* history,
                                     int* step_counter, int n, int max_steps, const int* slot_ids,
-                                    long long* records, cudaStream_t stream) {
+                                    long long* records, const int* status, int* status_out, cudaStream_t stream) {
   if (n <= 0) return 0;
+  if (status_out != nullptr && status == nullptr) return kRefusedSize;
   if ((records != nullptr) == (sample_pos != nullptr)) return kRefusedSize;    // one of the two
   return launch_kernel(decode_advance_kernel, dim3(1), dim3(n < 1024 ? ((n + 31) / 32) * 32 : 1024), 0,
                        stream, token_ids, positions, ctx_len, sample_pos, sampled, history,
-                       step_counter, n, max_steps, slot_ids, records);
+                       step_counter, n, max_steps, slot_ids, records, status, status_out);
 }
 
 // Turns programmatic dependent launch on or off for the kernels of this library.

@@ -368,6 +368,25 @@ int leone_cache_table_copy(void* h, int gid, long long rid, int from, int count,
   std::copy(it->second.begin() + from, it->second.begin() + from + count, out);
   return kOk;
 }
+// For row i of a mirror of the block tables (rows `stride` entries apart): request i's entries from done[i] on, and -1 behind them up to
+// end[i] (no more entries than end[i]; nothing where done[i] >= end[i]).
+int leone_cache_table_tails(void* h, int gid, int n, const long long* rids, const int* done, const int* end, int* out,
+                            long long stride) {
+  Manager* m = static_cast<Manager*>(h);
+  if (gid < 0 || gid >= (int)m->groups.size()) return fail(kBadArgument, "no such group");
+  Group& g = m->groups[gid];
+  for (int i = 0; i < n; ++i) {
+    if (done[i] >= end[i]) continue;
+    auto it = g.tables.find(rids[i]);
+    if (it == g.tables.end()) return unknown(rids[i]);
+    if (done[i] < 0 || end[i] > stride || (int)it->second.size() > end[i]) return fail(kBadArgument, "table range");
+    int* row = out + (size_t)i * stride;
+    const int have = std::max(done[i], (int)it->second.size());
+    std::copy(it->second.begin() + std::min<size_t>(done[i], it->second.size()), it->second.end(), row + done[i]);
+    std::fill(row + have, row + end[i], -1);
+  }
+  return kOk;
+}
 // The block tables of n requests as rows of `width` entries, -1 where there is no page.
 int leone_cache_block_table(void* h, int gid, int n, const long long* rids, int width, int* out) {
   Manager* m = static_cast<Manager*>(h);

@@ -41,24 +41,28 @@ class DecodeGraph:
         packed, offsets, bt_offsets, _ = pack_metadata(
             [[0]] * batch, [0] * batch, [0] * batch, [[0]] * batch, tables)
         # in front of them, the order in which the sequences' attention starts.  Every sequence grows by a token a step, so an
-        # order holds until the next fill
-        self.offsets = {"seq_order": (0, batch), **{name: (batch + o, s) for name, (o, s) in offsets.items()}}
-        self.bt_offsets = [(batch + o, shape) for o, shape in bt_offsets]
-        self.size = batch + packed.size
+        # order holds until the next fill.  Behind it, the row of the history that the next step writes: 0 from every fill on
+        first = batch + 1
+        self.offsets = {"seq_order": (0, batch), **{name: (first + o, s) for name, (o, s) in offsets.items()}}
+        self.bt_offsets = [(first + o, shape) for o, shape in bt_offsets]
+        self.size = first + packed.size
         self.meta = torch.zeros(self.size, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(self.size, dtype=torch.int32, pin_memory=True)
         self.sampled = torch.zeros(batch, dtype=torch.int32, device=dev)
-        self.history = torch.zeros((max_quantum, batch), dtype=torch.int32, device=dev)
-        self.history_host = torch.zeros((max_quantum, batch), dtype=torch.int32, pin_memory=True)
-        self.counter = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.status_host = torch.zeros(4, dtype=torch.int32, pin_memory=True)
+        # what a step leaves for the host, read back in one copy: the status word, then a row of ids per step of the quantum
+        self._readback = torch.zeros(4 + max_quantum * batch, dtype=torch.int32, device=dev)
+        self._readback_host = torch.zeros(4 + max_quantum * batch, dtype=torch.int32, pin_memory=True)
+        self.history = self._readback[4:].view(max_quantum, batch)
+        self.history_host = self._readback_host[4:].view(max_quantum, batch)
+        self.status_host = self._readback_host[:4]
+        self.counter = self.meta[batch:first]
         self.logits = engine.decode_logits_buffer()[:batch]      # one buffer for every batch size
         self.ctx = self._context()
         self.graphs = {}                   # context bucket -> captured step
         self.graph = None                  # the selected bucket's
         self.bucket = None
         self._filled_rids = None           # what fill() last wrote into the host copy
-        self._filled_pages = [[0] * batch for _ in engine.cache.groups]
+        self._filled_pages = [np.zeros(batch, dtype=np.int32) for _ in engine.cache.groups]
         self._tables_at = min((o for o, _ in self.bt_offsets), default=None)   # where the block tables start
         # A row as wide as a design without a position limit needs (65,536 entries and more) costs more to clear and to
         # copy whole than a copy call of its own for the entries in use: 2 to 4 MB a refill, 44 us on the GPU and more on the
@@ -67,7 +71,6 @@ class DecodeGraph:
         if self._wide:
             self.meta[self._tables_at:].fill_(-1)
         self._events = [torch.cuda.Event(), torch.cuda.Event()]
-        self._advance_host = [torch.zeros((2, batch), dtype=torch.int32, pin_memory=True) for _ in range(2)]
         self.launches_per_step = 0
         self.stream = torch.cuda.Stream(device=dev)
 
@@ -117,7 +120,8 @@ class DecodeGraph:
         records = e.slot_records.on_device
         e.ops.sample_slots(logits, self.ctx.slot_ids, records, self.sampled)
         e.ops.decode_advance(self.ctx.token_ids, self.ctx.positions, self.ctx.ctx_len, None, self.sampled,
-                             self.history, self.counter, slot_ids=self.ctx.slot_ids, records=records)
+                             self.history, self.counter, slot_ids=self.ctx.slot_ids, records=records,
+                             status_out=self._readback[:4])
 
     def fill(self, rids: Sequence[Hashable], last_tokens: Sequence[int], lengths: Sequence[int], params,
              versions=None, slots=None, table_lens=None):
@@ -154,42 +158,37 @@ class DecodeGraph:
         appended = []                       # [lo, hi) ranges of the host copy that gained entries
         for gi, (g, w, (o, shape)) in enumerate(zip(e.cache.groups, self.widths, self.bt_offsets)):
             view = host[o:o + shape[0] * shape[1]].reshape(shape)
-            for i, r in enumerate(rids):
-                n = int(table_lens[gi][i]) if table_lens is not None else g.tables.length(r)
-                if n > w:
-                    raise ValueError(f"block table needs {n} columns, only {w} given")
-                # (a window's table that lost entries at its front has a new version, so it is not the same)
-                before = self._filled_pages[gi][i]
-                done = before if same else 0
-                end = n                     # a wide row is cleared as far as it was in use
-                if done == 0 and not self._wide:
-                    view[i, :] = -1
-                elif not same and before > n:
-                    view[i, n:before] = -1
-                    end = before
-                if n > done:
-                    view[i, done:n] = g.tables.tail(r, done)
-                if end > done:
-                    appended.append((o + i * shape[1] + done, o + i * shape[1] + end))
-                self._filled_pages[gi][i] = n
+            n = np.array(table_lens[gi] if table_lens is not None else [g.tables.length(r) for r in rids], dtype=np.int32)
+            if int(n.max()) > w:
+                raise ValueError(f"block table needs {int(n.max())} columns, only {w} given")
+            # (a window's table that lost entries at its front has a new version, so it is not the same)
+            before = self._filled_pages[gi]
+            if same:
+                done, end = before, n
+            else:                           # a wide row is cleared as far as it was in use, others whole
+                done, end = np.zeros(b, dtype=np.int32), np.maximum(before, n) if self._wide else np.full(b, w, dtype=np.int32)
+            e.cache.copy_table_tails(gi, rids, done, end, view)
+            if same or self._wide:
+                appended += [(o + i * shape[1] + int(done[i]), o + i * shape[1] + int(end[i])) for i in np.flatnonzero(end > done)]
+            self._filled_pages[gi] = n
         self._filled_rids = key
         # the requests' slot records: sampling parameters, and where each stands (the position
         # of the token being fed is the position that is sampled at)
         records = e.slot_records
         row_slots = slots if slots is not None else [e.cache.slot(r) for r in rids]
-        for slot, p, length, tok in zip(row_slots, params, lengths, last_tokens):
-            records.set_sampling(int(slot), p.seed, p.temperature)
-            records.set_progress(int(slot), int(length), int(length), int(tok))
+        records.set_rows(row_slots, params, lengths, last_tokens)
         records.sync()
         if (same or self._wide) and self._tables_at is not None:
             # the per-token and per-sequence vectors, and the block-table entries that are new: those appended since the last
-            # call for the same requests in the same rows, or all that are in use
+            # call for the same requests in the same rows, or all that are in use (a copy call takes the host longer than the
+            # GPU takes for rows of ordinary width, so from three on they are one copy)
+            if len(appended) > 2 and not self._wide:
+                appended = [(appended[0][0], appended[-1][1])]
             self.meta[:self._tables_at].copy_(self.meta_host[:self._tables_at], non_blocking=True)
             for lo, hi in appended:
                 self.meta[lo:hi].copy_(self.meta_host[lo:hi], non_blocking=True)
         else:
             self.meta.copy_(self.meta_host, non_blocking=True)
-        self.counter.zero_()
 
     def capture(self, bucket: int):
         """Run one step eagerly on the filled buffers (so every scratch buffer exists), then
@@ -224,24 +223,15 @@ class DecodeGraph:
         cur.wait_stream(self.stream)
         self.counter.zero_()
 
-    def advance_from_host(self, rids: Sequence[Hashable], lengths, table_lens, slot: int) -> None:
-        """Inputs of a step that is launched before the step before it has been read: the host's
-        own record of every request's position and length (the cache manager's; the device has
-        advanced its copy to the same values) and the block-table entries of pages taken since
-        the last :meth:`fill`.  The token ids are where the device put them.  The pinned staging
-        rows alternate with ``slot``, so a row is rewritten only after the step that read it
-        has been waited for."""
+    def advance_from_host(self, rids: Sequence[Hashable], table_lens) -> None:
+        """Inputs of a step that is launched before the step before it has been read: the
+        block-table entries of pages taken since the last :meth:`fill`.  Token ids, positions and lengths are
+        where the step before puts them."""
         e = self.engine
-        b = self.batch
-        stage = self._advance_host[slot & 1]
-        stage[0].numpy()[:] = lengths                    # position of the token being fed
-        stage[1].numpy()[:] = lengths + 1                # the sequence's length after the step
-        self._view("positions").copy_(stage[0], non_blocking=True)
-        self._view("ctx_len").copy_(stage[1], non_blocking=True)
         host = self.meta_host.numpy()
         for gi, (g, w, (o, shape)) in enumerate(zip(e.cache.groups, self.widths, self.bt_offsets)):
             for i, r in enumerate(rids):
-                n, done = int(table_lens[gi][i]), self._filled_pages[gi][i]
+                n, done = int(table_lens[gi][i]), int(self._filled_pages[gi][i])
                 if n > w:
                     raise ValueError(f"block table needs {n} columns, only {w} given")
                 if n > done:
@@ -251,12 +241,15 @@ class DecodeGraph:
                     self.meta[at + done:at + n].copy_(self.meta_host[at + done:at + n], non_blocking=True)
                     self._filled_pages[gi][i] = n
 
+    def _read_back(self, rows: int) -> None:
+        end = 4 + rows * self.batch
+        self._readback_host[:end].copy_(self._readback[:end], non_blocking=True)
+
     def launch(self, slot: int) -> torch.cuda.Event:
         """Enqueue one step, whose sampled ids go to row ``slot`` of the history, and their
         read-back; returns the event that says the ids are on the host."""
         self.graph.replay()
-        self.history_host[slot].copy_(self.history[slot], non_blocking=True)
-        self.status_host.copy_(self.engine.status, non_blocking=True)
+        self._read_back(slot + 1)
         event = self._events[slot & 1]
         event.record()
         return event
@@ -272,8 +265,7 @@ class DecodeGraph:
         """Replay ``steps`` steps and read the sampled ids back: int32 [steps, batch]."""
         for _ in range(steps):
             self.graph.replay()
-        self.history_host[:steps].copy_(self.history[:steps], non_blocking=True)
-        self.status_host.copy_(self.engine.status, non_blocking=True)
+        self._read_back(steps)
         torch.cuda.current_stream(self.engine.device).synchronize()
         if int(self.status_host[0]) != 0:
             self.engine.check_status()

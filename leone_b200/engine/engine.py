@@ -29,11 +29,13 @@ from ..weights.loader import check_names_and_shapes, load_checkpoint, target_dty
 from .budget import check_memory_budget, plan_memory
 from .batch import ORDER_FROM, StepContext, StepEntry, longest_first, pack_metadata
 from .model import Model
+from ..sampling.sampler import SamplingParams
 
 _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16,
            "float32": torch.float32, "fp32": torch.float32, "f32": torch.float32}
 
 
+_GREEDY = SamplingParams()
 EMBEDDING = "embedding"      # stands for a run position where the embedding part's own state is named
 
 
@@ -433,12 +435,11 @@ class Engine:
         """One decode step of ``rids`` from the captured graph, for a caller that samples itself:
         returns the fp32 logits ``[len(rids), vocab]`` (the graph's own buffer, valid until the
         next decode step); lengths advance by one.  The graph's built-in greedy draw is ignored."""
-        from ..sampling.sampler import SamplingParams
         rids = list(rids)
         self.drop_lookahead()
         if self.device.type != "cuda":
             return self.step([(r, [int(t)], [0]) for r, t in zip(rids, last_tokens)])
-        params = [SamplingParams() for _ in rids]
+        params = [_GREEDY] * len(rids)
         lengths, versions, slots, table_lens = self.cache.reserve_steps(rids, 1)
         try:
             if int(lengths.max()) + 1 > self.spec.max_positions:
@@ -519,7 +520,7 @@ class Engine:
                 except OutOfPages:
                     pass                                                   # the next call decides what gives way
                 else:
-                    graph.advance_from_host(rids, lengths + 1, table_lens, slot + 1)
+                    graph.advance_from_host(rids, table_lens)
                     ahead = dict(rids=rids, params=params, graph=graph, lengths=lengths + 1, slot=slot + 1,
                                  event=graph.launch(slot + 1))
             tokens = graph.collect(slot, event)

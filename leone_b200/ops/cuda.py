@@ -1,8 +1,8 @@
 """The kernel table: Python calls into the engine's own CUDA libraries.
 
 Every call checks shapes, dtypes and contiguity on the host, then launches on
-the current torch stream through a C entry point of ``csrc`` (loaded with
-ctypes; compiled on first use by :mod:`leone_b200.csrc.build`).  There is no
+the current torch stream through a C entry point of ``csrc`` (called through
+:mod:`leone_b200.ops.entry_points`; compiled on first use by :mod:`leone_b200.csrc.build`).  There is no
 other implementation behind these calls: without a CUDA device or without the
 compiled libraries, construction raises.  The reference has the same split
 between checked wrappers and raw entry points
@@ -12,13 +12,15 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_void_p
+from ctypes import c_int
 from typing import Optional
 
 import numpy as np
 import torch
 
 from ..csrc.build import ensure_built
+from .entry_points import EntryPoints
+from .fast import leading_ones
 
 _STATUS_TEXT = {
     1: "a token id outside the vocabulary reached the embedding kernel",
@@ -38,16 +40,14 @@ class KernelError(RuntimeError):
     pass
 
 
+_DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1}
+
+
 def _dt(t: torch.dtype) -> int:
-    if t == torch.float32:
-        return 0
-    if t == torch.bfloat16:
-        return 1
-    raise KernelError(f"kernels take float32 or bfloat16, not {t}")
-
-
-def _ptr(t: Optional[torch.Tensor]):
-    return c_void_p(0 if t is None else t.data_ptr())
+    code = _DTYPE_CODES.get(t)
+    if code is None:
+        raise KernelError(f"kernels take float32 or bfloat16, not {t}")
+    return code
 
 
 def _check(code: int, what: str) -> None:
@@ -95,6 +95,7 @@ class CudaOps:
             raise KernelError(f"the kernels are built for sm_100a; device reports sm_{major}{minor}")
         self.dtype = dtype
         self.core = ctypes.CDLL(ensure_built("core"))
+        self.core_calls = EntryPoints(self.core)         # the launches (self.core: what is asked once in a while)
         self.fast = None
         self._pinned_stream = None
         if dtype == torch.bfloat16:
@@ -130,12 +131,12 @@ class CudaOps:
     def _stream(self):
         if self._pinned_stream is not None:        # (a handle of 0, the default stream, is a valid pin)
             return self._pinned_stream
-        return c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     def pin_stream(self, on: bool) -> None:
         """Between ``pin_stream(True)`` and ``pin_stream(False)`` every launch goes to the stream
         that was current at the first call: a step looks its stream up once, not once per launch."""
-        handle = c_void_p(torch.cuda.current_stream(self.device).cuda_stream) if on else None
+        handle = torch.cuda.current_stream(self.device).cuda_stream if on else None
         self._pinned_stream = handle
         if self.fast is not None:
             self.fast.pin_stream(handle)
@@ -170,8 +171,8 @@ class CudaOps:
         _need(ids.dtype == torch.int32 and ids.numel() == n, "embedding ids must be int32 [N]")
         _need(table.shape[1] == hidden and table.is_contiguous(), "embedding table shape")
         self.launches += 1
-        _check(self.core.leone_embedding(_dt(table.dtype), _ptr(table), _ptr(ids), _ptr(out), n,
-                                         hidden, table.shape[0], c_float(scale), _ptr(status), self._stream()),
+        _check(self.core_calls.leone_embedding(_dt(table.dtype), table, ids, out, n,
+                                         hidden, table.shape[0], float(scale), status, self._stream()),
                "embedding")
 
     def embedding_sum(self, ctx, table, out, scale=1.0, pairs=None, buckets=0, mul_prev=0, mul_cur=0, last_token=None,
@@ -189,33 +190,35 @@ class CudaOps:
             _need(pairs.shape[0] == buckets + 1 and last_token is not None and last_token.is_contiguous()
                   and last_token.element_size() == 4 and last_token.numel() == last_token.shape[0], "embedding_sum pairs/state")
         self.launches += 1
-        _check(self.core.leone_embedding_sum(
-            _dt(table.dtype), _ptr(table), _ptr(ctx.token_ids), _ptr(out), n, hidden, table.shape[0], c_float(scale),
-            _ptr(pairs), int(buckets), ctypes.c_longlong(mul_prev), ctypes.c_longlong(mul_cur), _ptr(last_token),
-            1 if write_state else 0, _ptr(places), 0 if places is None else places.shape[0], _ptr(ctx.positions),
-            _ptr(ctx.q_start), _ptr(ctx.seq_of_token), _ptr(ctx.slot_ids), ctx.n_seqs,
-            0 if last_token is None else last_token.shape[0], _ptr(ctx.status), self._stream()), "embedding_sum")
+        _check(self.core_calls.leone_embedding_sum(
+            _dt(table.dtype), table, ctx.token_ids, out, n, hidden, table.shape[0], float(scale),
+            pairs, int(buckets), mul_prev, mul_cur, last_token,
+            1 if write_state else 0, places, 0 if places is None else places.shape[0], ctx.positions,
+            ctx.q_start, ctx.seq_of_token, ctx.slot_ids, ctx.n_seqs,
+            0 if last_token is None else last_token.shape[0], ctx.status, self._stream()), "embedding_sum")
 
     def logit_post(self, logits, scale: float = 1.0, soft_cap: Optional[float] = None):
         """In place: ``logits * scale``, then ``cap * tanh(. / cap)`` if a soft cap is given."""
         _need(logits.dtype == torch.float32 and logits.is_contiguous(), "logits must be contiguous fp32")
         _need(soft_cap is None or soft_cap > 0, "a soft cap must be positive")
         self.launches += 1
-        _check(self.core.leone_logit_post(_ptr(logits), ctypes.c_longlong(logits.numel()), c_float(scale),
-                                          c_float(soft_cap or 0.0), self._stream()), "logit_post")
+        _check(self.core_calls.leone_logit_post(logits, logits.numel(), float(scale),
+                                          float(soft_cap or 0.0), self._stream()), "logit_post")
 
     def rms_norm(self, x, weight, out, eps, rows=None):
         n_out, hidden = out.shape
-        _need(x.dtype == torch.float32 and x.is_contiguous() and x.shape[1] == hidden,
-              "rms_norm input must be contiguous fp32 [*, hidden]")
-        _need(weight.numel() == hidden and out.is_contiguous(), "rms_norm weight/output shape")
+        n_in, width = x.shape
+        if x.dtype != torch.float32 or width != hidden or not x.is_contiguous():
+            raise KernelError("rms_norm input must be contiguous fp32 [*, hidden]")
+        if weight.numel() != hidden or not out.is_contiguous():
+            raise KernelError("rms_norm weight/output shape")
         if rows is not None:
             _need(rows.dtype == torch.int32 and rows.numel() == n_out, "rms_norm rows must be int32")
-        else:
-            _need(x.shape[0] >= n_out, "rms_norm input has fewer rows than the output")
+        elif n_in < n_out:
+            raise KernelError("rms_norm input has fewer rows than the output")
         self.launches += 1
-        _check(self.core.leone_rms_norm(_ptr(x), _ptr(rows), _ptr(weight), _dt(weight.dtype),
-                                        _ptr(out), _dt(out.dtype), n_out, hidden, c_float(eps),
+        _check(self.core_calls.leone_rms_norm(x, rows, weight, _dt(weight.dtype),
+                                        out, _dt(out.dtype), n_out, hidden, float(eps),
                                         self._stream()), "rms_norm")
 
     def layer_norm(self, x, weight, bias, out, eps, rows=None):
@@ -232,16 +235,16 @@ class CudaOps:
         else:
             _need(x.shape[0] >= n_out, "layer_norm input has fewer rows than the output")
         self.launches += 1
-        _check(self.core.leone_layer_norm(_ptr(x), _ptr(rows), _ptr(weight), _ptr(bias), _dt(weight.dtype), _ptr(out),
-                                          _dt(out.dtype), n_out, hidden, c_float(eps), self._stream()), "layer_norm")
+        _check(self.core_calls.leone_layer_norm(x, rows, weight, bias, _dt(weight.dtype), out,
+                                          _dt(out.dtype), n_out, hidden, float(eps), self._stream()), "layer_norm")
 
     def _gemm_simt(self, x, w, out, epilogue, residual, bias=None):
         m, k = x.shape
         n = w.shape[0]
         self.launches += 1
-        _check(self.core.leone_gemm_simt(_dt(x.dtype), epilogue, _ptr(x), _ptr(w), _ptr(out),
-                                         _ptr(residual), _ptr(bias), m, n, k, x.stride(0), w.stride(0),
-                                         out.stride(0), _ptr(self.status), self._stream()), "gemm_simt")
+        _check(self.core_calls.leone_gemm_simt(_dt(x.dtype), epilogue, x, w, out,
+                                         residual, bias, m, n, k, x.stride(0), w.stride(0),
+                                         out.stride(0), self.status, self._stream()), "gemm_simt")
 
     def linear_fuses_norm(self, n_tokens: int, w: PreparedMatrix) -> bool:
         """True if a product of ``n_tokens`` tokens with ``w`` can take part in a fused RMSNorm:
@@ -283,17 +286,21 @@ class CudaOps:
         ``residual`` may be added; it may be ``out`` itself).  ``norm_in`` / ``norm_out``: see
         :meth:`linear_fuses_norm`."""
         m, k = x.shape
-        _need(k == w.in_features and out.shape == (m, w.out_features), "linear: shapes do not chain")
-        _need(x.dtype == w.dtype and x.stride(1) == 1 and out.stride(1) == 1, "linear: dtype/stride")
+        dtype, out_dtype = x.dtype, out.dtype
+        if k != w.in_features or out.shape != (m, w.out_features):
+            raise KernelError("linear: shapes do not chain")
+        if dtype != w.weight.dtype or x.stride(1) != 1 or out.stride(1) != 1:
+            raise KernelError("linear: dtype/stride")
         if residual is not None:
-            _need(out.dtype == torch.float32 and residual.dtype == torch.float32
-                  and residual.shape == out.shape and residual.stride() == out.stride(),
-                  "linear: a residual needs fp32 output of the same layout")
+            if out_dtype != torch.float32 or not (residual is out or (
+                    residual.dtype == torch.float32 and residual.shape == out.shape and residual.stride() == out.stride())):
+                raise KernelError("linear: a residual needs fp32 output of the same layout")
             epilogue = 2
-        elif out.dtype == torch.float32 and x.dtype != torch.float32:
+        elif out_dtype == torch.float32 and dtype != torch.float32:
             epilogue = 1
         else:
-            _need(out.dtype == x.dtype, "linear: output dtype")
+            if out_dtype != dtype:
+                raise KernelError("linear: output dtype")
             epilogue = 0
         if m == 0:
             return
@@ -333,19 +340,19 @@ class CudaOps:
         self._gemm_simt(x, w_gate_up.weight, scratch, 0, None, w_gate_up.bias)
         self.launches += 1
         if gate_shape is None:
-            _check(self.core.leone_swiglu(_dt(x.dtype), _ptr(scratch), _ptr(out), m, inter,
+            _check(self.core_calls.leone_swiglu(_dt(x.dtype), scratch, out, m, inter,
                                           self._stream()), "swiglu")
         else:
             slope, limit, shift, cubic = gate_shape
-            _check(self.core.leone_gated_act(_dt(x.dtype), _ptr(scratch), _ptr(out), m, inter, c_float(slope),
-                                             c_float(limit), c_float(shift), c_float(cubic), self._stream()), "gated_act")
+            _check(self.core_calls.leone_gated_act(_dt(x.dtype), scratch, out, m, inter, float(slope),
+                                             float(limit), float(shift), float(cubic), self._stream()), "gated_act")
 
     def convert(self, src, out):
         """``out = src`` elementwise, ``src`` fp32, ``out`` fp32 or the run dtype (same shape)."""
         _need(src.dtype == torch.float32 and src.is_contiguous() and out.is_contiguous()
               and src.shape == out.shape, "convert: layout")
         self.launches += 1
-        _check(self.core.leone_convert(_dt(out.dtype), _ptr(src), _ptr(out), ctypes.c_longlong(src.numel()),
+        _check(self.core_calls.leone_convert(_dt(out.dtype), src, out, src.numel(),
                                        self._stream()), "convert")
 
     def swiglu(self, gate_up, out):
@@ -353,7 +360,7 @@ class CudaOps:
         _need(out.shape == (m, two_i // 2) and gate_up.is_contiguous() and out.is_contiguous(),
               "swiglu shapes")
         self.launches += 1
-        _check(self.core.leone_swiglu(_dt(gate_up.dtype), _ptr(gate_up), _ptr(out), m, two_i // 2,
+        _check(self.core_calls.leone_swiglu(_dt(gate_up.dtype), gate_up, out, m, two_i // 2,
                                       self._stream()), "swiglu")
 
     _scratch_bufs = None
@@ -374,35 +381,39 @@ class CudaOps:
                            rotary_dim, cache, pairing="half_split"):
         """``pairing``: which elements of a head form rotation pair ``i``: ``(i, i + rotary_dim/2)``
         ("half_split") or ``(2i, 2i + 1)`` ("adjacent")."""
-        _need(pairing in ("half_split", "adjacent"), f"rotary pairing '{pairing}'")
-        n = qkv.shape[0]
-        _need(qkv.is_contiguous() and qkv.shape[1] == (n_q + 2 * n_kv) * d, "qkv layout")
+        if pairing != "half_split" and pairing != "adjacent":
+            raise KernelError(f"rotary pairing '{pairing}'")
+        n, cols = qkv.shape
+        dtype = qkv.dtype
+        if cols != (n_q + 2 * n_kv) * d or not qkv.is_contiguous():
+            raise KernelError("qkv layout")
         w_dtype = 0
         if q_norm_w is not None:
-            _need(k_norm_w is not None and q_norm_w.dtype == k_norm_w.dtype
-                  and q_norm_w.numel() == d and k_norm_w.numel() == d, "q/k norm weights")
+            if k_norm_w is None or q_norm_w.dtype != k_norm_w.dtype or q_norm_w.numel() != d or k_norm_w.numel() != d:
+                raise KernelError("q/k norm weights")
             w_dtype = _dt(q_norm_w.dtype)
         max_pos = 0
         if table is not None:
-            _need(table.dtype == torch.float32 and table.is_contiguous() and table.dim() == 3
-                  and table.shape[1] * 2 == rotary_dim and table.shape[2] == 2, "rotary table layout")
-            max_pos = table.shape[0]
+            shape = table.shape
+            if table.dtype != torch.float32 or len(shape) != 3 or shape[1] * 2 != rotary_dim or shape[2] != 2 or not table.is_contiguous():
+                raise KernelError("rotary table layout")
+            max_pos = shape[0]
         if cache is not None:
             kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
-            _need(kp.is_contiguous() and vp.is_contiguous() and kp.dtype == qkv.dtype
-                  and kp.shape[1] == n_kv and kp.shape[3] == d and kp.shape[2] == cache.page_tokens,
-                  "cache pool layout")
-            _need(bt.dtype == torch.int32 and bt.is_contiguous(), "block table")
-            pool_args = (_ptr(bt), bt.shape[1], bt.shape[0], _ptr(kp), _ptr(vp), kp.shape[0],
-                         cache.page_tokens)
+            pages, heads, rows, width = kp.shape
+            if kp.dtype != dtype or heads != n_kv or width != d or rows != cache.page_tokens or not kp.is_contiguous() \
+                    or not vp.is_contiguous():
+                raise KernelError("cache pool layout")
+            n_seqs, table_width = bt.shape
+            if bt.dtype != torch.int32 or not bt.is_contiguous():
+                raise KernelError("block table")
+            pool_args = (bt, table_width, n_seqs, kp, vp, pages, rows)
         else:
-            pool_args = (c_void_p(0), 0, 0, c_void_p(0), c_void_p(0), 0, 0)
+            pool_args = (None, 0, 0, None, None, 0, 0)
         self.launches += 1
-        _check(self.core.leone_qk_norm_rope_write(
-            _dt(qkv.dtype), _ptr(qkv), n, n_q, n_kv, d, _ptr(q_norm_w), _ptr(k_norm_w), w_dtype,
-            c_float(eps), _ptr(table), rotary_dim, max_pos, _ptr(ctx.positions),
-            _ptr(ctx.seq_of_token), pool_args[0], pool_args[1], pool_args[2], pool_args[3],
-            pool_args[4], pool_args[5], pool_args[6], 1 if pairing == "adjacent" else 0, _ptr(ctx.status),
+        _check(self.core_calls.leone_qk_norm_rope_write(
+            _dt(dtype), qkv, n, n_q, n_kv, d, q_norm_w, k_norm_w, w_dtype, float(eps), table, rotary_dim, max_pos, ctx.positions,
+            ctx.seq_of_token, *pool_args, 1 if pairing == "adjacent" else 0, ctx.status,
             self._stream()), "qk_norm_rope_write")
 
     def can_fuse_decode(self, ctx, qkv, n_q, n_kv, d) -> bool:
@@ -415,10 +426,11 @@ class CudaOps:
     def attention(self, ctx, qkv, out, n_q, n_kv, d, scale, window, cache, fuse=None):
         n = qkv.shape[0]
         kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
-        _need(out.shape == (n, n_q * d) and out.is_contiguous() and out.dtype == qkv.dtype,
-              "attention output layout")
-        _need(kp.is_contiguous() and vp.is_contiguous() and kp.dtype == qkv.dtype
-              and kp.shape[1] == n_kv and kp.shape[3] == d, "cache pool layout")
+        dtype, shape = qkv.dtype, kp.shape
+        if out.shape != (n, n_q * d) or out.dtype != dtype or not out.is_contiguous():
+            raise KernelError("attention output layout")
+        if kp.dtype != dtype or shape[1] != n_kv or shape[3] != d or not kp.is_contiguous() or not vp.is_contiguous():
+            raise KernelError("cache pool layout")
         if self.fast is not None and self.fast.attention(ctx, qkv, out, n_q, n_kv, d, scale,
                                                          window, cache, fuse):
             self.launches += 1
@@ -427,11 +439,11 @@ class CudaOps:
         if self._attention_f32(ctx, qkv, out, n_q, n_kv, d, scale, window, cache):
             return
         self.launches += 1
-        _check(self.core.leone_attention_generic(
-            _dt(qkv.dtype), _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp),
-            _ptr(bt), bt.shape[1], _ptr(ctx.seq_of_token), _ptr(ctx.positions), n, n_q, n_kv, d,
-            c_float(scale), int(window or 0), cache.page_tokens, kp.shape[0], bt.shape[0],
-            _ptr(ctx.status), self._stream()), "attention_generic")
+        _check(self.core_calls.leone_attention_generic(
+            _dt(qkv.dtype), qkv, qkv.stride(0), out, out.stride(0), kp, vp,
+            bt, bt.shape[1], ctx.seq_of_token, ctx.positions, n, n_q, n_kv, d,
+            float(scale), int(window or 0), cache.page_tokens, kp.shape[0], bt.shape[0],
+            ctx.status, self._stream()), "attention_generic")
 
     @staticmethod
     def _leading_single_rows(ctx) -> int:
@@ -440,9 +452,7 @@ class CudaOps:
         q_lens = getattr(ctx, "q_lens", None)
         if ctx.decode_only or getattr(ctx, "fixed_shapes", False) or q_lens is None:
             return 0
-        n = 0
-        while n < len(q_lens) and q_lens[n] == 1:
-            n += 1
+        n = leading_ones(ctx, q_lens)
         return n if n < len(q_lens) else 0
 
     def _attention_f32(self, ctx, qkv, out, n_q, n_kv, d, scale, window, cache) -> bool:
@@ -461,10 +471,10 @@ class CudaOps:
                      (n, ctx.n_seqs - n, int(ctx.q_lens[n:].max()), int(ctx.ctx_lens[n:].max()))]
         for first, count, q_len, ctx_len in parts:
             self.launches += 1
-            _check(self.core.leone_attention_f32(
-                _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt[first:]), bt.stride(0),
-                _ptr(ctx.q_start[first:]), _ptr(ctx.ctx_len[first:]), count, q_len, ctx_len, n_q, n_kv, d, c_float(scale),
-                int(window or 0), cache.page_tokens, kp.shape[0], _ptr(ctx.status), self._stream()), "attention_f32")
+            _check(self.core_calls.leone_attention_f32(
+                qkv, qkv.stride(0), out, out.stride(0), kp, vp, bt[first:], bt.stride(0),
+                ctx.q_start[first:], ctx.ctx_len[first:], count, q_len, ctx_len, n_q, n_kv, d, float(scale),
+                int(window or 0), cache.page_tokens, kp.shape[0], ctx.status, self._stream()), "attention_f32")
         return True
 
     _MASKS = {"causal": 0, "window": 1, "chunk": 2}
@@ -496,14 +506,14 @@ class CudaOps:
             _need(vp is not None and kp.is_contiguous() and vp.is_contiguous() and kp.dtype == qkv.dtype == vp.dtype
                   and kp.shape[1] == n_kv and kp.shape[2] == cache.page_tokens and kp.shape[3] == dk
                   and vp.shape[3] == dv and bt.dtype == torch.int32 and bt.is_contiguous(), "attention_prepare: cache layout")
-            pool_args = (_ptr(bt), bt.shape[1], bt.shape[0], _ptr(kp), _ptr(vp), kp.shape[0], cache.page_tokens)
+            pool_args = (bt, bt.shape[1], bt.shape[0], kp, vp, kp.shape[0], cache.page_tokens)
         else:
-            pool_args = (c_void_p(0), 0, ctx.n_seqs, c_void_p(0), c_void_p(0), 0, 0)
+            pool_args = (None, 0, ctx.n_seqs, None, None, 0, 0)
         self.launches += 1
-        _check(self.mixers.leone_attention_prepare(
-            _dt(qkv.dtype), _ptr(qkv), qkv.stride(0), n, n_q, n_kv, dk, dv, mode, _ptr(q_w), _ptr(k_w), c_float(eps),
-            _ptr(freqs), rot, 1 if pairing == "adjacent" else 0, c_float(coef), int(every), _ptr(ctx.positions),
-            _ptr(ctx.seq_of_token), *pool_args, _ptr(ctx.status), self._stream()), "attention_prepare")
+        _check(self.mixer_calls.leone_attention_prepare(
+            _dt(qkv.dtype), qkv, qkv.stride(0), n, n_q, n_kv, dk, dv, mode, q_w, k_w, float(eps),
+            freqs, rot, 1 if pairing == "adjacent" else 0, float(coef), int(every), ctx.positions,
+            ctx.seq_of_token, *pool_args, ctx.status, self._stream()), "attention_prepare")
 
     def attention_masked(self, ctx, qkv, out, n_q, n_kv, dk, dv, scale, mask, mask_size, weights, bias, cache):
         """Attention with a mask (``"causal"``, ``"window"``, ``"chunk"`` of ``mask_size``) and a
@@ -523,11 +533,11 @@ class CudaOps:
         if self.fast is not None and self.attention_masked_tiled(ctx, qkv, out, n_q, n_kv, dk, dv, scale, mask,
                                                                  mask_size, weights, bias, cache):
             return
-        _check(self.mixers.leone_attention_masked(
-            _dt(qkv.dtype), _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt),
-            bt.shape[1], _ptr(ctx.seq_of_token), _ptr(ctx.positions), n, n_q, n_kv, dk, dv, c_float(scale),
-            self._MASKS[mask], int(mask_size), self._WEIGHTS[weights], _ptr(bias), cache.page_tokens, kp.shape[0],
-            bt.shape[0], _ptr(ctx.status), self._stream()), "attention_masked")
+        _check(self.mixer_calls.leone_attention_masked(
+            _dt(qkv.dtype), qkv, qkv.stride(0), out, out.stride(0), kp, vp, bt,
+            bt.shape[1], ctx.seq_of_token, ctx.positions, n, n_q, n_kv, dk, dv, float(scale),
+            self._MASKS[mask], int(mask_size), self._WEIGHTS[weights], bias, cache.page_tokens, kp.shape[0],
+            bt.shape[0], ctx.status, self._stream()), "attention_masked")
 
     def attention_masked_tiled(self, ctx, qkv, out, n_q, n_kv, dk, dv, scale, mask, mask_size, weights, bias, cache) -> bool:
         """The tensor-core form of :meth:`attention_masked` (``csrc/attention_masked_mma.cu``) where
@@ -557,11 +567,11 @@ class CudaOps:
                 need = int(self.mixers.leone_attention_masked_mma_scratch(ctx.n_seqs, n_kv, dv, splits))
                 partial = self._scratch("masked_partial", -(-need // 64), 64, torch.float32)
                 self.launches += 1
-        _check(self.mixers.leone_attention_masked_mma(
-            _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt), bt.shape[1],
-            _ptr(ctx.q_start), _ptr(ctx.ctx_len), ctx.n_seqs, 1 if decode else int(ctx.max_q_len), n_q, n_kv, dk, dv,
-            c_float(scale), self._MASKS[mask], int(mask_size), self._WEIGHTS[weights], _ptr(bias), cache.page_tokens,
-            kp.shape[0], 1 if decode else 0, splits, _ptr(partial), _ptr(ctx.status), self._stream()),
+        _check(self.mixer_calls.leone_attention_masked_mma(
+            qkv, qkv.stride(0), out, out.stride(0), kp, vp, bt, bt.shape[1],
+            ctx.q_start, ctx.ctx_len, ctx.n_seqs, 1 if decode else int(ctx.max_q_len), n_q, n_kv, dk, dv,
+            float(scale), self._MASKS[mask], int(mask_size), self._WEIGHTS[weights], bias, cache.page_tokens,
+            kp.shape[0], 1 if decode else 0, splits, partial, ctx.status, self._stream()),
             "attention_masked_mma")
         return True
 
@@ -574,6 +584,13 @@ class CudaOps:
             lib.leone_mixers_set_pdl(1 if self._pdl and self._mixers_pdl else 0)
         return lib
 
+    @property
+    def mixer_calls(self):
+        calls = self.__dict__.get("_mixer_calls")
+        if calls is None:
+            calls = self.__dict__["_mixer_calls"] = EntryPoints(self.mixers)
+        return calls
+
     def rms_norm_pair(self, x, w_a, w_b, out_a, out_b, eps):
         """Two RMS norms (weights ``w_a``, ``w_b``, one eps) of the same fp32 rows in one pass."""
         n, width = out_a.shape
@@ -582,14 +599,14 @@ class CudaOps:
               and out_b.is_contiguous() and w_a.dtype == w_b.dtype and w_a.numel() == width == w_b.numel(),
               "rms_norm_pair outputs/weights")
         self.launches += 1
-        _check(self.mixers.leone_rms_norm_pair(_ptr(x), _ptr(w_a), _ptr(w_b), _dt(w_a.dtype), _ptr(out_a), _ptr(out_b),
-                                               _dt(out_a.dtype), n, width, c_float(eps), self._stream()), "rms_norm_pair")
+        _check(self.mixer_calls.leone_rms_norm_pair(x, w_a, w_b, _dt(w_a.dtype), out_a, out_b,
+                                               _dt(out_a.dtype), n, width, float(eps), self._stream()), "rms_norm_pair")
 
     def relu_squared(self, t):
         """In place: ``max(t, 0)^2``."""
         _need(t.is_contiguous(), "relu_squared needs a contiguous tensor")
         self.launches += 1
-        _check(self.mixers.leone_relu_squared(_dt(t.dtype), _ptr(t), ctypes.c_longlong(t.numel()), self._stream()),
+        _check(self.mixer_calls.leone_relu_squared(_dt(t.dtype), t, t.numel(), self._stream()),
                "relu_squared")
 
     def linear_per_head(self, a, a_head_stride, w, c, c_head_stride, heads, k, n):
@@ -601,9 +618,9 @@ class CudaOps:
         _need((heads - 1) * a_head_stride + k <= a.shape[1] and (heads - 1) * c_head_stride + n <= c.shape[1],
               "linear_per_head: heads run past a row")
         self.launches += 1
-        _check(self.mixers.leone_gemm_batched(_dt(a.dtype), _ptr(a), _ptr(w), _ptr(c), m, n, k, a.stride(0), k,
-                                              c.stride(0), ctypes.c_longlong(a_head_stride),
-                                              ctypes.c_longlong(n * k), ctypes.c_longlong(c_head_stride), heads,
+        _check(self.mixer_calls.leone_gemm_batched(_dt(a.dtype), a, w, c, m, n, k, a.stride(0), k,
+                                              c.stride(0), a_head_stride,
+                                              n * k, c_head_stride, heads,
                                               self._stream()), "linear_per_head")
 
     def linear_attention(self, ctx, proj, out, state, decay, heads, dim, vdim, q_off, k_off, v_off, chunk=0):
@@ -625,28 +642,28 @@ class CudaOps:
             lead = self._leading_single_rows(ctx)
             if lead:
                 self.launches += 1
-                _check(self.mixers.leone_linear_attention(
-                    _dt(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
-                    _ptr(ctx.q_start), _ptr(ctx.slot_ids), _ptr(decay), lead, heads, dim, vdim, state.shape[0], 0, 0,
-                    c_void_p(0), _ptr(ctx.status), self._stream()), "linear_attention")
+                _check(self.mixer_calls.leone_linear_attention(
+                    _dt(proj.dtype), proj, proj.stride(0), q_off, k_off, v_off, out, out.stride(0), state,
+                    ctx.q_start, ctx.slot_ids, decay, lead, heads, dim, vdim, state.shape[0], 0, 0,
+                    None, ctx.status, self._stream()), "linear_attention")
             chunks = [-(-int(q) // 64) for q in ctx.q_lens[lead:]]
             entries = sum(c - 1 for c in chunks if c > 1)
             if entries:
                 chunk_state = self._scratch("linattn_chunks", entries, heads * dim * vdim, torch.float32)
             self.launches += 4 if entries else 2
-            _check(self.mixers.leone_linear_attention_tiles(
-                _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
-                _ptr(ctx.q_start[lead:]), _ptr(ctx.slot_ids[lead:]), _ptr(decay), len(chunks), heads, dim, vdim, state.shape[0],
-                sum(chunks), entries, _ptr(chunk_state), _ptr(ctx.status), self._stream()), "linear_attention_tiles")
+            _check(self.mixer_calls.leone_linear_attention_tiles(
+                proj, proj.stride(0), q_off, k_off, v_off, out, out.stride(0), state,
+                ctx.q_start[lead:], ctx.slot_ids[lead:], decay, len(chunks), heads, dim, vdim, state.shape[0],
+                sum(chunks), entries, chunk_state, ctx.status, self._stream()), "linear_attention_tiles")
             return
         if chunk > 0:
             n_chunks = int(sum(-(-int(q) // chunk) for q in ctx.q_lens))
             chunk_state = self._scratch("linattn_chunks", n_chunks, heads * dim * vdim, torch.float32)
         self.launches += 1 if chunk == 0 else 3
-        _check(self.mixers.leone_linear_attention(
-            _dt(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), out.stride(0), _ptr(state),
-            _ptr(ctx.q_start), _ptr(ctx.slot_ids), _ptr(decay), ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk,
-            n_chunks, _ptr(chunk_state), _ptr(ctx.status), self._stream()), "linear_attention")
+        _check(self.mixer_calls.leone_linear_attention(
+            _dt(proj.dtype), proj, proj.stride(0), q_off, k_off, v_off, out, out.stride(0), state,
+            ctx.q_start, ctx.slot_ids, decay, ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk,
+            n_chunks, chunk_state, ctx.status, self._stream()), "linear_attention")
 
     def gated_linear_attention(self, ctx, proj, gated, state, w2, w2_bias, norm_w, heads, dim, vdim, rank, tau, q_scale,
                                eps, q_off, k_off, v_off, u_off, gate_off, chunk=0, act="silu"):
@@ -673,7 +690,7 @@ class CudaOps:
         # a head wider than a block's columns is normed and gated by a kernel of its own
         whole = vdim <= (128 if dim <= 128 else 64 if dim <= 256 else 32)
         o = None if whole else self._scratch("gla_out", n, hv, torch.float32)
-        gated_arg = _ptr(gated) if whole else c_void_p(0)
+        gated_arg = gated if whole else None
         offsets = (q_off, k_off, v_off, u_off, gate_off)
         if (self.fast is not None and gated.dtype == torch.bfloat16 and not ctx.decode_only and ctx.max_q_len >= 16
                 and os.environ.get("LEONE_NO_GLA_MMA", "0") != "1" and chunk % 16 == 0 and rank <= 512
@@ -682,22 +699,22 @@ class CudaOps:
             # prompt portions in bfloat16: 16 tokens at a time on tensor cores
             alpha = self._scratch("gla_alpha", n, heads * dim, torch.float32)
             self.launches += 2 if chunk == 0 else 4
-            _check(self.mixers.leone_gla_mma(
-                _ptr(proj), proj.stride(0), *offsets, _ptr(w2), _ptr(w2_bias), rank, c_float(1.0 / tau), c_float(q_scale),
-                _ptr(o), 0 if o is None else o.stride(0), gated_arg, gated.stride(0), _ptr(norm_w),
-                1 if act == "silu" else 0, c_float(eps), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.slot_ids), n, ctx.n_seqs,
-                heads, dim, vdim, state.shape[0], chunk, n_chunks, _ptr(chunk_state), _ptr(chunk_decay), _ptr(alpha),
-                _ptr(ctx.status), self._stream()), "gated_linear_attention (tensor cores)")
+            _check(self.mixer_calls.leone_gla_mma(
+                proj, proj.stride(0), *offsets, w2, w2_bias, rank, float(1.0 / tau), float(q_scale),
+                o, 0 if o is None else o.stride(0), gated_arg, gated.stride(0), norm_w,
+                1 if act == "silu" else 0, float(eps), state, ctx.q_start, ctx.slot_ids, n, ctx.n_seqs,
+                heads, dim, vdim, state.shape[0], chunk, n_chunks, chunk_state, chunk_decay, alpha,
+                ctx.status, self._stream()), "gated_linear_attention (tensor cores)")
             if not whole:
                 self.group_gate_norm(o, norm_w, proj[:, gate_off:gate_off + hv], gated, eps, heads, vdim, act=act)
             return
         self.launches += 1 if chunk == 0 else 3
-        _check(self.mixers.leone_gla(
-            _dt(gated.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, u_off, gate_off, _ptr(w2), _ptr(w2_bias), rank,
-            c_float(1.0 / tau), c_float(q_scale), _ptr(o), 0 if o is None else o.stride(0), gated_arg,
-            gated.stride(0), _ptr(norm_w), 1 if act == "silu" else 0, c_float(eps), _ptr(state), _ptr(ctx.q_start),
-            _ptr(ctx.slot_ids), ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk, n_chunks, _ptr(chunk_state),
-            _ptr(chunk_decay), _ptr(ctx.status), self._stream()), "gated_linear_attention")
+        _check(self.mixer_calls.leone_gla(
+            _dt(gated.dtype), proj, proj.stride(0), q_off, k_off, v_off, u_off, gate_off, w2, w2_bias, rank,
+            float(1.0 / tau), float(q_scale), o, 0 if o is None else o.stride(0), gated_arg,
+            gated.stride(0), norm_w, 1 if act == "silu" else 0, float(eps), state, ctx.q_start,
+            ctx.slot_ids, ctx.n_seqs, heads, dim, vdim, state.shape[0], chunk, n_chunks, chunk_state,
+            chunk_decay, ctx.status, self._stream()), "gated_linear_attention")
         if not whole:
             self.group_gate_norm(o, norm_w, proj[:, gate_off:gate_off + hv], gated, eps, heads, vdim, act=act)
 
@@ -708,8 +725,8 @@ class CudaOps:
               and gate.shape == o.shape and gate.stride(1) == 1 and gate.dtype == out.dtype
               and weight.numel() == width, "gate_norm layout")
         self.launches += 1
-        _check(self.mixers.leone_gate_norm(_dt(out.dtype), _ptr(o), n, width, _ptr(weight), _dt(weight.dtype), _ptr(gate),
-                                           gate.stride(0), _ptr(out), c_float(eps), self._stream()), "gate_norm")
+        _check(self.mixer_calls.leone_gate_norm(_dt(out.dtype), o, n, width, weight, _dt(weight.dtype), gate,
+                                           gate.stride(0), out, float(eps), self._stream()), "gate_norm")
 
     def latent_prepare(self, ctx, proj, q_abs, heads, dim, rot_dim, rank, norm_w, eps, freqs, magnitude, pairing,
                        cache, q_off, dkv_off):
@@ -728,15 +745,15 @@ class CudaOps:
             _need(cache.v_pool is None and kp.is_contiguous() and kp.dtype == proj.dtype and kp.shape[1] == 1
                   and kp.shape[2] == cache.page_tokens and kp.shape[3] == dk and bt.dtype == torch.int32
                   and bt.is_contiguous(), "latent cache layout")
-            pool_args = (_ptr(bt), bt.shape[1], bt.shape[0], _ptr(kp), kp.shape[0], cache.page_tokens)
+            pool_args = (bt, bt.shape[1], bt.shape[0], kp, kp.shape[0], cache.page_tokens)
         else:
-            pool_args = (c_void_p(0), 0, ctx.n_seqs, c_void_p(0), 0, 0)
+            pool_args = (None, 0, ctx.n_seqs, None, 0, 0)
         self.launches += 1
-        _check(self.mixers.leone_latent_prepare(
-            _dt(proj.dtype), _ptr(proj), proj.stride(0), q_off, dkv_off, _ptr(q_abs), n, heads, dim, rot_dim, rank,
-            _ptr(norm_w), _dt(norm_w.dtype), c_float(eps), _ptr(freqs), rot_dims, c_float(magnitude),
-            1 if pairing == "adjacent" else 0, _ptr(ctx.positions), _ptr(ctx.seq_of_token), pool_args[0],
-            pool_args[1], pool_args[2], pool_args[3], pool_args[4], pool_args[5], _ptr(ctx.status), self._stream()),
+        _check(self.mixer_calls.leone_latent_prepare(
+            _dt(proj.dtype), proj, proj.stride(0), q_off, dkv_off, q_abs, n, heads, dim, rot_dim, rank,
+            norm_w, _dt(norm_w.dtype), float(eps), freqs, rot_dims, float(magnitude),
+            1 if pairing == "adjacent" else 0, ctx.positions, ctx.seq_of_token, pool_args[0],
+            pool_args[1], pool_args[2], pool_args[3], pool_args[4], pool_args[5], ctx.status, self._stream()),
             "latent_prepare")
 
     def attention_latent(self, ctx, q_abs, out, cache, heads, dk, dv, scale, window, sink=None, gate=None):
@@ -763,18 +780,18 @@ class CudaOps:
             if splits > 1:
                 partial = self._scratch("latent_partial", n * groups * splits * 16, dv + 2, torch.float32)
                 self.launches += 1
-            _check(self.mixers.leone_attention_latent_mma(
-                _ptr(q_abs), _ptr(out), _ptr(kp), _ptr(bt), bt.shape[1], _ptr(ctx.seq_of_token), _ptr(ctx.positions),
-                n, heads, dk, dv, c_float(scale), int(window or 0), _ptr(sink), 0 if sink is None else _dt(sink.dtype),
-                _ptr(gate), 0 if gate is None else gate.stride(0), cache.page_tokens, kp.shape[0], bt.shape[0],
-                splits, _ptr(partial), 1 if os.environ.get("LEONE_NO_SHARED_KEY_TILES", "0") == "1" else 0,
-                _ptr(ctx.status), self._stream()), "attention_latent_mma")
+            _check(self.mixer_calls.leone_attention_latent_mma(
+                q_abs, out, kp, bt, bt.shape[1], ctx.seq_of_token, ctx.positions,
+                n, heads, dk, dv, float(scale), int(window or 0), sink, 0 if sink is None else _dt(sink.dtype),
+                gate, 0 if gate is None else gate.stride(0), cache.page_tokens, kp.shape[0], bt.shape[0],
+                splits, partial, 1 if os.environ.get("LEONE_NO_SHARED_KEY_TILES", "0") == "1" else 0,
+                ctx.status, self._stream()), "attention_latent_mma")
             return
-        _check(self.mixers.leone_attention_latent(
-            _dt(q_abs.dtype), _ptr(q_abs), _ptr(out), _ptr(kp), _ptr(bt), bt.shape[1], _ptr(ctx.seq_of_token),
-            _ptr(ctx.positions), n, heads, dk, dv, c_float(scale), int(window or 0), _ptr(sink),
-            0 if sink is None else _dt(sink.dtype), _ptr(gate), 0 if gate is None else gate.stride(0),
-            cache.page_tokens, kp.shape[0], bt.shape[0], _ptr(ctx.status), self._stream()), "attention_latent")
+        _check(self.mixer_calls.leone_attention_latent(
+            _dt(q_abs.dtype), q_abs, out, kp, bt, bt.shape[1], ctx.seq_of_token,
+            ctx.positions, n, heads, dk, dv, float(scale), int(window or 0), sink,
+            0 if sink is None else _dt(sink.dtype), gate, 0 if gate is None else gate.stride(0),
+            cache.page_tokens, kp.shape[0], bt.shape[0], ctx.status, self._stream()), "attention_latent")
 
     def experts_route(self, x, w_router, chosen, weight, top, softmax=False, renormalize=False, groups=1,
                       groups_kept=None, weight_scale=1.0, bias=None, experts=None, correction=None):
@@ -802,9 +819,9 @@ class CudaOps:
         self.linear(x, w_router, logits)
         self.launches += 1
         mode = 2 if softmax == "chosen" else (1 if softmax else 0)
-        _check(self.mixers.leone_experts_select(_ptr(logits), logits.stride(0), _ptr(bias), _ptr(correction), n, experts, top, mode,
+        _check(self.mixer_calls.leone_experts_select(logits, logits.stride(0), bias, correction, n, experts, top, mode,
                                                 1 if renormalize else 0, int(groups), int(groups_kept or groups),
-                                                c_float(weight_scale), _ptr(chosen), _ptr(weight), self._stream()),
+                                                float(weight_scale), chosen, weight, self._stream()),
                "experts_select")
         return logits
 
@@ -827,10 +844,10 @@ class CudaOps:
         _need(taps == 1 or (state.dtype == torch.float32 and state.is_contiguous()
                             and tuple(state.shape[1:]) == (taps - 1, channels)), "short_conv state")
         self.launches += 1
-        _check(self.mixers.leone_short_conv(
-            _dt(x.dtype), _dt(out.dtype), _ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(state), _ptr(out), out.stride(0),
-            _ptr(ctx.q_start), _ptr(ctx.seq_of_token), _ptr(ctx.slot_ids), n, channels, taps,
-            (1 if add_input else 0) | (2 if activation == "silu" else 0), 1 if update_state else 0, ctx.n_seqs, state.shape[0] if state is not None else 0, _ptr(ctx.status),
+        _check(self.mixer_calls.leone_short_conv(
+            _dt(x.dtype), _dt(out.dtype), x, x.stride(0), weight, bias, state, out, out.stride(0),
+            ctx.q_start, ctx.seq_of_token, ctx.slot_ids, n, channels, taps,
+            (1 if add_input else 0) | (2 if activation == "silu" else 0), 1 if update_state else 0, ctx.n_seqs, state.shape[0] if state is not None else 0, ctx.status,
             self._stream()), "short_conv")
 
     def short_conv_state(self, ctx, x, state):
@@ -842,9 +859,9 @@ class CudaOps:
         if keep == 0:
             return
         self.launches += 1
-        _check(self.mixers.leone_short_conv_state(
-            _dt(x.dtype), _ptr(x), x.stride(0), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.slot_ids), ctx.n_seqs,
-            channels, keep + 1, state.shape[0], _ptr(ctx.status), self._stream()), "short_conv_state")
+        _check(self.mixer_calls.leone_short_conv_state(
+            _dt(x.dtype), x, x.stride(0), state, ctx.q_start, ctx.slot_ids, ctx.n_seqs,
+            channels, keep + 1, state.shape[0], ctx.status, self._stream()), "short_conv_state")
 
     def min_gru(self, ctx, proj, z_bias, x_bias, state, out, out_scale=1.0, chunk=0):
         """``S_t = (1 - z) S_(t-1) + z c`` per channel with ``z = sigmoid(pz + bz)``, ``u = px + bx``,
@@ -856,7 +873,7 @@ class CudaOps:
               and state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] == width, "min_gru layout")
         for b in (z_bias, x_bias):
             _need(b is None or (b.dtype == torch.float32 and b.is_contiguous() and b.numel() == width), "min_gru bias")
-        n_chunks, chunk_args = 0, (c_void_p(0),) * 5
+        n_chunks, chunk_args = 0, (None,) * 5
         if chunk > 0:
             cuts = ctx.__dict__.setdefault("_token_chunks", {})      # the cut is the same for every layer of the step
             if chunk not in cuts:
@@ -869,12 +886,12 @@ class CudaOps:
                 cuts[chunk] = (len(first), torch.tensor(first + last + seq_start, dtype=torch.int32).to(self.device))
             n_chunks, meta = cuts[chunk]
             sums = self._scratch("min_gru_chunks", 2 * n_chunks, width, torch.float32)
-            chunk_args = (_ptr(meta), _ptr(meta[n_chunks:]), _ptr(meta[2 * n_chunks:]), _ptr(sums), _ptr(sums[n_chunks:]))
+            chunk_args = (meta, meta[n_chunks:], meta[2 * n_chunks:], sums, sums[n_chunks:])
         self.launches += 1 if n_chunks == 0 else 3
-        _check(self.mixers.leone_min_gru(
-            _dt(proj.dtype), _dt(out.dtype), _ptr(proj), proj.stride(0), 0, width, 2 * width, _ptr(z_bias), _ptr(x_bias),
-            _ptr(state), _ptr(out), out.stride(0), _ptr(ctx.q_start), _ptr(ctx.slot_ids), ctx.n_seqs, width,
-            state.shape[0], c_float(out_scale), n_chunks, *chunk_args, _ptr(ctx.status), self._stream()), "min_gru")
+        _check(self.mixer_calls.leone_min_gru(
+            _dt(proj.dtype), _dt(out.dtype), proj, proj.stride(0), 0, width, 2 * width, z_bias, x_bias,
+            state, out, out.stride(0), ctx.q_start, ctx.slot_ids, ctx.n_seqs, width,
+            state.shape[0], float(out_scale), n_chunks, *chunk_args, ctx.status, self._stream()), "min_gru")
 
     def scale_rows(self, a, gate, scale=1.0):
         """In place: ``a[t, :] *= scale * sigmoid(gate[t])``; ``gate``: one fp32 logit per row (a
@@ -882,8 +899,8 @@ class CudaOps:
         n, cols = a.shape
         _need(a.stride(1) == 1 and (gate is None or (gate.dtype == torch.float32 and gate.shape[0] == n)), "scale_rows layout")
         self.launches += 1
-        _check(self.mixers.leone_scale_rows(_dt(a.dtype), _ptr(a), a.stride(0), n, cols, _ptr(gate),
-                                            0 if gate is None else gate.stride(0), c_float(scale), self._stream()),
+        _check(self.mixer_calls.leone_scale_rows(_dt(a.dtype), a, a.stride(0), n, cols, gate,
+                                            0 if gate is None else gate.stride(0), float(scale), self._stream()),
                "scale_rows")
 
     def add_scaled(self, x, y, scale=1.0):
@@ -891,7 +908,7 @@ class CudaOps:
         _need(x.dtype == torch.float32 and y.dtype == torch.float32 and x.shape == y.shape and x.is_contiguous()
               and y.is_contiguous(), "add_scaled layout")
         self.launches += 1
-        _check(self.mixers.leone_add_scaled(_ptr(x), _ptr(y), ctypes.c_longlong(x.numel()), c_float(scale),
+        _check(self.mixer_calls.leone_add_scaled(x, y, x.numel(), float(scale),
                                             self._stream()), "add_scaled")
 
     def attention_pooled_prepare(self, ctx, proj, q_out, n_q, n_kv, dk, dv, conv_w, conv_state, freqs, pairing,
@@ -922,14 +939,14 @@ class CudaOps:
               and kp.shape[1] == n_kv and kp.shape[2] == cache.page_tokens and kp.shape[3] == dk and vp.shape[3] == dv
               and bt.dtype == torch.int32 and bt.is_contiguous(), "attention_pooled_prepare cache layout")
         self.launches += 1
-        _check(self.mixers.leone_attention_pooled_prepare(
-            _dt(proj.dtype), _dt(q_out.dtype), _ptr(proj), proj.stride(0), n, n_q, n_kv, dk, dv, _ptr(conv_w), taps,
-            _ptr(conv_state), 1 if (update_state and ctx.decode_only) else 0, _ptr(freqs), rot, 1 if pairing == "adjacent" else 0, c_float(magnitude),
-            1 if unit_norm else 0, c_float(eps), _ptr(q_out), q_out.stride(0), _ptr(ctx.positions),
-            _ptr(ctx.seq_of_token), _ptr(ctx.q_start), _ptr(ctx.slot_ids),
-            conv_state.shape[0] if conv_state is not None else 0, _ptr(bt), bt.shape[1], bt.shape[0],
-            _ptr(kp) if cache.writes else c_void_p(0), _ptr(vp) if cache.writes else c_void_p(0), kp.shape[0],
-            cache.page_tokens, _ptr(ctx.status), self._stream()), "attention_pooled_prepare")
+        _check(self.mixer_calls.leone_attention_pooled_prepare(
+            _dt(proj.dtype), _dt(q_out.dtype), proj, proj.stride(0), n, n_q, n_kv, dk, dv, conv_w, taps,
+            conv_state, 1 if (update_state and ctx.decode_only) else 0, freqs, rot, 1 if pairing == "adjacent" else 0, float(magnitude),
+            1 if unit_norm else 0, float(eps), q_out, q_out.stride(0), ctx.positions,
+            ctx.seq_of_token, ctx.q_start, ctx.slot_ids,
+            conv_state.shape[0] if conv_state is not None else 0, bt, bt.shape[1], bt.shape[0],
+            kp if cache.writes else None, vp if cache.writes else None, kp.shape[0],
+            cache.page_tokens, ctx.status, self._stream()), "attention_pooled_prepare")
 
     @staticmethod
     def _pooled_args(tokens, blocks, n_kv, dk, dv, pool):
@@ -942,17 +959,17 @@ class CudaOps:
               and blocks.page_tokens == tokens.page_tokens and blocks.tokens_per_row == pool
               and rows == -(-tokens.page_tokens // pool) and bt.dtype == torch.int32 and pt.dtype == torch.int32
               and bt.is_contiguous() and pt.is_contiguous() and bt.shape[0] == pt.shape[0], "pooled attention cache layout")
-        return (_ptr(kp), _ptr(vp), _ptr(bt), bt.shape[1], kp.shape[0], tokens.page_tokens,
-                _ptr(kb), _ptr(vb), _ptr(pt), pt.shape[1], kb.shape[0], rows)
+        return (kp, vp, bt, bt.shape[1], kp.shape[0], tokens.page_tokens,
+                kb, vb, pt, pt.shape[1], kb.shape[0], rows)
 
     def attention_pool_blocks(self, ctx, tokens, blocks, n_kv, dk, dv, pool):
         """Every block of ``pool`` positions that one of the step's tokens ends gets its mean key
         and mean value (over the rows as the token cache holds them) in the cache of blocks."""
         args = self._pooled_args(tokens, blocks, n_kv, dk, dv, pool)
         self.launches += 1
-        _check(self.mixers.leone_attention_pool_blocks(
-            _dt(tokens.k_pool.dtype), *args, _ptr(ctx.positions), _ptr(ctx.seq_of_token), ctx.n_tokens, ctx.n_seqs,
-            n_kv, dk, dv, pool, _ptr(ctx.status), self._stream()), "attention_pool_blocks")
+        _check(self.mixer_calls.leone_attention_pool_blocks(
+            _dt(tokens.k_pool.dtype), *args, ctx.positions, ctx.seq_of_token, ctx.n_tokens, ctx.n_seqs,
+            n_kv, dk, dv, pool, ctx.status, self._stream()), "attention_pool_blocks")
 
     def attention_pooled(self, ctx, q, out, tokens, blocks, n_q, n_kv, dk, dv, scale, window, pool, out_scale=1.0):
         """Softmax attention of every token over the last ``window`` cached keys and the mean keys
@@ -966,10 +983,10 @@ class CudaOps:
         if self.fast is not None and self.attention_pooled_tiled(ctx, q, out, args, n_q, n_kv, dk, dv, scale, window,
                                                                  pool, out_scale):
             return
-        _check(self.mixers.leone_attention_pooled(
-            _dt(q.dtype), _ptr(q), q.stride(0), _ptr(out), out.stride(0), *args, _ptr(ctx.seq_of_token),
-            _ptr(ctx.positions), n, n_q, n_kv, dk, dv, c_float(scale), int(window), int(pool), c_float(out_scale),
-            ctx.n_seqs, _ptr(ctx.status), self._stream()), "attention_pooled")
+        _check(self.mixer_calls.leone_attention_pooled(
+            _dt(q.dtype), q, q.stride(0), out, out.stride(0), *args, ctx.seq_of_token,
+            ctx.positions, n, n_q, n_kv, dk, dv, float(scale), int(window), int(pool), float(out_scale),
+            ctx.n_seqs, ctx.status, self._stream()), "attention_pooled")
 
     def attention_pooled_tiled(self, ctx, q, out, args, n_q, n_kv, dk, dv, scale, window, pool, out_scale) -> bool:
         """The tensor-core form of :meth:`attention_pooled`: the masked attention of
@@ -997,10 +1014,10 @@ class CudaOps:
                 need = int(self.mixers.leone_attention_masked_mma_scratch(ctx.n_seqs, n_kv, dv, splits))
                 partial = self._scratch("masked_partial", -(-need // 64), 64, torch.float32)
                 self.launches += 1
-        _check(self.mixers.leone_attention_pooled_mma(
-            _ptr(q), q.stride(0), _ptr(out), out.stride(0), *args, _ptr(ctx.q_start), _ptr(ctx.ctx_len), ctx.n_seqs,
-            1 if decode else int(ctx.max_q_len), n_q, n_kv, dk, dv, c_float(scale), int(window), int(pool),
-            c_float(out_scale), 1 if decode else 0, splits, _ptr(partial), _ptr(ctx.status), self._stream()),
+        _check(self.mixer_calls.leone_attention_pooled_mma(
+            q, q.stride(0), out, out.stride(0), *args, ctx.q_start, ctx.ctx_len, ctx.n_seqs,
+            1 if decode else int(ctx.max_q_len), n_q, n_kv, dk, dv, float(scale), int(window), int(pool),
+            float(out_scale), 1 if decode else 0, splits, partial, ctx.status, self._stream()),
             "attention_pooled_mma")
         return True
 
@@ -1009,7 +1026,7 @@ class CudaOps:
         """``t = 0`` (a contiguous tensor)."""
         _need(t.is_contiguous(), "zero needs a contiguous tensor")
         self.launches += 1
-        _check(self.mixers.leone_zero(_ptr(t), ctypes.c_longlong(t.numel() * t.element_size()), self._stream()), "zero")
+        _check(self.mixer_calls.leone_zero(t, t.numel() * t.element_size(), self._stream()), "zero")
 
     def rms_norm_add(self, dst, a, w_a, eps, b=None, w_b=None, coef=1.0, accumulate=True, rounded=None, then=None,
                      following=None):
@@ -1035,15 +1052,15 @@ class CudaOps:
                   and next_out.shape == dst.shape and next_out.is_contiguous(), "rms_norm_add: the norm that follows")
         side = rounded if rounded is not None else next_out
         w_b = w_b if b is not None else None
-        args = (_ptr(dst), _ptr(a), _ptr(w_a), _ptr(b), _ptr(w_b), _dt(w_a.dtype), n, width, c_float(coef), c_float(eps),
-                1 if accumulate else 0, _ptr(rounded), 0 if side is None else _dt(side.dtype), _ptr(then))
+        args = (dst, a, w_a, b, w_b, _dt(w_a.dtype), n, width, float(coef), float(eps),
+                1 if accumulate else 0, rounded, 0 if side is None else _dt(side.dtype), then)
         self.launches += 1
         if (width % 4 == 0 and width <= 8192 and (rounded is None or next_out is None or rounded.dtype == next_out.dtype)
                 and not any(t is not None and t.data_ptr() % 16 for t in (dst, a, w_a, b, w_b, rounded, then, next_w, next_out))):
-            _check(self.mixers.leone_rms_norm_add_next(*args, _ptr(next_w), c_float(next_eps), _ptr(next_out), self._stream()),
+            _check(self.mixer_calls.leone_rms_norm_add_next(*args, next_w, float(next_eps), next_out, self._stream()),
                    "rms_norm_add")
             return
-        _check(self.mixers.leone_rms_norm_add(*args, self._stream()), "rms_norm_add")
+        _check(self.mixer_calls.leone_rms_norm_add(*args, self._stream()), "rms_norm_add")
         if following is not None:
             self.rms_norm(dst, next_w, next_out, next_eps)
 
@@ -1053,7 +1070,7 @@ class CudaOps:
         _need(gate.shape == a.shape and gate.dtype == a.dtype and a.stride(1) == 1 and gate.stride(1) == 1
               and act in ("sigmoid", "silu"), "gate_rows layout")
         self.launches += 1
-        _check(self.mixers.leone_gate_rows(_dt(a.dtype), _ptr(a), a.stride(0), _ptr(gate), gate.stride(0), n, cols,
+        _check(self.mixer_calls.leone_gate_rows(_dt(a.dtype), a, a.stride(0), gate, gate.stride(0), n, cols,
                                            1 if act == "silu" else 0, self._stream()), "gate_rows")
 
     def gelu_gate(self, z, rows, offset, out):
@@ -1063,8 +1080,8 @@ class CudaOps:
               and rows.stride(1) == 1 and rows.shape[0] == n and 0 <= offset and offset + cols <= rows.shape[1]
               and out.stride(1) == 1, "gelu_gate layout")
         self.launches += 1
-        _check(self.mixers.leone_gelu_gate(_dt(out.dtype), _ptr(z), z.stride(0), _ptr(rows), rows.stride(0), int(offset),
-                                           _ptr(out), out.stride(0), n, cols, self._stream()), "gelu_gate")
+        _check(self.mixer_calls.leone_gelu_gate(_dt(out.dtype), z, z.stride(0), rows, rows.stride(0), int(offset),
+                                           out, out.stride(0), n, cols, self._stream()), "gelu_gate")
 
     def attention_mixed_heads(self, ctx, q, out, cache, n_q, n_kv, dk, dv, scale, temp, cap, mix, sink, mask, mask_size):
         """Softmax attention whose scores are mixed across heads before the softmax
@@ -1092,11 +1109,11 @@ class CudaOps:
             partial = self._scratch("mixed_heads_partial", n * splits, n_q * (dv + 2), torch.float32)
             self.launches += 1
         self.launches += 1
-        _check(self.mixers.leone_attention_mixed_heads(
-            _dt(q.dtype), _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(partial), _ptr(kp), _ptr(vp), _ptr(bt),
-            bt.shape[1], _ptr(ctx.seq_of_token), _ptr(ctx.positions), n, n_q, n_kv, dk, dv, c_float(scale), _ptr(temp),
-            c_float(cap or 0.0), _ptr(mix), _ptr(sink), self._MASKS[mask], size, cache.page_tokens, kp.shape[0],
-            bt.shape[0], splits, _ptr(ctx.status), self._stream()), "attention_mixed_heads")
+        _check(self.mixer_calls.leone_attention_mixed_heads(
+            _dt(q.dtype), q, q.stride(0), out, out.stride(0), partial, kp, vp, bt,
+            bt.shape[1], ctx.seq_of_token, ctx.positions, n, n_q, n_kv, dk, dv, float(scale), temp,
+            float(cap or 0.0), mix, sink, self._MASKS[mask], size, cache.page_tokens, kp.shape[0],
+            bt.shape[0], splits, ctx.status, self._stream()), "attention_mixed_heads")
 
     def attention_mixed_heads_tiled(self, ctx, q, out, cache, n_q, n_kv, dk, dv, scale, temp, cap, mix, sink, mask, size) -> bool:
         """The tensor-core form of :meth:`attention_mixed_heads` (``csrc/attention_mixed_heads_mma.cu``) for
@@ -1118,10 +1135,10 @@ class CudaOps:
             tiles = ctx.__dict__["_row_tiles"] = (len(rows) // 3, torch.tensor(rows, dtype=torch.int32).to(self.device))
         kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
         self.launches += 1
-        _check(self.mixers.leone_attention_mixed_heads_mma(
-            _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt), bt.shape[1], _ptr(ctx.positions),
-            _ptr(tiles[1]), tiles[0], n_q, n_kv, dk, dv, c_float(scale), _ptr(temp), c_float(cap or 0.0), _ptr(mix),
-            _ptr(sink), self._MASKS[mask], size, cache.page_tokens, kp.shape[0], bt.shape[0], _ptr(ctx.status),
+        _check(self.mixer_calls.leone_attention_mixed_heads_mma(
+            q, q.stride(0), out, out.stride(0), kp, vp, bt, bt.shape[1], ctx.positions,
+            tiles[1], tiles[0], n_q, n_kv, dk, dv, float(scale), temp, float(cap or 0.0), mix,
+            sink, self._MASKS[mask], size, cache.page_tokens, kp.shape[0], bt.shape[0], ctx.status,
             self._stream()), "attention_mixed_heads_mma")
         return True
 
@@ -1150,18 +1167,18 @@ class CudaOps:
                 groups = int(sum(-(-int(q) // 16) for q in ctx.q_lens))
                 images = self._scratch("delta_images", groups * heads, image, torch.uint8)
                 self.launches += 2
-                _check(self.mixers.leone_gated_delta_mma(
-                    _ptr(act), act.stride(0), q_off, k_off, v_off, _dt(raw.dtype), _ptr(raw), raw.stride(0), a_off, b_off,
-                    _ptr(z), 0 if z is None else z.stride(0), _ptr(a_log), _ptr(dt_bias), c_float(q_scale), _ptr(out),
-                    out.stride(0), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.slot_ids), ctx.n_seqs, heads, kv_heads, dim, vdim,
-                    state.shape[0], _ptr(images), groups, _ptr(ctx.status), self._stream()), "gated_delta (tensor cores)")
+                _check(self.mixer_calls.leone_gated_delta_mma(
+                    act, act.stride(0), q_off, k_off, v_off, _dt(raw.dtype), raw, raw.stride(0), a_off, b_off,
+                    z, 0 if z is None else z.stride(0), a_log, dt_bias, float(q_scale), out,
+                    out.stride(0), state, ctx.q_start, ctx.slot_ids, ctx.n_seqs, heads, kv_heads, dim, vdim,
+                    state.shape[0], images, groups, ctx.status, self._stream()), "gated_delta (tensor cores)")
                 return
         self.launches += 1
-        _check(self.mixers.leone_gated_delta(
-            _ptr(act), act.stride(0), q_off, k_off, v_off, _dt(raw.dtype), _ptr(raw), raw.stride(0), a_off, b_off,
-            _ptr(z), 0 if z is None else z.stride(0), _ptr(a_log), _ptr(dt_bias), c_float(q_scale), _ptr(out), out.stride(0), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.slot_ids),
+        _check(self.mixer_calls.leone_gated_delta(
+            act, act.stride(0), q_off, k_off, v_off, _dt(raw.dtype), raw, raw.stride(0), a_off, b_off,
+            z, 0 if z is None else z.stride(0), a_log, dt_bias, float(q_scale), out, out.stride(0), state, ctx.q_start, ctx.slot_ids,
             ctx.n_seqs, heads, kv_heads, dim, vdim, state.shape[0],
-            1 if ctx.decode_only else 0, _ptr(ctx.status), self._stream()), "gated_delta")
+            1 if ctx.decode_only else 0, ctx.status, self._stream()), "gated_delta")
 
     def group_gate_norm(self, o, weight, gate, out, eps, heads, vdim, act="sigmoid"):
         """``out[t, h, :] = rms_norm(o[t, h, :]) * weight * act(gate[t, h, :])``: every head normed on its own,
@@ -1173,9 +1190,9 @@ class CudaOps:
         _need(gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == o.shape),
               "group_gate_norm gate")
         self.launches += 1
-        _check(self.mixers.leone_group_gate_norm(
-            _dt(out.dtype), _ptr(o), o.stride(0), n, heads, vdim, _ptr(weight), _dt(weight.dtype), _ptr(gate),
-            0 if gate is None else gate.stride(0), 1 if act == "silu" else 0, _ptr(out), out.stride(0), c_float(eps),
+        _check(self.mixer_calls.leone_group_gate_norm(
+            _dt(out.dtype), o, o.stride(0), n, heads, vdim, weight, _dt(weight.dtype), gate,
+            0 if gate is None else gate.stride(0), 1 if act == "silu" else 0, out, out.stride(0), float(eps),
             self._stream()), "group_gate_norm")
 
     def ssd(self, ctx, act, raw, out, state, a_log, dt_bias, d_skip, heads, groups, n_state, vdim, x_off, b_off, c_off, dt_off,
@@ -1204,18 +1221,18 @@ class CudaOps:
                 chunk_state = self._scratch("ssd_chunk_state", n_chunks, heads * n_state * vdim, torch.float32)
                 chunk_decay = self._scratch("ssd_chunk_decay", n_chunks, heads * n_state, torch.float32)
             self.launches += 1 if chunk == 0 else 3
-            _check(self.mixers.leone_ssd_mma(
-                _ptr(act), act.stride(0), x_off, b_off, c_off, _ptr(raw), raw.stride(0), dt_off, _ptr(a_log), _ptr(dt_bias),
-                _ptr(d_skip), _ptr(out), out.stride(0), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.slot_ids), ctx.n_seqs, heads,
-                groups, n_state, vdim, state.shape[0], chunk, n_chunks, _ptr(chunk_state), _ptr(chunk_decay),
-                _ptr(ctx.status), self._stream()), "ssd (tensor cores)")
+            _check(self.mixer_calls.leone_ssd_mma(
+                act, act.stride(0), x_off, b_off, c_off, raw, raw.stride(0), dt_off, a_log, dt_bias,
+                d_skip, out, out.stride(0), state, ctx.q_start, ctx.slot_ids, ctx.n_seqs, heads,
+                groups, n_state, vdim, state.shape[0], chunk, n_chunks, chunk_state, chunk_decay,
+                ctx.status, self._stream()), "ssd (tensor cores)")
             return
         self.launches += 1
-        _check(self.mixers.leone_ssd(
-            _dt(act.dtype), _ptr(act), act.stride(0), x_off, b_off, c_off, _dt(raw.dtype), _ptr(raw), raw.stride(0), dt_off,
-            _ptr(a_log), _ptr(dt_bias), _ptr(d_skip), _ptr(out), out.stride(0), _ptr(state), _ptr(ctx.q_start),
-            _ptr(ctx.slot_ids), ctx.n_seqs, heads, groups, n_state, vdim, state.shape[0],
-            1 if ctx.decode_only else 0, _ptr(ctx.status), self._stream()),
+        _check(self.mixer_calls.leone_ssd(
+            _dt(act.dtype), act, act.stride(0), x_off, b_off, c_off, _dt(raw.dtype), raw, raw.stride(0), dt_off,
+            a_log, dt_bias, d_skip, out, out.stride(0), state, ctx.q_start,
+            ctx.slot_ids, ctx.n_seqs, heads, groups, n_state, vdim, state.shape[0],
+            1 if ctx.decode_only else 0, ctx.status, self._stream()),
             "ssd")
 
     def grouped_gate_norm(self, y, z, weight, out, eps, groups):
@@ -1226,9 +1243,9 @@ class CudaOps:
               and out.shape == y.shape and out.stride(1) == 1 and width % groups == 0 and weight.dtype == torch.float32
               and weight.numel() == width and weight.is_contiguous(), "grouped_gate_norm layout")
         self.launches += 1
-        _check(self.mixers.leone_grouped_gate_norm(
-            _dt(out.dtype), _ptr(y), y.stride(0), _dt(z.dtype), _ptr(z), z.stride(0), _ptr(weight), _ptr(out), out.stride(0),
-            n, groups, width // groups, c_float(eps), self._stream()), "grouped_gate_norm")
+        _check(self.mixer_calls.leone_grouped_gate_norm(
+            _dt(out.dtype), y, y.stride(0), _dt(z.dtype), z, z.stride(0), weight, out, out.stride(0),
+            n, groups, width // groups, float(eps), self._stream()), "grouped_gate_norm")
 
     def experts_forward(self, x, w_gate, w_up, w_down, chosen, weight, top, scale_input, hidden, rt, identity=0,
                         fresh=False):
@@ -1252,14 +1269,14 @@ class CudaOps:
         pair_out = rt.flat_buffer("experts_pair_out", pairs * width, torch.float32, reserve=cap * width)
         tensor_cores = 0 if os.environ.get("LEONE_NO_EXPERT_MMA", "0") == "1" else 1
         # grouping, two products, the sum over a token's experts; on tcgen05 the rows are sorted first
-        self.launches += 4 + self.mixers.leone_experts_on_tcgen05(
-            _dt(x.dtype), _ptr(x), x.stride(0), _ptr(w_gate), _ptr(w_up), _ptr(w_down), n, width, ff, experts, top, _ptr(act),
-            _ptr(pair_out), tensor_cores)
-        _check(self.mixers.leone_experts_forward(
-            _dt(x.dtype), _ptr(x), x.stride(0), _ptr(w_gate), _ptr(w_up), _ptr(w_down), _ptr(chosen), _ptr(weight), n,
-            width, ff, experts, top, 1 if scale_input else 0, _ptr(offsets), _ptr(order), _ptr(act), _ptr(pair_out),
-            _ptr(hidden), tensor_cores, int(identity),
-            1 if fresh else 0, _ptr(self.status), self._stream()), "experts_forward")
+        self.launches += 4 + self.mixer_calls.leone_experts_on_tcgen05(
+            _dt(x.dtype), x, x.stride(0), w_gate, w_up, w_down, n, width, ff, experts, top, act,
+            pair_out, tensor_cores)
+        _check(self.mixer_calls.leone_experts_forward(
+            _dt(x.dtype), x, x.stride(0), w_gate, w_up, w_down, chosen, weight, n,
+            width, ff, experts, top, 1 if scale_input else 0, offsets, order, act, pair_out,
+            hidden, tensor_cores, int(identity),
+            1 if fresh else 0, self.status, self._stream()), "experts_forward")
 
     def sample(self, logits, temperature, seeds, positions, out):
         rows, vocab = logits.shape
@@ -1269,8 +1286,8 @@ class CudaOps:
         _need(temperature.numel() >= rows and seeds.numel() >= rows and positions.numel() >= rows
               and out.numel() >= rows, "sample argument lengths")
         self.launches += 1
-        _check(self.core.leone_sample(_ptr(logits), rows, vocab, _ptr(temperature), _ptr(seeds),
-                                      _ptr(positions), _ptr(out), self._stream()), "sample")
+        _check(self.core_calls.leone_sample(logits, rows, vocab, temperature, seeds,
+                                      positions, out, self._stream()), "sample")
 
     def sample_slots(self, logits, slot_ids, records, out):
         """One token per row with the row's temperature, seed and position taken from the slot
@@ -1282,7 +1299,7 @@ class CudaOps:
               and records.is_contiguous() and records.shape[1] == 8 and out.dtype == torch.int32
               and out.numel() >= rows, "sample_slots arguments")
         self.launches += 1
-        _check(self.core.leone_sample_slots(_ptr(logits), rows, vocab, _ptr(slot_ids), _ptr(records), _ptr(out),
+        _check(self.core_calls.leone_sample_slots(logits, rows, vocab, slot_ids, records, out,
                                             self._stream()), "sample_slots")
 
     def penalize(self, logits, entries, penalties):
@@ -1299,9 +1316,9 @@ class CudaOps:
         per_row = torch.tensor([[p.repetition for p in penalties], [p.presence for p in penalties],
                                 [p.frequency for p in penalties]], dtype=torch.float64, device=dev)
         self.launches += 1
-        _check(self.core.leone_penalize(_ptr(logits), vocab, len(entries), _ptr(ints[0]), _ptr(ints[1]),
-                                        _ptr(ints[2]), _ptr(dry), _ptr(per_row[0]), _ptr(per_row[1]),
-                                        _ptr(per_row[2]), self._stream()), "penalize")
+        _check(self.core_calls.leone_penalize(logits, vocab, len(entries), ints[0], ints[1],
+                                        ints[2], dry, per_row[0], per_row[1],
+                                        per_row[2], self._stream()), "penalize")
 
     def sample_truncated(self, logits, temperatures, seeds, positions, stages, want_probs: bool = False,
                          maximum_surprise=None, rows=None, out=None):
@@ -1326,35 +1343,44 @@ class CudaOps:
         if self._sample_scratch is None or self._sample_scratch.numel() < need:
             self._sample_scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
         dev = self.device
-        t = torch.tensor(temperatures, dtype=torch.float64, device=dev)
-        sd = torch.tensor(np.array([s_ & 0xFFFF_FFFF_FFFF_FFFF for s_ in seeds], dtype=np.uint64).view(np.int64),
-                          device=dev)
-        pos = torch.tensor(positions, dtype=torch.int64, device=dev)
-        row_map = None if rows is None else torch.tensor(members, dtype=torch.int32, device=dev)
         if out is None:
             out = torch.empty(n_rows, dtype=torch.int32, device=dev)
         _need(out.dtype == torch.int32 and out.numel() >= n_rows and out.is_contiguous(), "out: int32, a place per logits row")
         probs = torch.empty((count, vocab), dtype=torch.float64, device=dev) if want_probs else None
-        mu = chosen = None
+        _need(maximum_surprise is None or len(maximum_surprise) == count, "one maximum surprise a row")
+        chosen = None if maximum_surprise is None else torch.zeros(count, dtype=torch.float64, device=dev)
+        # the rows' arguments go over in one copy: temperature and maximum surprise as fp64, seed and position as int64, row number
+        # (torch's caches of pinned and device memory know which stream uses what)
+        host = torch.empty(5 * count, dtype=torch.int64, pin_memory=True)
+        words, floats = host.numpy(), host.view(torch.float64).numpy()
+        floats[:count] = temperatures
+        words[count:2 * count] = np.array([s_ & 0xFFFF_FFFF_FFFF_FFFF for s_ in seeds], dtype=np.uint64).view(np.int64)
+        words[2 * count:3 * count] = positions
         if maximum_surprise is not None:
-            _need(len(maximum_surprise) == count, "one maximum surprise a row")
-            mu = torch.tensor([float(m) for m in maximum_surprise], dtype=torch.float64, device=dev)
-            chosen = torch.zeros(count, dtype=torch.float64, device=dev)
+            floats[3 * count:4 * count] = maximum_surprise
+        words[4 * count:].view(np.int32)[:count] = members
+        args = host.to(dev, non_blocking=True)
+        t, sd, pos, mu, row_map = (args.data_ptr() + 8 * count * i for i in range(5))
+        if maximum_surprise is None:
+            mu = None
+        if rows is None:
+            row_map = None
         n = len(stages)
         types = (ctypes.c_int * max(n, 1))(*[int(a) for a, _ in stages])
         values = (ctypes.c_double * max(n, 1))(*[float(b) for _, b in stages])
         self.launches += 1
-        _check(self.core.leone_sample_truncated(_ptr(logits), count, vocab, _ptr(t), _ptr(sd), _ptr(pos), n,
-                                                types, values, _ptr(self._sample_scratch), _ptr(out),
-                                                _ptr(probs), _ptr(mu), _ptr(chosen), _ptr(row_map), self._stream()),
+        _check(self.core_calls.leone_sample_truncated(logits, count, vocab, t, sd, pos, n,
+                                                ctypes.addressof(types), ctypes.addressof(values), self._sample_scratch, out,
+                                                probs, mu, chosen, row_map, self._stream()),
                "sample_truncated")
-        result = (out,) + ((probs,) if want_probs else ()) + ((chosen,) if mu is not None else ())
+        result = (out,) + ((probs,) if want_probs else ()) + ((chosen,) if chosen is not None else ())
         return result if len(result) > 1 else out
 
     def decode_advance(self, token_ids, positions, ctx_len, sample_pos, sampled, history, counter,
-                       slot_ids=None, records=None):
+                       slot_ids=None, records=None, status_out=None):
         """Feeds the sampled ids back as the next step's inputs.  Either ``sample_pos`` (int64 per
-        row) is advanced, or, with ``slot_ids`` and ``records``, each request's slot record."""
+        row) is advanced, or, with ``slot_ids`` and ``records``, each request's slot record.
+        ``status_out``: int32 [4], gets the status word as the step left it."""
         n = token_ids.numel()
         _need(history.dtype == torch.int32 and history.shape[1] == n and counter.dtype == torch.int32,
               "decode_advance arguments")
@@ -1364,8 +1390,8 @@ class CudaOps:
         else:
             _need(sample_pos is not None and sample_pos.dtype == torch.int64, "decode_advance: sample positions")
         self.launches += 1
-        _check(self.core.leone_decode_advance(_ptr(token_ids), _ptr(positions), _ptr(ctx_len),
-                                              _ptr(sample_pos), _ptr(sampled), _ptr(history),
-                                              _ptr(counter), n, history.shape[0], _ptr(slot_ids), _ptr(records),
-                                              self._stream()),
+        _check(self.core_calls.leone_decode_advance(token_ids, positions, ctx_len,
+                                              sample_pos, sampled, history,
+                                              counter, n, history.shape[0], slot_ids, records,
+                                              None if status_out is None else self.status, status_out, self._stream()),
                "decode_advance")

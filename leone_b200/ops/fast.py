@@ -8,21 +8,30 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_longlong, c_void_p, byref
+from ctypes import addressof, byref, c_float, c_int, c_longlong
 
 import torch
 
 from ..csrc.build import ensure_built
+from .entry_points import EntryPoints
 
 
-def _ptr(t):
-    return c_void_p(0 if t is None else t.data_ptr())
+def leading_ones(ctx, q_lens) -> int:
+    """How many of a step's first sequences bring one token; counted once a step (a context is made for one step)."""
+    n = getattr(ctx, "leading_ones", None)
+    if n is None:
+        n = 0
+        while n < len(q_lens) and q_lens[n] == 1:
+            n += 1
+        ctx.leading_ones = n
+    return n
 
 
 class FastKernels:
     def __init__(self, device):
         self.device = torch.device(device)
         self.lib = ctypes.CDLL(ensure_built("bf16"))
+        self.calls = EntryPoints(self.lib)
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self._configure()
         self.lib.leone_attention_decode_scratch.restype = ctypes.c_longlong
@@ -85,7 +94,7 @@ class FastKernels:
     def _stream(self):
         if self._pinned_stream is not None:        # (a handle of 0, the default stream, is a valid pin)
             return self._pinned_stream
-        return c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     def pin_stream(self, handle) -> None:
         """The stream every launch goes to until ``pin_stream(None)``: a step looks its stream up
@@ -158,13 +167,6 @@ class FastKernels:
             return 1, tiles, False
         s = min(sms // rem, k_blocks // 12, 8)
         return (s, tiles - rem, False) if s > 1 else (1, tiles, False)
-
-    def _tc_ok(self, x, w, out) -> bool:
-        if not self.use_tensor_cores or x.dtype != torch.bfloat16:
-            return False
-        k = x.shape[1]
-        return (k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
-                and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def token_major(self, m: int, n: int) -> bool:
         """Which form of the product runs: tokens on the MMA's 128-row side and 256 weight rows
@@ -299,6 +301,26 @@ class FastKernels:
         plan = self._plans.get(key)
         if plan is None:
             plan = self._plans[key] = self._plan_gemm(*key)
+        return self._launch_gemm(plan, x, x.stride(0), w, w.stride(0), out, out.stride(0), epilogue, residual, m, n_rows, k, norm_in,
+                                 norm_out, gate_shape, bias)
+
+    def _product(self, x, w, out, epilogue, residual, norm_in, norm_out, gate_shape=None) -> bool:
+        """A product with a prepared matrix in the form that the rules choose; False if it cannot run on tensor cores."""
+        weight = w.weight
+        m, k = x.shape
+        ldx, ldw = x.stride(0), weight.stride(0)
+        if not self.use_tensor_cores or x.dtype != torch.bfloat16 or (k | ldx | ldw) & 7 or (x.data_ptr() | weight.data_ptr()) & 15:
+            return False
+        n_rows = w.out_features
+        key = (m, n_rows, k, epilogue, norm_in is not None, norm_out is not None)
+        plan = self._plans.get(key)
+        if plan is None:
+            plan = self._plans[key] = self._plan_gemm(m, n_rows, k, epilogue, None, 0, False, None, norm_in is not None,
+                                                      norm_out is not None)
+        return self._launch_gemm(plan, x, ldx, weight, ldw, out, out.stride(0), epilogue, residual, m, n_rows, k, norm_in, norm_out,
+                                 gate_shape, w.bias)
+
+    def _launch_gemm(self, plan, x, ldx, w, ldw, out, ldc, epilogue, residual, m, n_rows, k, norm_in, norm_out, gate_shape, bias) -> bool:
         pairs, token_major, splits, full_tiles, cluster, ws_floats, ws_counters, parts, width = plan
         ws = ct = None
         if ws_floats or ws_counters:
@@ -308,22 +330,23 @@ class FastKernels:
         if norm_out is not None and norm_out[2].shape[0] != parts:
             raise ValueError(f"the sums of squares have {norm_out[2].shape[0]} parts, this product leaves {parts}")
         no = (None, None, None, 0) if norm_out is None else \
-            (_ptr(norm_out[0]), _ptr(norm_out[1]), _ptr(norm_out[2]), norm_out[0].stride(0))
-        ni = (None, 0, c_float(0.0)) if norm_in is None else (_ptr(norm_in[0]), int(norm_in[1]), c_float(norm_in[2]))
+            (norm_out[0], norm_out[1], norm_out[2], norm_out[0].stride(0))
+        ni = (None, 0, 0.0) if norm_in is None else (norm_in[0], int(norm_in[1]), float(norm_in[2]))
         # the gate's shape of the gated epilogue: four host floats, or null for SwiGLU
-        gs = None if gate_shape is None else (c_float * 4)(*[float(v) for v in gate_shape])
+        shape = None if gate_shape is None else (c_float * 4)(*[float(v) for v in gate_shape])
+        gs = None if shape is None else addressof(shape)
         if pairs:
             # pairs of SMs on tiles of 256 tokens (gemm_pair.cu)
-            code = self.lib.leone_gemm_pair(_ptr(x), _ptr(w), _ptr(out), _ptr(residual), m, n_rows, k,
-                                            x.stride(0), w.stride(0), out.stride(0), epilogue, width, splits, _ptr(ws),
-                                            _ptr(self.status), self.sm_count, *no, *ni, gs, _ptr(bias), self._stream())
+            code = self.calls.leone_gemm_pair(x, w, out, residual, m, n_rows, k,
+                                            ldx, ldw, ldc, epilogue, width, splits, ws,
+                                            self.status, self.sm_count, *no, *ni, gs, bias, self._stream())
             if code != 0:
                 raise RuntimeError(f"gemm_pair refused or failed with code {code} for m={m} n={n_rows} k={k}")
             return True
-        code = self.lib.leone_gemm_tc(_ptr(x), _ptr(w), _ptr(out), _ptr(residual), m, n_rows, k,
-                                      x.stride(0), w.stride(0), out.stride(0), epilogue, splits,
-                                      full_tiles, _ptr(ws), _ptr(ct), _ptr(self.status), self.sm_count,
-                                      1 if cluster else 0, 1 if token_major else 0, *no, *ni, gs, _ptr(bias), self._stream())
+        code = self.calls.leone_gemm_tc(x, w, out, residual, m, n_rows, k,
+                                      ldx, ldw, ldc, epilogue, splits,
+                                      full_tiles, ws, ct, self.status, self.sm_count,
+                                      1 if cluster else 0, 1 if token_major else 0, *no, *ni, gs, bias, self._stream())
         if code != 0:
             raise RuntimeError(f"gemm_tc refused or failed with code {code} for m={m} n={n_rows} k={k} "
                                f"splits={splits} cluster={cluster} token_major={token_major}")
@@ -387,10 +410,7 @@ class FastKernels:
         return int(self.lib.leone_gemm_tc_norm_parts(m, n))
 
     def linear(self, x, w, out, epilogue, residual, norm_in=None, norm_out=None) -> bool:
-        if not self._tc_ok(x, w.weight, out):
-            return False
-        return self._gemm(x, w.weight, out, epilogue, residual, w.out_features, norm_in=norm_in, norm_out=norm_out,
-                          bias=w.bias)
+        return self._product(x, w, out, epilogue, residual, norm_in, norm_out)
 
     # -- gate/up --------------------------------------------------------------------------
     def prepare_gate_up(self, gate, up, gate_bias=None, up_bias=None):
@@ -412,10 +432,9 @@ class FastKernels:
         return m
 
     def linear_swiglu(self, x, w, out, norm_in=None, gate_shape=None) -> bool:
-        if getattr(w, "gate_up_layout", None) != "interleaved16" or not self._tc_ok(x, w.weight, out):
+        if getattr(w, "gate_up_layout", None) != "interleaved16":
             return False
-        return self._gemm(x, w.weight, out, 3, None, w.out_features, norm_in=norm_in, gate_shape=gate_shape,
-                          bias=w.bias)
+        return self._product(x, w, out, 3, None, norm_in, None, gate_shape)
 
     # -- attention ------------------------------------------------------------------------
     def decode_splits(self, n_seqs: int, n_kv: int, g: int, max_ctx: int) -> int:
@@ -489,9 +508,7 @@ class FastKernels:
         q_lens = getattr(ctx, "q_lens", None)
         if ctx.decode_only or getattr(ctx, "fixed_shapes", False) or q_lens is None or not self.divide_mixed_steps:
             return 0
-        n = 0
-        while n < len(q_lens) and q_lens[n] == 1:
-            n += 1
+        n = leading_ones(ctx, q_lens)
         return n if self.mixed_decode_rows_from <= n < len(q_lens) else 0
 
     def attention(self, ctx, qkv, out, n_q, n_kv, d, scale, window, cache, fuse=None) -> bool:
@@ -509,33 +526,34 @@ class FastKernels:
         if n_dec:
             self._attention_decode(*args, ctx.q_start[:n_dec + 1], ctx.ctx_len[:n_dec], bt[:n_dec], n_dec,
                                    int(ctx.ctx_lens[:n_dec].max()), ctx.status, None, getattr(ctx, "seq_order", None))
-        self._attention_prompt(*args, ctx.q_start[n_dec:], ctx.ctx_len[n_dec:], bt[n_dec:], ctx.n_seqs - n_dec,
-                               int(ctx.q_lens[n_dec:].max()) if n_dec else ctx.max_q_len, ctx.status)
+            self._attention_prompt(*args, ctx.q_start[n_dec:], ctx.ctx_len[n_dec:], bt[n_dec:], ctx.n_seqs - n_dec,
+                                   int(ctx.q_lens[n_dec:].max()), ctx.status)
+        else:
+            self._attention_prompt(*args, ctx.q_start, ctx.ctx_len, bt, ctx.n_seqs, ctx.max_q_len, ctx.status)
         return True
 
     def _attention_decode(self, qkv, out, n_q, n_kv, d, scale, window, cache, q_start, ctx_len, bt, n_seqs,
                           max_ctx, status, fuse, order=None) -> None:
         """Sequences with one query token each (row ``q_start[s]``); ``order``: these sequences, the longest first."""
-        from ctypes import c_float
         if order is not None and order.numel() != n_seqs:
             raise ValueError(f"an order of {order.numel()} sequences for {n_seqs}")
         g = n_q // n_kv
         kp, vp = cache.k_pool, cache.v_pool
-        common = (_ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt),
-                  bt.stride(0), _ptr(q_start), _ptr(ctx_len), n_seqs)
+        common = (qkv, qkv.stride(0), out, out.stride(0), kp, vp, bt,
+                  bt.stride(0), q_start, ctx_len, n_seqs)
         splits = self.decode_splits(n_seqs, n_kv, g, max_ctx)
         if self.decode_in_clusters(n_seqs, n_kv, g, max_ctx):
             # the splits of a (sequence, KV head) merge inside a cluster; optionally the
             # kernel norms and rotates q and the new k and writes the cache itself
-            fz = (0, None, None, c_float(0.0), None, 0, 0, 0)
+            fz = (0, None, None, 0.0, None, 0, 0, 0)
             if fuse is not None:
                 rope = fuse["rope"]
-                fz = (1, _ptr(fuse["q_w"]), _ptr(fuse["k_w"]), c_float(fuse["eps"]), _ptr(rope),
+                fz = (1, fuse["q_w"], fuse["k_w"], float(fuse["eps"]), rope,
                       rope.shape[0] if rope is not None else 0, 1 if fuse["write_cache"] else 0,
                       1 if fuse.get("pairing", "half_split") == "adjacent" else 0)
-            code = self.lib.leone_attention_decode_cluster_ordered(
-                *common, n_q, n_kv, d, c_float(scale), int(window or 0), cache.page_tokens,
-                kp.shape[0], splits, *fz, _ptr(order), _ptr(status), self._stream())
+            code = self.calls.leone_attention_decode_cluster_ordered(
+                *common, n_q, n_kv, d, float(scale), int(window or 0), cache.page_tokens,
+                kp.shape[0], splits, *fz, order, status, self._stream())
         else:
             if fuse is not None:
                 raise RuntimeError("fused decode attention asked for where decode_fusable() is false")
@@ -543,25 +561,23 @@ class FastKernels:
             if splits > 1:
                 need = self.lib.leone_attention_decode_scratch(n_seqs, n_q, d, splits)
                 scratch = self._attn_scratch(need)
-            code = self.lib.leone_attention_decode(
-                *common, n_q, n_kv, d, c_float(scale), int(window or 0), cache.page_tokens,
-                kp.shape[0], splits, _ptr(scratch), _ptr(status), self._stream())
+            code = self.calls.leone_attention_decode(
+                *common, n_q, n_kv, d, float(scale), int(window or 0), cache.page_tokens,
+                kp.shape[0], splits, scratch, status, self._stream())
         if code != 0:
             raise RuntimeError(f"decode attention refused or failed with code {code}")
 
     def _attention_prompt(self, qkv, out, n_q, n_kv, d, scale, window, cache, q_start, ctx_len, bt, n_seqs,
                           max_q_len, status) -> None:
         """Sequences with any number of query tokens (rows ``q_start[s] .. q_start[s + 1]``)."""
-        from ctypes import c_float
         g = n_q // n_kv
         kp, vp = cache.k_pool, cache.v_pool
         # head sizes 64 and 128 run on tcgen05; the others on the mma.sync kernel
-        tc = self.use_tc_attention and d in (64, 128) and g <= 128 and out.stride(0) % 8 == 0
-        entry = self.lib.leone_attention_prefill_pingpong if tc else self.lib.leone_attention_prefill
-        code = entry(_ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt),
-                     bt.stride(0), _ptr(q_start), _ptr(ctx_len), n_seqs, max_q_len, n_q, n_kv, d,
-                     c_float(scale), int(window or 0), cache.page_tokens, kp.shape[0], _ptr(status),
-                     self._stream())
+        ldo = out.stride(0)
+        tc = self.use_tc_attention and d in (64, 128) and g <= 128 and ldo % 8 == 0
+        entry = self.calls.leone_attention_prefill_pingpong if tc else self.calls.leone_attention_prefill
+        code = entry(qkv, qkv.stride(0), out, ldo, kp, vp, bt, bt.stride(0), q_start, ctx_len, n_seqs, max_q_len, n_q, n_kv, d,
+                     float(scale), int(window or 0), cache.page_tokens, kp.shape[0], status, self._stream())
         if code != 0:
             raise RuntimeError(f"prompt attention refused or failed with code {code}")
 
@@ -575,11 +591,11 @@ class FastKernels:
                 and d in (64, 128) and g <= 128 and out.stride(0) % 8 == 0 and not ctx.decode_only):
             return False
         kp, vp, bt = cache.k_pool, cache.v_pool, cache.block_table
-        code = self.lib.leone_attention_prefill_pingpong_rules(
-            _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(kp), _ptr(vp), _ptr(bt), bt.stride(0),
-            _ptr(ctx.q_start), _ptr(ctx.ctx_len), ctx.n_seqs, ctx.max_q_len, n_q, n_kv, d, c_float(scale),
-            int(window or 0), int(weights), int(chunk or 0), _ptr(bias), cache.page_tokens, kp.shape[0],
-            _ptr(ctx.status), self._stream())
+        code = self.calls.leone_attention_prefill_pingpong_rules(
+            qkv, qkv.stride(0), out, out.stride(0), kp, vp, bt, bt.stride(0),
+            ctx.q_start, ctx.ctx_len, ctx.n_seqs, ctx.max_q_len, n_q, n_kv, d, float(scale),
+            int(window or 0), int(weights), int(chunk or 0), bias, cache.page_tokens, kp.shape[0],
+            ctx.status, self._stream())
         if code != 0:
             raise RuntimeError(f"prompt attention refused or failed with code {code}")
         return True
@@ -595,10 +611,10 @@ class FastKernels:
                 and not ctx.decode_only):
             return False
         kp, vp, bt, bt_width, pages, page_tokens, kb, vb, pt, pt_width, pool_pages, rows = args
-        code = self.lib.leone_attention_prefill_pingpong_pooled(
-            _ptr(q), q.stride(0), _ptr(out), out.stride(0), kp, vp, bt, bt_width, pages, page_tokens, kb, vb, pt, pt_width,
-            pool_pages, rows, _ptr(ctx.q_start), _ptr(ctx.ctx_len), ctx.n_seqs, int(ctx.max_q_len), n_q, n_kv, d,
-            c_float(scale), int(window), int(pool), c_float(out_scale), _ptr(ctx.status), self._stream())
+        code = self.calls.leone_attention_prefill_pingpong_pooled(
+            q, q.stride(0), out, out.stride(0), kp, vp, bt, bt_width, pages, page_tokens, kb, vb, pt, pt_width,
+            pool_pages, rows, ctx.q_start, ctx.ctx_len, ctx.n_seqs, int(ctx.max_q_len), n_q, n_kv, d,
+            float(scale), int(window), int(pool), float(out_scale), ctx.status, self._stream())
         if code != 0:
             raise RuntimeError(f"prompt attention with pooled blocks refused or failed with code {code}")
         return True

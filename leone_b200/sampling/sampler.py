@@ -236,16 +236,15 @@ class Sampler:
                                                     for p in params])
         if rows > self._cap:
             self._grow(max(rows, 2 * self._cap))
-        host = self._host.numpy()
-        temps = np.array([p.temperature for p in params], dtype=np.float32)
-        host_f = self._host[:self._cap].view(torch.float32).numpy()      # first `cap` int64 = 2*cap floats
-        host_f[:rows] = temps
-        host[self._cap:self._cap + rows] = np.array([p.seed & 0xFFFF_FFFF_FFFF_FFFF for p in params],
-                                                    dtype=np.uint64).view(np.int64)
-        host[2 * self._cap:2 * self._cap + rows] = np.asarray(positions, dtype=np.int64)
         out = self._out[:rows]
         # rows without stages and without Mirostat; where there are none the plain kernel has nothing to draw
         if not all(p.temperature > 0 and (p.truncations or p.mirostat) for p in params):
+            host = self._host.numpy()
+            host_f = self._host[:self._cap].view(torch.float32).numpy()      # first `cap` int64 = 2*cap floats
+            host_f[:rows] = np.array([p.temperature for p in params], dtype=np.float32)
+            host[self._cap:self._cap + rows] = np.array([p.seed & 0xFFFF_FFFF_FFFF_FFFF for p in params],
+                                                        dtype=np.uint64).view(np.int64)
+            host[2 * self._cap:2 * self._cap + rows] = np.asarray(positions, dtype=np.int64)
             self._dev.copy_(self._host, non_blocking=True)
             t = self._dev[:self._cap].view(torch.float32)[:rows]
             seeds = self._dev[self._cap:self._cap + rows]
