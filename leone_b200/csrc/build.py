@@ -37,7 +37,7 @@ MODULES: Dict[str, List[str]] = {
     # of mask and weight rule, routed experts, short convolutions with state, the minGRU recurrence, attention
     # over a window of tokens and pooled blocks before it, attention whose scores are mixed across heads, the gated
     # delta rule, gated linear attention with a decay per key channel, the Mamba-2 recurrence
-    "mixers": ["linear_attention.cu", "linear_attention_tiles.cu", "attention_latent.cu", "attention_latent_mma.cu", "attention_masked.cu",
+    "mixers": ["linear_attention.cu", "linear_attention_tiles.cu", "attention_latent.cu", "attention_latent_mma.cu", "attention_latent_tc.cu", "attention_masked.cu",
                "attention_masked_mma.cu", "experts.cu", "experts_tc.cu", "norm_act.cu", "short_conv.cu", "attention_pooled.cu",
                "attention_mixed_heads.cu", "attention_mixed_heads_mma.cu", "gated_delta.cu", "gated_delta_mma.cu",
                "gated_linear_attention.cu", "gated_linear_attention_mma.cu", "ssd.cu", "ssd_mma.cu"],

@@ -102,6 +102,7 @@ class CudaOps:
             from .fast import FastKernels
             self.fast = FastKernels(self.device)
         self.launches = 0
+        self.latent_tc_from = 8            # tokens of a portion from which latent attention runs on tcgen05
         self._sample_scratch = None
         self.status = None
         # LEONE_NO_PDL=1 launches every kernel fully serialised after its predecessor
@@ -769,12 +770,31 @@ class CudaOps:
                   "attention_latent gate")
         if sink is not None:
             _need(sink.numel() == heads and sink.is_contiguous(), "attention_latent sink")
+        q_start = getattr(ctx, "q_start", None)
+        if (q_abs.dtype == torch.bfloat16 and not ctx.decode_only and q_start is not None and ctx.max_q_len >= self.latent_tc_from
+                and os.environ.get("LEONE_NO_LATENT_TC", "0") != "1" and scale > 0
+                and self.mixers.leone_attention_latent_tc_supported(dk, dv)
+                and not (q_abs.data_ptr() | out.data_ptr() | kp.data_ptr()) & 15):
+            # prompt portions on tcgen05, eight tokens of a sequence a tile; in a mixed step the decode rows in front, each of
+            # which would be such a tile, take the form below
+            lead = self._leading_single_rows(ctx)
+            self.launches += 1
+            _check(self.mixer_calls.leone_attention_latent_tc(
+                q_abs, out, kp, bt[lead:], bt.stride(0), q_start[lead:], ctx.ctx_len[lead:], ctx.n_seqs - lead,
+                int(ctx.max_q_len), heads, dk, dv, float(scale), int(window or 0), sink, 0 if sink is None else _dt(sink.dtype),
+                gate, 0 if gate is None else gate.stride(0), cache.page_tokens, kp.shape[0], ctx.status, self._stream()),
+                "attention_latent_tc")
+            if lead == 0:
+                return
+            n, max_ctx_len = lead, int(ctx.ctx_lens[:lead].max())
+        else:
+            max_ctx_len = ctx.max_ctx_len
         self.launches += 1
         if (q_abs.dtype == torch.bfloat16 and os.environ.get("LEONE_NO_LATENT_MMA", "0") != "1"
                 and self.mixers.leone_attention_latent_mma_supported(dk, dv)):
             # few tokens (decode): a token's keys are split over blocks until the SMs are busy
             groups = -(-heads // 16)
-            keys = min(int(window), ctx.max_ctx_len) if window else ctx.max_ctx_len
+            keys = min(int(window), max_ctx_len) if window else max_ctx_len
             splits = max(1, min(16, -(-keys // 64), 148 // max(n * groups, 1)))
             partial = None
             if splits > 1:
