@@ -161,10 +161,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
           const uint32_t a_addr = tiles_base + stage * kExStage;
-          const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(a_addr + kExStageA);
-#pragma unroll
-          for (int k = 0; k < kExK / 16; ++k)
-            umma_bf16(tmem_base + buf * kExCols, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_k64(tmem_base + buf * kExCols, desc_low(a_addr), desc_low(a_addr + kExStageA), idesc, kb > 0 ? 1u : 0u);
           umma_commit(empty0 + 8 * stage);
           if (++stage == kExStages) { stage = 0; phase ^= 1; }
         }

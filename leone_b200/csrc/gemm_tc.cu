@@ -106,46 +106,56 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---------------- producer ----------------
     // The weights do not depend on the kernels before this one: the weight halves of the
     // first stages are requested at once, and only then does the producer wait for the
-    // predecessor (whose output is the token operand).  Pass 0 issues those early weight
-    // loads, pass 1 is the steady loop, which for the first stages adds the token half only.
+    // predecessor, whose output is the token operand; then the token halves follow
     if (elect_one()) {
-      int early = 0;                       // stages whose weight half was requested in pass 0
-      for (int pass = 0; pass < 2; ++pass) {
-        int stage = 0, filled = 0;
-        uint32_t phase = 0;
-        bool stop = false;
-        for (int t = blockIdx.x; t < total && !*giveup && !stop; t += gridDim.x) {
-          const Unit un = unit_of(t, p);
-          const int m_tile = un.tile % m_tiles, n_tile = un.tile / m_tiles;
+      // where the next stage's data comes from: unit t, k-block kb of its kb1
+      struct Cursor { int t, kb, kb1, w_row, x_row; };
+      auto start = [&](Cursor& c) {
+        for (; c.t < total; c.t += gridDim.x) {
+          const Unit un = unit_of(c.t, p);
           const int per = (k_blocks + un.nsplit - 1) / un.nsplit;
-          const int kb0 = un.split * per, kb1 = min(k_blocks, kb0 + per);
-          for (int kb = kb0; kb < kb1; ++kb, ++filled) {
-            if (pass == 0 && filled >= kStages) {
-              // further weight tiles cannot land yet (no free stage): the L2 may fetch them
-              if (filled >= kStages + p.l2_ahead) { stop = true; break; }
-              tma_prefetch_2d(&map_w, kb * kTileK, n_tile * (kSwap ? kTileW : BN));
-              continue;
-            }
-            const bool had_weights = pass == 1 && filled < early;
-            if (pass == 1 && !had_weights && !mbar_wait(empty0 + 8 * stage, phase ^ 1, giveup)) {
-              stop = true;
-              break;
-            }
-            const uint32_t dst = tiles_base + stage * Cfg::kStageBytes;
-            const uint32_t bar = full0 + 8 * stage;
-            if (!had_weights) mbar_expect_tx(bar, Cfg::kStageBytes);
-            const uint32_t w_dst = kSwap ? dst : dst + kTileW * kTileK * 2;
-            const uint32_t x_dst = kSwap ? dst + kTileW * kTileK * 2 : dst;
-            if (!had_weights) tma_load_2d(w_dst, &map_w, bar, kb * kTileK, n_tile * (kSwap ? kTileW : BN));
-            if (pass == 1) tma_load_2d(x_dst, &map_x, bar, kb * kTileK, m_tile * (kSwap ? BN : kTileW));
-            if (++stage == kStages) { stage = 0; phase ^= 1; }
-          }
+          c.kb = un.split * per;
+          c.kb1 = min(k_blocks, c.kb + per);
+          c.x_row = un.tile % m_tiles * kTokRows;
+          c.w_row = un.tile / m_tiles * kWRows;
+          if (c.kb < c.kb1) break;         // (else a share without k-blocks)
         }
-        if (pass == 0) {
-          early = min(filled, kStages);
-          stamp(p, 1);                                     // early weight requests issued
-          pdl_wait();
-          stamp(p, 2);                                     // predecessor complete
+      };
+      auto advance = [&](Cursor& c) {
+        if (++c.kb >= c.kb1) {
+          c.t += gridDim.x;
+          start(c);
+        }
+      };
+      constexpr uint32_t kWAt = kSwap ? 0 : kTileW * kTileK * 2, kXAt = kSwap ? kTileW * kTileK * 2 : 0;      // in a stage
+      Cursor c{(int)blockIdx.x, 0, 0, 0, 0};
+      start(c);
+      const Cursor first = c;
+      int early = 0;                       // stages whose weights are requested now
+      for (; early < kStages && c.t < total; ++early, advance(c)) {
+        mbar_expect_tx(full0 + 8 * early, Cfg::kStageBytes);
+        tma_load_2d(tiles_base + early * Cfg::kStageBytes + kWAt, &map_w, full0 + 8 * early, c.kb * kTileK, c.w_row);
+      }
+      // further weight tiles cannot land yet (no free stage): the L2 may fetch them
+      for (int i = 0; i < p.l2_ahead && c.t < total; ++i, advance(c)) tma_prefetch_2d(&map_w, c.kb * kTileK, c.w_row);
+      stamp(p, 1);                                         // early weight requests issued
+      pdl_wait();
+      stamp(p, 2);                                         // predecessor complete
+      c = first;
+      for (int i = 0; i < early; ++i, advance(c))
+        tma_load_2d(tiles_base + i * Cfg::kStageBytes + kXAt, &map_x, full0 + 8 * i, c.kb * kTileK, c.x_row);
+      uint32_t dst = tiles_base, bar = full0, phase = 0;   // (the ring was filled once where anything is left)
+      for (; c.t < total; advance(c)) {
+        if (!mbar_wait(bar + 8 * kStages, phase, giveup)) break;
+        mbar_expect_tx(bar, Cfg::kStageBytes);
+        tma_load_2d(dst + kWAt, &map_w, bar, c.kb * kTileK, c.w_row);
+        tma_load_2d(dst + kXAt, &map_x, bar, c.kb * kTileK, c.x_row);
+        dst += Cfg::kStageBytes;
+        bar += 8;
+        if (bar == empty0) {
+          dst = tiles_base;
+          bar = full0;
+          phase ^= 1;
         }
       }
     }
@@ -153,34 +163,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t idesc = instr_desc_bf16(kTileW, BN);
-      int stage = 0;
-      uint32_t phase = 0;
+      constexpr uint32_t kStep = Cfg::kStageBytes >> 4, kBAt = (kTileW * kTileK * 2) >> 4;
+      const uint32_t first = desc_low(tiles_base);
+      uint32_t a = first, bar = full0, phase = 0;
       int it = 0;
       for (int t = blockIdx.x; t < total && !*giveup; t += gridDim.x, ++it) {
         const Unit un = unit_of(t, p);
         const int per = (k_blocks + un.nsplit - 1) / un.nsplit;
-        const int kb0 = un.split * per, kb1 = min(k_blocks, kb0 + per);
+        const int kb0 = un.split * per;
+        int left = min(k_blocks, kb0 + per) - kb0;
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         if (!mbar_wait(acc_empty0 + 8 * buf, acc_phase ^ 1, giveup)) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * BN;
-        bool ok = true;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
-          if (it == 0 && kb == kb0) stamp(p, 3);           // first stage complete in shared memory
-          const uint32_t a_addr = tiles_base + stage * Cfg::kStageBytes;
-          const uint32_t b_addr = a_addr + kTileW * kTileK * 2;
-          const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(b_addr);
-#pragma unroll
-          for (int k = 0; k < kTileK / 16; ++k) {
-            // 16 bf16 = 32 bytes further along K inside the swizzled row: +2 in 16-byte units
-            umma_bf16(tmem_d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+        uint32_t sum = 0;                                  // the first MMA of a unit sets the accumulator
+        for (; left > 0; --left) {
+          if (!mbar_wait(bar, phase, giveup)) break;
+          if (it == 0 && sum == 0) stamp(p, 3);            // first stage complete in shared memory
+          umma_k64(tmem_d, a, a + kBAt, idesc, sum);
+          sum = 1;
+          umma_commit(bar + 8 * kStages);
+          bar += 8;
+          a += kStep;
+          if (bar == empty0) {
+            bar = full0;
+            a = first;
+            phase ^= 1;
           }
-          umma_commit(empty0 + 8 * stage);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
+        if (left > 0) break;                               // a wait ran out
         umma_commit(acc_full0 + 8 * buf);
         stamp(p, 4);                                       // last MMA of the (latest) unit issued
       }

@@ -150,6 +150,24 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The four MMAs of a k-block of 64 bf16 whose operand tiles (both K-major with the 128-byte swizzle) start at `a` and `b`: the low words
+// of their descriptors, desc_low(address).  Written as one piece because the thread that issues them is what bounds a product
+// with narrow tiles: the descriptors' high words are constants, and 16 elements further along K are 32 bytes, 2 in the low word.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);       // as in smem_desc_sw128
+__device__ __forceinline__ uint32_t desc_low(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+#define LEONE_UMMA_K64(group)                                                                                                  \
+  "{\n\t.reg .pred p, t;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"                                                            \
+  "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, %0, %0;\n\t"                                                                       \
+  "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\ttcgen05.mma.cta_group::" group ".kind::f16 [%0], a, b, %3, p;\n\t"           \
+  "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 a, {x, %5};\n\tmov.b64 b, {y, %5};\n\t"                                   \
+  "tcgen05.mma.cta_group::" group ".kind::f16 [%0], a, b, %3, t;\n\t"                                                          \
+  "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 a, {x, %5};\n\tmov.b64 b, {y, %5};\n\t"                                   \
+  "tcgen05.mma.cta_group::" group ".kind::f16 [%0], a, b, %3, t;\n\t"                                                          \
+  "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 a, {x, %5};\n\tmov.b64 b, {y, %5};\n\t"                                   \
+  "tcgen05.mma.cta_group::" group ".kind::f16 [%0], a, b, %3, t;\n\t}"
+__device__ __forceinline__ void umma_k64(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(LEONE_UMMA_K64("1") ::"r"(tmem_d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(kDescHigh) : "memory");
+}
 // The mbarrier gets one arrival when every MMA issued so far by this thread is done.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
