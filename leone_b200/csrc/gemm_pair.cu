@@ -6,9 +6,8 @@
 // 128 token rows and HALF of the tile's weight rows (at BN = 256: 32 KB per k-block and SM, a
 // third less, and seven stages instead of four in the same shared memory), the first block issues one MMA of
 // M = 256 per 16 elements of K that reads both blocks' shared memory, and each block's tensor
-// memory receives the accumulators of its own 128 token rows, which it finishes exactly as the
-// single-block kernel does (same epilogue code: bf16 / fp32 / fp32 + residual / SwiGLU, and the
-// RMSNorm folded into the products around it).
+// memory receives the accumulators of its own 128 token rows, which it finishes (finish_rows) into bf16 / fp32 / fp32 + residual /
+// SwiGLU, with the RMSNorm folded into the products around it.
 //
 // BN is a launch argument, any multiple of 16 from 32 to 256 (of 32 with the SwiGLU epilogue): the
 // caller picks the width whose tiles cost the fewest rounds over the pairs (the k-loop's time
@@ -17,7 +16,8 @@
 //
 // Per block: warp 0 loads (TMA loads into its own shared memory, no multicast; both blocks' loads
 // count their bytes on the FIRST block's barrier, which is what the cta_group::2 form of the copy
-// is for), warp 1 of the first block issues the MMAs, warps 2..5 run the epilogue.  The MMAs' completion is
+// is for), warp 1 of the first block issues the MMAs, warps 2..9 run the epilogue, two for
+// every 32 rows.  The MMAs' completion is
 // committed to both blocks' barriers (tcgen05.commit with a two-block mask): stage free, and
 // accumulator ready.  The second block's epilogue warps release an accumulator by arriving on
 // the first block's barrier.  Every wait is bounded; a wait that runs out sets the status word
@@ -27,34 +27,37 @@
 
 namespace leone {
 namespace tc {
-
 constexpr int kPairMaxStages = 10;
-constexpr int kPairThreads = 192;
-constexpr int kPairSmemLimit = 226 * 1024;             // dynamic shared memory of a block (the static part is beside it)
+constexpr int kPairEpilogueWarps = 8;               // two for every 32 rows: each finishes half of the tile's columns
+constexpr int kPairThreads = 64 + 32 * kPairEpilogueWarps;
+constexpr int kPairSmemLimit = 227 * 1024 - 64;        // dynamic shared memory of a block (the static part is beside it)
+constexpr int kPairSumsBytes = 2 * 4 * 32 * 4;         // two buffers of the sums of squares that pass between the epilogue's halves
 
 // Shared memory of a pair's block for tiles of bn weight rows: stages of 128 token rows and bn / 2
 // weight rows (each operand tile starts on a 1024-byte boundary, as the 128-byte swizzle wants).
 struct PairShape {
-  int half, stage_bytes, stages, smem_bytes;
+  int half, blocks, b_bytes, stage_bytes, stages, smem_bytes;     // blocks: k-blocks of a stage, b_bytes of weights in one
 };
-__host__ __device__ inline PairShape pair_shape(int bn) {
+__host__ __device__ inline PairShape pair_shape(int bn, int blocks) {
   PairShape c;
   c.half = bn / 2;
-  c.stage_bytes = kTileW * kTileK * 2 + ((c.half * kTileK * 2 + 1023) & ~1023);
-  c.stages = (kPairSmemLimit - 1024 /*alignment*/ - 256 /*barriers*/) / c.stage_bytes;
+  c.b_bytes = (c.half * kTileK * 2 + 1023) & ~1023;
+  c.blocks = blocks;
+  c.stage_bytes = c.blocks * (kTileW * kTileK * 2 + c.b_bytes);
+  constexpr int other = 1024 /*alignment*/ + 256 /*barriers*/ + kPairSumsBytes + kPairEpilogueWarps * kBoxBytes;
+  c.stages = (kPairSmemLimit - other) / c.stage_bytes;
   if (c.stages > kPairMaxStages) c.stages = kPairMaxStages;
-  c.smem_bytes = c.stages * c.stage_bytes + 1024 + 256;
+  c.smem_bytes = c.stages * c.stage_bytes + other;
   return c;
 }
 
-__device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// k-blocks of a stage.  Two halve what the waits and commits cost the thread that issues the MMAs, which is what bounds narrow tiles
+// (2048 weight rows, K 2048 / 6144, 256 tokens: 8.9 / 18.8 us against 9.2 / 19.3 at 64 rows a tile, 10.3 / 21.0 either way at 96);
+// wider tiles lose more to the ring's fewer stages (10.9 against 10.6 at 128, 14.9 against 13.9 at 192).
+inline int pair_blocks(int bn) { return bn <= 96 ? 2 : 1; }
+
+__device__ __forceinline__ void umma2_k64(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(LEONE_UMMA_K64("2") ::"r"(tmem_d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(kDescHigh) : "memory");
 }
 // One arrival on the barrier at this offset in both blocks of the pair when every MMA issued so
 // far by this thread is done.
@@ -124,9 +127,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 // them in split order on top of the residual values and runs the epilogue (no folded norm).
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                 const GemmParams p, const int BN) {
-  const PairShape cfg = pair_shape(BN);
+                 const GemmParams p, const int BN, const int blocks) {
+  const PairShape cfg = pair_shape(BN, blocks);
   const int kStages = cfg.stages;
+  constexpr int kABytes = kTileW * kTileK * 2;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles_base = (raw + 1023u) & ~1023u;
@@ -136,7 +140,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   // and for the split mode: the pieces of a chunk have landed, and all four warps have read them
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kStages;
   const uint32_t acc_full0 = empty0 + 8 * kStages, acc_empty0 = acc_full0 + 16;
-  const uint32_t landed = acc_empty0 + 16, pieces_read = landed + 8;
+  // and, where a norm follows, the second half's sums of squares of a quarter of the rows are in place (4)
+  const uint32_t landed = acc_empty0 + 16, pieces_read = landed + 8, sums_there = pieces_read + 8;
   __shared__ uint32_t tmem_holder;
   __shared__ int gave_up;
 
@@ -163,10 +168,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);
-      mbar_init(acc_empty0 + 8 * b, 8);               // four epilogue warps of each block (used in the first)
+      mbar_init(acc_empty0 + 8 * b, 2 * kPairEpilogueWarps);     // the epilogue warps of both blocks (used in the first)
     }
     mbar_init(landed, 1);
-    mbar_init(pieces_read, 4);
+    for (int q = 0; q < 4; ++q) mbar_init(sums_there + 8 * q, 1);
+    mbar_init(pieces_read, (uint32_t)(BN / 32));
     mbar_fence_init();
     tma_prefetch_desc(&map_w);
     tma_prefetch_desc(&map_x);
@@ -186,33 +192,51 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // As in the single-block kernel the weight halves of the first stages are requested before
     // the wait for the kernel before this one, whose output is the token operand.
     if (elect_one()) {
-      int early = 0;
-      for (int pass = 0; pass < 2; ++pass) {
-        int stage = 0, filled = 0;
-        uint32_t phase = 0;
-        bool stop = false;
-        for (int t = pair; t < total && !*giveup && !stop; t += pairs) {
-          const int m_tile = (t % m_pairs) * 2 + (int)rank, n_tile = t / m_pairs;
-          for (int kb = kb_lo; kb < kb_hi; ++kb, ++filled) {
-            if (pass == 0 && filled == kStages) { stop = true; break; }
-            const bool had_weights = pass == 1 && filled < early;
-            if (pass == 1 && !had_weights && !mbar_wait_cluster(empty0 + 8 * stage, phase ^ 1, giveup)) {
-              stop = true;
-              break;
-            }
-            const uint32_t dst = tiles_base + stage * cfg.stage_bytes;
-            const uint32_t bar = cluster_map(full0 + 8 * stage, lead);   // the first block's barrier counts both blocks' bytes
-            if (!had_weights) {
-              if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * (kTileW * kTileK * 2 + cfg.half * kTileK * 2));
-              tma_load_2d_pair(dst + kTileW * kTileK * 2, &map_w, bar, kb * kTileK, n_tile * BN + (int)rank * cfg.half);
-            }
-            if (pass == 1) tma_load_2d_pair(dst, &map_x, bar, kb * kTileK, m_tile * kTileW);
-            if (++stage == kStages) { stage = 0; phase ^= 1; }
-          }
+      // where the next stage's data comes from: tile t, k-block kb
+      struct Cursor { int t, kb, m, n; };
+      auto start = [&](Cursor& c) {
+        c.kb = kb_lo;
+        c.m = (c.t % m_pairs * 2 + (int)rank) * kTileW;
+        c.n = c.t / m_pairs * BN + (int)rank * cfg.half;
+      };
+      auto advance = [&](Cursor& c) {
+        if ((c.kb += blocks) >= kb_hi) {
+          c.t += pairs;
+          start(c);
         }
-        if (pass == 0) {
-          early = filled;
-          pdl_wait();
+      };
+      // (the first block's barrier, `bar`, counts both blocks' bytes)
+      auto load_w = [&](const Cursor& c, uint32_t dst, uint32_t bar_here, uint32_t bar) {
+        const int here = min(blocks, kb_hi - c.kb);
+        if (rank == 0) mbar_expect_tx(bar_here, (uint32_t)(2 * here * (kABytes + cfg.half * kTileK * 2)));
+        tma_load_2d_pair(dst + blocks * kABytes, &map_w, bar, c.kb * kTileK, c.n);
+        if (here == 2) tma_load_2d_pair(dst + 2 * kABytes + cfg.b_bytes, &map_w, bar, (c.kb + 1) * kTileK, c.n);
+      };
+      auto load_x = [&](const Cursor& c, uint32_t dst, uint32_t bar) {
+        tma_load_2d_pair(dst, &map_x, bar, c.kb * kTileK, c.m);
+        if (min(blocks, kb_hi - c.kb) == 2) tma_load_2d_pair(dst + kABytes, &map_x, bar, (c.kb + 1) * kTileK, c.m);
+      };
+      const uint32_t lead_full0 = cluster_map(full0, lead);
+      Cursor c{pair, kb_lo, 0, 0};
+      start(c);
+      const Cursor first = c;
+      int early = 0;
+      for (; early < kStages && c.t < total; ++early, advance(c))
+        load_w(c, tiles_base + early * cfg.stage_bytes, full0 + 8 * early, lead_full0 + 8 * early);
+      pdl_wait();
+      c = first;
+      for (int i = 0; i < early; ++i, advance(c)) load_x(c, tiles_base + i * cfg.stage_bytes, lead_full0 + 8 * i);
+      uint32_t dst = tiles_base, bar = full0, phase = 0;         // (the ring was filled once where anything is left)
+      for (; c.t < total; advance(c)) {
+        if (!mbar_wait_cluster(bar + 8 * kStages, phase, giveup)) break;
+        load_w(c, dst, bar, lead_full0 + (bar - full0));
+        load_x(c, dst, lead_full0 + (bar - full0));
+        dst += cfg.stage_bytes;
+        bar += 8;
+        if (bar == empty0) {
+          dst = tiles_base;
+          bar = full0;
+          phase ^= 1;
         }
       }
     }
@@ -222,47 +246,80 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // ---------------- MMA issuer (the first block) ----------------
     if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(2 * kTileW, BN);
-      int stage = 0;
-      uint32_t phase = 0;
+      const uint32_t first = desc_low(tiles_base), step = cfg.stage_bytes >> 4;
+      const uint32_t b_step = cfg.b_bytes >> 4, b_at = blocks * (kABytes >> 4);
+      uint32_t a = first, bar = full0, phase = 0;
       int it = 0;
       for (int t = pair; t < total && !*giveup; t += pairs, ++it) {
         const int buf = it & 1;
         if (!mbar_wait_cluster(acc_empty0 + 8 * buf, (((it >> 1) & 1) ^ 1), giveup)) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * 256;
-        bool ok = true;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait_cluster(full0 + 8 * stage, phase, giveup)) { ok = false; break; }
-          const uint32_t a_addr = tiles_base + stage * cfg.stage_bytes;
-          const uint32_t b_addr = a_addr + kTileW * kTileK * 2;
-          const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(b_addr);
-#pragma unroll
-          for (int k = 0; k < kTileK / 16; ++k)
-            umma2_bf16(tmem_d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > kb_lo || k > 0) ? 1u : 0u);
-          umma2_commit_both(empty0 + 8 * stage, lead);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        uint32_t sum = 0;                              // the first MMA of a tile sets the accumulator
+        int left = kb_hi - kb_lo;
+        for (; left > 0; left -= blocks) {
+          if (!mbar_wait_cluster(bar, phase, giveup)) break;
+          umma2_k64(tmem_d, a, a + b_at, idesc, sum);
+          sum = 1;
+          if (blocks == 2 && left > 1) umma2_k64(tmem_d, a + (kABytes >> 4), a + b_at + b_step, idesc, 1);
+          umma2_commit_both(bar + 8 * kStages, lead);
+          bar += 8;
+          a += step;
+          if (bar == empty0) {
+            bar = full0;
+            a = first;
+            phase ^= 1;
+          }
         }
-        if (!ok) break;
+        if (left > 0) break;                           // a wait ran out
         umma2_commit_both(acc_full0 + 8 * buf, lead);
       }
     }
   } else {
     // ---------------- epilogue (both blocks) ----------------
     const int quarter = warp & 3;                     // TMEM lanes 32*quarter .. +31
+    const int half = (warp - 2) >> 2;                 // which columns of the tile
+    const int unit = p.epilogue == 3 || S > 1 ? 32 : 16, middle = (BN / unit + 1) / 2 * unit;
+    const int c_lo = half == 0 ? 0 : middle, c_hi = half == 0 ? middle : BN;
+    float* sums = reinterpret_cast<float*>(bars + 32);
+    const uint32_t box = smem_u32(bars) + 256 + kPairSumsBytes + (warp - 2) * kBoxBytes;
     int it = 0;
     pdl_wait();      // outputs and residual may be in use until here
     for (int t = pair; t < total && !*giveup; t += pairs, ++it) {
       const int m_tile = (t % m_pairs) * 2 + (int)rank, n_tile = t / m_pairs;
       const int buf = it & 1;
-      bool ok = mbar_wait_cluster(acc_full0 + 8 * buf, (it >> 1) & 1, giveup);
-      ok = __all_sync(0xffffffffu, ok);                // the loads from tensor memory are warp-wide
-      if (!ok) break;
-      tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * 256;
+      auto complete = [&]() {
+        bool ok = mbar_wait_cluster(acc_full0 + 8 * buf, (it >> 1) & 1, giveup);
+        ok = __all_sync(0xffffffffu, ok);              // the loads from tensor memory are warp-wide
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      // the two warps of these rows each have the sums of squares of half of the tile's columns: the second hands its own to
+      // the first (its next tile's go to the other buffer, and the one after that waits for this tile's release)
+      auto squares = [&](const float (&s)[8]) {
+        float* there = sums + (buf * 4 + quarter) * 32;
+        const int row = lane >> 3;
+        if (half == 1) {
+          if ((lane & 7) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) there[4 * i + row] = s[i];
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sums_there + 8 * quarter);
+        } else if (mbar_wait(sums_there + 8 * quarter, it & 1, giveup) && (lane & 7) == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int m = m_tile * kTileW + quarter * 32 + 4 * i + row;
+            if (m < p.M) p.norm_out_ss[(size_t)n_tile * p.M + m] = s[i] + there[4 * i + row];
+          }
+        }
+      };
       if (S > 1) {
+        if (!complete()) break;
         // this block's 128 rows of partial sums go to the workspace; one tile per cluster
         float* ws = p.workspace + (size_t)blockIdx.x * ((size_t)BN * kTileW) + (size_t)quarter * (BN * 32) + lane;
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c_lo; c < c_hi; c += 32) {
           uint32_t r[32];
           tmem_ld32_issue(taddr + c, r);
           tmem_ld_wait();
@@ -272,7 +329,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         __threadfence();
         break;
       }
-      finish_token_major_row(p, taddr, m_tile * kTileW + quarter * 32 + lane, n_tile * BN, n_tile, BN);
+      if (!finish_rows(p, taddr, m_tile * kTileW + quarter * 32, n_tile * BN, c_lo, c_hi, box, complete, squares)) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -286,25 +343,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // Every thread of every block of the cluster comes here (all loops above are bounded).
     __syncwarp();
     cluster_sync_all();                                // all partial tiles are in the workspace
-    if (warp >= 2 && pair < total && !*giveup) {
+    if (warp >= 2 && warp < 2 + BN / 32 && pair < total && !*giveup) {
       const int m_pair = pair % m_pairs, n_tile = pair / m_pairs;
-      const int groups = BN / 128;                     // groups of 32 columns per warp: 1 or 2
       const uint32_t piece = (uint32_t)BN * 32 * 4;    // one block's partial sums of a chunk
       const float* ws_cluster = p.workspace + (size_t)(blockIdx.x - crank) * ((size_t)BN * kTileW);
-      const float* box = reinterpret_cast<const float*>(aligned);
-      const int et = (warp - 2) * 32 + lane;
+      const float* pieces = reinterpret_cast<const float*>(aligned);
+      const int c = (warp - 2) * 32;                   // this warp's 32 columns
       uint32_t landed_phase = 0, read_phase = 0;
       bool first = true;
       for (int ch = (int)crank; ch < 8; ch += 2 * S) { // chunk ch: rows 32 ch .. of the tile's 256
         const int half = ch >> 2, q4 = ch & 3;         // whose rows they are in every pair, and which quarter
         const int m = (m_pair * 2 + half) * kTileW + q4 * 32 + lane;
-        const int n0 = n_tile * BN + (warp & 3) * (BN / 4);
-        float v[2][32];
-#pragma unroll
-        for (int g = 0; g < 2; ++g)
-          if (g < groups) fetch_residual32(p, v[g], m, n0 + g * 32);
-        if (et == 0) {
-          // the pieces of the chunk before have been read by all four warps (a wait that runs out
+        float v[32];
+        fetch_residual32(p, v, m, n_tile * BN + c);
+        if (warp == 2 && lane == 0) {
+          // the pieces of the chunk before have been read by all warps (a wait that runs out
           // requests nothing, and the others' waits run out too)
           bool go = true;
           if (!first) {
@@ -322,21 +375,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         first = false;
         if (!mbar_wait(landed, landed_phase, giveup)) break;
         landed_phase ^= 1;
+        for (int u = 0; u < S; ++u) {                  // split order
+          const float* src = pieces + (size_t)u * (BN * 32) + c * 32 + lane;
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          if (g < groups) {
-            const float* src = box + (size_t)((warp & 3) * (BN / 4) + g * 32) * 32 + lane;
-            for (int u = 0; u < S; ++u) {                // split order
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[g][j] += src[(size_t)u * (BN * 32) + j * 32];
-            }
-          }
+          for (int j = 0; j < 32; ++j) v[j] += src[j * 32];
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(pieces_read);
-#pragma unroll
-        for (int g = 0; g < 2; ++g)
-          if (g < groups) finish_token_major32(p, v[g], m, n0 + g * 32, true);
+        finish_token_major32(p, v, m, n_tile * BN + c, true);
       }
     }
   }
@@ -374,7 +420,7 @@ int pair_cluster_capacity(int bn, int splits) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2u * (unsigned)splits * 64u);
   cfg.blockDim = dim3(kPairThreads);
-  cfg.dynamicSmemBytes = (size_t)pair_shape(bn).smem_bytes;
+  cfg.dynamicSmemBytes = (size_t)pair_shape(bn, pair_blocks(bn)).smem_bytes;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2u * (unsigned)splits;
@@ -400,11 +446,11 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
     // one tile per cluster of 2 * splits blocks, all clusters resident at once
     if (total > pair_cluster_capacity(bn, p.splits)) return kRefusedSize;
     return launch_kernel_cluster(gemm_pair_kernel, dim3((unsigned)(total * 2 * p.splits)), dim3(kPairThreads),
-                                 (size_t)pair_shape(bn).smem_bytes, stream, dim3(2u * (unsigned)p.splits), mw, mx, p, bn);
+                                 (size_t)pair_shape(bn, pair_blocks(bn)).smem_bytes, stream, dim3(2u * (unsigned)p.splits), mw, mx, p, bn, pair_blocks(bn));
   }
   const int pairs = (int)(total < sm_count / 2 ? total : sm_count / 2);
   return launch_kernel_cluster(gemm_pair_kernel, dim3(2u * (unsigned)pairs), dim3(kPairThreads),
-                               (size_t)pair_shape(bn).smem_bytes, stream, dim3(2), mw, mx, p, bn);
+                               (size_t)pair_shape(bn, pair_blocks(bn)).smem_bytes, stream, dim3(2), mw, mx, p, bn, pair_blocks(bn));
 }
 
 }  // namespace tc
@@ -455,6 +501,7 @@ extern "C" int leone_gemm_pair(const void* x, const void* w, void* out, const fl
 
 // Tiles of `width` weight rows whose clusters of 2 * splits blocks can be resident at once, and the
 // workspace floats a product split that way needs.
+// Tuning only: k-blocks a stage (0: the rule).
 extern "C" int leone_gemm_pair_capacity(int width, int splits) {
   if ((splits != 2 && splits != 4) || (width != 128 && width != 256)) return 0;
   return pair_cluster_capacity(width, splits);

@@ -482,5 +482,243 @@ __device__ __forceinline__ void finish_token_major_row(const GemmParams& p, uint
   finish_token_major_row(p, taddr, m, n0, n_tile, BN);
 }
 
+// Token-major form, the pairs' epilogue: a warp finishes its 32 token rows (m0 ..; tensor memory at `taddr`, lane = row) for
+// the accumulator columns [c_lo, c_hi) of the tile whose first weight row is n0 (multiples of 16, of 32 with the gate).
+// Sums go through 4 KB of the warp's own shared memory, 32 rows of 128 bytes with their 16-byte pieces swizzled by the row, so
+// that every access to global memory is four rows of 128 bytes side by side.  (A thread per row, as above, touches 32 rows with
+// 16 bytes each: half sectors, and 32 cache lines an instruction.)
+// The row's factor of a norm before the product (1 without one).
+__device__ __forceinline__ float norm_in_factor(const GemmParams& p, int m) {
+  if (p.norm_in_ss == nullptr) return 1.f;
+  float ss = 0.f;
+  if (m < p.M) {
+#pragma unroll 8
+    for (int q = 0; q < p.norm_in_parts; ++q) ss += p.norm_in_ss[(size_t)q * p.M + m];
+  }
+  return rsqrtf(ss / (float)p.K + p.norm_eps);
+}
+
+constexpr int kBoxBytes = 32 * 128;                // a warp's shared memory for finish_rows
+constexpr int kResidualAhead = 2;                  // chunks of residual values in flight ahead of their use
+
+// The residual values of one chunk of 32 columns, as finish_rows' lanes own them: rows 4 i + lane / 8, columns 4 (lane % 8) ..
+__device__ __forceinline__ void fetch_residual_chunk(const GemmParams& p, float4 (&r)[8], int m0, int n, int c, int c_hi, bool vec) {
+  const int lane = threadIdx.x & 31, col = n + c + 4 * (lane & 7);
+  const bool here = c + 4 * (lane & 7) < c_hi;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + 4 * i + (lane >> 3);
+    r[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!here || m >= p.M) continue;
+    const float* src = p.residual + (size_t)m * p.ldc + col;
+    if (vec && col + 4 <= p.N) {
+      r[i] = *reinterpret_cast<const float4*>(src);
+    } else {
+      if (col < p.N) r[i].x = src[0];
+      if (col + 1 < p.N) r[i].y = src[1];
+      if (col + 2 < p.N) r[i].z = src[2];
+      if (col + 3 < p.N) r[i].w = src[3];
+    }
+  }
+}
+
+// A product's kernel runs once in a layer, with the step's other kernels in between, so the code of its epilogue comes from memory
+// again: what every tile of the gate executes is kept short (a loop over 16 outputs at a time, the edges of tiles and unaligned rows
+// in paths of their own).  12288 x 2048 with the gate in a step of 1,027 tokens 54.7 us with the loop unrolled, 42.8 as it is (48.8
+// with a thread a row); at 64 tokens 22.9 and 10.3.  (The unrolled one over and over, its code at hand: 44.9.)
+//
+// `ready`: waits until the accumulator is complete (false: gave up); the first residual values are requested before it.
+// Called by whole warps.  `squares(s)`: s[i] is the sum of squares of output row m0 + 4 i + lane / 8 over these
+// columns, for the norm after the product (the row's eight lanes have it).
+template <class Ready, class Squares>
+__device__ __forceinline__ bool finish_rows(const GemmParams& p, uint32_t taddr, int m0, int n0, int c_lo, int c_hi,
+                                            uint32_t box, Ready ready, Squares squares) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t mine = box + lane * 128;                             // this thread's row of the box
+  const int sw = lane & 7;
+  const int row_out = lane >> 3, unit = lane & 7;                     // on the way out: rows 4 i + row_out, 16-byte piece `unit`
+  if (m0 >= p.M) return ready();                                      // no such tokens: nothing to store
+  const float rs = norm_in_factor(p, m0 + lane);
+  auto put = [&](int u, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(mine + ((u ^ sw) << 4)), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+  };
+  auto get = [&](int i) {
+    const int r = 4 * i + row_out;
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(box + r * 128 + ((unit ^ (r & 7)) << 4)) : "memory");
+    return v;
+  };
+  auto pack = [](float a, float b) {
+    __nv_bfloat162 v2 = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&v2);
+  };
+  if (p.epilogue == 1 || p.epilogue == 2) {
+    const bool vec = ((p.ldc & 3) | ((uintptr_t)p.out & 15) | ((uintptr_t)p.residual & 15)) == 0;
+    const bool vec_x = ((p.ld_norm_out & 3) | ((uintptr_t)p.norm_out_x & 7)) == 0;
+    float4 ahead[kResidualAhead][8];
+    float ssq[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ssq[i] = 0.f;
+    if (p.epilogue == 2) {
+#pragma unroll
+      for (int a = 0; a < kResidualAhead; ++a)
+        if (c_lo + 32 * a < c_hi) fetch_residual_chunk(p, ahead[a], m0, n0, c_lo + 32 * a, c_hi, vec);
+    }
+    if (!ready()) return false;
+    for (int c0 = c_lo; c0 < c_hi; c0 += 32 * kResidualAhead) {
+#pragma unroll
+      for (int a = 0; a < kResidualAhead; ++a) {                      // chunk c uses and refills slot a
+        const int c = c0 + 32 * a;
+        if (c >= c_hi) break;
+        uint32_t r[32];
+        const bool whole = c + 32 <= c_hi;
+        if (whole) tmem_ld32_issue(taddr + c, r);
+        else tmem_ld16_issue(taddr + c, r);
+        tmem_ld_wait();
+        __syncwarp();                                                 // the chunk before has left the box
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (q == 1 && !whole) break;
+          float v[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[16 * q + j]) * rs;
+          if (p.bias != nullptr) add_bias16(p, v, n0 + c + 16 * q);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            put(4 * q + j, __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]),
+                __float_as_uint(v[4 * j + 3]));
+        }
+        __syncwarp();
+        const int n = n0 + c + 4 * unit;
+        const bool here = c + 4 * unit < c_hi && n < p.N, full = vec && n + 4 <= p.N;
+        float w[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p.norm_out_x != nullptr && here) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (n + j < p.N) w[j] = __ldg(p.norm_out_w + n + j);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int m = m0 + 4 * i + row_out;
+          const uint4 raw = get(i);
+          float4 v = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z), __uint_as_float(raw.w));
+          if (p.epilogue == 2) {
+            v.x += ahead[a][i].x;
+            v.y += ahead[a][i].y;
+            v.z += ahead[a][i].z;
+            v.w += ahead[a][i].w;
+          }
+          if (!here || m >= p.M) continue;
+          float* dst = (float*)p.out + (size_t)m * p.ldc + n;
+          if (full) {
+            *reinterpret_cast<float4*>(dst) = v;
+          } else {
+            dst[0] = v.x;
+            if (n + 1 < p.N) dst[1] = v.y; else v.y = 0.f;
+            if (n + 2 < p.N) dst[2] = v.z; else v.z = 0.f;
+            if (n + 3 < p.N) dst[3] = v.w; else v.w = 0.f;
+          }
+          if (p.norm_out_x != nullptr) {
+            ssq[i] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ssq[i]))));
+            __nv_bfloat16* x = p.norm_out_x + (size_t)m * p.ld_norm_out + n;
+            if (full && vec_x) {
+              *reinterpret_cast<uint2*>(x) = make_uint2(pack(v.x * w[0], v.y * w[1]), pack(v.z * w[2], v.w * w[3]));
+            } else {
+              x[0] = __float2bfloat16_rn(v.x * w[0]);
+              if (n + 1 < p.N) x[1] = __float2bfloat16_rn(v.y * w[1]);
+              if (n + 2 < p.N) x[2] = __float2bfloat16_rn(v.z * w[2]);
+              if (n + 3 < p.N) x[3] = __float2bfloat16_rn(v.w * w[3]);
+            }
+          }
+        }
+        if (p.epilogue == 2 && c + 32 * kResidualAhead < c_hi)
+          fetch_residual_chunk(p, ahead[a], m0, n0, c + 32 * kResidualAhead, c_hi, vec);
+      }
+    }
+    if (p.norm_out_x != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float s = ssq[i];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        ssq[i] = s;
+      }
+      squares(ssq);
+    }
+    return true;
+  }
+  // bfloat16 outputs: 64 of them a chunk, from 64 accumulator columns or, with the gate, from 128
+  if (!ready()) return false;
+  const bool gated = p.epilogue == 3;
+  const bool vec = ((p.ldc & 7) | ((uintptr_t)p.out & 15)) == 0;
+  const int step = gated ? 128 : 64;
+  const int n_out = gated ? p.N >> 1 : p.N;
+#pragma unroll 1
+  for (int c = c_lo; c < c_hi; c += step) {
+    __syncwarp();                                                     // the chunk before has left the box
+    const int parts = min(step, c_hi - c) / (gated ? 32 : 16);        // 16 outputs each
+#pragma unroll 1
+    for (int h = 0; h < parts; ++h) {
+      uint32_t r[32];
+      float v[16];
+      if (gated) {
+        const int at = c + 32 * h;
+        tmem_ld32_issue(taddr + at, r);
+        tmem_ld_wait();
+        float u[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          v[j] = __uint_as_float(r[j]) * rs;
+          u[j] = __uint_as_float(r[16 + j]) * rs;
+        }
+        if (__builtin_expect(p.bias != nullptr, 0) && n0 + at < p.N) {
+          add_bias16(p, v, n0 + at);
+          add_bias16(p, u, n0 + at + 16);
+        }
+        if (__builtin_expect(p.gate_plain, 1)) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = silu_mul(v[j], u[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = gate_mul(p, v[j], u[j]);
+        }
+      } else {
+        const int at = c + 16 * h;
+        tmem_ld16_issue(taddr + at, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) * rs;
+        if (__builtin_expect(p.bias != nullptr, 0)) add_bias16(p, v, n0 + at);
+      }
+      put(2 * h, pack(v[0], v[1]), pack(v[2], v[3]), pack(v[4], v[5]), pack(v[6], v[7]));
+      put(2 * h + 1, pack(v[8], v[9]), pack(v[10], v[11]), pack(v[12], v[13]), pack(v[14], v[15]));
+    }
+    __syncwarp();
+    const int first = gated ? (n0 + c) >> 1 : n0 + c, n = first + 8 * unit, m1 = m0 + row_out;
+    const bool here = n < n_out && unit < 2 * parts;
+    __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)m1 * p.ldc + n;
+    if (__all_sync(0xffffffffu, !here || (vec && n + 8 <= n_out))) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i, dst += 4 * (size_t)p.ldc) {
+        const uint4 v = get(i);
+        if (here && m1 + 4 * i < p.M) *reinterpret_cast<uint4*>(dst) = v;
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < 8; ++i, dst += 4 * (size_t)p.ldc) {
+        const uint4 v = get(i);
+        if (!here || m1 + 4 * i >= p.M) continue;
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (n + j < n_out) dst[j] = __ushort_as_bfloat16((unsigned short)(w[j >> 1] >> (16 * (j & 1))));
+      }
+    }
+  }
+  return true;
+}
+
 }  // namespace tc
 }  // namespace leone
