@@ -31,7 +31,7 @@ MODULES: Dict[str, List[str]] = {
     # every run needs these: both dtypes, every size
     "core": ["elementwise.cu", "gemm_simt.cu", "gemm_f32_tc.cu", "attention_generic.cu", "attention_f32.cu", "sampling_pipeline.cu", "random_weights.cu"],
     # the bfloat16 serving path: tensor-core products and tiled attention
-    "bf16": ["gemm_tc.cu", "gemm_pair.cu", "attention_tiled.cu", "attention_prefill_pingpong.cu"],
+    "bf16": ["gemm_tc.cu", "gemm_pair.cu", "gemm_narrow.cu", "attention_tiled.cu", "attention_prefill_pingpong.cu"],
     # mixers and feed-forwards beyond softmax attention over K/V pages and the dense gated layer:
     # linear attention with a decaying state, attention through a cached latent, attention with a choice
     # of mask and weight rule, routed experts, short convolutions with state, the minGRU recurrence, attention

@@ -71,6 +71,8 @@ class FastKernels:
         self.pair_padding = 0.8            # a pair's half tile against a single block's tile, at most (see in_pairs)
         self.pair_width_override = 0       # > 0: the tile width of every product on pairs (kernel_bench sets it)
         self.pair_split_override = 0       # > 0: pairs per tile of every product on pairs (tests set it)
+        # LEONE_NO_NARROW=1 leaves the products with few tiles to the forms that split K
+        self.use_narrow = os.environ.get("LEONE_NO_NARROW", "0") != "1"
         self._pair_widths = {}
         self._plans = {}                   # _gemm's decisions per (sizes, arguments)
         self.decode_cluster_rounds = 1     # rounds of blocks a clustered decode attention may take (kernel_bench sets it)
@@ -274,6 +276,55 @@ class FastKernels:
             self._cluster_capacity[key] = int(self.lib.leone_gemm_tc_cluster_capacity_token_major(splits))
         return self._cluster_capacity[key]
 
+    def narrow_width(self, m: int, n: int, k: int, gated: bool) -> int:
+        """Weight rows per tile of an unsplit product on single SMs (gemm_narrow.cu) where that is the best form, else 0: from 33
+        to 128 tokens, if the estimate below is under that of the swapped form's split along K.  Both in us, fitted to products of
+        40, 77 and 128 tokens with 11 matrices of 2048 x 2048 to 24576 x 4096.  Narrow tiles: 3.2, 0.012 for every tile past 64, and
+        for every round of tiles over the SMs and k-block 0.12 + 0.0007 a weight row (what the thread that issues the MMAs
+        takes); no less than the weights at 4.8 MB a us.  The split: 7.3 + 0.165 a MB of weights up to 64 tokens, 9.2 + 0.215
+        above (partial tiles of 128 columns are exchanged).  So K decides: 2048 x 2048 at 77 tokens 7.6 us against 10.6,
+        12288 x 2048 14.8 against 18.8, 2048 x 6144 17.0 against 14.3 (stays split).  Not for an output head, whose time is its
+        logits."""
+        if not self.use_narrow or not 32 < m <= 128:
+            return 0
+        k_blocks, mb, best = -(-k // 64), n * k * 2e-6, None
+        if n > 256 * self.sm_count:
+            return 0
+        for w in range(256, 15, -32 if gated else -16):
+            tiles = -(-n // w)
+            cost = 3.2 + 0.012 * max(0, min(tiles, self.sm_count) - 64) + -(-tiles // self.sm_count) * k_blocks * (0.12 + 0.0007 * w)
+            if best is None or cost < 0.99 * best[0]:
+                best = (cost, w)
+        split = 7.3 + 0.165 * mb if m <= 64 else 9.2 + 0.215 * mb
+        return best[1] if max(best[0], 3.2 + mb / 4.8) < split else 0
+
+    def pairs_unsplit(self, m: int, n: int, k: int) -> bool:
+        """Whether a product that carries no norm runs unsplit on pairs of SMs with tiles of :meth:`pair_tile`'s width: from 129 tokens
+        on, but not where the single blocks would split a long K (6,144 and more) four ways or more, which matches narrow tiles'
+        k-loops there (4096 x 12288 at 256 tokens 34.8 us split, 38.9 unsplit; 2048 x 6144 at 300 tokens 19.9 and 21.0; but
+        4096 x 4096 at 256 tokens 18.3 and 17.0, 2048 x 3072 15.4 and 11.4)."""
+        if not self.use_pairs or m < self.pairs_from or self.pair_split_override:
+            return False
+        return k < 6144 or self.token_major_split(m, n, k) < 4
+
+    def pair_tile(self, m: int, n: int, k: int, gated: bool) -> int:
+        """Weight rows per tile of an unsplit product on pairs of SMs that carries no norm behind it: the width of the lowest
+        estimate, in us: 2.3 + 0.024 a weight row (start, and the epilogue of the last tile), and for every round of tiles over the
+        pairs and k-block the MMAs' time (0.00111 a weight row), what the issuing thread takes (0.16), or the operands' way from
+        the L2 (16 MB a us), whichever is longest.  Against 130 measured products of 144 to 2,048 tokens the width that it chooses is
+        within 5 percent of the best of seven.  Unlike :meth:`pair_width` it knows K: short products take narrow tiles for the
+        sake of their epilogue (2048 x 2048 at 256 tokens: 8.9 us at 64 rows, 17.5 at 256)."""
+        if self.pair_width_override:
+            return self.pair_width_override
+        pairs, m_pairs, k_blocks, best = self.sm_count // 2, -(-m // 256), -(-k // 64), None
+        for w in range(256, 63, -32 if gated else -16):
+            tiles = -(-n // w) * m_pairs
+            block = max(0.16, 0.00111 * w, min(tiles, pairs) * (256 + w) * 128 / 16e6)
+            cost = 2.3 + 0.024 * w + -(-tiles // pairs) * k_blocks * block
+            if best is None or cost < 0.99 * best[0]:
+                best = (cost, w)
+        return best[1]
+
     def plan_product(self, m: int, n: int, k: int):
         """``(token_major, splits, full_tiles, cluster)`` for a product without a folded norm."""
         if self.in_pairs(m, n, k):
@@ -335,6 +386,13 @@ class FastKernels:
         # the gate's shape of the gated epilogue: four host floats, or null for SwiGLU
         shape = None if gate_shape is None else (c_float * 4)(*[float(v) for v in gate_shape])
         gs = None if shape is None else addressof(shape)
+        if pairs == 2:
+            # unsplit on single SMs, tiles as narrow as fill the chip (gemm_narrow.cu)
+            code = self.calls.leone_gemm_narrow(x, w, out, residual, m, n_rows, k, ldx, ldw, ldc, epilogue,
+                                                width, self.status, self.sm_count, *ni, gs, bias, self._stream())
+            if code != 0:
+                raise RuntimeError(f"gemm_narrow refused or failed with code {code} for m={m} n={n_rows} k={k} width={width}")
+            return True
         if pairs:
             # pairs of SMs on tiles of 256 tokens (gemm_pair.cu)
             code = self.calls.leone_gemm_pair(x, w, out, residual, m, n_rows, k,
@@ -356,8 +414,15 @@ class FastKernels:
         """What :meth:`_gemm` does for one combination of sizes and arguments (kept per combination;
         every change of a switch of this object forgets the plans): ``(pairs, token_major, splits,
         full_tiles, cluster, workspace floats, counters, parts of a folded norm's sums, tile width
-        on pairs)``.  On pairs, ``splits`` is the number of pairs per tile."""
+        on pairs or of narrow tiles)``.  ``pairs`` is 2 for narrow tiles on single SMs; on pairs, ``splits`` is the number of pairs
+        per tile."""
         no_norm = not has_norm_in and not has_norm_out
+        if token_major is None and splits is None and no_norm and not cluster:
+            width = self.narrow_width(m, n_rows, k, epilogue == 3)
+            if width:
+                return 2, True, 1, 0, False, 0, 0, 0, width
+            if self.use_narrow and self.pairs_unsplit(m, n_rows, k):
+                return True, True, 1, 0, False, 0, 0, self.norm_parts(m, n_rows, True), self.pair_tile(m, n_rows, k, epilogue == 3)
         # on pairs of SMs unless the caller forces another form
         pairs = token_major is None and splits in (None, 1) and not cluster and self.in_pairs(m, n_rows, k)
         if pairs:
