@@ -298,29 +298,28 @@ class FastKernels:
         split = 7.3 + 0.165 * mb if m <= 64 else 9.2 + 0.215 * mb
         return best[1] if max(best[0], 3.2 + mb / 4.8) < split else 0
 
-    def pairs_unsplit(self, m: int, n: int, k: int) -> bool:
+    def pairs_unsplit(self, m: int) -> bool:
         """Whether a product that carries no norm runs unsplit on pairs of SMs with tiles of :meth:`pair_tile`'s width: from 129 tokens
-        on, but not where the single blocks would split a long K (6,144 and more) four ways or more, which matches narrow tiles'
-        k-loops there (4096 x 12288 at 256 tokens 34.8 us split, 38.9 unsplit; 2048 x 6144 at 300 tokens 19.9 and 21.0; but
-        4096 x 4096 at 256 tokens 18.3 and 17.0, 2048 x 3072 15.4 and 11.4)."""
-        if not self.use_pairs or m < self.pairs_from or self.pair_split_override:
-            return False
-        return k < 6144 or self.token_major_split(m, n, k) < 4
+        on.  A split along K is faster alone where K is long (4096 x 12288 at 256 tokens 35.1 us against 39.2), but its exchange
+        holds up the next kernel's start: a layer's products with their norms take 56.3 us unsplit and 59.3 with only the
+        2048 x 6144 one split (129 tokens; 58.5 and 62.0 at 256, 69.3 and 71.1 at 400), and 119.5 and 116.5 in the 8B shape."""
+        return self.use_pairs and m >= self.pairs_from and not self.pair_split_override
 
     def pair_tile(self, m: int, n: int, k: int, gated: bool) -> int:
-        """Weight rows per tile of an unsplit product on pairs of SMs that carries no norm behind it: the width of the lowest
-        estimate, in us: 2.3 + 0.024 a weight row (start, and the epilogue of the last tile), and for every round of tiles over the
-        pairs and k-block the MMAs' time (0.00111 a weight row), what the issuing thread takes (0.16), or the operands' way from
-        the L2 (16 MB a us), whichever is longest.  Against 130 measured products of 144 to 2,048 tokens the width that it chooses is
-        within 5 percent of the best of seven.  Unlike :meth:`pair_width` it knows K: short products take narrow tiles for the
-        sake of their epilogue (2048 x 2048 at 256 tokens: 8.9 us at 64 rows, 17.5 at 256)."""
+        """Weight rows per tile of an unsplit product on pairs of SMs that carries no norm around it: the width of the lowest
+        estimate, in us: 2.3 + 0.016 a weight row (start, and the epilogue of the last tile), and for every round of tiles over the
+        pairs and k-block the MMAs' time (0.0013 a weight row), what the issuing thread takes (0.18), or the operands' way from
+        the L2 (18 MB a us), whichever is longest.  Fitted to 56 products of 144 to 2,048 tokens and 2,048 to 24,576 weight rows, measured
+        on 7 to 11 widths each: its width is 0.3 percent slower than the best of them on average, 5.4 at most.  Unlike
+        :meth:`pair_width` it knows K: short products take narrow tiles for the sake of their epilogue (2048 x 2048 at 256
+        tokens: 8.9 us at 64 rows, 17.5 at 256)."""
         if self.pair_width_override:
             return self.pair_width_override
         pairs, m_pairs, k_blocks, best = self.sm_count // 2, -(-m // 256), -(-k // 64), None
         for w in range(256, 63, -32 if gated else -16):
             tiles = -(-n // w) * m_pairs
-            block = max(0.16, 0.00111 * w, min(tiles, pairs) * (256 + w) * 128 / 16e6)
-            cost = 2.3 + 0.024 * w + -(-tiles // pairs) * k_blocks * block
+            block = max(0.18, 0.0013 * w, min(tiles, pairs) * (256 + w) * 128 / 18e6)
+            cost = 2.3 + 0.016 * w + -(-tiles // pairs) * k_blocks * block
             if best is None or cost < 0.99 * best[0]:
                 best = (cost, w)
         return best[1]
@@ -421,7 +420,7 @@ class FastKernels:
             width = self.narrow_width(m, n_rows, k, epilogue == 3)
             if width:
                 return 2, True, 1, 0, False, 0, 0, 0, width
-            if self.use_narrow and self.pairs_unsplit(m, n_rows, k):
+            if self.use_narrow and self.pairs_unsplit(m):
                 return True, True, 1, 0, False, 0, 0, self.norm_parts(m, n_rows, True), self.pair_tile(m, n_rows, k, epilogue == 3)
         # on pairs of SMs unless the caller forces another form
         pairs = token_major is None and splits in (None, 1) and not cluster and self.in_pairs(m, n_rows, k)

@@ -76,7 +76,7 @@ def test_widths_are_what_the_kernels_take(fast, n, k):
                 assert 64 <= w <= 256 and w % step == 0
             plan = _plan(fast, m, n, k, 3 if gated else 0)
             assert (plan[0] == 2) == (fast.narrow_width(m, n, k, gated) > 0)
-            if m > 128 and fast.pairs_unsplit(m, n, k):
+            if m > 128 and fast.pairs_unsplit(m):
                 assert plan[:3] == (True, True, 1) and plan[8] == fast.pair_tile(m, n, k, gated)
 
 
@@ -85,8 +85,7 @@ def test_measured_choices(fast):
     assert fast.narrow_width(77, 2048, 6144, False) == 0            # a long K stays split
     assert fast.narrow_width(77, 151936, 4096, False) == 0
     assert fast.pair_tile(256, 2048, 2048, False) == 64 and fast.pair_tile(2048, 24576, 4096, True) >= 224
-    assert fast.pairs_unsplit(256, 4096, 4096) and not fast.pairs_unsplit(256, 4096, 12288)
-    assert not fast.pairs_unsplit(300, 2048, 6144) and fast.pairs_unsplit(1027, 2048, 6144)
+    assert not fast.pairs_unsplit(128) and fast.pairs_unsplit(129) and fast.pairs_unsplit(300)
 
 
 def test_what_a_caller_asks_for_stays(fast):
