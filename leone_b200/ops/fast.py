@@ -188,8 +188,8 @@ class FastKernels:
         return self.token_major_fill * self.sm_count <= tiles <= 2 * self.sm_count
 
     def in_pairs(self, m: int, n: int = 0, k: int = 0) -> bool:
-        """Whether an unsplit product of ``m`` tokens runs on pairs of SMs (tiles of 256 tokens,
-        the width chosen by :meth:`pair_width`): from 129 tokens on, except from 257 to 384
+        """Whether an unsplit product of ``m`` tokens with a norm around it runs on pairs of SMs (tiles of 256 tokens,
+        the width chosen by :meth:`pair_width`; one without a norm: :meth:`pairs_unsplit`): from 129 tokens on, except from 257 to 384
         tokens, where the second of two tiles of 256 would be half empty and the single-block
         kernel's three tiles of 128 measured faster (gate/up at 384 tokens 62.3 us against 67.2;
         at 640 tokens three pairs already beat five single tiles, 95.9 against 105.6).  With
