@@ -423,7 +423,8 @@ class FastKernels:
             if self.use_narrow and self.pairs_unsplit(m):
                 return True, True, 1, 0, False, 0, 0, self.norm_parts(m, n_rows, True), self.pair_tile(m, n_rows, k, epilogue == 3)
         # on pairs of SMs unless the caller forces another form
-        pairs = token_major is None and splits in (None, 1) and not cluster and self.in_pairs(m, n_rows, k)
+        pairs = token_major is None and splits in (None, 1) and not cluster and \
+            (self.in_pairs(m, n_rows, k) or (not no_norm and self._pairs_fit(m)))
         if pairs:
             ps = self.pair_split(m, n_rows, k) if no_norm else 1
             width, floats = self.pair_width(m, n_rows, epilogue == 3), 0
@@ -459,10 +460,12 @@ class FastKernels:
         (up to 32 tokens; from there to 256 the extra work in the two epilogues was measured to
         cost more than the norm kernel it replaces) and prompt-sized ones (over 256 tokens,
         where a thread owns a token row and the sums are its own).  With ``n`` and ``k``: whether
-        this ``[n x k]`` product does; one that is split in the token-major form does not."""
+        this ``[n x k]`` product does; one that is split in the token-major form does not, and where an unsplit one fits pairs of
+        SMs (:meth:`in_pairs`) none is split for it (a step of 1,027 tokens on the 1.7B
+        shape 5.80 ms with norm kernels, 5.57 without)."""
         if not (self.use_tensor_cores and self.fuse_norm and (0 < m <= self.fuse_norm_tokens or m > 256)):
             return False
-        return not (n and k and self.token_major_split(m, n, k) > 1)
+        return self._pairs_fit(m) or not (n and k and self.token_major_split(m, n, k) > 1)
 
     def norm_parts(self, m: int, n: int, pairs=None) -> int:
         """Parts of the sums of squares that a product of ``m`` tokens with ``n`` outputs leaves

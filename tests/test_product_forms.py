@@ -88,6 +88,20 @@ def test_measured_choices(fast):
     assert not fast.pairs_unsplit(128) and fast.pairs_unsplit(129) and fast.pairs_unsplit(300)
 
 
+def test_norms_are_folded_where_pairs_fit(fast):
+    for n, k in ((2048, 2048), (4096, 12288), (6144, 4096)):
+        for m in (385, 512, 600, 1027, 2048):
+            assert fast.fuses_norm(m, n, k)
+            for kw in (dict(norm_in=True), dict(norm_out=True, epilogue=2)):
+                plan = _plan(fast, m, n, k, **kw)
+                width = fast.pair_width(m, n, False)
+                assert plan[:3] == (True, True, 1) and plan[5] == 0 and plan[7] == -(-n // width) == fast.norm_parts(m, n) and plan[8] == width
+    # elsewhere as it was: not where tiles of 256 tokens would be half empty and K is split, nor from 33 to 256 tokens
+    assert not fast.fuses_norm(300, 4096, 4096) and fast.fuses_norm(300, 640, 64) and not fast.fuses_norm(100, 2048, 2048)
+    fast.use_pairs = False
+    assert not fast.fuses_norm(400, 4096, 4096)
+
+
 def test_what_a_caller_asks_for_stays(fast):
     """Forced forms, norms around the product and every switch give the plan they gave without the narrow forms."""
     cases = [dict(splits=1), dict(splits=4, cluster=True), dict(token_major=True), dict(token_major=False), dict(norm_in=True), dict(norm_out=True)]
