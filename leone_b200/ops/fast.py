@@ -281,9 +281,9 @@ class FastKernels:
         to 128 tokens, if the estimate below is under that of the swapped form's split along K.  Both in us, fitted to products of
         40, 77 and 128 tokens with 11 matrices of 2048 x 2048 to 24576 x 4096.  Narrow tiles: 3.2, 0.012 for every tile past 64, and
         for every round of tiles over the SMs and k-block 0.12 + 0.0007 a weight row (what the thread that issues the MMAs
-        takes); no less than the weights at 4.8 MB a us.  The split: 7.3 + 0.165 a MB of weights up to 64 tokens, 9.2 + 0.215
-        above (partial tiles of 128 columns are exchanged).  So K decides: 2048 x 2048 at 77 tokens 7.6 us against 10.6,
-        12288 x 2048 14.8 against 18.8, 2048 x 6144 17.0 against 14.3 (stays split).  Not for an output head, whose time is its
+        takes); no less than the weights at 6 MB a us (24576 x 4096 at 64 tokens 36.8 us against 40.7 split).  The split: 7.3 + 0.165 a
+        MB of weights up to 64 tokens, 9.2 + 0.215 above (partial tiles of 128 columns are exchanged).  So K decides: 2048 x 2048 at 77 tokens 7.5 us against 10.3,
+        12288 x 2048 11.6 against 18.5, 2048 x 6144 16.0 against 13.7 (stays split).  Not for an output head, whose time is its
         logits."""
         if not self.use_narrow or not 32 < m <= 128:
             return 0
@@ -296,7 +296,7 @@ class FastKernels:
             if best is None or cost < 0.99 * best[0]:
                 best = (cost, w)
         split = 7.3 + 0.165 * mb if m <= 64 else 9.2 + 0.215 * mb
-        return best[1] if max(best[0], 3.2 + mb / 4.8) < split else 0
+        return best[1] if max(best[0], 3.2 + mb / 6) < split else 0
 
     def pairs_unsplit(self, m: int) -> bool:
         """Whether a product that carries no norm runs unsplit on pairs of SMs with tiles of :meth:`pair_tile`'s width: from 129 tokens

@@ -83,7 +83,7 @@ def test_widths_are_what_the_kernels_take(fast, n, k):
 def test_measured_choices(fast):
     assert 16 <= fast.narrow_width(77, 2048, 2048, False) <= 32 and fast.narrow_width(77, 12288, 2048, True) == 96
     assert fast.narrow_width(77, 2048, 6144, False) == 0            # a long K stays split
-    assert fast.narrow_width(77, 151936, 4096, False) == 0
+    assert fast.narrow_width(77, 151936, 4096, False) == 0 and fast.narrow_width(64, 24576, 4096, True) == 192
     assert fast.pair_tile(256, 2048, 2048, False) == 64 and fast.pair_tile(2048, 24576, 4096, True) >= 224
     assert not fast.pairs_unsplit(128) and fast.pairs_unsplit(129) and fast.pairs_unsplit(300)
 
