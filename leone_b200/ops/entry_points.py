@@ -24,8 +24,11 @@ def _through_ctypes(fn):
         if isinstance(a, float):
             return ctypes.c_float(a)
         if isinstance(a, int):
-            # (an int without a type is a C int to ctypes)
-            return a if -(1 << 31) <= a < 1 << 31 else ctypes.c_void_p(a & (1 << 64) - 1)
+            # As 64 bits whatever its size: an int without a type is a C int to ctypes, which writes four of the eight bytes of a place
+            # on the stack, and the callee may read all eight (a stride, a stream).  One that reads an int takes the low half.
+            if not -(1 << 63) <= a < 1 << 64:
+                raise OverflowError("an argument does not fit 64 bits")
+            return ctypes.c_longlong(a)
         return ctypes.c_void_p(a.data_ptr())
 
     return lambda *args: fn(*[as_argument(a) for a in args])

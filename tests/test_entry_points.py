@@ -24,6 +24,11 @@ extern "C" int many(void* p, int a1, float f1, int a2, int a3, long long a4, voi
   out[0] = (int)(h & 0x7fffffff);
   return -3;
 }
+// places on the stack that the callee reads as 64 bits
+extern "C" int wide(int, int, int, int, int, int, int a, long long b, long long c, void* d, long long e, long long* out) {
+  out[0] = a; out[1] = b; out[2] = c; out[3] = (long long)d; out[4] = e;
+  return 0;
+}
 """
 
 
@@ -61,6 +66,27 @@ def test_arguments_arrive(lib, native, monkeypatch):
     assert int(out[0]) == h & 0x7FFFFFFF
     with pytest.raises((AttributeError, TypeError)):
         calls.few("x", 1.0, 1, 1)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_small_numbers_in_64_bit_places(lib, native, monkeypatch):
+    """Zero, small and negative numbers behind the sixth integer, where the stack held other bits before."""
+    if native:
+        if entry_points._bind() is entry_points._through_ctypes:
+            pytest.skip("the extension is not built here")
+    else:
+        monkeypatch.setattr(entry_points, "_BIND", entry_points._through_ctypes)
+    calls = entry_points.EntryPoints(lib)
+    out = torch.zeros(5, dtype=torch.int64)
+    full = (1 << 62) + 0x5A5A5A5A5A5A5A5A % (1 << 60)
+    for row in ([0, 0, 0, 0, 0], [-1, 5, -5, 0, 7], [3, -1, 1, 1 << 20, -(1 << 31)], [9, 1 << 31, -(1 << 31) - 1, (1 << 64) - 16, 0],
+                [2, (1 << 31) - 1, 0, 0, -2]):
+        assert calls.wide(*[full] * 11, out) == 0
+        assert calls.wide(1, 2, 3, 4, 5, 6, *row, out) == 0
+        assert out.tolist() == [*row[:3], row[3] if row[3] < 1 << 63 else row[3] - (1 << 64), row[4]]
+    for too_long in (1 << 64, -(1 << 63) - 1):
+        with pytest.raises(OverflowError):
+            calls.wide(1, 2, 3, 4, 5, 6, 7, too_long, 9, 10, 11, out)
 
 
 def test_tails_of_block_tables():
