@@ -52,7 +52,7 @@ MODULES: Dict[str, List[str]] = {
 HOST_ONLY = {"host", "call"}
 OPTIONAL = {"call"}                # what the package does without where it cannot be built
 HEADERS = ["common.cuh", "mma_tile.cuh", "tc_common.cuh", "gemm_parts.cuh", "leone_static.h", "attention_tiled.cu", "random_draw.h",
-           "gla_parts.cuh", "ssd_parts.cuh", "experts_tc.h", "gemm_f32.h"]
+           "pair_sums.h", "gla_parts.cuh", "ssd_parts.cuh", "experts_tc.h", "gemm_f32.h"]
 
 # -fno-gnu-unique: statics inside inline functions and templates (the once-per-kernel set-up
 # flags, the launch mode switch) must belong to one library image each; with GNU unique

@@ -24,6 +24,7 @@
 // and the block goes on to the end, where one cluster barrier keeps either block's shared
 // memory and barriers alive until both are done.
 #include "gemm_parts.cuh"
+#include "pair_sums.h"
 
 namespace leone {
 namespace tc {
@@ -31,7 +32,9 @@ constexpr int kPairMaxStages = 10;
 constexpr int kPairEpilogueWarps = 8;               // two for every 32 rows: each finishes half of the tile's columns
 constexpr int kPairThreads = 64 + 32 * kPairEpilogueWarps;
 constexpr int kPairSmemLimit = 227 * 1024 - 64;        // dynamic shared memory of a block (the static part is beside it)
-constexpr int kPairSumsBytes = 2 * 4 * 32 * 4;         // two buffers of the sums of squares that pass between the epilogue's halves
+constexpr int kPairBarrierBytes = 320;
+constexpr int kPairSumsBytes = kSumsBarriers * 32 * 4; // the sums of squares that pass between the epilogue's halves (pair_sums.h)
+static_assert(8 * (2 * kPairMaxStages + 6 + kSumsBarriers) <= kPairBarrierBytes, "the barriers' place");
 
 // Shared memory of a pair's block for tiles of bn weight rows: stages of 128 token rows and bn / 2
 // weight rows (each operand tile starts on a 1024-byte boundary, as the 128-byte swizzle wants).
@@ -44,7 +47,7 @@ __host__ __device__ inline PairShape pair_shape(int bn, int blocks) {
   c.b_bytes = (c.half * kTileK * 2 + 1023) & ~1023;
   c.blocks = blocks;
   c.stage_bytes = c.blocks * (kTileW * kTileK * 2 + c.b_bytes);
-  constexpr int other = 1024 /*alignment*/ + 256 /*barriers*/ + kPairSumsBytes + kPairEpilogueWarps * kBoxBytes;
+  constexpr int other = 1024 /*alignment*/ + kPairBarrierBytes + kPairSumsBytes + kPairEpilogueWarps * kBoxBytes;
   c.stages = (kPairSmemLimit - other) / c.stage_bytes;
   if (c.stages > kPairMaxStages) c.stages = kPairMaxStages;
   c.smem_bytes = c.stages * c.stage_bytes + other;
@@ -140,7 +143,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   // and for the split mode: the pieces of a chunk have landed, and all four warps have read them
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kStages;
   const uint32_t acc_full0 = empty0 + 8 * kStages, acc_empty0 = acc_full0 + 16;
-  // and, where a norm follows, the second half's sums of squares of a quarter of the rows are in place (4)
+  // and, where a norm follows, the second half's sums of squares of a buffer and quarter of the rows are in place (8)
   const uint32_t landed = acc_empty0 + 16, pieces_read = landed + 8, sums_there = pieces_read + 8;
   __shared__ uint32_t tmem_holder;
   __shared__ int gave_up;
@@ -171,7 +174,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       mbar_init(acc_empty0 + 8 * b, 2 * kPairEpilogueWarps);     // the epilogue warps of both blocks (used in the first)
     }
     mbar_init(landed, 1);
-    for (int q = 0; q < 4; ++q) mbar_init(sums_there + 8 * q, 1);
+    for (int q = 0; q < kSumsBarriers; ++q) mbar_init(sums_there + 8 * q, 1);
     mbar_init(pieces_read, (uint32_t)(BN / 32));
     mbar_fence_init();
     tma_prefetch_desc(&map_w);
@@ -281,9 +284,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int half = (warp - 2) >> 2;                 // which columns of the tile
     const int unit = p.epilogue == 3 || S > 1 ? 32 : 16, middle = (BN / unit + 1) / 2 * unit;
     const int c_lo = half == 0 ? 0 : middle, c_hi = half == 0 ? middle : BN;
-    float* sums = reinterpret_cast<float*>(bars + 32);
-    const uint32_t box = smem_u32(bars) + 256 + kPairSumsBytes + (warp - 2) * kBoxBytes;
+    float* sums = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kPairBarrierBytes);
+    const uint32_t box = smem_u32(bars) + kPairBarrierBytes + kPairSumsBytes + (warp - 2) * kBoxBytes;
     int it = 0;
+    SumsHandover handover;
     pdl_wait();      // outputs and residual may be in use until here
     for (int t = pair; t < total && !*giveup; t += pairs, ++it) {
       const int m_tile = (t % m_pairs) * 2 + (int)rank, n_tile = t / m_pairs;
@@ -296,9 +300,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         return ok;
       };
       // the two warps of these rows each have the sums of squares of half of the tile's columns: the second hands its own to
-      // the first (its next tile's go to the other buffer, and the one after that waits for this tile's release)
+      // the first.  (Not called where the rows lie past the last token.)
       auto squares = [&](const float (&s)[8]) {
-        float* there = sums + (buf * 4 + quarter) * 32;
+        const int place = SumsHandover::place(buf, quarter);
+        const unsigned parity = handover.next(buf);
+        float* there = sums + place * 32;
         const int row = lane >> 3;
         if (half == 1) {
           if ((lane & 7) == 0) {
@@ -306,8 +312,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             for (int i = 0; i < 8; ++i) there[4 * i + row] = s[i];
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive(sums_there + 8 * quarter);
-        } else if (mbar_wait(sums_there + 8 * quarter, it & 1, giveup) && (lane & 7) == 0) {
+          if (lane == 0) mbar_arrive(sums_there + 8 * place);
+        } else if (mbar_wait(sums_there + 8 * place, parity, giveup) && (lane & 7) == 0) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int m = m_tile * kTileW + quarter * 32 + 4 * i + row;

@@ -135,6 +135,36 @@ def test_real_layer_sizes_a_prompt_on_pairs_of_sms(setup):
         torch.cuda.empty_cache()
 
 
+def test_real_layer_sizes_a_prompt_with_ragged_tiles_in_several_rounds():
+    """A prompt of 1,100 tokens of the 8B shape in one step: the products with a norm behind them have more tiles than there are
+    pairs of SMs, the last of them ragged."""
+    from leone_b200.config.qwen3 import Qwen3Config
+    from leone_b200.engine.engine import Engine
+    cfg = _cfg("8b", positions=2048)
+    tensors = _plain_weights(cfg)
+    reqs = {"a": replay.random_tokens(VOCAB, 1100, 9)}
+    want = _plain_logits(cfg, tensors, reqs["a"], True).cpu()
+    del tensors
+    torch.cuda.empty_cache()
+
+    class Plain:
+        def logits(self, tokens):
+            return want
+
+    steps = replay.trace_whole(reqs)
+    for st in steps:
+        for e in st["entries"]:
+            e["want"] = [w for w in e["want"] if w % 29 == 0 or w == len(e["tokens"]) - 1]
+    engine = Engine.from_config(Qwen3Config.from_dict(cfg), SEED, dtype="bfloat16", page_tokens=16,
+                                max_tokens=replay.max_live_tokens(steps), max_requests=2, max_batch_tokens=1152)
+    if not engine.ops.fast.use_pairs:
+        pytest.skip("LEONE_NO_PAIRS is set")
+    assert engine.ops.fast.fuses_norm(1100, 4096, 4096) and engine.ops.fast.norm_parts(1100, 4096) * 5 > engine.ops.fast.sm_count // 2
+    out = replay.run_trace_engine(engine, steps)
+    worst = replay.compare(steps, out, Plain(), reqs, *replay.tolerance("bfloat16"), "8b layer sizes, 1,100 tokens on pairs")
+    replay.check_worst(("real-pairs-rounds", "8b"), worst)
+
+
 @pytest.mark.parametrize("context", [5, 130, 2100])
 def test_decode_graph_at_the_models_real_position_limit(context):
     """A real ``config.json`` allows 40,960 positions.  The captured decode step must give the
