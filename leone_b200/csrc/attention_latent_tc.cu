@@ -255,7 +255,7 @@ attention_latent_tc_kernel(const Params p) {
       float m_run = -INFINITY, l_run = 0.f;
       if (p.sink != nullptr && here) {                           // the sink is the first score
         m_run = (p.sink_bf16 ? __bfloat162float(((const __nv_bfloat16*)p.sink)[head]) : ((const float*)p.sink)[head]) * kLog2e;
-        l_run = 1.f;
+        l_run = m_run == -INFINITY ? 0.f : 1.f;                  // (a sink of -inf, or one that is after the factor, has no weight)
       }
       const int first_seen = p.window > 0 ? max(0, pos - p.window + 1) : 0;
       bool ok = true;
@@ -332,8 +332,8 @@ attention_latent_tc_kernel(const Params p) {
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
       if (ok) {
-        const bool zeros = *(volatile int*)&bad != 0 || !(l_run > 0.f);
-        float f = zeros ? 0.f : 1.f / l_run;
+        const bool zeros = *(volatile int*)&bad != 0;            // (a sum that is NaN stays one: its outputs are too)
+        float f = l_run > 0.f ? 1.f / l_run : 0.f;
         if (p.gate != nullptr && here) f *= 1.f / (1.f + expf(-__bfloat162float(p.gate[(size_t)(q0 + tok) * p.ldg + head])));
         uint4* dst = reinterpret_cast<uint4*>(p.out + ((size_t)(q0 + (here ? tok : tok0)) * p.heads + (here ? head : h0)) * kDv + half * kHalf);
         for (int c = 0; c < kHalf; c += 32) {

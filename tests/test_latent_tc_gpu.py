@@ -113,3 +113,26 @@ def test_a_missing_page_is_reported(ops):
     out = torch.empty((100, 16 * DV), device=DEV, dtype=torch.bfloat16)
     ops.attention_latent(ctx, q, out, cache, 16, DK, DV, DK ** -0.5, None)
     assert int(ctx.status[0]) == 2 and int(ctx.status[3]) in range(32, 48)
+
+
+def test_sinks_without_weight_and_rows_that_are_nan(ops, monkeypatch):
+    """A sink of -inf, or of the type's lowest value, adds nothing to the denominator; a query that is NaN gives NaN in its token's rows
+    and in no other's.  As in the other kernel."""
+    ctx, cache, q, rows = _case([40, 30], [0, 100], 16, 16, 21, stale=0.0)
+    sink = torch.randn(16, device=DEV, generator=torch.Generator(device=DEV).manual_seed(8))
+    sink[3], sink[7], sink[9] = float("-inf"), torch.finfo(torch.float32).min, torch.finfo(torch.bfloat16).min
+    want = _exact([40, 30], [0, 100], 16, q, rows, DK ** -0.5, 50, sink, None)
+    for form in ("0", "1"):
+        monkeypatch.setenv("LEONE_NO_LATENT_TC", form)
+        for s_ in (sink, sink.to(torch.bfloat16)):
+            out = torch.empty((70, 16 * DV), device=DEV, dtype=torch.bfloat16)
+            ops.attention_latent(ctx, q, out, cache, 16, DK, DV, DK ** -0.5, 50, s_)
+            heads = (out.double() - want).view(70, 16, DV)[:, [3, 7, 9]]
+            assert float(heads.norm() / want.view(70, 16, DV)[:, [3, 7, 9]].norm()) < 4e-3        # as in test_against_float64
+        poisoned = q.clone()
+        poisoned[13, 5] = float("nan")                      # head 0 of token 13
+        out = torch.empty((70, 16 * DV), device=DEV, dtype=torch.bfloat16)
+        ops.attention_latent(ctx, poisoned, out, cache, 16, DK, DV, DK ** -0.5, 50, sink)
+        nan = out.view(70, 16, DV).isnan()
+        assert bool(nan[13, 0].all()) and int(nan.sum()) == DV
+    assert int(ctx.status.abs().sum()) == 0
