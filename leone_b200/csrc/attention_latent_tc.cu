@@ -22,6 +22,8 @@
 // A tile's chain bounds it (the gather of 73 KB, scores, softmax), not the tensor cores.  One sequence of 2,048 tokens, 16 heads, a
 // window of 1,024: 415 us in the mma.sync form, 197 in this (0.17 of the bf16 rate, from 0.08); a prompt of the eight-layer decoder
 // with two such layers 4.51 to 4.08 ms.  Its error against 64 bits is no larger than that form's.
+// A tile walks its keys alone, so few tokens behind many keys take the other form, which splits them over blocks (8 tokens behind 16,384:
+// 824 us here, 150 there); the rule and its measurements are latent_times in ops/cuda.py.
 #include "tc_common.cuh"
 
 namespace leone {

@@ -63,6 +63,53 @@ def _need(cond: bool, msg: str) -> None:
         raise KernelError(msg)
 
 
+def latent_times(q_lens, ctx_lens, groups: int, window, lead: int, sms: int = 148):
+    """What a step's latent attention takes in us, ``(tcgen05, mma.sync)``: sequences of ``q_lens`` tokens that end at ``ctx_lens``,
+    ``groups`` groups of 16 heads, the first ``lead`` sequences decode rows (which the mma.sync form takes either way).
+
+    The forms differ in what they do with many keys and few tokens.  On tcgen05 a tile of eight tokens walks all its keys in two
+    blocks: 12 us and 3.2 for every 64 keys.  The other form splits the keys of up to 74 (token, head group) pairs over blocks: 10 us and
+    7.8 for every 64 keys of a split; from there on it walks them whole, 2 us (7 with four tokens a block, from 64 tokens) and 7.3.
+    A block each an SM, so more blocks than SMs take rounds.  Fitted to 1 to 16 sequences of 2 to 2,048 tokens behind 0 to 32,768 cached ones, 16 to 128 heads, with and
+    without a window.  8 tokens behind 16,384: 824 us on tcgen05, 150 in the other form; 48: 824 and 681; 64: 823 and 1,012;
+    8 tokens behind 1,024: 68 and 31; a prompt of 2,048: 233 and 562, of 64: 15.4 and 14.2, of 96: 17.8 and 20.7."""
+    q, ctx = np.asarray(q_lens, dtype=np.int64), np.asarray(ctx_lens, dtype=np.int64)
+
+    def tiles_of(ctx, tokens):                        # of 64 keys, that `tokens` tokens up to the one at ctx read together
+        return -(-(np.minimum(ctx, window + tokens - 1) if window else ctx) // 64)
+
+    def mma(q, ctx):
+        n = int(q.sum())
+        splits = latent_splits(n * groups, int(tiles_of(ctx, 1).max()))
+        if splits > 1:
+            return 10 + 7.8 * -(-int(tiles_of(ctx, 1).max()) // splits)
+        per, start = (4, 7) if n >= 64 else (1, 2)    # tokens of a block
+        blocks, longest = -(-q // per) * groups, tiles_of(ctx, per)
+        each = start + 3.65 * (tiles_of(ctx - q + np.minimum(q, per), per) + longest)          # on average
+        rounds = float((blocks * each).sum()) / sms + (float(each.mean()) / 2 if blocks.sum() > sms else 0)
+        return max(start + 7.3 * int(longest.max()), rounds)
+
+    def tcgen05(q, ctx):
+        blocks, longest = 2 * groups * -(-q // 8), tiles_of(ctx, 8)
+        each = 12 + 1.6 * (tiles_of(ctx - q + np.minimum(q, 8), 8) + longest)
+        return max(12 + 3.2 * int(longest.max()), float((blocks * each).sum()) / sms)
+
+    other = mma(q, ctx)
+    return tcgen05(q[lead:], ctx[lead:]) + (mma(q[:lead], ctx[:lead]) if lead else 0), other
+
+
+def latent_portions_are_long(tokens: int, seqs: int, max_ctx_len: int, window) -> bool:
+    """Whether :func:`latent_times` need not be asked of a step without decode rows: portions of so many tokens that the mma.sync form splits no keys, of eight
+    and more on average, and contexts of two tiles of keys and more."""
+    return tokens >= max(96, 8 * seqs) and (min(max_ctx_len, window) if window else max_ctx_len) > 64
+
+
+def latent_splits(rows: int, tiles: int) -> int:
+    """Blocks that share the keys (``tiles`` of 64) of each of ``rows`` (token, group of 16 heads) pairs in the mma.sync form of
+    the latent attention: until the SMs are busy."""
+    return max(1, min(16, tiles, 148 // max(rows, 1)))
+
+
 class PreparedMatrix:
     """A weight matrix ``[out, in]`` with what the kernels precompute for it, and the bias ``[out]`` (fp32, or
     None) that every product with it adds to its sums."""
@@ -102,7 +149,7 @@ class CudaOps:
             from .fast import FastKernels
             self.fast = FastKernels(self.device)
         self.launches = 0
-        self.latent_tc_from = 8            # tokens of a portion from which latent attention runs on tcgen05
+        self.use_latent_tc = None          # True, False: latent attention of prompt portions on tcgen05 or not, whatever the rule says
         self._sample_scratch = None
         self.status = None
         # LEONE_NO_PDL=1 launches every kernel fully serialised after its predecessor
@@ -771,10 +818,12 @@ class CudaOps:
         if sink is not None:
             _need(sink.numel() == heads and sink.is_contiguous(), "attention_latent sink")
         q_start = getattr(ctx, "q_start", None)
-        if (q_abs.dtype == torch.bfloat16 and not ctx.decode_only and q_start is not None and ctx.max_q_len >= self.latent_tc_from
-                and os.environ.get("LEONE_NO_LATENT_TC", "0") != "1" and scale > 0
-                and self.mixers.leone_attention_latent_tc_supported(dk, dv)
-                and not (q_abs.data_ptr() | out.data_ptr() | kp.data_ptr()) & 15):
+        mma = (q_abs.dtype == torch.bfloat16 and os.environ.get("LEONE_NO_LATENT_MMA", "0") != "1"
+               and self.mixers.leone_attention_latent_mma_supported(dk, dv))
+        if (q_abs.dtype == torch.bfloat16 and not ctx.decode_only and q_start is not None and scale > 0
+                and os.environ.get("LEONE_NO_LATENT_TC", "0") != "1" and self.mixers.leone_attention_latent_tc_supported(dk, dv)
+                and not (q_abs.data_ptr() | out.data_ptr() | kp.data_ptr()) & 15
+                and (not mma or self._latent_on_tcgen05(ctx, n, -(-heads // 16), int(window or 0)))):
             # prompt portions on tcgen05, eight tokens of a sequence a tile; in a mixed step the decode rows in front, each of
             # which would be such a tile, take the form below
             lead = self._leading_single_rows(ctx)
@@ -790,12 +839,11 @@ class CudaOps:
         else:
             max_ctx_len = ctx.max_ctx_len
         self.launches += 1
-        if (q_abs.dtype == torch.bfloat16 and os.environ.get("LEONE_NO_LATENT_MMA", "0") != "1"
-                and self.mixers.leone_attention_latent_mma_supported(dk, dv)):
-            # few tokens (decode): a token's keys are split over blocks until the SMs are busy
+        if mma:
+            # few tokens (decode): a token's keys are split over blocks
             groups = -(-heads // 16)
             keys = min(int(window), max_ctx_len) if window else max_ctx_len
-            splits = max(1, min(16, -(-keys // 64), 148 // max(n * groups, 1)))
+            splits = latent_splits(n * groups, -(-keys // 64))
             partial = None
             if splits > 1:
                 partial = self._scratch("latent_partial", n * groups * splits * 16, dv + 2, torch.float32)
@@ -812,6 +860,22 @@ class CudaOps:
             ctx.positions, n, heads, dk, dv, float(scale), int(window or 0), sink,
             0 if sink is None else _dt(sink.dtype), gate, 0 if gate is None else gate.stride(0),
             cache.page_tokens, kp.shape[0], bt.shape[0], ctx.status, self._stream()), "attention_latent")
+
+    def _latent_on_tcgen05(self, ctx, n: int, groups: int, window: int) -> bool:
+        """Whether the prompt portions of a step of ``n`` tokens take the tcgen05 form of the latent attention."""
+        if self.use_latent_tc is not None:
+            return self.use_latent_tc
+        q_lens, ctx_lens = getattr(ctx, "q_lens", None), getattr(ctx, "ctx_lens", None)
+        if q_lens is None or ctx_lens is None:
+            return n >= 96
+        lead = self._leading_single_rows(ctx)
+        if lead == 0 and latent_portions_are_long(n, ctx.n_seqs, ctx.max_ctx_len, window):
+            return True
+        known = ctx.__dict__.setdefault("_latent_on_tcgen05", {})      # once a step and window (50 us)
+        if (groups, window) not in known:
+            tcgen05, mma = latent_times(q_lens, ctx_lens, groups, window, lead)
+            known[groups, window] = tcgen05 < mma
+        return known[groups, window]
 
     def experts_route(self, x, w_router, chosen, weight, top, softmax=False, renormalize=False, groups=1,
                       groups_kept=None, weight_scale=1.0, bias=None, experts=None, correction=None):

@@ -15,6 +15,7 @@ def ops():
     from leone_b200.ops.cuda import CudaOps
     o = CudaOps(DEV, torch.bfloat16)
     o.bind_status(torch.zeros(4, dtype=torch.int32, device=DEV))
+    o.use_latent_tc = True              # also where the rule takes the other kernel
     return o
 
 
