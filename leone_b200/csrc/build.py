@@ -23,7 +23,7 @@ import tempfile
 import threading
 import time
 from concurrent.futures import ThreadPoolExecutor
-from typing import Dict, List
+from typing import Dict, List, Optional
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -98,6 +98,8 @@ def build_dir() -> str:
 def _digest(module: str) -> str:
     h = hashlib.sha256()
     h.update(" ".join(HOST_FLAGS if module in HOST_ONLY else NVCC_FLAGS).encode())
+    if module == "call":
+        h.update(f"{sys.version} {sysconfig.get_config_var('SOABI')}".encode())
     for name in MODULES[module] + HEADERS:
         path = os.path.join(HERE, name)
         if os.path.isfile(path):
@@ -107,8 +109,11 @@ def _digest(module: str) -> str:
     return h.hexdigest()
 
 
-def library_path(module: str) -> str:
-    return os.path.join(build_dir(), f"libleone_{module}.so")
+def library_path(module: str, out_dir: Optional[str] = None) -> str:
+    """Where the module's library is, or will be.  ``call`` uses the interpreter's own structures, so each interpreter that shares
+    this directory has one of its own, named by its ABI."""
+    abi = f".{sysconfig.get_config_var('SOABI') or sys.implementation.cache_tag}" if module == "call" else ""
+    return os.path.join(out_dir or build_dir(), f"libleone_{module}{abi}.so")
 
 
 def _run_with_heartbeat(cmd: List[str], what: str) -> None:
@@ -135,7 +140,7 @@ def ensure_built(module: str, verbose: bool = True) -> str:
     if module not in MODULES:
         raise BuildError(f"unknown kernel module '{module}'")
     out_dir = build_dir()
-    lib = os.path.join(out_dir, f"libleone_{module}.so")
+    lib = library_path(module, out_dir)
     stamp = lib + ".stamp"
     digest = _digest(module)
 

@@ -68,6 +68,21 @@ def test_arguments_arrive(lib, native, monkeypatch):
         calls.few("x", 1.0, 1, 1)
 
 
+def test_the_extension_belongs_to_its_interpreter(monkeypatch):
+    """Another interpreter, or another version of it, neither finds this one's file nor takes it for its own."""
+    import sys
+    import sysconfig
+    from leone_b200.csrc import build
+    path, digest, others = build.library_path("call"), build._digest("call"), {m: build.library_path(m) for m in build.MODULES if m != "call"}
+    real = sysconfig.get_config_var
+    monkeypatch.setattr(sysconfig, "get_config_var", lambda name: "cpython-399-test" if name == "SOABI" else real(name))
+    assert build.library_path("call") != path and build._digest("call") != digest
+    monkeypatch.undo()
+    monkeypatch.setattr(sys, "version", sys.version + "+1")
+    assert build.library_path("call") == path and build._digest("call") != digest
+    assert others == {m: build.library_path(m) for m in others}
+
+
 @pytest.mark.parametrize("native", [True, False])
 def test_small_numbers_in_64_bit_places(lib, native, monkeypatch):
     """Zero, small and negative numbers behind the sixth integer, where the stack held other bits before."""
