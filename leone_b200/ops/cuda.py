@@ -312,6 +312,10 @@ class CudaOps:
         the norm after it."""
         return self.fast.norm_parts(n_tokens, n)
 
+    def norm_sums_floats(self, max_tokens: int, n: int) -> int:
+        """The most floats the ``ss`` buffer needs for steps of up to ``max_tokens`` tokens."""
+        return self.fast.norm_sums_floats(max_tokens, n)
+
     def _norm_args(self, m, w, norm_in, norm_out):
         ni = no = None
         if norm_in is not None:

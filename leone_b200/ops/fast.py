@@ -476,6 +476,16 @@ class FastKernels:
             return -(-n // self.pair_width(m, n, False))
         return int(self.lib.leone_gemm_tc_norm_parts(m, n))
 
+    def norm_sums_floats(self, max_tokens: int, n: int) -> int:
+        """The most floats that products with ``n`` outputs of up to ``max_tokens`` tokens leave for the norm after them
+        (:meth:`norm_parts` times the tokens).  Not the parts of the largest step: one of 512 tokens with 2,048 outputs leaves 32, one
+        of 2,048 tokens 9.  The parts are the same for up to 32 tokens and for every 128 from there on."""
+        key = ("sums", max_tokens, n)
+        if key not in self._pair_widths:
+            steps = [min(max_tokens, self.fuse_norm_tokens), *range(384, max_tokens, 128), max_tokens]
+            self._pair_widths[key] = max((m * self.norm_parts(m, n) for m in steps if self.fuses_norm(m)), default=0)
+        return self._pair_widths[key]
+
     def linear(self, x, w, out, epilogue, residual, norm_in=None, norm_out=None) -> bool:
         return self._product(x, w, out, epilogue, residual, norm_in, norm_out)
 

@@ -173,15 +173,14 @@ class DeferredNorm:
     def prepare(self, rt, parts: int) -> None:
         """Buffers for a step of ``n`` tokens: ``xn [n, size]`` and the partial sums ``ss
         [parts, n]``, a view of one flat allocation per tag that is large enough for any step
-        (``parts`` never exceeds the row width; a step never exceeds ``rt.max_tokens``), so its
+        (a step never exceeds ``rt.max_tokens``), so its
         address is the same for every step size and a captured graph keeps seeing it."""
         n, size = self.hidden.shape
         self.parts = parts
         self.xn = rt.buffer(f"deferred_norm_x_{self.tag}", n, size, rt.dtype)
-        # up to 32 tokens a part is 32 weight rows (parts * n <= size); prompt-sized steps have a
-        # part per tile of at least 240 weight rows: reserve for the larger of the two at once
+        # the parts follow the tiles of each step's product: the most that any step leaves is reserved at once
         flat = rt.flat_buffer(f"deferred_norm_ss_{self.tag}", parts * n, torch.float32,
-                              reserve=max(size, (size // 240 + 2) * rt.max_tokens))
+                              reserve=rt.ops.norm_sums_floats(rt.max_tokens, size))
         self.ss = flat[:parts * n].view(parts, n)
 
     def materialize(self) -> torch.Tensor:

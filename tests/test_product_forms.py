@@ -124,3 +124,25 @@ def test_what_a_caller_asks_for_stays(fast):
     assert _plan(fast, 512, 2048, 2048)[2] == 2
     fast.pair_split_override, fast.use_pairs = 0, False
     assert _plan(fast, 512, 2048, 2048)[0] is False
+
+
+@pytest.mark.parametrize("max_tokens,size", [(24, 2048), (200, 2048), (512, 2048), (512, 4096), (1100, 4096), (2048, 2048), (2048, 5120), (3000, 1024)])
+def test_a_norms_sums_are_allocated_once(fast, monkeypatch, max_tokens, size):
+    """A decode step first, then steps of every size up to the largest: the buffer of the sums of squares stays where it is."""
+    import types
+
+    import torch
+    from leone_b200.parts.base import DeferredNorm, Runtime
+    # as the library has it: 32 weight rows a part for few tokens, tiles of at least 240 for prompts on single SMs
+    monkeypatch.setattr(_Sizes, "leone_gemm_tc_norm_parts", staticmethod(lambda m, n: -(-n // (32 if m <= 256 else 240))))
+    rt = Runtime("cpu", torch.bfloat16, types.SimpleNamespace(norm_sums_floats=fast.norm_sums_floats), max_tokens)
+    at, most = set(), 0
+    for m in [*range(1, 33, 5), 32, *range(257, max_tokens, 37), *range(384, max_tokens, 128), *range(385, max_tokens, 128), max_tokens]:
+        if m > max_tokens or not fast.fuses_norm(m):
+            continue
+        d = DeferredNorm(None, None, torch.empty((m, size)), None, 1e-6)
+        d.prepare(rt, fast.norm_parts(m, size))
+        at.add(d.ss.data_ptr())
+        most = max(most, d.ss.numel())
+    assert len(at) == 1
+    assert fast.norm_sums_floats(max_tokens, size) >= most
