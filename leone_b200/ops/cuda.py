@@ -98,10 +98,15 @@ def latent_times(q_lens, ctx_lens, groups: int, window, lead: int, sms: int = 14
     return tcgen05(q[lead:], ctx[lead:]) + (mma(q[:lead], ctx[:lead]) if lead else 0), other
 
 
-def latent_portions_are_long(tokens: int, seqs: int, max_ctx_len: int, window) -> bool:
-    """Whether :func:`latent_times` need not be asked of a step without decode rows: portions of so many tokens that the mma.sync form splits no keys, of eight
-    and more on average, and contexts of two tiles of keys and more."""
-    return tokens >= max(96, 8 * seqs) and (min(max_ctx_len, window) if window else max_ctx_len) > 64
+def latent_short_answer(tokens: int, seqs: int, groups: int, max_ctx_len: int, window) -> Optional[bool]:
+    """Where a step without decode rows need not ask :func:`latent_times` (50 us of the host): True (tcgen05) for portions
+    of eight tokens and more on average, so many that the mma.sync form splits no keys, and contexts of two tiles of keys and more; False
+    for so few tokens that it splits the keys at least four ways; else None."""
+    if tokens * groups <= 37:
+        return False
+    if tokens >= max(96, 8 * seqs) and (min(max_ctx_len, window) if window else max_ctx_len) > 64:
+        return True
+    return None
 
 
 def latent_splits(rows: int, tiles: int) -> int:
@@ -873,9 +878,10 @@ class CudaOps:
         if q_lens is None or ctx_lens is None:
             return n >= 96
         lead = self._leading_single_rows(ctx)
-        if lead == 0 and latent_portions_are_long(n, ctx.n_seqs, ctx.max_ctx_len, window):
-            return True
-        known = ctx.__dict__.setdefault("_latent_on_tcgen05", {})      # once a step and window (50 us)
+        answer = latent_short_answer(n, ctx.n_seqs, groups, ctx.max_ctx_len, window) if lead == 0 else None
+        if answer is not None:
+            return answer
+        known = ctx.__dict__.setdefault("_latent_on_tcgen05", {})      # once a step and window
         if (groups, window) not in known:
             tcgen05, mma = latent_times(q_lens, ctx_lens, groups, window, lead)
             known[groups, window] = tcgen05 < mma

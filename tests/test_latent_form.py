@@ -1,10 +1,10 @@
 """Which form of the latent attention a step's prompt portions take, on the CPU: the estimate against times measured of both forms, and
-the short answer for long portions against the estimate."""
+the short answers against the estimate."""
 import random
 
 import pytest
 
-from leone_b200.ops.cuda import latent_portions_are_long, latent_times
+from leone_b200.ops.cuda import latent_short_answer, latent_times
 
 # tokens, cached tokens before them, sequences, heads, window, us on tcgen05, us on mma.sync
 MEASURED = [
@@ -23,15 +23,16 @@ def test_the_faster_form_is_chosen(q, before, seqs, heads, window, tcgen05, mma)
     assert (a < b) == (tcgen05 < mma)
 
 
-def test_long_portions_need_no_estimate():
+def test_short_answers_agree_with_the_estimate():
     rng = random.Random(5)
-    asked = 0
-    for _ in range(3000):
-        q = [max(2, int(2 ** rng.uniform(1, 11))) for _ in range(rng.randint(1, 12))]
+    given = {True: 0, False: 0}
+    for _ in range(4000):
+        q = [max(1, int(2 ** rng.uniform(0, 11))) for _ in range(rng.choice([1, 1, 2, rng.randint(1, 12)]))]
         ctx = [n + int(2 ** rng.uniform(0, 15)) - 1 for n in q]
-        window = rng.choice([0, 0, 100, 1024])
-        if latent_portions_are_long(sum(q), len(q), max(ctx), window):
-            a, b = latent_times(q, ctx, rng.choice([1, 2, 8]), window, 0)
-            assert a < 1.25 * b, (q, ctx, window, a, b)
-            asked += 1
-    assert asked > 500
+        window, groups = rng.choice([0, 0, 100, 1024]), rng.choice([1, 2, 8])
+        answer = latent_short_answer(sum(q), len(q), groups, max(ctx), window)
+        if answer is not None:
+            a, b = latent_times(q, ctx, groups, window, 0)
+            assert a < 1.25 * b if answer else b < a, (q, ctx, window, groups, a, b)
+            given[answer] += 1
+    assert min(given.values()) > 300
