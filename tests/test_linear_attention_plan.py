@@ -38,7 +38,8 @@ def _plan(q_lens, heads, dim, vdim, dtype=torch.bfloat16, chunk=64):
                                 q_start=torch.zeros(len(q_lens) + 1, dtype=torch.int32),
                                 slot_ids=torch.zeros(len(q_lens), dtype=torch.int32), status=torch.zeros(4, dtype=torch.int32))
     cols = heads * (2 * dim + vdim)
-    ops.linear_attention(ctx, torch.zeros((n, cols), dtype=dtype), torch.zeros((n, heads * vdim)),
+    # (nothing reads them, and clearing gigabytes would take the caller's time limit on a slow host)
+    ops.linear_attention(ctx, torch.empty((n, cols), dtype=dtype), torch.empty((n, heads * vdim)),
                          torch.zeros((1, heads, dim, vdim)), torch.ones(heads), heads, dim, vdim, 0, heads * dim, 2 * heads * dim,
                          chunk=chunk)
     return scratch, [c for c in lib.calls if not c[0].endswith("_supported")]
