@@ -9,6 +9,10 @@
 // Warp 0 loads (TMA, 128-byte swizzle; the token tile only as many rows as there are tokens, in whole groups of eight: the MMA reads
 // 128 rows whatever they hold, and a row reaches nothing but its own sums, which are not stored), warp 1 issues tcgen05.mma, the
 // others finish rows (finish_rows).  Two accumulators where a block has several tiles.  Every wait is bounded.
+//
+// All of K is added in one accumulator, as in every unsplit product: a relative error against 64 bits of 2.1e-6 at K 2048 and 4.4e-6
+// at 4096, where a split, whose shorter sums meet in fp32, has 0.2 to 2.1e-6.  The operands' rounding to bfloat16 is 2e-3, and
+// the logits of whole steps are as far from 64 bits in either form.
 #include "gemm_parts.cuh"
 
 namespace leone {
@@ -204,7 +208,8 @@ using namespace leone;
 using namespace leone::tc;
 
 // The arguments and epilogues of leone_gemm_pair (0 bf16, 1 fp32, 2 fp32 += residual, 3 gate) with tiles of 128 tokens x `width` weight
-// rows (a multiple of 16 from 16 to 256, of 32 with the gate); a norm before the product, none after it.
+// rows (a multiple of 16 from 16 to 256, of 32 with the gate); a norm before the product, none after it.  (The callers' rules
+// take it for products without a norm on either side.)
 extern "C" int leone_gemm_narrow(const void* x, const void* w, void* out, const float* residual, int m, int n, int k, int ldx,
                                  int ldw, int ldc, int epilogue, int width, int* status, int sm_count,
                                  const float* norm_in_ss, int norm_in_parts, float norm_eps, const float* gate_shape,

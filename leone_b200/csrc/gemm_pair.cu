@@ -127,7 +127,8 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 // rows of partial sums in the workspace (L2), [block][chunk of 32 rows][column][row of the chunk];
 // after a cluster barrier the tile's eight chunks are dealt to the 2 S blocks, and the block that
 // finishes a chunk copies its S pieces into the (now free) stages with the copy engine, adds
-// them in split order on top of the residual values and runs the epilogue (no folded norm).
+// them in split order on top of the residual values and runs the epilogue (no folded norm).  The caller's rule takes
+// this form only where its unsplit pairs are switched off.
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const GemmParams p, const int BN, const int blocks) {
@@ -140,7 +141,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   uint8_t* aligned = smem_raw + (tiles_base - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + kStages * cfg.stage_bytes);
   // barriers: full[kStages] (used in the pair's first block), empty[kStages], acc_full[2], acc_empty[2],
-  // and for the split mode: the pieces of a chunk have landed, and all four warps have read them
+  // and for the split mode: the pieces of a chunk have landed, and the BN / 32 warps that add them have read them
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kStages;
   const uint32_t acc_full0 = empty0 + 8 * kStages, acc_empty0 = acc_full0 + 16;
   // and, where a norm follows, the second half's sums of squares of a buffer and quarter of the rows are in place (8)
@@ -465,7 +466,7 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
 using namespace leone;
 using namespace leone::tc;
 
-// The token-major product of gemm_tc.cu for more than 256 tokens on pairs of SMs: the same
+// The token-major product of gemm_tc.cu on pairs of SMs (any number of tokens; the caller's rule takes it from 129 on): the same
 // arguments and epilogues (0 bf16, 1 fp32, 2 fp32 += residual, 3 SwiGLU) and the same norm
 // arguments; `width`: weight rows per tile, a multiple of 16 from 32 to 256 (of 32 with the SwiGLU
 // epilogue); the sums of squares of a folded norm have one part per tile of that width.
@@ -507,7 +508,6 @@ extern "C" int leone_gemm_pair(const void* x, const void* w, void* out, const fl
 
 // Tiles of `width` weight rows whose clusters of 2 * splits blocks can be resident at once, and the
 // workspace floats a product split that way needs.
-// Tuning only: k-blocks a stage (0: the rule).
 extern "C" int leone_gemm_pair_capacity(int width, int splits) {
   if ((splits != 2 && splits != 4) || (width != 128 && width != 256)) return 0;
   return pair_cluster_capacity(width, splits);

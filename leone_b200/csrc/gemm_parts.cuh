@@ -482,11 +482,6 @@ __device__ __forceinline__ void finish_token_major_row(const GemmParams& p, uint
   finish_token_major_row(p, taddr, m, n0, n_tile, BN);
 }
 
-// Token-major form, the pairs' epilogue: a warp finishes its 32 token rows (m0 ..; tensor memory at `taddr`, lane = row) for
-// the accumulator columns [c_lo, c_hi) of the tile whose first weight row is n0 (multiples of 16, of 32 with the gate).
-// Sums go through 4 KB of the warp's own shared memory, 32 rows of 128 bytes with their 16-byte pieces swizzled by the row, so
-// that every access to global memory is four rows of 128 bytes side by side.  (A thread per row, as above, touches 32 rows with
-// 16 bytes each: half sectors, and 32 cache lines an instruction.)
 // The row's factor of a norm before the product (1 without one).
 __device__ __forceinline__ float norm_in_factor(const GemmParams& p, int m) {
   if (p.norm_in_ss == nullptr) return 1.f;
@@ -522,6 +517,12 @@ __device__ __forceinline__ void fetch_residual_chunk(const GemmParams& p, float4
   }
 }
 
+// Token-major form, the epilogue of pairs and of narrow tiles: a warp finishes its 32 token rows (m0 ..; tensor memory at `taddr`, lane = row) for
+// the accumulator columns [c_lo, c_hi) of the tile whose first weight row is n0 (multiples of 16, of 32 with the gate).
+// Sums go through 4 KB of the warp's own shared memory, 32 rows of 128 bytes with their 16-byte pieces swizzled by the row, so
+// that every access to global memory is four rows of 128 bytes side by side.  (A thread per row, as above, touches 32 rows with
+// 16 bytes each: half sectors, and 32 cache lines an instruction.)
+//
 // A product's kernel runs once in a layer, with the step's other kernels in between, so the code of its epilogue comes from memory
 // again: what every tile of the gate executes is kept short (a loop over 16 outputs at a time, the edges of tiles and unaligned rows
 // in paths of their own).  12288 x 2048 with the gate in a step of 1,027 tokens 54.7 us with the loop unrolled, 42.8 as it is (48.8

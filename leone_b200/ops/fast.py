@@ -66,12 +66,13 @@ class FastKernels:
         # LEONE_NO_PAIRS=1 keeps prompt-sized products on single SMs (cta_group::1)
         self.use_pairs = os.environ.get("LEONE_NO_PAIRS", "0") != "1"
         self.pairs_from = 129              # tokens from which unsplit products run on pairs
-        # LEONE_NO_PAIR_SPLITS=1 leaves the narrow products' split along K to the single-block kernel
+        # LEONE_NO_PAIR_SPLITS=1 leaves the narrow products' split along K to the single-block kernel (only where pairs_unsplit is off)
         self.use_pair_splits = os.environ.get("LEONE_NO_PAIR_SPLITS", "0") != "1"
         self.pair_padding = 0.8            # a pair's half tile against a single block's tile, at most (see in_pairs)
         self.pair_width_override = 0       # > 0: the tile width of every product on pairs (kernel_bench sets it)
         self.pair_split_override = 0       # > 0: pairs per tile of every product on pairs (tests set it)
-        # LEONE_NO_NARROW=1 leaves the products with few tiles to the forms that split K
+        # LEONE_NO_NARROW=1 leaves products without a norm around them to the rules from before the unsplit forms: those of 33 to 128
+        # tokens (narrow_width) and those from 129 on (pairs_unsplit) to plan_product, which splits K where tiles are few
         self.use_narrow = os.environ.get("LEONE_NO_NARROW", "0") != "1"
         self._pair_widths = {}
         self._plans = {}                   # _gemm's decisions per (sizes, arguments)
@@ -193,10 +194,8 @@ class FastKernels:
         tokens, where the second of two tiles of 256 would be half empty and the single-block
         kernel's three tiles of 128 measured faster (gate/up at 384 tokens 62.3 us against 67.2;
         at 640 tokens three pairs already beat five single tiles, 95.9 against 105.6).  With
-        ``n`` and ``k``: whether this ``[n x k]`` product does; the narrow products of a layer,
-        which up to about 600 tokens are split along K, do not (with tiles narrow enough to fill
-        the pairs, all pairs read the same few token tiles at once, and that measured slower
-        than the split: o_proj at 256 tokens 25.3 us against 18.7, down 61.7 against 37.1)."""
+        ``n`` and ``k``: whether this ``[n x k]`` product does where :meth:`pairs_unsplit` is
+        switched off; the narrow products of a layer are then split along K up to about 600 tokens."""
         if n and k and self.token_major_split(m, n, k) > 1:
             return self.pair_split(m, n, k) > 1
         return self._pairs_fit(m)
@@ -206,7 +205,8 @@ class FastKernels:
 
     def pair_split(self, m: int, n: int, k: int) -> int:
         """Pairs of SMs per tile of a narrow product (one that the single-block kernel would split
-        along K): 4 or 2 pairs share the k-blocks of a tile of 256 tokens x 256 weight rows when
+        along K), asked only where :meth:`pairs_unsplit` is switched off (the times below are from before its epilogue and are kept as
+        the reason of this rule): 4 or 2 pairs share the k-blocks of a tile of 256 tokens x 256 weight rows when
         their clusters of 8 or 4 blocks are all resident at once and a pair keeps at least 8
         k-blocks; 1: not split on pairs.  Only where the pairs can split as many ways as the single
         blocks would: with the same number of splits the pairs' k-loop wins (down at 512 tokens
@@ -255,7 +255,9 @@ class FastKernels:
         """Splits along K of the token-major form, summed inside thread-block clusters (1: none).
         A product whose token-major tiles fill at most half of the SMs (the narrow products of a
         layer between 65 and about 600 tokens) is split so that tiles x splits blocks fill them;
-        a split keeps at least 8 k-blocks.  Such a product takes no folded norm."""
+        a split keeps at least 8 k-blocks.  Such a product takes no folded norm.  Products without one that :meth:`narrow_width` or
+        :meth:`pairs_unsplit` takes do not ask; from 257 to 384 tokens, where no pairs fit a norm, the answer decides whether
+        the norm is folded (:meth:`fuses_norm`)."""
         if not (self.use_clusters and self.use_token_major) or m <= self.token_major_split_from:
             return 1
         tiles = int(self.lib.leone_gemm_tc_tiles_token_major(m, n))
@@ -325,7 +327,8 @@ class FastKernels:
         return best[1]
 
     def plan_product(self, m: int, n: int, k: int):
-        """``(token_major, splits, full_tiles, cluster)`` for a product without a folded norm."""
+        """``(token_major, splits, full_tiles, cluster)`` for a product without a folded norm that :meth:`narrow_width` and
+        :meth:`pairs_unsplit` leave: decode sizes, the output head up to 128 tokens, everything where those are switched off."""
         if self.in_pairs(m, n, k):
             return True, 1, 0, False                 # on pairs of SMs (_gemm takes them where nothing is forced)
         s = self.token_major_split(m, n, k)

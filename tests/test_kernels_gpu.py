@@ -252,13 +252,17 @@ def test_gemm_tc_token_major_cluster_split(ops16, m, n, k, splits):
 
 
 def test_the_dispatcher_splits_narrow_products_in_the_token_major_form(ops16, monkeypatch):
-    """(In single blocks: the splits on pairs of SMs, which take some of these, are switched off.)"""
+    """Where the unsplit forms are switched off, which take these from 33 tokens on.  (In single blocks: the splits on pairs of SMs,
+    which take some of these, are switched off too.)"""
     fast = ops16.fast
+    assert fast._plan_gemm(300, 4096, 4096, 0, None, 0, False, None, False, False)[:3] == (True, True, 1)
     monkeypatch.setattr(fast, "use_pair_splits", False)
+    monkeypatch.setattr(fast, "use_narrow", False)
     sms = fast.sm_count
     assert fast.plan_product(8, 4096, 4096)[0] is False                     # decode-sized: swapped
     tm, s, full, cluster = fast.plan_product(300, 4096, 4096)                # 3 x 16 tiles
     assert tm and cluster and full == 0 and 2 <= s <= 8 and 48 * s <= sms
+    assert fast._plan_gemm(300, 4096, 4096, 0, None, 0, False, None, False, False)[:5] == (False, tm, s, full, cluster)
     assert fast.plan_product(2048, 4096, 4096) == (True, 1, 0, False)        # fills the SMs unsplit
     assert not fast.fuses_norm(300, 4096, 4096) and fast.fuses_norm(2048, 4096, 4096)
     assert fast.plan_product(300, 4096, 256)[:2] == (True, 1)                # too few k-blocks to split
